@@ -5,22 +5,32 @@
  * hidden layers, a linear output layer, mean-squared error and Adam.  No
  * reference counterpart.
  *
+ * Matrices: see lbib_mlp_tc.cuh for the chunk layout of the BF16 ones
+ * (activations, dZ, weights); Z (FP32) has the same order, 8 consecutive
+ * columns of a row together.  Row padding (to 128) is written as zeros by
+ * every epilogue, column padding (to 128) is zero from the start.
+ *
  * Shapes: widths w_0 .. w_L (input, hidden..., output); layer l maps w_l to
  * w_{l+1}.  Every width is padded to a multiple of 16 inside (the padded
  * weight rows and columns are zero and stay zero: their gradients vanish);
  * the ABI sees the unpadded shapes.  Parameters, in ABI order: for each
  * layer W_l [w_{l+1}][w_l] row-major, then b_l [w_{l+1}].
  *
- * One GEMM kernel serves all products, C[M][N] = sum_k A(m,k) B(k,n), with
- * A and B read through element strides (so a transposed operand needs no
- * copy): tcgen05.mma on 128 x 64 tiles with the accumulator in TMEM
- * (mlp_gemm_tc below, device helpers in lbib_mlp_tc.cuh), the weight
- * gradients' long K split four ways with a fixed-order reduction.
+ * One tile routine serves all products, C[M][N] = sum_k A(m,k) B(k,n), with
+ * any operand transposed in place (so a transposed one needs no copy):
+ * tcgen05.mma on 128 x 32 tiles with the accumulator in TMEM (gemm_tile
+ * below), the weight gradients' long K split four ways with a fixed-order
+ * reduction.  A training step is one
+ * launch per layer forward, one per layer backward (that layer's dW, db and
+ * the dZ of the layer below, which all need only its dZ) and Adam: 2L + 1
+ * launches, chained by programmatic dependent launch.
  */
 #include <math.h>
 #include <stdint.h>
 #include <stdlib.h>
 #include <string.h>
+
+#include <type_traits>
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -31,11 +41,14 @@
 namespace {
 
 
-/* Epilogues of the GEMM. */
+/* Epilogues of a tile. */
 enum Epi {
-  EPI_STORE = 0,        /* C (fp32) = acc                                  */
-  EPI_BIAS_GELU = 1,    /* Z = acc + b (fp32 out0), A = gelu(Z) (bf16 out1) */
-  EPI_BIAS = 2,         /* Y = acc + b (fp32 out0)                          */
+  EPI_STORE = 0,        /* C (fp32 out0) = acc, or a split-K partial            */
+  EPI_GELU = 1,         /* A = gelu(acc + b) (bf16 out1)                        */
+  EPI_GELU_KEEP = 2,    /* the same, and Z = acc + b (fp32 out0) for training   */
+  EPI_OUT = 3,          /* Y = acc + b (fp32 out0, the first w columns)         */
+  EPI_MSE = 4,          /* out1 = d(mean squared error)/dY (bf16), loss partial */
+  EPI_GELU_BACK = 5,    /* out1 = acc * gelu'(Z) (bf16)                         */
 };
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
@@ -46,175 +59,373 @@ __device__ __forceinline__ float gelu_grad(float z) {
   return cdf + z * pdf;
 }
 
+using lbib_tc::BK;
+using lbib_tc::BM;
+using lbib_tc::kStages;
+using lbib_tc::NT;
+using lbib_tc::Operand;
 
-/* C[M][N] (row-major, ldc) = A(m,k) B(k,n), A(m,k) = A[m*am + k*ak],
- * B(k,n) = B[k*bk + n*bn], out-of-range elements read as 0, on the tcgen05
- * tensor cores (FP32 accumulator in TMEM; lbib_mlp_tc.cuh): a 128 x BN tile
- * per 128-thread CTA, K in double-buffered slices of 64.  `err` is set if an mbarrier wait
- * ran out (the tile is then not written).
- *
- * Split K (gridDim.z = S > 1, EPI_STORE only): CTA z sums the K slices
- * [z Kc, (z+1) Kc) and writes its partial tile to ws[z]; the CTA that
- * finishes a tile last (a per-tile counter) adds the S partials in z order
- * into out0 and resets the counter -- the same bits whatever the order in
- * which the CTAs run.  `aux` is the bias. */
-constexpr int TC_BN = 64;
+/* 128 x 32 tiles: at a batch of 1024 and a width of 256 (the sweep
+ * surrogate) that is 64 tiles; 64-column tiles were 32 CTAs on 148 SMs. */
+constexpr int BN = 32;
 constexpr int kMaxSplit = 8;      /* split-K factors 1, 2, 4, 8             */
-constexpr int kMaxTiles = 4096;   /* output tiles a split GEMM may have     */
-constexpr int TC_SMEM = 2 * (lbib_tc::BM + TC_BN) * lbib_tc::BK * 2 + 64;
+constexpr int kStageBytes = (BM + BN) * BK * 2;
+constexpr int kSmem = kStages * kStageBytes + (2 * kStages + 1) * 8 + 16;
+constexpr int kChunks = BN / 8;   /* column chunks of a tile: one per group of 4 warps */
+constexpr int kEpiLd = BN + 1;    /* row stride of a split's partial tile */
+static_assert(BM * kEpiLd * 4 <= kStages * kStageBytes, "the partial tile reuses the operand buffers");
+static_assert(NT == 32 * 4 * kChunks, "an epilogue thread per chunk");
 
-template <int EPI>
-__global__ void __launch_bounds__(lbib_tc::NT) mlp_gemm_tc(const __nv_bfloat16* __restrict__ A, long am, long ak,
-                                                         const __nv_bfloat16* __restrict__ B, long bk, long bn, int M,
-                                                         int N, int K, float* __restrict__ out0,
-                                                         __nv_bfloat16* __restrict__ out1, long ldc,
-                                                         const float* __restrict__ aux, int* __restrict__ err,
-                                                         float* __restrict__ ws, int* __restrict__ tile_cnt) {
-  const float* bias = aux;
-  using namespace lbib_tc;
-  constexpr int BN = TC_BN;
-  extern __shared__ __align__(1024) uint8_t smem[];
-  __nv_bfloat16* sA = reinterpret_cast<__nv_bfloat16*>(smem);             /* [2][BM * BK] */
-  __nv_bfloat16* sB = sA + 2 * BM * BK;                                    /* [2][BN * BK] */
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sB + 2 * BN * BK);           /* [2]          */
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  if (warp == 0) tmem_alloc<BN>(tslot);
-  if (t == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tslot;
-  /* the B operand is staged as X(n, k) = B[n*bn + k*bk] */
-  const int ma = stage_mode(A, am, ak, M, K), mb = stage_mode(B, bn, bk, N, K);
-  const uint32_t idesc = instr_desc_bf16(BM, BN, ma == ST_MN_VEC, mb == ST_MN_VEC);
-  /* this CTA's K slices: all of them, or its share of a split */
-  const int nk_all = (K + BK - 1) / BK;
-  const int S = gridDim.z, per = (nk_all + S - 1) / S;
-  const int kt0 = blockIdx.z * per;
-  const int nk = kt0 + per <= nk_all ? per : (nk_all > kt0 ? nk_all - kt0 : 0);
-  bool ok = true;
-  for (int kk = 0; kk < nk; ++kk) {
-    const int kt = kt0 + kk;
-    const int b = kk & 1;
-    if (kk >= 2 && !__syncthreads_and(mbar_wait(&bar[b], ((kk - 2) >> 1) & 1))) {
-      ok = false;
-      break;
-    }
-    __nv_bfloat16* a_s = sA + b * BM * BK;
-    __nv_bfloat16* b_s = sB + b * BN * BK;
-    stage_operand<BM>(a_s, A, am, ak, m0, M, kt * BK, K, ma);
-    stage_operand<BN>(b_s, B, bn, bk, n0, N, kt * BK, K, mb);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (t == 0) {
-      tc_fence_after();
+/* One product and what is done with it. */
+struct Gemm {
+  Operand A, B;           /* A(m, k), and B as X(n, k)                      */
+  const float* X;         /* A instead: FP32 rows [M][xw], rounded on the way in */
+  int xw;
+  __nv_bfloat16* copy;    /* with X: the rounded rows, in A's layout, or NULL */
+  int M, N, K;
+  int tn, tiles, split;   /* tiles along N, tiles, K splits                 */
+  float* out0;            /* row-major, row stride ldc (EPI_STORE, EPI_OUT); Z (EPI_GELU_KEEP) */
+  long ldc;
+  __nv_bfloat16* out1;    /* BF16 result, in blocks of 128 rows of oC chunks */
+  int oC;
+  const float* aux;       /* bias                                           */
+  const float* z;         /* EPI_GELU_BACK: pre-activations, in out1's order */
+  const float* T;         /* EPI_MSE: targets [M][w]                        */
+  int w;                  /* EPI_OUT, EPI_MSE: unpadded columns             */
+  float* loss;            /* EPI_MSE: per-tile squared-error sums, or NULL  */
+};
+
+/* 8 floats of 32-byte aligned memory. */
+__device__ __forceinline__ void load8(const float* p, float* v) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void store8(float* p, const float* v) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ uint4 pack8(const float* v) {
+  __align__(16) __nv_bfloat16 e[8];
 #pragma unroll
-      for (int s = 0; s < BK / 16; ++s) {
-        const uint64_t da = smem_desc(smem_u32(a_s) + s * 2 * (BM / 8) * 128, (BM / 8) * 128, 128);
-        const uint64_t db = smem_desc(smem_u32(b_s) + s * 2 * (BN / 8) * 128, (BN / 8) * 128, 128);
-        mma_bf16(tmem, da, db, idesc, (kk > 0 || s > 0) ? 1u : 0u);
+  for (int i = 0; i < 8; ++i) e[i] = __float2bfloat16(v[i]);
+  return *reinterpret_cast<const uint4*>(e);
+}
+
+/* The barriers and the TMEM address of a CTA, after its operand buffers. */
+struct TileCtx {
+  uint64_t *full, *done;   /* [kStages] slice arrived / its MMAs finished */
+  uint32_t tmem;
+};
+
+/* Tile `tile` of product g, split z of g.split.
+ *
+ * Split K (EPI_STORE only): the g.split CTAs of a cluster share a tile;
+ * CTA z sums the K elements [z Kc, (z+1) Kc), then each adds the partials of
+ * its share of the tile's rows in z order, read from the others' shared
+ * memory -- the same bits whatever the order in which the CTAs run.
+ * `err` is set if an mbarrier wait ran out (the tile is then not written).
+ *
+ * An epilogue thread holds 8 columns of one row, as tcgen05.ld delivers
+ * them; what it reads (Z, targets, bias) is loaded before it waits for the
+ * products. */
+template <int EPI>
+__device__ __forceinline__ void gemm_tile(const Gemm& g, int tile, int z, uint8_t* smem, const TileCtx& c,
+                                          int* __restrict__ err) {
+  using namespace lbib_tc;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int m0 = (tile / g.tn) * BM, n0 = (tile % g.tn) * BN;
+  /* this CTA's K range, all of it or its share of a split (shares in units
+     of 64), and the slices of BK it lies in */
+  const int units = (g.K + 63) / 64, per = (units + g.split - 1) / g.split;
+  const int kbeg = min(z * per * 64, g.K), kend = min((z + 1) * per * 64, g.K);
+  const int k00 = kbeg / BK * BK, nk = kend > kbeg ? (kend - k00 + BK - 1) / BK : 0;
+  const uint32_t s0 = smem_u32(smem);
+  const bool fp32_in = (EPI == EPI_GELU || EPI == EPI_GELU_KEEP || EPI == EPI_OUT || EPI == EPI_MSE) && g.X;
+  auto extent = [&](int kk) { return min(BK, (kend - (k00 + kk * BK) + 15) / 16 * 16); };
+  auto fetch = [&](int kk) {   /* one thread: the copies of slice kk */
+    const int b = kk % kStages, kn = extent(kk), k0 = k00 + kk * BK;
+    const uint32_t s = s0 + b * kStageBytes;
+    mbar_expect(&c.full[b], (fp32_in ? 0 : slice_bytes<BM>(g.A, kn)) + slice_bytes<BN>(g.B, kn));
+    if (!fp32_in) fetch_slice<BM>(s, g.A, m0, k0, kn, &c.full[b]);
+    fetch_slice<BN>(s + BM * BK * 2, g.B, n0, k0, kn, &c.full[b]);
+  };
+  /* the FP32 input's slice kk (a layer of few columns: rarely more than
+     one), by all threads */
+  auto convert = [&](int kk) {
+    const int b = kk % kStages, kn = extent(kk), k0 = k00 + kk * BK;
+    for (int v = t; v < BM * (kn / 8); v += NT) {
+      const int r = v % BM, kb = v / BM, m = m0 + r, k = k0 + kb * 8;
+      float x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = m < g.M && k + i < g.xw ? g.X[(long)m * g.xw + k + i] : 0.0f;
+      const uint4 u = pack8(x);
+      *reinterpret_cast<uint4*>(smem + b * kStageBytes + (kb * BM + r) * 16) = u;
+      if (g.copy && n0 == 0) *reinterpret_cast<uint4*>(g.copy + (((long)(m0 / BM) * g.A.C + k / 8) * BM + r) * 8) = u;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  };
+  bool ok = true;
+  const int lead = nk < kStages ? nk : kStages;
+  if (t == 0)
+    for (int kk = 0; kk < lead; ++kk) fetch(kk);
+  if (fp32_in) {
+    for (int kk = 0; kk < lead; ++kk) convert(kk);
+    __syncthreads();
+  }
+  const uint32_t idesc = instr_desc_bf16(BM, BN, g.A.mn, g.B.mn);
+  auto multiply = [&](int kk) {   /* one thread: the MMAs of slice kk */
+    const int b = kk % kStages, k0 = k00 + kk * BK;
+    if (!mbar_wait(&c.full[b], (kk / kStages) & 1)) return false;
+    tc_fence_after();
+    const uint32_t a = s0 + b * kStageBytes;
+    const int j0 = kk == 0 ? (kbeg - k0) / 16 : 0, j1 = extent(kk) / 16;
+#pragma unroll 4
+    for (int j = j0; j < j1; ++j)
+      mma_bf16(c.tmem, operand_desc<BM>(a, g.A.mn, j), operand_desc<BN>(a + BM * BK * 2, g.B.mn, j), idesc,
+               (kk > 0 || j > j0) ? 1u : 0u);
+    mma_commit(&c.done[b]);
+    return true;
+  };
+  if (!fp32_in) {
+    if (t == 32)
+      for (int kk = 0; kk < nk && ok; ++kk) ok = multiply(kk);
+    /* refills, each once the MMAs that read the buffer are done */
+    if (t == 0)
+      for (int kk = kStages; kk < nk && ok; ++kk) {
+        ok = mbar_wait(&c.done[kk % kStages], (kk / kStages - 1) & 1);
+        if (ok) fetch(kk);
       }
-      mma_commit(&bar[b]);
+  } else {
+    /* a wide FP32 input: the later slices in step, all threads converting */
+    for (int kk = 0; kk < nk; ++kk) {
+      if (kk >= kStages) {
+        if (!__syncthreads_and(ok && mbar_wait(&c.done[kk % kStages], (kk / kStages - 1) & 1))) { ok = false; break; }
+        if (t == 0) fetch(kk);
+        convert(kk);
+        __syncthreads();
+      }
+      if (t == 32) ok = ok && multiply(kk);
+    }
+  }
+  /* warp w holds TMEM lanes 32 (w % 4) .., columns 8 (w / 4) .. */
+  const int row = (warp & 3) * 32 + lane, ch = warp >> 2;
+  const int m = m0 + row, n = n0 + 8 * ch;
+  const bool nin = n < g.N, live = nin && m < g.M;
+  const long at = (((long)(m0 / BM) * g.oC + n / 8) * BM + row) * 8;   /* the thread's chunk */
+  float pre[8], bias[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) { pre[i] = 0.0f; bias[i] = 0.0f; }
+  if constexpr (EPI == EPI_GELU_BACK) {
+    if (live) load8(g.z + at, pre);
+  } else if constexpr (EPI != EPI_STORE) {
+    if (nin) load8(g.aux + n, bias);
+    if constexpr (EPI == EPI_MSE) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (live && n + i < g.w) pre[i] = g.T[(long)m * g.w + n + i];
     }
   }
   /* the last commit covers every MMA of the tile */
-  if (nk > 0) ok = __syncthreads_and(ok && mbar_wait(&bar[(nk - 1) & 1], ((nk - 1) >> 1) & 1));
+  if (nk > 0) ok = ok && mbar_wait(&c.done[(nk - 1) % kStages], ((nk - 1) / kStages) & 1);
+  ok = __syncthreads_and(ok);
   tc_fence_after();
-  __shared__ int s_last;
-  if (ok) {
-    const int m = m0 + warp * 32 + lane;
-    float* part = S > 1 ? ws + (long)blockIdx.z * M * ldc : nullptr;
-    for (int c = 0; c < BN; c += 16) {
-      float v[16];
-      if (nk > 0) tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
-      else for (int i = 0; i < 16; ++i) v[i] = 0.0f;   /* no K slice in this split */
-      if (m >= M) continue;
+  const bool split = EPI == EPI_STORE && g.split > 1;
+  if (!ok) {
+    if (t == 0) atomicExch(err, 1);
+    if (split) { cluster_sync(); cluster_sync(); }   /* the cluster's other CTAs meet here */
+    return;
+  }
+  float v[8];
+  if (nk > 0) tmem_ld8(c.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(8 * ch), v);
+  else
+    for (int i = 0; i < 8; ++i) v[i] = 0.0f;   /* no K slice in this split */
+  tc_fence_before();
+  if constexpr (EPI == EPI_STORE) {
+    if (!split) {
+      if (live) store8(g.out0 + (long)m * g.ldc + n, v);
+      return;
+    }
+    float* ep = reinterpret_cast<float*>(smem);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int n = n0 + c + i;
-        if (n >= N) continue;
-        float x = v[i];
-        if (EPI == EPI_STORE) {
-          if (S > 1) part[(long)m * ldc + n] = x;
-          else out0[(long)m * ldc + n] = x;
+    for (int i = 0; i < 8; ++i) ep[row * kEpiLd + 8 * ch + i] = v[i];
+    cluster_sync();
+    const int rows = BM / g.split;   /* this CTA's share: rows z * rows .. */
+    for (int r = z * rows + warp; r < (z + 1) * rows; r += NT / 32) {
+      float p[kMaxSplit];
+#pragma unroll
+      for (int k = 0; k < kMaxSplit; ++k) p[k] = k < g.split ? ld_cluster(ep + r * kEpiLd + lane, k) : 0.0f;
+      float acc = 0.0f;
+#pragma unroll
+      for (int k = 0; k < kMaxSplit; ++k)
+        if (k < g.split) acc += p[k];
+      if (m0 + r < g.M && n0 + lane < g.N) g.out0[(long)(m0 + r) * g.ldc + n0 + lane] = acc;
+    }
+    cluster_sync();   /* no CTA leaves while its partials are read */
+    return;
+  } else {
+    float loss = 0.0f, y[8];
+    const float mse_n = (float)g.M * (float)g.w;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float x = v[i];
+      if constexpr (EPI == EPI_GELU_BACK) {
+        y[i] = x * gelu_grad(pre[i]);
+      } else {
+        x += bias[i];
+        v[i] = x;
+        if constexpr (EPI == EPI_MSE) {
+          float d = 0.0f;
+          if (live && n + i < g.w) {
+            const float e = x - pre[i];
+            loss += e * e;
+            d = 2.0f * e / mse_n;
+          }
+          y[i] = d;
         } else {
-          x += bias[n];
-          out0[(long)m * ldc + n] = x;
-          if (EPI == EPI_BIAS_GELU) out1[(long)m * ldc + n] = __float2bfloat16(gelu(x));
+          y[i] = EPI == EPI_OUT ? x : gelu(x);
+        }
+      }
+      if (!live) y[i] = 0.0f;   /* the padding rows */
+    }
+    if constexpr (EPI == EPI_OUT) {
+      if (live) {
+        float* o = g.out0 + (long)m * g.ldc + n;
+        if (n + 8 <= g.w && ((reinterpret_cast<uintptr_t>(o) | (uintptr_t)(g.ldc * 4)) & 15) == 0) {
+          store8(o, y);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (n + i < g.w) o[i] = y[i];
+        }
+      }
+    } else if (nin) {
+      *reinterpret_cast<uint4*>(g.out1 + at) = pack8(y);
+      if (EPI == EPI_GELU_KEEP) store8(g.out0 + at, v);
+    }
+    if constexpr (EPI == EPI_MSE) {
+      if (g.loss) {
+        /* the tile's squared error, in a fixed order (the operand buffers
+           are free: every MMA is done) */
+        float* ep = reinterpret_cast<float*>(smem);
+        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+        if (lane == 0) ep[warp] = loss;
+        __syncthreads();
+        if (t == 0) {
+          float s = 0.0f;
+          for (int k = 0; k < NT / 32; ++k) s += ep[k];
+          g.loss[tile] = s;
         }
       }
     }
-    if (EPI == EPI_STORE && S > 1) {
-      /* the last CTA of this tile adds the partials in split order */
-      __threadfence();
-      __syncthreads();
-      if (t == 0) {
-        const int tile = blockIdx.y * gridDim.x + blockIdx.x;
-        s_last = atomicAdd(&tile_cnt[tile], 1) == S - 1;
-        if (s_last) tile_cnt[tile] = 0;
-      }
-      __syncthreads();
-      if (s_last) {
-        __threadfence();
-        for (int e = t; e < BM * BN; e += NT) {
-          const int mm = m0 + e / BN, nn = n0 + e % BN;
-          if (mm >= M || nn >= N) continue;
-          float acc = 0.0f;
-          for (int z = 0; z < S; ++z) acc += ws[(long)z * M * ldc + (long)mm * ldc + nn];
-          out0[(long)mm * ldc + nn] = acc;
-        }
-      }
-    }
-  } else if (t == 0) {
-    atomicExch(err, 1);
+  }
+}
+
+/* TMEM columns and the slice barriers, before the kernel's first global
+ * access (so that they overlap the tail of the kernel before it). */
+__device__ __forceinline__ TileCtx tile_begin(uint8_t* smem) {
+  using namespace lbib_tc;
+  TileCtx c;
+  c.full = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
+  c.done = c.full + kStages;
+  uint32_t* slot = reinterpret_cast<uint32_t*>(c.done + kStages);
+  if (threadIdx.x < 32) tmem_alloc<BN>(slot);
+  if (threadIdx.x == 32) {
+    for (int k = 0; k < 2 * kStages; ++k) mbar_init(&c.full[k], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_free<BN>(tmem);
+  tc_fence_after();
+  c.tmem = *slot;
+  return c;
 }
 
-/* X (fp32, [B][w_in]) -> bf16 [B][w_pad], pad columns 0. */
-__global__ void mlp_input(const float* __restrict__ X, int B, int w, int wp, __nv_bfloat16* __restrict__ out) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long)B * wp) return;
-  const int r = (int)(i / wp), c = (int)(i % wp);
-  out[i] = __float2bfloat16(c < w ? X[(long)r * w + c] : 0.0f);
-}
-
-/* Mean-squared error over the unpadded outputs: dY = 2 (Y - T) / (B w)
- * (bf16, pad columns 0), and per-block loss partials. */
-__global__ void mlp_mse(const float* __restrict__ Y, const float* __restrict__ T, int B, int w, int wp,
-                        __nv_bfloat16* __restrict__ dY, float* __restrict__ part) {
-  __shared__ float s[256];
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  float l = 0.0f;
-  if (i < (long)B * wp) {
-    const int r = (int)(i / wp), c = (int)(i % wp);
-    float d = 0.0f;
-    if (c < w) {
-      const float e = Y[i] - T[(long)r * w + c];
-      l = e * e;
-      d = 2.0f * e / ((float)B * (float)w);
-    }
-    dY[i] = __float2bfloat16(d);
-  }
-  s[threadIdx.x] = l;
+__device__ __forceinline__ void tile_end(uint32_t tmem) {
+  lbib_tc::tc_fence_before();
   __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = s[0];
+  if (threadIdx.x < 32) lbib_tc::tmem_free<BN>(tmem);
 }
 
+/* A layer forward: C = A W^T + b and its epilogue, a CTA per tile.  At
+ * 1024 x 256 x 256 with GELU 6.0 us (46 us with 128 x 64 tiles staged one K
+ * slice at a time by dependent loads): 3.5 us in the CTA -- the copies'
+ * latency, 16 MMAs, 2000 cycles of erf -- and the launch.  A training step
+ * of the sweep surrogate (batch 1024, 5 -> 4 x 256 -> 192) went from 27
+ * launches and 590 us to 11 and 76 us. */
+template <int EPI>
+__global__ void __launch_bounds__(NT) mlp_layer(const __grid_constant__ Gemm g, int* __restrict__ err) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  lbib_tc::pdl_trigger();
+  const TileCtx c = tile_begin(smem);
+  lbib_tc::pdl_wait();
+  gemm_tile<EPI>(g, blockIdx.x, 0, smem, c, err);
+  tile_end(c.tmem);
+}
+
+/* db[n] = sum over the batch of dZ[:, n] for the 16 columns of block j, in a
+ * fixed order: 32 row groups r, r + 32, ... summed in turn, then the 32
+ * partial sums of a column in order. */
+constexpr int kBiasCols = 16;
+__device__ __forceinline__ void bias_grad(const Operand& dZ, int B, int w, int j, float* __restrict__ db,
+                                          float* __restrict__ part) {
+  /* 8 consecutive threads on a chunk, consecutive rows next */
+  const int r0 = (threadIdx.x >> 3) & 31, c = (threadIdx.x & 7) + 8 * (threadIdx.x >> 8);
+  const int n = j * kBiasCols + c;
+  float s = 0.0f;
+  if (n < w) {
+    const __nv_bfloat16* p = dZ.p + (long)(n / 8) * BM * 8 + n % 8;
+#pragma unroll 16
+    for (int r = r0; r < B; r += 32) s += __bfloat162float(p[((long)(r / BM) * dZ.C * BM + r % BM) * 8]);
+  }
+  part[r0 * kBiasCols + c] = s;
+  __syncthreads();
+  if (threadIdx.x < kBiasCols && j * kBiasCols + threadIdx.x < w) {
+    float t = 0.0f;
+    for (int k = 0; k < 32; ++k) t += part[k * kBiasCols + threadIdx.x];
+    db[j * kBiasCols + threadIdx.x] = t;
+  }
+}
+static_assert(NT / kBiasCols == 32, "32 row groups");
+
+/* A layer backward, from its dZ: the CTAs of one launch share three
+ * independent jobs -- the tiles of dW = dZ^T X (split along the batch), the
+ * tiles of dZ_below = (dZ W) gelu'(Z_below), and the bias gradient's column
+ * blocks -- so that a layer costs one launch and its jobs fill the chip
+ * together (64 + 64 + 16 CTAs at the surrogate's hidden layers). */
+struct LayerBack {
+  Gemm dW, dA;
+  int n_dW, n_dA;                /* CTAs of each (dA: 0 at the first layer), whole clusters */
+  Operand dZ;
+  int batch, w;
+  float* db;
+};
+
+__global__ void __launch_bounds__(NT, 2) mlp_layer_back(const __grid_constant__ LayerBack a, int* __restrict__ err) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  lbib_tc::pdl_trigger();
+  const int b = blockIdx.x;
+  if (b >= a.n_dW + a.n_dA) {
+    lbib_tc::pdl_wait();
+    bias_grad(a.dZ, a.batch, a.w, b - a.n_dW - a.n_dA, a.db, reinterpret_cast<float*>(smem));
+    return;
+  }
+  const TileCtx c = tile_begin(smem);
+  lbib_tc::pdl_wait();
+  if (b >= a.n_dA) {
+    /* a cluster's CTAs are consecutive: rank z sums split z of the tile */
+    gemm_tile<EPI_STORE>(a.dW, (b - a.n_dA) / a.dW.split, (b - a.n_dA) % a.dW.split, smem, c, err);
+  } else if (b < a.dA.tiles) {
+    gemm_tile<EPI_GELU_BACK>(a.dA, b, 0, smem, c, err);
+  }
+  tile_end(c.tmem);
+}
+
+/* The loss from the tiles' squared-error sums. */
 __global__ void mlp_sum(const float* __restrict__ part, int n, float scale, float* __restrict__ out) {
   __shared__ float s[256];
+  lbib_tc::pdl_trigger();
+  lbib_tc::pdl_wait();
   float v = 0.0f;
   for (int i = threadIdx.x; i < n; i += 256) v += part[i];
   s[threadIdx.x] = v;
@@ -226,37 +437,12 @@ __global__ void mlp_sum(const float* __restrict__ part, int n, float scale, floa
   if (threadIdx.x == 0) *out = s[0] * scale;
 }
 
-/* dZ = dA * gelu'(Z), bf16. */
-__global__ void mlp_gelu_back(const float* __restrict__ dA, const float* __restrict__ Z, long n,
-                              __nv_bfloat16* __restrict__ dZ) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dZ[i] = __float2bfloat16(dA[i] * gelu_grad(Z[i]));
-}
-
-/* db[n] = sum over the batch of dZ[:, n], in a fixed order: thread
- * (c, g) of a 32 x 32 block sums rows g, g + 32, ... of column 32 blockIdx.x
- * + c, then the 32 partial sums of a column are added in g order. */
-__global__ void __launch_bounds__(1024) mlp_bias_grad(const __nv_bfloat16* __restrict__ dZ, int B, int w,
-                                                     float* __restrict__ db) {
-  __shared__ float part[32][33];
-  const int c = threadIdx.x, g = threadIdx.y;
-  const int n = blockIdx.x * 32 + c;
-  float s = 0.0f;
-  if (n < w)
-    for (int r = g; r < B; r += 32) s += __bfloat162float(dZ[(long)r * w + n]);
-  part[g][c] = s;
-  __syncthreads();
-  if (g == 0 && n < w) {
-    float t = 0.0f;
-    for (int k = 0; k < 32; ++k) t += part[k][c];
-    db[n] = t;
-  }
-}
-
 /* Adam on the fp32 master copy; refresh the bf16 weights. */
 __global__ void mlp_adam(float* __restrict__ p, const float* __restrict__ gr, float* __restrict__ m,
                          float* __restrict__ v, long n, float lr, float b1, float b2, float eps, float c1, float c2,
-                         __nv_bfloat16* __restrict__ wbf, const int* __restrict__ is_w) {
+                         __nv_bfloat16* __restrict__ wbf, const int2* __restrict__ is_w) {
+  lbib_tc::pdl_trigger();
+  lbib_tc::pdl_wait();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float g = gr[i];
@@ -266,10 +452,15 @@ __global__ void mlp_adam(float* __restrict__ p, const float* __restrict__ gr, fl
   v[i] = vi;
   const float x = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
   p[i] = x;
-  if (is_w[i] >= 0) wbf[is_w[i]] = __float2bfloat16(x);
+  const int2 at = is_w[i];
+  if (at.x >= 0) {
+    const __nv_bfloat16 w = __float2bfloat16(x);
+    wbf[at.x] = w;   /* W_l, and its transpose */
+    wbf[at.y] = w;
+  }
 }
 
-long align16(long v) { return (v + 15) / 16 * 16; }
+long align_up(long v, long a) { return (v + a - 1) / a * a; }
 
 }  // namespace
 
@@ -280,24 +471,23 @@ struct lbib_mlp {
   int* w;               /* [L+1] widths */
   int* wp;              /* [L+1] padded */
   int max_batch;
+  char* mem;            /* the device allocation the buffers below are parts of */
   long np;              /* padded parameter count */
   float *p, *g, *m, *v; /* master params, grads, Adam moments (padded layout) */
-  int* wmap;            /* padded param index -> bf16 weight index, or -1 */
-  __nv_bfloat16* wbf;   /* bf16 weights, layer after layer, [wp_{l+1}][wp_l] */
+  int2* wmap;           /* padded param index -> its places in wbf, or -1 */
+  /* the chunk-layout matrices (lbib_mlp_tc.cuh) */
+  long rows;            /* batch rows: max_batch to a multiple of 128     */
+  __nv_bfloat16* wbf;   /* bf16 weights: per layer W [wp_{l+1}][wp_l] and its transpose, */
+  long nw;              /*   rows padded to 32, in blocks of 32           */
   long* woff;           /* [L] offset of W_l in p (padded) */
   long* boff;           /* [L] offset of b_l in p */
-  long* wbo;            /* [L] offset of W_l in wbf */
-  __nv_bfloat16** act;  /* [L+1] bf16 activations [B][wp_l] (act[0] = input) */
-  float** z;            /* [L] pre-activations fp32 [B][wp_{l+1}] */
-  float* dA;            /* fp32 [B][max wp]                               */
-  __nv_bfloat16* dZ;    /* bf16 [2][B][max wp]: layer l's dZ, and l-1's  */
-  float* ws;            /* split-K partial tiles                          */
-  long ws_elems;
-  int* tile_cnt;        /* split-K arrivals per output tile (kMaxTiles)   */
-  float* part;
+  long* wbo;            /* [2 L] offsets of W_l and its transpose in wbf  */
+  __nv_bfloat16** act;  /* [L] activations, rows x wp_l (to 128); act[0] = input */
+  __nv_bfloat16** dz;   /* [L] dZ, rows x wp_{l+1} (to 128)               */
+  float** z;            /* [L-1] pre-activations fp32, rows x wp_{l+1}    */
+  float* part;          /* squared-error sums of the output layer's tiles */
   float* d_loss;
   int* d_err;           /* a tensor-core GEMM's mbarrier wait ran out     */
-  int maxw;             /* largest padded width                           */
   long steps;
   cudaStream_t stream;  /* where the work runs: own_stream or the caller's */
   cudaStream_t own_stream;
@@ -305,83 +495,135 @@ struct lbib_mlp {
 
 namespace {
 
-int launch_gemm(lbib_mlp* n, int epi, const __nv_bfloat16* A, long am, long ak, const __nv_bfloat16* B, long bk,
-                long bn, int M, int N, int K, float* out0, __nv_bfloat16* out1, long ldc, const float* bias) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(mlp_gemm_tc<EPI_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
-    cudaFuncSetAttribute(mlp_gemm_tc<EPI_BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
-    cudaFuncSetAttribute(mlp_gemm_tc<EPI_BIAS_GELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
-    attr = true;
-  }
-  dim3 grid((unsigned)((N + TC_BN - 1) / TC_BN), (unsigned)((M + lbib_tc::BM - 1) / lbib_tc::BM), 1);
-  /* a long K over few tiles (the weight gradients, K = batch) is split so
-     that ~32 CTAs share it; the split depends on the shape only */
-  if (epi == EPI_STORE) {
-    const int tiles = (int)(grid.x * grid.y), nkt = (K + lbib_tc::BK - 1) / lbib_tc::BK;
-    int sk = 1;
-    while (sk * 2 <= kMaxSplit && tiles * sk < 32 && nkt >= 4 * sk * 2) sk *= 2;
-    if ((long)sk * M * ldc > n->ws_elems || tiles > kMaxTiles) sk = 1;
-    grid.z = (unsigned)sk;
-  }
-  switch (epi) {
-    case EPI_BIAS_GELU:
-      mlp_gemm_tc<EPI_BIAS_GELU><<<grid, lbib_tc::NT, TC_SMEM, n->stream>>>(A, am, ak, B, bk, bn, M, N, K, out0,
-                                                                            out1, ldc, bias, n->d_err, n->ws,
-                                                                            n->tile_cnt);
-      break;
-    case EPI_BIAS:
-      mlp_gemm_tc<EPI_BIAS><<<grid, lbib_tc::NT, TC_SMEM, n->stream>>>(A, am, ak, B, bk, bn, M, N, K, out0, out1,
-                                                                       ldc, bias, n->d_err, n->ws, n->tile_cnt);
-      break;
-    default:
-      mlp_gemm_tc<EPI_STORE><<<grid, lbib_tc::NT, TC_SMEM, n->stream>>>(A, am, ak, B, bk, bn, M, N, K, out0, out1,
-                                                                        ldc, bias, n->d_err, n->ws, n->tile_cnt);
-  }
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+int set_smem_limits() {
+  const void* k[] = {(const void*)mlp_layer<EPI_GELU>, (const void*)mlp_layer<EPI_GELU_KEEP>,
+                     (const void*)mlp_layer<EPI_OUT>, (const void*)mlp_layer<EPI_MSE>, (const void*)mlp_layer_back};
+  for (const void* f : k)
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return -2;
+  return 0;
 }
 
-/* Forward pass of `batch` rows; the output (fp32) is z[L-1]. */
-int forward(lbib_mlp* n, const float* X, int batch) {
-  const unsigned nb = (unsigned)(((long)batch * n->wp[0] + 255) / 256);
-  mlp_input<<<nb, 256, 0, n->stream>>>(X, batch, n->w[0], n->wp[0], n->act[0]);
+/* A launch whose kernel may start while the one before it on the stream
+ * finishes (it waits, before its first global access, until that one is
+ * done: pdl_wait). */
+template <typename... P, typename... A>
+int launch(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st, unsigned cluster,
+           A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(blocks);
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  c.attrs = at;
+  c.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&c, kernel, (P)args...) == cudaSuccess ? 0 : -2;
+}
+
+/* Chunks of a row of a rows x wp matrix. */
+int row_chunks(int wp) { return (int)(align_up(wp, 128) / 8); }
+
+/* Layer l's matrices as operands: rows as the tile's rows, or columns; W_l
+ * [out][in] or its transpose. */
+Operand act_op(const lbib_mlp* n, int l, int mn) { return Operand{n->act[l], row_chunks(n->wp[l]), BM, mn}; }
+Operand dz_op(const lbib_mlp* n, int l, int mn) { return Operand{n->dz[l], row_chunks(n->wp[l + 1]), BM, mn}; }
+Operand w_op(const lbib_mlp* n, int l, int transposed) {
+  return Operand{n->wbf + n->wbo[2 * l + transposed], n->wp[l + transposed] / 8, BN, 0};
+}
+
+Gemm product(Operand A, Operand B, int M, int N, int K) {
+  Gemm g;
+  memset(&g, 0, sizeof(g));
+  g.A = A; g.B = B;
+  g.M = M; g.N = N; g.K = K;
+  g.tn = (N + BN - 1) / BN;
+  g.tiles = g.tn * ((M + BM - 1) / BM);
+  g.split = 1;
+  return g;
+}
+
+/* Layer l forward of `batch` rows; layer 0 reads the caller's FP32 rows. */
+Gemm layer_product(lbib_mlp* n, int l, const float* X, int batch) {
+  Gemm g = product(act_op(n, l, 0), w_op(n, l, 0), batch, n->wp[l + 1], n->wp[l]);
+  if (l == 0) { g.X = X; g.xw = n->w[0]; }
+  g.aux = n->p + n->boff[l];
+  g.oC = row_chunks(n->wp[l + 1]);
+  if (l + 1 < n->L) g.out1 = n->act[l + 1];
+  return g;
+}
+
+/* Y [batch][w_L] of `batch` rows. */
+int forward(lbib_mlp* n, const float* X, int batch, float* Y) {
   for (int l = 0; l < n->L; ++l) {
-    const int in = n->wp[l], out = n->wp[l + 1];
-    const __nv_bfloat16* W = n->wbf + n->wbo[l];
-    const float* b = n->p + n->boff[l];
-    const int epi = l + 1 < n->L ? EPI_BIAS_GELU : EPI_BIAS;
-    if (launch_gemm(n, epi, n->act[l], in, 1, W, 1, in, batch, out, in, n->z[l], n->act[l + 1], out, b)) return -2;
+    Gemm g = layer_product(n, l, X, batch);
+    int rc;
+    if (l + 1 < n->L) {
+      rc = launch(mlp_layer<EPI_GELU>, g.tiles, NT, kSmem, n->stream, 1, g, n->d_err);
+    } else {
+      g.out0 = Y; g.w = n->w[n->L]; g.ldc = n->w[n->L];
+      rc = launch(mlp_layer<EPI_OUT>, g.tiles, NT, kSmem, n->stream, 1, g, n->d_err);
+    }
+    if (rc) return rc;
   }
   return 0;
 }
 
-/* Gradients of the mean-squared error into n->g (padded layout). */
-int backward(lbib_mlp* n, const float* T, int batch) {
+/* Gradients of the mean-squared error on one batch into n->g (padded
+ * layout), and the loss into n->d_loss when it is wanted. */
+int gradients(lbib_mlp* n, const float* X, const float* T, int batch, bool want_loss) {
   const int L = n->L;
-  const long ny = (long)batch * n->wp[L];
-  const unsigned nb = (unsigned)((ny + 255) / 256);
-  const long zst = (long)n->max_batch * n->maxw;       /* the two dZ buffers */
-  mlp_mse<<<nb, 256, 0, n->stream>>>(n->z[L - 1], T, batch, n->w[L], n->wp[L], n->dZ, n->part);
-  mlp_sum<<<1, 256, 0, n->stream>>>(n->part, (int)nb, 1.0f / ((float)batch * (float)n->w[L]), n->d_loss);
+  for (int l = 0; l < L; ++l) {
+    Gemm g = layer_product(n, l, X, batch);
+    if (l == 0) g.copy = n->act[0];                     /* read again by dW of layer 0 */
+    int rc;
+    if (l + 1 < L) {
+      g.out0 = n->z[l];
+      rc = launch(mlp_layer<EPI_GELU_KEEP>, g.tiles, NT, kSmem, n->stream, 1, g, n->d_err);
+    } else {
+      g.out1 = n->dz[l]; g.T = T; g.w = n->w[L];
+      g.loss = want_loss ? n->part : NULL;
+      rc = launch(mlp_layer<EPI_MSE>, g.tiles, NT, kSmem, n->stream, 1, g, n->d_err);
+      if (!rc && want_loss)
+        rc = launch(mlp_sum, 1, 256, 0, n->stream, 1, (const float*)n->part, g.tiles,
+                    1.0f / ((float)batch * (float)n->w[L]), n->d_loss);
+    }
+    if (rc) return rc;
+  }
   for (int l = L - 1; l >= 0; --l) {
     const int in = n->wp[l], out = n->wp[l + 1];
-    __nv_bfloat16* dZ = n->dZ + ((L - 1 - l) & 1) * zst;
-    __nv_bfloat16* dZ_prev = n->dZ + ((L - l) & 1) * zst;
-    /* dW = dZ^T X: M = out, N = in, K = batch */
-    if (launch_gemm(n, EPI_STORE, dZ, 1, out, n->act[l], in, 1, out, in, batch, n->g + n->woff[l], NULL, in, NULL))
-      return -2;
-    mlp_bias_grad<<<(out + 31) / 32, dim3(32, 32), 0, n->stream>>>(dZ, batch, out, n->g + n->boff[l]);
-    if (l == 0) break;
-    /* dZ_{l-1} = (dZ W) * gelu'(Z_{l-1}): M = batch, N = in, K = out */
-    const __nv_bfloat16* W = n->wbf + n->wbo[l];
-    /* the GELU derivative (erf and exp per element) is an element-wise
-       kernel of its own: inside the GEMM's epilogue it ran on the GEMM's
-       few CTAs and took longer than the separate launch */
-    if (launch_gemm(n, EPI_STORE, dZ, out, 1, W, in, 1, batch, in, out, n->dA, NULL, in, NULL)) return -2;
-    const long na = (long)batch * in;
-    mlp_gelu_back<<<(unsigned)((na + 255) / 256), 256, 0, n->stream>>>(n->dA, n->z[l - 1], na, dZ_prev);
+    LayerBack a;
+    memset(&a, 0, sizeof(a));
+    /* dW = dZ^T X: M = out, N = in, K = batch.  A long K over few output
+       tiles is split so that enough CTAs share it; the factor depends on
+       the shape only (counted in tiles of 64 columns and K slices of 64;
+       4 ways at the surrogate's hidden layers) */
+    a.dW = product(dz_op(n, l, 1), act_op(n, l, 1), out, in, batch);
+    const int wide = ((in + 63) / 64) * ((out + BM - 1) / BM), nkt = (batch + 63) / 64;
+    int sk = 1;
+    while (sk * 2 <= kMaxSplit && wide * sk < 32 && nkt >= 4 * sk * 2) sk *= 2;
+    a.dW.split = sk;
+    a.dW.out0 = n->g + n->woff[l];
+    a.dW.ldc = in;
+    a.n_dW = a.dW.tiles * sk;
+    a.dZ = dz_op(n, l, 0); a.batch = batch; a.w = out;
+    a.db = n->g + n->boff[l];
+    if (l > 0) {
+      /* dZ_{l-1} = (dZ W) * gelu'(Z_{l-1}): M = batch, N = in, K = out */
+      a.dA = product(dz_op(n, l, 0), w_op(n, l, 1), batch, in, out);
+      a.dA.out1 = n->dz[l - 1];
+      a.dA.oC = row_chunks(in);
+      a.dA.z = n->z[l - 1];
+      a.n_dA = (a.dA.tiles + sk - 1) / sk * sk;
+    }
+    const int n_db = ((out + kBiasCols - 1) / kBiasCols + sk - 1) / sk * sk;
+    if (launch(mlp_layer_back, (unsigned)(a.n_dW + a.n_dA + n_db), NT, kSmem, n->stream, sk, a, n->d_err)) return -2;
   }
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return 0;
 }
 
 /* ABI parameter index <-> padded index. */
@@ -404,16 +646,16 @@ void for_each_param(const lbib_mlp* n, F f) {
 int refresh_bf16(lbib_mlp* n) {
   /* wbf from the master copy (host round trip; set-up only) */
   float* hp = (float*)malloc(sizeof(float) * n->np);
-  int* map = (int*)malloc(sizeof(int) * n->np);
-  long nw = n->wbo[n->L - 1] + (long)n->wp[n->L] * n->wp[n->L - 1];
+  int2* map = (int2*)malloc(sizeof(int2) * n->np);
+  const long nw = n->nw;
   __nv_bfloat16* hw = (__nv_bfloat16*)malloc(sizeof(__nv_bfloat16) * nw);
   int rc = (!hp || !map || !hw) ? -5 : 0;
   if (!rc && cudaMemcpy(hp, n->p, sizeof(float) * n->np, cudaMemcpyDeviceToHost) != cudaSuccess) rc = -2;
-  if (!rc && cudaMemcpy(map, n->wmap, sizeof(int) * n->np, cudaMemcpyDeviceToHost) != cudaSuccess) rc = -2;
+  if (!rc && cudaMemcpy(map, n->wmap, sizeof(int2) * n->np, cudaMemcpyDeviceToHost) != cudaSuccess) rc = -2;
   if (!rc) {
     for (long i = 0; i < nw; ++i) hw[i] = __float2bfloat16(0.0f);
     for (long i = 0; i < n->np; ++i)
-      if (map[i] >= 0) hw[map[i]] = __float2bfloat16(hp[i]);
+      if (map[i].x >= 0) hw[map[i].x] = hw[map[i].y] = __float2bfloat16(hp[i]);
     if (cudaMemcpy(n->wbf, hw, sizeof(__nv_bfloat16) * nw, cudaMemcpyHostToDevice) != cudaSuccess) rc = -2;
   }
   free(hp);
@@ -448,79 +690,80 @@ lbib_mlp* lbib_mlp_create(int n_layers, const int* widths, int max_batch, unsign
   n->wp = (int*)calloc(L + 1, sizeof(int));
   n->woff = (long*)calloc(L, sizeof(long));
   n->boff = (long*)calloc(L, sizeof(long));
-  n->wbo = (long*)calloc(L, sizeof(long));
+  n->wbo = (long*)calloc(2 * L, sizeof(long));
   n->act = (__nv_bfloat16**)calloc(L + 1, sizeof(void*));
+  n->dz = (__nv_bfloat16**)calloc(L, sizeof(void*));
   n->z = (float**)calloc(L, sizeof(void*));
-  int rc = (!n->w || !n->wp || !n->woff || !n->boff || !n->wbo || !n->act || !n->z) ? -5 : 0;
-  int maxw = 0;
+  int rc = (!n->w || !n->wp || !n->woff || !n->boff || !n->wbo || !n->act || !n->dz || !n->z) ? -5 : 0;
+  n->rows = align_up(max_batch, BM);
   long np = 0, nw = 0;
   for (int l = 0; l <= L && !rc; ++l) {
     n->w[l] = widths[l];
-    n->wp[l] = (int)align16(widths[l]);
-    if (n->wp[l] > maxw) maxw = n->wp[l];
+    n->wp[l] = (int)align_up(widths[l], 16);
   }
   for (int l = 0; l < L && !rc; ++l) {
     n->woff[l] = np;
     np += (long)n->wp[l + 1] * n->wp[l];
     n->boff[l] = np;
     np += n->wp[l + 1];
-    n->wbo[l] = nw;
-    nw += (long)n->wp[l + 1] * n->wp[l];
+    n->wbo[2 * l] = nw;
+    nw += align_up(n->wp[l + 1], BN) * n->wp[l];
+    n->wbo[2 * l + 1] = nw;
+    nw += align_up(n->wp[l], BN) * n->wp[l + 1];
   }
   n->np = np;
-  n->maxw = maxw;
+  n->nw = nw;
   if (!rc && cudaStreamCreateWithFlags(&n->own_stream, cudaStreamNonBlocking) != cudaSuccess) rc = -2;
   n->stream = n->own_stream;
+  /* every device buffer in one allocation (256-byte aligned parts), zeroed */
   const size_t fp = sizeof(float) * np;
-  if (!rc && cudaMalloc(&n->p, fp) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&n->g, fp) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&n->m, fp) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&n->v, fp) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&n->wmap, sizeof(int) * np) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&n->wbf, sizeof(__nv_bfloat16) * nw) != cudaSuccess) rc = -5;
-  for (int l = 0; l <= L && !rc; ++l)
-    if (cudaMalloc(&n->act[l], sizeof(__nv_bfloat16) * max_batch * n->wp[l]) != cudaSuccess) rc = -5;
-  for (int l = 0; l < L && !rc; ++l)
-    if (cudaMalloc(&n->z[l], sizeof(float) * max_batch * n->wp[l + 1]) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&n->dA, sizeof(float) * max_batch * maxw) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&n->dZ, sizeof(__nv_bfloat16) * 2 * max_batch * maxw) != cudaSuccess) rc = -5;
-  /* split-K partials: up to kMaxSplit copies of the largest weight matrix */
-  n->ws_elems = 0;
-  for (int l = 0; l < L; ++l)
-    if ((long)n->wp[l + 1] * n->wp[l] > n->ws_elems) n->ws_elems = (long)n->wp[l + 1] * n->wp[l];
-  n->ws_elems *= kMaxSplit;
-  if (!rc && cudaMalloc(&n->ws, sizeof(float) * n->ws_elems) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&n->tile_cnt, sizeof(int) * kMaxTiles) != cudaSuccess) rc = -5;
-  if (!rc && cudaMemset(n->tile_cnt, 0, sizeof(int) * kMaxTiles) != cudaSuccess) rc = -2;
-  if (!rc && cudaMalloc(&n->part, sizeof(float) * ((long)max_batch * maxw / 256 + 2)) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&n->d_loss, sizeof(float)) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&n->d_err, sizeof(int)) != cudaSuccess) rc = -5;
-  if (!rc && cudaMemset(n->d_err, 0, sizeof(int)) != cudaSuccess) rc = -2;
+  const long out_tiles = (n->rows / BM) * ((widths[L] + BN - 1) / BN + 1);
+  for (int pass = 0; pass < 2 && !rc; ++pass) {
+    size_t at = 0;
+    auto part = [&](auto& ptr, size_t bytes) {
+      if (pass) ptr = reinterpret_cast<std::decay_t<decltype(ptr)>>(n->mem + at);
+      at += (bytes + 255) / 256 * 256;
+    };
+    part(n->p, fp); part(n->g, fp); part(n->m, fp); part(n->v, fp);
+    part(n->wmap, sizeof(int2) * np);
+    part(n->wbf, sizeof(__nv_bfloat16) * nw);
+    for (int l = 0; l < L; ++l) {
+      const size_t z = n->rows * align_up(n->wp[l + 1], 128);
+      part(n->act[l], sizeof(__nv_bfloat16) * n->rows * align_up(n->wp[l], 128));
+      part(n->dz[l], sizeof(__nv_bfloat16) * z);
+      if (l + 1 < L) part(n->z[l], sizeof(float) * z);
+    }
+    part(n->part, sizeof(float) * out_tiles);
+    part(n->d_loss, sizeof(float));
+    part(n->d_err, sizeof(int));
+    if (pass) break;
+    if (cudaMalloc(&n->mem, at) != cudaSuccess) rc = -5;
+    else if (cudaMemset(n->mem, 0, at) != cudaSuccess) rc = -2;
+  }
+  if (!rc) rc = set_smem_limits();
   if (!rc) {
     /* He-uniform weights for the GELU layers (bound sqrt(6 / fan_in)),
        zero biases, zero padding */
     float* hp = (float*)calloc(np, sizeof(float));
-    int* map = (int*)malloc(sizeof(int) * np);
+    int2* map = (int2*)malloc(sizeof(int2) * np);
     uint64_t s = seed;
     if (!hp || !map) rc = -5;
-    for (long i = 0; i < np && !rc; ++i) map[i] = -1;
+    for (long i = 0; i < np && !rc; ++i) map[i] = make_int2(-1, -1);
     for (int l = 0; l < L && !rc; ++l) {
       const double bound = sqrt(6.0 / n->w[l]);
       for (int r = 0; r < n->wp[l + 1]; ++r)
         for (int c = 0; c < n->wp[l]; ++c) {
           const long i = n->woff[l] + (long)r * n->wp[l] + c;
-          map[i] = (int)(n->wbo[l] + (long)r * n->wp[l] + c);
+          auto at = [](int row, int col, int cols) { return ((long)(row / BN * (cols / 8) + col / 8) * BN + row % BN) * 8 + col % 8; };
+          map[i] = make_int2((int)(n->wbo[2 * l] + at(r, c, n->wp[l])), (int)(n->wbo[2 * l + 1] + at(c, r, n->wp[l + 1])));
           if (r < n->w[l + 1] && c < n->w[l]) hp[i] = (float)((2.0 * uniform01(&s) - 1.0) * bound);
         }
     }
     if (!rc && cudaMemcpy(n->p, hp, fp, cudaMemcpyHostToDevice) != cudaSuccess) rc = -2;
-    if (!rc && cudaMemcpy(n->wmap, map, sizeof(int) * np, cudaMemcpyHostToDevice) != cudaSuccess) rc = -2;
+    if (!rc && cudaMemcpy(n->wmap, map, sizeof(int2) * np, cudaMemcpyHostToDevice) != cudaSuccess) rc = -2;
     free(hp);
     free(map);
   }
-  if (!rc && (cudaMemset(n->m, 0, fp) != cudaSuccess || cudaMemset(n->v, 0, fp) != cudaSuccess ||
-              cudaMemset(n->g, 0, fp) != cudaSuccess))
-    rc = -2;
   if (!rc) rc = refresh_bf16(n);
   if (rc) {
     lbib_mlp_free(n);
@@ -532,13 +775,9 @@ lbib_mlp* lbib_mlp_create(int n_layers, const int* widths, int max_batch, unsign
 void lbib_mlp_free(lbib_mlp* n) {
   if (!n) return;
   if (n->stream) cudaStreamSynchronize(n->stream);
-  cudaFree(n->p); cudaFree(n->g); cudaFree(n->m); cudaFree(n->v); cudaFree(n->wmap); cudaFree(n->wbf);
-  for (int l = 0; l <= n->L && n->act; ++l) cudaFree(n->act[l]);
-  for (int l = 0; l < n->L && n->z; ++l) cudaFree(n->z[l]);
-  cudaFree(n->dA); cudaFree(n->dZ); cudaFree(n->part); cudaFree(n->d_loss); cudaFree(n->d_err);
-  cudaFree(n->ws); cudaFree(n->tile_cnt);
+  cudaFree(n->mem);
   if (n->own_stream) cudaStreamDestroy(n->own_stream);
-  free(n->w); free(n->wp); free(n->woff); free(n->boff); free(n->wbo); free(n->act); free(n->z);
+  free(n->w); free(n->wp); free(n->woff); free(n->boff); free(n->wbo); free(n->act); free(n->dz); free(n->z);
   free(n);
 }
 
@@ -581,11 +820,7 @@ int lbib_mlp_set_params(lbib_mlp* n, const float* in) {
 /* X [batch][w_0] fp32 and Y [batch][w_L] fp32, device pointers. */
 int lbib_mlp_forward(lbib_mlp* n, const float* X, int batch, float* Y) {
   if (!n || !X || !Y || batch < 1 || batch > n->max_batch) return LBIB_E_ARG;
-  if (forward(n, X, batch)) return LBIB_E_CUDA;
-  const int L = n->L;
-  if (cudaMemcpy2DAsync(Y, sizeof(float) * n->w[L], n->z[L - 1], sizeof(float) * n->wp[L], sizeof(float) * n->w[L],
-                        batch, cudaMemcpyDeviceToDevice, n->stream) != cudaSuccess)
-    return LBIB_E_CUDA;
+  if (forward(n, X, batch, Y)) return LBIB_E_CUDA;
   return lbib_mlp_synchronize(n);
 }
 
@@ -593,7 +828,7 @@ int lbib_mlp_forward(lbib_mlp* n, const float* X, int batch, float* Y) {
  * of the mean-squared error on one batch, without updating anything. */
 int lbib_mlp_gradient(lbib_mlp* n, const float* X, const float* T, int batch, float* grad, float* loss) {
   if (!n || !X || !T || batch < 1 || batch > n->max_batch) return LBIB_E_ARG;
-  if (forward(n, X, batch) || backward(n, T, batch)) return LBIB_E_CUDA;
+  if (gradients(n, X, T, batch, loss != NULL)) return LBIB_E_CUDA;
   float* hg = (float*)malloc(sizeof(float) * n->np);
   if (!hg) return LBIB_E_NOMEM;
   int rc = 0;
@@ -612,13 +847,13 @@ int lbib_mlp_gradient(lbib_mlp* n, const float* X, const float* T, int batch, fl
  * the step.  Asynchronous unless loss is asked for. */
 int lbib_mlp_train_step(lbib_mlp* n, const float* X, const float* T, int batch, float lr, float* loss) {
   if (!n || !X || !T || batch < 1 || batch > n->max_batch || !(lr > 0)) return LBIB_E_ARG;
-  if (forward(n, X, batch) || backward(n, T, batch)) return LBIB_E_CUDA;
+  if (gradients(n, X, T, batch, loss != NULL)) return LBIB_E_CUDA;
   n->steps++;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = (float)(1.0 - pow(b1, (double)n->steps)), c2 = (float)(1.0 - pow(b2, (double)n->steps));
-  mlp_adam<<<(unsigned)((n->np + 255) / 256), 256, 0, n->stream>>>(n->p, n->g, n->m, n->v, n->np, lr, b1, b2, 1e-8f,
-                                                                    c1, c2, n->wbf, n->wmap);
-  if (cudaGetLastError() != cudaSuccess) return LBIB_E_CUDA;
+  if (launch(mlp_adam, (unsigned)((n->np + 255) / 256), 256, 0, n->stream, 1, n->p, (const float*)n->g, n->m, n->v, n->np,
+             lr, b1, b2, 1e-8f, c1, c2, n->wbf, (const int2*)n->wmap))
+    return LBIB_E_CUDA;
   if (loss) {
     if (cudaMemcpyAsync(loss, n->d_loss, sizeof(float), cudaMemcpyDeviceToHost, n->stream) != cudaSuccess ||
         cudaStreamSynchronize(n->stream) != cudaSuccess)

@@ -4,22 +4,33 @@
  * accumulator in tensor memory (TMEM), read back with tcgen05.ld for the
  * bias / GELU epilogue.
  *
- * C[M][N] = sum_k A(m,k) B(k,n), A(m,k) = A[m*am + k*ak], B(k,n) =
- * B[k*bk + n*bn] (element strides, so W^T and dZ^T need no copies), rows
- * and columns beyond M, N, K read as zero.  One CTA of 128 threads computes
- * a 128 x BN tile: TMEM lane i holds row m0 + i, BN FP32 columns.
+ * C[M][N] = sum_k A(m,k) B(k,n).  One CTA computes a 128 x BN tile: TMEM
+ * lane i holds row m0 + i, BN FP32 columns.
  *
- * Operands are staged in K slices of 64 (four MMAs of K = 16), double
- * buffered: the threads load a slice from global memory (16-byte vectors
- * when the operand is contiguous along K, single elements otherwise) and
- * write it in the canonical K-major layout without swizzle -- 8 x 16-byte
- * "core matrices", core (kb, g) of rows 8g..8g+7 and K elements 8kb..8kb+7
- * at byte (kb * G + g) * 128, so the descriptor's stride byte offset (next
- * 8 rows) is 128 and its leading byte offset (next 8 K elements) G * 128.
- * One thread issues the MMAs of a slice and commits them to the slice's
- * mbarrier; a buffer is refilled only after that mbarrier says the MMAs
- * that read it are done.  Every wait is bounded: on a timeout the CTA
- * records an error, skips the rest and still frees its TMEM.
+ * Every BF16 matrix of the network (activations, dZ, weights) lies in global
+ * memory as 16-byte chunks of 8 consecutive columns, in blocks of `blk`
+ * rows: chunk (c, r) of columns 8c..8c+7 of row r at chunk index
+ * ((r / blk) * C + c) * blk + r % blk, with C the chunks of a row.  Eight
+ * consecutive chunks are one 8 x 16-byte "core matrix" of the tensor cores'
+ * no-swizzle layout, whichever way the matrix is used -- rows as M or N and
+ * columns as K (K-major), or columns as M or N and rows as K (MN-major) --
+ * so that with blk = 128 (activations, dZ) or 32 (weights, each also kept
+ * transposed) a K slice of an operand is ONE contiguous run of global
+ * memory, as it lies in the operand buffer.  An epilogue thread, which holds
+ * 8 columns of one row, writes one chunk, a warp's 32 rows contiguous.
+ *
+ * These products are small (K is a layer's width or a share of the batch)
+ * and bound by latency.  For the 80 KB of a tile with K = 256: the threads'
+ * own 16-byte cp.async from row-major matrices took ~6000 cycles to issue;
+ * bulk copies of 0.5 to 2 KB runs ~65 cycles each, 48 or more of them; one
+ * copy per operand and slice of 128 (four in all) is what remains.
+ *
+ * Operands are staged in K slices of 128 (eight MMAs of K = 16), kStages
+ * slices deep: a K of 256 is in flight whole.  One thread issues the copies
+ * of a slice to its mbarrier, another its MMAs when that mbarrier completes,
+ * and commits them to a second one, on which a refill of the buffer waits.
+ * Every wait is bounded: on a timeout the CTA records an error, skips the
+ * rest and still frees its TMEM.
  */
 #ifndef LBIB_MLP_TC_CUH
 #define LBIB_MLP_TC_CUH
@@ -31,8 +42,9 @@
 namespace lbib_tc {
 
 constexpr int BM = 128;   /* rows per CTA = TMEM lanes                 */
-constexpr int BK = 64;    /* K per stage: four MMAs of K = 16          */
-constexpr int NT = 128;   /* threads per CTA                           */
+constexpr int BK = 128;   /* K per stage: up to eight MMAs of K = 16   */
+constexpr int NT = 512;   /* threads per CTA: four warps per TMEM quadrant */
+constexpr int kStages = 2;   /* K slices staged at once                  */
 constexpr long kSpin = 1L << 24;   /* try_wait polls before giving up  */
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -114,80 +126,77 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                : "memory");
 }
 
-/* 16 consecutive FP32 columns of this thread's TMEM lane. */
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
+/* 8 consecutive FP32 columns of this thread's TMEM lane. */
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-/* How an operand tile is staged. */
-enum Stage {
-  ST_K_VEC = 0,    /* contiguous along K: 16-byte vectors, K-major tile      */
-  ST_MN_VEC = 1,   /* contiguous along the rows: 16-byte vectors, MN-major   */
-  ST_ELEM = 2,     /* any strides: element by element, K-major tile          */
+/* `bytes` (a multiple of 16) global -> shared by the bulk copy engine;
+ * the barrier counts them. */
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
+/* Programmatic dependent launch: let the next kernel of the stream start
+ * its set-up; wait until the kernels before this one are done and their
+ * writes visible (nothing global is read or written before that). */
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+/* An operand X(r, k) in the chunk layout above: the matrix's rows are the
+ * tile's rows and its columns K (mn = 0), or the other way round (mn = 1,
+ * blk = 128 = BK only). */
+struct Operand {
+  const __nv_bfloat16* p;
+  int C, blk, mn;
 };
 
-/* The staging mode for X(r, k) = X[r*xr + k*xk] with nr valid rows. */
-__host__ __device__ inline int stage_mode(const void* X, long xr, long xk, int nr, int K) {
-  const bool al = (reinterpret_cast<uintptr_t>(X) & 15) == 0;
-  if (al && xk == 1 && xr % 8 == 0 && K % 8 == 0) return ST_K_VEC;
-  if (al && xr == 1 && xk % 8 == 0 && nr % 8 == 0) return ST_MN_VEC;
-  return ST_ELEM;
+/* All CTAs of the cluster; shared-memory writes before it are visible to
+ * their readers after it. */
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+/* A float at the same shared-memory place of CTA `rank` of the cluster. */
+__device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
 }
 
-/* Rows [r0, r0 + R) x K elements [k0, k0 + BK) of X(r, k) = X[r*xr + k*xk]
- * into shared memory at s, as 8 x 16-byte core matrices, core (kb, g) of
- * rows 8g..8g+7 and K elements 8kb..8kb+7 at byte (kb * G + g) * 128
- * (G = R / 8).  K-major (ST_K_VEC, ST_ELEM): core row i holds row 8g+i's
- * eight K elements; MN-major (ST_MN_VEC): core row i holds K element 8kb+i
- * of the eight rows.  Either way the descriptor's leading byte offset (next
- * 8 K elements) is G * 128 and its stride byte offset (next 8 rows) 128.
- * Outside [0, nr) x [0, K): zero (r0 and nr are multiples of 8 in the
- * MN-major mode). */
+/* The operand's rows [r0, r0 + R) (r0 a multiple of R; R = blk when K-major)
+ * at K elements [k0, k0 + kn), k0 a multiple of BK and kn <= BK of 16: its
+ * bytes, and their copy to shared memory at s.  MN-major copies the whole
+ * block of BK rows. */
 template <int R>
-__device__ __forceinline__ void stage_operand(__nv_bfloat16* __restrict__ s, const __nv_bfloat16* __restrict__ X,
-                                              long xr, long xk, int r0, int nr, int k0, int K, int mode) {
-  constexpr int G = R / 8;
-  const int t = threadIdx.x;
-  if (mode == ST_MN_VEC) {
-    /* BK x G vectors, consecutive threads along the rows (contiguous) */
-    for (int v = t; v < BK * G; v += NT) {
-      const int g = v % G, k = v / G;
-      const int gr = r0 + 8 * g, gk = k0 + k;
-      uint4 val = make_uint4(0u, 0u, 0u, 0u);
-      if (gr < nr && gk < K) val = *reinterpret_cast<const uint4*>(X + (long)gk * xk + gr);
-      *reinterpret_cast<uint4*>(s + (((k >> 3) * G + g) * 64 + (k & 7) * 8)) = val;
-    }
-  } else if (mode == ST_K_VEC) {
-    /* R x (BK / 8) vectors, eight consecutive threads per row (128
-       contiguous bytes); vector (kb, r) -> core (kb, r / 8), row r % 8 */
-    for (int v = t; v < R * (BK / 8); v += NT) {
-      const int kb = v % (BK / 8), r = v / (BK / 8);
-      const int gr = r0 + r, gk = k0 + kb * 8;
-      uint4 val = make_uint4(0u, 0u, 0u, 0u);
-      if (gr < nr && gk < K) val = *reinterpret_cast<const uint4*>(X + (long)gr * xr + gk);
-      *reinterpret_cast<uint4*>(s + ((kb * G + (r >> 3)) * 64 + (r & 7) * 8)) = val;
-    }
-  } else {
-    /* consecutive threads take consecutive addresses: along the rows when
-       they are contiguous (a transposed operand), along K otherwise */
-    const __nv_bfloat16 zero = __float2bfloat16(0.0f);
-    const bool rows_fast = xr == 1;
-    for (int e = t; e < R * BK; e += NT) {
-      const int r = rows_fast ? e % R : e / BK, k = rows_fast ? e / R : e % BK;
-      const int gr = r0 + r, gk = k0 + k;
-      const __nv_bfloat16 val = (gr < nr && gk < K) ? X[(long)gr * xr + (long)gk * xk] : zero;
-      s[((k >> 3) * G + (r >> 3)) * 64 + (r & 7) * 8 + (k & 7)] = val;
-    }
-  }
+__device__ __forceinline__ uint32_t slice_bytes(const Operand& X, int kn) {
+  return X.mn ? R * BK * 2 : R * kn * 2;
+}
+template <int R>
+__device__ __forceinline__ void fetch_slice(uint32_t s, const Operand& X, int r0, int k0, int kn, uint64_t* bar) {
+  const long chunk = X.mn ? ((long)(k0 / BK) * X.C + r0 / 8) * BK : ((long)(r0 / R) * X.C + k0 / 8) * R;
+  bulk_copy(s, X.p + chunk * 8, slice_bytes<R>(X, kn), bar);
+}
+
+/* The descriptor of a staged operand's K = 16 step j: core matrices along K
+ * are 16 R bytes apart and along the rows 128 (K-major), or 128 and 16 BK
+ * (MN-major); the leading byte offset is the one along K. */
+template <int R>
+__device__ __forceinline__ uint64_t operand_desc(uint32_t s, int mn, int j) {
+  return mn ? smem_desc(s + j * 2 * 128, 128, BK * 16) : smem_desc(s + j * 2 * R * 16, R * 16, 128);
 }
 
 }  // namespace lbib_tc
