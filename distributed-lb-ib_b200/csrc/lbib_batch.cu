@@ -46,101 +46,78 @@ using namespace lbib;
 /* ------------------------------------------------------------ kernels */
 namespace {
 
-__global__ void lbib_b_forces(double* __restrict__ nodes, const int* __restrict__ node_inst,
-                              const BatchDesc* __restrict__ D, const int* __restrict__ err, long SP, int bend_bug) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= SP) return;
-  const int k = node_inst[i];
-  if (k < 0 || err[2 * k]) return;
+/* A block per 32-node chunk, all of one problem (every problem's nodes start
+ * at a multiple of 32), as the one-grid lbib_node_prep: four warps evaluate
+ * the delta factors, the first also reduces the chunk's box and enters the
+ * touched tiles, the fifth computes the fiber forces.  step_no: the batch's
+ * device step counter (graph replays see the live value), 1 for the first
+ * step. */
+__global__ void __launch_bounds__(160, 5) lbib_b_node_prep(double* __restrict__ nodes, const int* __restrict__ node_inst,
+                                                        const BatchDesc* __restrict__ D, double* __restrict__ W,
+                                                        int* __restrict__ st, int* __restrict__ chunk_box,
+                                                        int* __restrict__ slot, int* __restrict__ list,
+                                                        int* __restrict__ count, int* err, long SP,
+                                                        const int* __restrict__ step_no, int bend_bug) {
+  const long i0 = (long)blockIdx.x * 32, i = i0 + (threadIdx.x & 31);
+  const int part = threadIdx.x >> 5, k = node_inst[i0];
+  if (k < 0 || *(volatile int*)(err + 2 * k)) return;   /* uniform over the block, but for a node that fails right now */
   const BatchDesc& d = D[k];
-  fiber_forces_node(nodes + d.node0 * 12, d.rows, d.cols, d.bc, d.sc, d.sc2, d.ds1, d.ds2, bend_bug,
-                    (int)(i - d.node0));
-}
-
-/* step_no: the batch's device step counter (graph replays see the live
- * value), 1 for the first step. */
-__global__ void lbib_b_node_prep(const double* __restrict__ nodes, const int* __restrict__ node_inst,
-                                 const BatchDesc* __restrict__ D, double* __restrict__ W, int* __restrict__ st,
-                                 int* __restrict__ tile_cnt, int* __restrict__ chunk_box, int* err, long SP,
-                                 const int* __restrict__ step_no) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int step = *step_no;
-  int b0 = INT_MAX, b1 = INT_MIN, b2 = INT_MAX, b3 = INT_MIN, b4 = INT_MAX, b5 = INT_MIN;
-  const int k = i < SP ? node_inst[i] : -1;
-  if (k >= 0 && !err[2 * k]) {
-    const BatchDesc& d = D[k];
-    node_prep_one(nodes, i, d.nx, d.ny, d.nz, d.ntx, d.nty, d.tile0, W, st, tile_cnt, err + 2 * k, step, b0, b1, b2,
-                  b3, b4, b5);
+  const bool mine = i < d.node0 + d.S;
+  if (part == 4) {
+    if (mine)
+      fiber_forces_node(nodes + d.node0 * 12, d.rows, d.cols, d.bc, d.sc, d.sc2, d.ds1, d.ds2, bend_bug,
+                        (int)(i - d.node0));
+    return;
   }
-  chunk_box_reduce(i, SP, chunk_box, b0, b1, b2, b3, b4, b5);
+  int is = 0, js = 0, ks = 0;
+  const bool ok = mine && node_prep_part(nodes, i, part, d.nx, d.ny, d.nz, W, st, err + 2 * k, *step_no, is, js, ks);
+  if (part == 0) {
+    chunk_box_reduce(i, SP, chunk_box, nullptr, is, js, ks, ok);
+    touch_tiles(is, js, ks, ok, d.ntx, d.nty, d.tile0, slot, list, count, nullptr);
+  }
 }
 
-/* Entries {chunk, lane mask} per tile, as the one-grid spread's: a warp's
- * 32 nodes belong to one problem (every problem's nodes start at a
- * multiple of 32), so the warp works with that problem's grid; warps of
- * padding nodes or of a failed problem append nothing. */
-__global__ void lbib_b_pair_scatter(const int* __restrict__ st, const int* __restrict__ node_inst,
-                                    const BatchDesc* __restrict__ D, const int* __restrict__ slot,
-                                    const int* __restrict__ slot_off, int* __restrict__ slot_cursor,
-                                    int2* __restrict__ ent, const int* err, long SP) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long i0 = i & ~31L;   /* the warp's first node: its problem is the warp's */
-  const int k = i0 < SP ? node_inst[i0] : -1;
-  if (k < 0 || *(volatile const int*)(err + 2 * k)) return;   /* uniform over the warp */
-  const BatchDesc& d = D[k];
-  const long S = i < SP && node_inst[i] == k ? i + 1 : i;   /* lanes past the problem's nodes: no node */
-  pair_scatter_warp(st, i, S, d.ntx, d.nty, d.nx, d.ny, d.nz, 0, d.ntx, slot + d.tile0, slot_off, slot_cursor, ent);
-}
-
-/* Every listed tile of the batch from its entries (gather_tile_ent), or,
- * with more than kListCap nodes, by scanning its problem's node chunks in
- * order (gather_tile_scan), in one launch. */
-__global__ void __launch_bounds__(64) lbib_b_gather(const double* __restrict__ nodes, const double* __restrict__ W,
-                                                    const int* __restrict__ st, const int* __restrict__ chunk_box,
-                                                    const int* __restrict__ list, const int* __restrict__ count,
-                                                    const int* __restrict__ slot_off, const int* __restrict__ slot_len,
-                                                    const int* __restrict__ slot_cursor, const int2* __restrict__ ent,
-                                                    const int* __restrict__ tile_inst, const BatchDesc* __restrict__ D,
-                                                    double* __restrict__ Ftile, const int* err) {
-  __shared__ union {
-    GatherSmemE e;
-    ScanSmem s;
-  } sm;
+/* Every listed tile of the batch: its force into its slot. */
+__global__ void __launch_bounds__(kGatherTPB) lbib_b_gather(GatherNodes g, const int* __restrict__ list,
+                                                            const int* __restrict__ count,
+                                                            const int* __restrict__ tile_inst,
+                                                            const BatchDesc* __restrict__ D,
+                                                            double* __restrict__ Ftile, const int* err) {
+  __shared__ GatherShared sm;
   const int n = *count;
   for (int it = blockIdx.x; it < n; it += gridDim.x) {
-    const int tile = list[it];
-    const int k = tile_inst[tile];
+    const int k = tile_inst[list[it]];
     if (*(volatile const int*)(err + 2 * k)) continue;
     const BatchDesc& d = D[k];
-    const int L = slot_len[it];
-    if (L <= kListCap) {
-      gather_tile_ent(sm.e, nodes, W, st, it, (int)(tile - d.tile0), L, slot_cursor[it], ent + slot_off[it], d.ntx,
-                      d.nty, Ftile);
-    } else {
-      __syncthreads();   /* the union's previous contents are no longer read */
-      const long end = d.node0 + d.S;
-      gather_tile_scan(sm.s, nodes, W, st, chunk_box, end, d.node0 >> 5, (end + 31) >> 5, it, (int)(tile - d.tile0),
-                       d.ntx, d.nty, Ftile);
+    const int tile = (int)(list[it] - d.tile0);
+    double Fx, Fy, Fz;
+    gather_tile(sm, batch_nodes(g, d), tile % d.ntx * 4, tile / d.ntx % d.nty * 4, tile / (d.ntx * d.nty) * 4, Fx, Fy,
+                Fz);
+    if (threadIdx.x < 64) {
+      double* Ft = Ftile + (long)it * 192;
+      Ft[threadIdx.x] = Fx; Ft[64 + threadIdx.x] = Fy; Ft[128 + threadIdx.x] = Fz;
     }
   }
 }
 
-/* The move, a warp per 32 nodes of one problem with the union box of their
- * stencils staged in shared memory (move_warp); a pinned leading row stays. */
-__global__ void __launch_bounds__(64) lbib_b_move(double* __restrict__ nodes, const double* __restrict__ W,
-                                                  const int* __restrict__ st, const int* __restrict__ node_inst,
-                                                  const BatchDesc* __restrict__ D, const int* __restrict__ slot,
-                                                  const double* __restrict__ Utile, const int* err, long SP,
-                                                  int* __restrict__ step_no) {
-  __shared__ double sU[2][3 * kMoveCap + kMoveTiles / 2];
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) ++*step_no;   /* the last kernel of the step; node_prep has read it */
-  const long i0 = i & ~31L;
-  const int k = i0 < SP ? node_inst[i0] : -1;
-  if (k < 0 || *(volatile const int*)(err + 2 * k)) return;   /* uniform over the warp */
+/* The move, a CTA per 32-node chunk of one problem (move_chunk); a pinned
+ * leading row stays. */
+__global__ void __launch_bounds__(kMoveTPB) lbib_b_move(double* __restrict__ nodes, const double* __restrict__ W,
+                                                        const int* __restrict__ st, const int* __restrict__ node_inst,
+                                                        const BatchDesc* __restrict__ D, const int* __restrict__ slot,
+                                                        const double* __restrict__ Utile, const int* err,
+                                                        int* __restrict__ step_no, int* __restrict__ old_count) {
+  __shared__ MoveSmem sm;
+  const long i0 = (long)blockIdx.x * 32, i = i0 + (threadIdx.x & 31);
+  if (i0 == 0 && threadIdx.x == 0) {   /* the last kernel of the step */
+    ++*step_no;
+    *old_count = 0;   /* the next step's tile list starts empty */
+  }
+  const int k = node_inst[i0];
+  if (k < 0 || *(volatile const int*)(err + 2 * k)) return;   /* uniform over the CTA */
   const BatchDesc& d = D[k];
-  const bool live = i < SP && node_inst[i] == k && !(d.pinned && i - d.node0 < d.cols);
-  move_warp(nodes, W, st, i, live, d.ntx, d.nty, slot + d.tile0, Utile, d.dt, sU[threadIdx.x >> 5]);
+  const bool live = i < d.node0 + d.S && !(d.pinned && i - d.node0 < d.cols);
+  move_chunk(sm, nodes, W, st, i, live, d.ntx, d.nty, slot + d.tile0, Utile, d.dt);
 }
 
 /* FP64 rows away from the walls: the two-cell step, a block per 128 pairs of
@@ -172,16 +149,18 @@ int rest_f64_t(const BatchFluid& f) {
 
 namespace lbib {
 
-int batch_fluid_rest_f64(const BatchFluid& f) { return f.par ? rest_f64_t<1>(f) : rest_f64_t<0>(f); }
+int batch_rows_f64(const BatchFluid& f) { return f.par ? rest_f64_t<1>(f) : rest_f64_t<0>(f); }
 
 int batch_tile_moments_f64(const BatchFluid& f) {
   const FluidParamsT<double>* P = static_cast<const FluidParamsT<double>*>(f.P);
   if (f.par == 0)
     lbib_b_tile_moments<double, 0><<<f.grid_tiles, 64, 0, f.stream>>>(P, f.desc, f.list, f.count, f.tile_inst, f.Ftile,
-                                                                       f.Utile, f.err);
+                                                                       f.Utile, f.err, f.old_slot, f.old_list,
+                                                                       f.old_count);
   else
     lbib_b_tile_moments<double, 1><<<f.grid_tiles, 64, 0, f.stream>>>(P, f.desc, f.list, f.count, f.tile_inst, f.Ftile,
-                                                                       f.Utile, f.err);
+                                                                       f.Utile, f.err, f.old_slot, f.old_list,
+                                                                       f.old_count);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -285,7 +264,7 @@ struct lbib_batch {
   /* pools */
   unsigned char* f;
   unsigned char* tab;
-  int *tile_cnt, *tile_inst, *scan_tmp, *slot_off, *slot_len, *slot_cursor, *pair_node;
+  int* tile_inst;
   int *tile_slot[2], *tile_list[2], *tile_count[2];
   double *Ftile[2], *Utile[2];
   double *nodes, *W;
@@ -473,58 +452,51 @@ BatchFluid fluid_args(lbib_batch* b, int par, const void* P, const void* WP, int
   f.Utile = b->Utile[c];
   f.err = b->err;
   f.grid_tiles = b->grid_tiles;
+  f.nodes = GatherNodes{b->nodes, b->W, b->st, b->chunk_box, NULL, 0, 0, 0};
+  f.old_slot = b->tile_slot[c ^ 1];
+  f.old_list = b->tile_list[c ^ 1];
+  f.old_count = b->tile_count[c ^ 1];
   return f;
 }
-
-constexpr int kScan = 1024;
 
 /* One step of the batch, launched on b->stream (eagerly or into a capture). */
 int batch_step(lbib_batch* b) {
   const int c = b->cur ^ 1, par = b->parity, first = b->steps == 0;
   cudaStream_t s = b->stream;
   const long SP = b->SP;
-  const unsigned nb = (unsigned)((SP + 127) / 128);
-  const int bend_bug = (b->compat & 1) != 0;
-  lbib_b_forces<<<nb, 128, 0, s>>>(b->nodes, b->node_inst, b->desc, b->err, SP, bend_bug);
-  CK(cudaMemsetAsync(b->tile_cnt, 0, sizeof(int) * b->NT, s));
-  CK(cudaMemsetAsync(b->tile_slot[c], 0xff, sizeof(int) * b->NT, s));
-  lbib_b_node_prep<<<nb, 128, 0, s>>>(b->nodes, b->node_inst, b->desc, b->W, b->st, b->tile_cnt, b->chunk_box, b->err,
-                                      SP, b->step_no);
-  const unsigned nblk = (unsigned)((b->NT + kScan - 1) / kScan);
-  int* block_tiles = b->scan_tmp;
-  int* block_pairs = b->scan_tmp + nblk + 1;
-  lbib_compact_count<<<nblk, kScan, 0, s>>>(b->tile_cnt, b->NT, block_tiles, block_pairs);
-  lbib_compact_scan<<<1, kScan, 0, s>>>(block_tiles, block_pairs, (int)nblk, b->tile_count[c]);
-  lbib_compact_write<<<nblk, kScan, 0, s>>>(b->tile_cnt, b->NT, block_tiles, block_pairs, b->tile_list[c],
-                                            b->tile_slot[c], b->slot_off, b->slot_len, b->slot_cursor);
-  int2* ent = reinterpret_cast<int2*>(b->pair_node);
-  lbib_b_pair_scatter<<<nb, 128, 0, s>>>(b->st, b->node_inst, b->desc, b->tile_slot[c], b->slot_off, b->slot_cursor,
-                                         ent, b->err, SP);
-  lbib_b_gather<<<b->grid_tiles, 64, 0, s>>>(b->nodes, b->W, b->st, b->chunk_box, b->tile_list[c], b->tile_count[c],
-                                             b->slot_off, b->slot_len, b->slot_cursor, ent, b->tile_inst, b->desc,
-                                             b->Ftile[c], b->err);
-  b->launches += 8;
+  lbib_b_node_prep<<<(unsigned)(SP / 32), 160, 0, s>>>(b->nodes, b->node_inst, b->desc, b->W, b->st, b->chunk_box,
+                                                       b->tile_slot[c], b->tile_list[c], b->tile_count[c], b->err, SP,
+                                                       b->step_no, (b->compat & 1) != 0);
+  b->launches += 1;
   /* the fused fluid step */
   const void* P = first ? b->P_first : b->P[c];
   const void* WP = first ? b->WP_first : b->WP[c];
   BatchFluid f = fluid_args(b, par, P, WP, c);
+  if (is_lp(b)) {
+    if (batch_gather_lp(f)) return -2;
+  } else {
+    lbib_b_gather<<<b->grid_tiles, kGatherTPB, 0, s>>>(f.nodes, f.list, f.count, b->tile_inst, b->desc, b->Ftile[c],
+                                                       b->err);
+  }
+  b->launches++;
   if (is_lp(b)) {
     for (int v = 0; v < MAXV; ++v)
       if (b->nwblk[v]) {
         if (batch_words_lp(f, v, b->wblk[v], b->nwblk[v])) return -2;
         b->launches++;
       }
-    if (batch_fluid_rest_lp(f)) return -2;
-    b->launches += 1 + (b->nrblk > 0);
+    if (batch_rows_lp(f)) return -2;
+    b->launches += b->nrblk > 0;
   } else {
-    if (batch_fluid_rest_f64(f)) return -2;
+    if (batch_rows_f64(f)) return -2;
     b->launches += (b->nxblk > 0) + (b->nrblk > 0);
   }
   /* moments of the touched tiles, read by the next step and the move */
   BatchFluid g = fluid_args(b, par ^ 1, b->P[c], b->WP[c], c);
   if ((is_lp(b) ? batch_tile_moments_lp(g) : batch_tile_moments_f64(g))) return -2;
-  lbib_b_move<<<(unsigned)((SP + 63) / 64), 64, 0, s>>>(b->nodes, b->W, b->st, b->node_inst, b->desc, b->tile_slot[c],
-                                                        b->Utile[c], b->err, SP, b->step_no);
+  lbib_b_move<<<(unsigned)(SP / 32), kMoveTPB, 0, s>>>(b->nodes, b->W, b->st, b->node_inst, b->desc, b->tile_slot[c],
+                                                        b->Utile[c], b->err, b->step_no,
+                                                        b->tile_count[c ^ 1]);
   b->launches += 2;
   b->cur = c;
   b->parity ^= 1;
@@ -561,6 +533,7 @@ int init_state(lbib_batch* b) {
   }
   CK(cudaMemsetAsync(b->tile_slot[0], 0xff, sizeof(int) * b->NT, b->stream));
   CK(cudaMemsetAsync(b->tile_slot[1], 0xff, sizeof(int) * b->NT, b->stream));
+  for (int c = 0; c < 2; ++c) CK(cudaMemsetAsync(b->tile_count[c], 0, sizeof(int), b->stream));
   const int one = 1;
   CK(cudaMemcpyAsync(b->step_no, &one, sizeof(int), cudaMemcpyHostToDevice, b->stream));
   CK(cudaStreamSynchronize(b->stream));
@@ -664,14 +637,7 @@ lbib_batch* lbib_batch_create(int n, const lbib_problem* problems, int precision
   if (!rc && big_malloc((void**)&b->f, foff) != cudaSuccess) rc = -5;
   if (!rc && big_malloc((void**)&b->tab, toff) != cudaSuccess) rc = -5;
   const long NT = b->NT, CAP = b->CAP, SP = b->SP;
-  const long nblk = (NT + kScan - 1) / kScan;
-  if (!rc && cudaMalloc(&b->tile_cnt, sizeof(int) * NT) != cudaSuccess) rc = -5;
   if (!rc && cudaMalloc(&b->tile_inst, sizeof(int) * NT) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&b->scan_tmp, sizeof(int) * (2 * nblk + 2)) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&b->slot_off, sizeof(int) * CAP) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&b->slot_len, sizeof(int) * CAP) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&b->slot_cursor, sizeof(int) * CAP) != cudaSuccess) rc = -5;
-  if (!rc && cudaMalloc(&b->pair_node, sizeof(int2) * 8 * SP) != cudaSuccess) rc = -5;
   for (int c = 0; c < 2 && !rc; ++c) {
     if (cudaMalloc(&b->tile_slot[c], sizeof(int) * NT) != cudaSuccess) rc = -5;
     if (!rc && cudaMalloc(&b->tile_list[c], sizeof(int) * CAP) != cudaSuccess) rc = -5;
@@ -786,8 +752,7 @@ void lbib_batch_free(lbib_batch* b) {
   }
   free(b->sh);
   big_free(b->f); big_free(b->tab);
-  cudaFree(b->tile_cnt); cudaFree(b->tile_inst); cudaFree(b->scan_tmp);
-  cudaFree(b->slot_off); cudaFree(b->slot_len); cudaFree(b->slot_cursor); cudaFree(b->pair_node);
+  cudaFree(b->tile_inst);
   for (int c = 0; c < 2; ++c) {
     cudaFree(b->tile_slot[c]); cudaFree(b->tile_list[c]); cudaFree(b->tile_count[c]);
     big_free(b->Ftile[c]); big_free(b->Utile[c]);

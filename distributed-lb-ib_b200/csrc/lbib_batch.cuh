@@ -5,8 +5,8 @@
  * Every problem keeps its own populations, tables and parameters (a
  * FluidParamsT<T> per problem in device memory, whose pointers reach into
  * the batch's pools); its tiles are a slice [tile0, tile0 + ntiles) of one
- * global tile space, so one touched-tile list, one slot space and one
- * compaction serve the whole batch.  Work is enumerated across problems:
+ * global tile space, so one touched-tile list and one slot space serve the
+ * whole batch.  Work is enumerated across problems:
  *   rows     blocks of 128 cells over the rows the generic kernel takes,
  *            each problem's rows laid end to end;
  *   pairs    (FP64) blocks of 128 cell pairs of the two-cell kernel;
@@ -24,6 +24,7 @@
 #ifndef LBIB_BATCH_CUH
 #define LBIB_BATCH_CUH
 
+#include "lbib_ib.cuh"
 #include "lbib_words.cuh"
 
 namespace lbib {
@@ -90,20 +91,42 @@ __global__ void __launch_bounds__(WTPB, MINB) lbib_b_words(const WordsParams<T>*
   for (long i = threadIdx.x; i < 4 * (r1 - r0); i += WTPB) edge_cell<T, PAR>(sb.p, sb.nry, (int)(r0 + i / 4), (int)(i & 3));
 }
 
-/* Cells of forced tiles in the word kernel's range, over the global list. */
+/* The batch's sheets as problem d's gather sees them: its own chunks. */
+__device__ __forceinline__ GatherNodes batch_nodes(GatherNodes g, const BatchDesc& d) {
+  g.S = d.node0 + d.S;
+  g.c_lo = d.node0 >> 5;
+  g.c_hi = (g.S + 31) >> 5;
+  return g;
+}
+
+/* Every listed tile: its spread force into its slot, and the step of its
+ * cells in the word kernel's range (which leaves them out), by the CTA that
+ * has just written the force.  Launched before the word blocks and the
+ * generic rows, which read the forces of their own cells. */
 template <typename T, int PAR>
-__global__ void __launch_bounds__(64) lbib_b_forced(const FluidParamsT<T>* __restrict__ P,
-                                                    const BatchDesc* __restrict__ D, const int* __restrict__ list,
-                                                    const int* __restrict__ count, const int* __restrict__ tile_inst,
-                                                    const int* __restrict__ err) {
-  const int n = *count;
+__global__ void __launch_bounds__(kGatherTPB, 5) lbib_b_gather_step(const FluidParamsT<T>* __restrict__ P,
+                                                                    const BatchDesc* __restrict__ D, GatherNodes g,
+                                                                    const int* __restrict__ list,
+                                                                    const int* __restrict__ count,
+                                                                    const int* __restrict__ tile_inst,
+                                                                    double* __restrict__ Ftile,
+                                                                    const int* __restrict__ err) {
+  __shared__ GatherShared sm;
+  const int n = *count, t = threadIdx.x;
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
-    const int tile = list[i];
-    const int k = tile_inst[tile];
-    if (err[2 * k] || !D[k].bulk) continue;
+    const int k = tile_inst[list[i]];
+    if (err[2 * k]) continue;
+    const BatchDesc& d = D[k];
+    const int tile = (int)(list[i] - d.tile0);
+    double Fx, Fy, Fz;
+    gather_tile(sm, batch_nodes(g, d), tile % d.ntx * 4, tile / d.ntx % d.nty * 4, tile / (d.ntx * d.nty) * 4, Fx, Fy,
+                Fz);
+    if (t >= 64) continue;
+    double* Ft = Ftile + (long)i * 192;
+    Ft[t] = Fx; Ft[64 + t] = Fy; Ft[128 + t] = Fz;
     const FluidParamsT<T>& p = P[k];
-    const int zb = min(p.nz - 4, p.zin_hi);
-    forced_cell<T, PAR>(p, (int)(tile - D[k].tile0), threadIdx.x, zb);
+    /* the thread reads back the force it has just written */
+    if (d.bulk) forced_cell<T, PAR>(p, tile, t, min(p.nz - 4, p.zin_hi));
   }
 }
 
@@ -112,7 +135,10 @@ template <typename T, int PAR>
 __global__ void lbib_b_tile_moments(const FluidParamsT<T>* __restrict__ P, const BatchDesc* __restrict__ D,
                                     const int* __restrict__ list, const int* __restrict__ count,
                                     const int* __restrict__ tile_inst, const double* __restrict__ Ftile,
-                                    double* __restrict__ Utile, const int* __restrict__ err) {
+                                    double* __restrict__ Utile, const int* __restrict__ err,
+                                    int* __restrict__ old_slot, const int* __restrict__ old_list,
+                                    const int* __restrict__ old_count) {
+  clear_slots(old_slot, old_list, old_count);
   const int n = *count;
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
     const int tile = list[i];

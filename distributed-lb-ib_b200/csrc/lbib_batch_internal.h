@@ -8,6 +8,8 @@
 
 #include <cuda_runtime_api.h>
 
+#include "lbib_ib.cuh"
+
 namespace lbib {
 
 struct BatchDesc;
@@ -29,16 +31,22 @@ struct BatchFluid {
   const int* list;         /* touched tiles (global ids) */
   const int* count;
   const int* tile_inst;
-  const double* Ftile;
+  GatherNodes nodes;       /* the batch's sheets (a problem's chunks: batch_nodes) */
+  double* Ftile;
   double* Utile;
+  int* old_slot;           /* the other buffer's tile map, list and count: cleared for the next step */
+  const int* old_list;
+  const int* old_count;
   const int* err;
   int grid_tiles;          /* persistent grid for tile-list kernels */
 };
 
-/* Generic rows + forced cells (the word blocks, with the edge cells, are separate);
- * FP64: two-cell blocks + generic rows. */
-int batch_fluid_rest_f64(const BatchFluid& f);
-int batch_fluid_rest_lp(const BatchFluid& f);
+/* The spread's gather, and in low precision the forced cells with it: before
+ * everything that reads the forces. */
+int batch_gather_lp(const BatchFluid& f);
+/* Generic rows (FP64: two-cell blocks too). */
+int batch_rows_lp(const BatchFluid& f);
+int batch_rows_f64(const BatchFluid& f);
 /* Word-kernel blocks of one variant. */
 int batch_words_lp(const BatchFluid& f, int variant, const int2* blk, long nblk);
 int batch_variants_lp(int prec);

@@ -11,14 +11,24 @@ namespace lbib {
 namespace {
 
 template <typename T>
-int rest(const BatchFluid& f) {
+int gather(const BatchFluid& f) {
+  const FluidParamsT<T>* P = static_cast<const FluidParamsT<T>*>(f.P);
+  if (f.par == 0)
+    lbib_b_gather_step<T, 0><<<f.grid_tiles, kGatherTPB, 0, f.stream>>>(P, f.desc, f.nodes, f.list, f.count,
+                                                                         f.tile_inst, f.Ftile, f.err);
+  else
+    lbib_b_gather_step<T, 1><<<f.grid_tiles, kGatherTPB, 0, f.stream>>>(P, f.desc, f.nodes, f.list, f.count,
+                                                                         f.tile_inst, f.Ftile, f.err);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+template <typename T>
+int rows(const BatchFluid& f) {
   const FluidParamsT<T>* P = static_cast<const FluidParamsT<T>*>(f.P);
   if (f.nrblk > 0) {
     if (f.par == 0) lbib_b_rows<T, 0><<<(unsigned)f.nrblk, 128, 0, f.stream>>>(P, f.rowyz, f.rblk, f.err);
     else lbib_b_rows<T, 1><<<(unsigned)f.nrblk, 128, 0, f.stream>>>(P, f.rowyz, f.rblk, f.err);
   }
-  if (f.par == 0) lbib_b_forced<T, 0><<<f.grid_tiles, 64, 0, f.stream>>>(P, f.desc, f.list, f.count, f.tile_inst, f.err);
-  else lbib_b_forced<T, 1><<<f.grid_tiles, 64, 0, f.stream>>>(P, f.desc, f.list, f.count, f.tile_inst, f.err);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -40,19 +50,30 @@ template <typename T>
 int moments(const BatchFluid& f) {
   const FluidParamsT<T>* P = static_cast<const FluidParamsT<T>*>(f.P);
   if (f.par == 0)
-    lbib_b_tile_moments<T, 0><<<f.grid_tiles, 64, 0, f.stream>>>(P, f.desc, f.list, f.count, f.tile_inst, f.Ftile, f.Utile, f.err);
+    lbib_b_tile_moments<T, 0><<<f.grid_tiles, 64, 0, f.stream>>>(P, f.desc, f.list, f.count, f.tile_inst, f.Ftile, f.Utile, f.err,
+                                                                 f.old_slot, f.old_list, f.old_count);
   else
-    lbib_b_tile_moments<T, 1><<<f.grid_tiles, 64, 0, f.stream>>>(P, f.desc, f.list, f.count, f.tile_inst, f.Ftile, f.Utile, f.err);
+    lbib_b_tile_moments<T, 1><<<f.grid_tiles, 64, 0, f.stream>>>(P, f.desc, f.list, f.count, f.tile_inst, f.Ftile, f.Utile, f.err,
+                                                                 f.old_slot, f.old_list, f.old_count);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 }  // namespace
 
-int batch_fluid_rest_lp(const BatchFluid& f) {
+int batch_gather_lp(const BatchFluid& f) {
   switch (LBIB_PREC_TYPE(f.prec)) {
-    case LBIB_PREC_F32: return rest<float>(f);
-    case LBIB_PREC_F16: return rest<__half>(f);
-    case LBIB_PREC_BF16: return rest<__nv_bfloat16>(f);
+    case LBIB_PREC_F32: return gather<float>(f);
+    case LBIB_PREC_F16: return gather<__half>(f);
+    case LBIB_PREC_BF16: return gather<__nv_bfloat16>(f);
+    default: return -1;
+  }
+}
+
+int batch_rows_lp(const BatchFluid& f) {
+  switch (LBIB_PREC_TYPE(f.prec)) {
+    case LBIB_PREC_F32: return rows<float>(f);
+    case LBIB_PREC_F16: return rows<__half>(f);
+    case LBIB_PREC_BF16: return rows<__nv_bfloat16>(f);
     default: return -1;
   }
 }

@@ -2,10 +2,11 @@
  * GPU state of one LBM-IB problem and the order of a time step.
  *
  * A step (cube_pthread/lbm_ib.c:3124-3563, mpi/do_thread.c:50-386) is
- *   fiber forces -> spread (node prep, tile compaction, gather) -> fused
- *   fluid step -> moments on the touched tiles -> interpolate and move
+ *   fiber forces and node preparation -> spread (gather) -> fused fluid
+ *   step -> moments on the touched tiles -> interpolate and move
  * all stream-ordered on one CUDA stream, with no host synchronisation.
  */
+#include <limits.h>
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -23,10 +24,11 @@ int lbdev_launch_sums(lbib_device* d, double* part, double* out);
 int lbdev_lp_variants(int prec);
 int lbdev_launch_fiber_forces(lbib_device* d, int k);
 int lbdev_can_fuse_forces(const lbib_device* d);
+int lbdev_launch_prep(lbib_device* d, int step);
 int lbdev_launch_spread(lbib_device* d, int step);
 int lbdev_launch_move(lbib_device* d);
 int lbdev_launch_stencil_box(lbib_device* d);
-int lbdev_launch_box_cells(lbib_device* d);
+int lbdev_launch_spread_box(lbib_device* d);
 int lbdev_launch_scatter_force(lbib_device* d, double* fx, double* fy, double* fz);
 }
 
@@ -43,11 +45,7 @@ static void free_tiles(lbib_device* d) {
     cudaFree(d->Ftile[b]); d->Ftile[b] = NULL;
     cudaFree(d->Utile[b]); d->Utile[b] = NULL;
   }
-  cudaFree(d->tile_cnt); d->tile_cnt = NULL;
-  cudaFree(d->slot_off); d->slot_off = NULL;
-  cudaFree(d->slot_len); d->slot_len = NULL;
-  cudaFree(d->slot_cursor); d->slot_cursor = NULL;
-  cudaFree(d->pair_node); d->pair_node = NULL;
+  cudaFree(d->tile_mark); d->tile_mark = NULL;
   cudaFree(d->scan_tmp); d->scan_tmp = NULL;
   cudaFree(d->scan_state); d->scan_state = NULL;
 }
@@ -59,6 +57,8 @@ static void free_sheets(lbib_device* d) {
   cudaFree(d->W); d->W = NULL;
   cudaFree(d->st); d->st = NULL;
   cudaFree(d->chunk_box); d->chunk_box = NULL;
+  for (int b = 0; b < 2; ++b) { cudaFree(d->super[b]); d->super[b] = NULL; }
+  d->nsuper = 0;
   free(d->sh); d->sh = NULL;
   d->nsheets = 0; d->S = 0; d->nchunks = 0;
 }
@@ -226,10 +226,10 @@ extern "C" int lbdev_create(lbib_device** out, const lbdev_config* c) {
   const char* pf = getenv("LBIB_L2_PREFETCH");
   d->l2_pf = pf ? atoi(pf) : 0;
   d->fluid_stream = d->stream;
-  /* box-mode steps for a whole grid: 1 in stream order (default), 2 with
-     the fluid's bulk concurrent to the spread, 0 off (LBIB_OVERLAP) */
+  /* box-mode steps for a whole grid: 2 with the fluid's bulk beside the
+     spread (default), 1 in stream order, 0 off (LBIB_OVERLAP) */
   const char* ov = getenv("LBIB_OVERLAP");
-  d->overlap = (d->x_lo == 0 && d->x_hi == d->nx) ? (ov ? atoi(ov) : 1) : 0;
+  d->overlap = lbdev_is_slab(d) ? 0 : (ov ? atoi(ov) : 2);
   if (d->overlap &&
       (cudaStreamCreateWithPriority(&d->side, cudaStreamNonBlocking, prio_lo) != cudaSuccess ||
        cudaEventCreateWithFlags(&d->ev_box, cudaEventDisableTiming) != cudaSuccess ||
@@ -322,6 +322,20 @@ extern "C" int lbdev_set_sheets(lbib_device* d, int nsheets, const lbib_sheet_de
     CK(cudaMalloc(&d->W, sizeof(double) * 12 * S));
     CK(cudaMalloc(&d->st, sizeof(int) * 3 * S));
     CK(cudaMalloc(&d->chunk_box, sizeof(int) * 6 * d->nchunks));
+    if (d->nchunks > LBIB_SUPER_MIN) {
+      /* empty boxes: {INT_MAX, INT_MIN} per axis */
+      d->nsuper = (d->nchunks + 31) / 32;
+      int* e = (int*)malloc(sizeof(int) * 6 * d->nsuper);
+      if (!e) return -5;
+      for (long i = 0; i < 6 * d->nsuper; ++i) e[i] = i & 1 ? INT_MIN : INT_MAX;
+      int rc = 0;
+      for (int b = 0; b < 2 && !rc; ++b)
+        if (cudaMalloc(&d->super[b], sizeof(int) * 6 * d->nsuper) != cudaSuccess ||
+            cudaMemcpy(d->super[b], e, sizeof(int) * 6 * d->nsuper, cudaMemcpyHostToDevice) != cudaSuccess)
+          rc = -2;
+      free(e);
+      if (rc) return rc;
+    }
     /* every node touches at most 8 tiles, so 8 S slots can never overflow */
     d->cap = 8 * S < d->ntiles ? 8 * S : d->ntiles;
     for (int b = 0; b < 2; ++b) {
@@ -333,15 +347,13 @@ extern "C" int lbdev_set_sheets(lbib_device* d, int nsheets, const lbib_sheet_de
       CK(cudaMemsetAsync(d->tile_slot[b], 0xff, sizeof(int) * d->ntiles, d->stream));
       CK(cudaMemsetAsync(d->tile_count[b], 0, sizeof(int), d->stream));
     }
-    CK(cudaMalloc(&d->tile_cnt, sizeof(int) * d->ntiles));
-    CK(cudaMemsetAsync(d->tile_cnt, 0, sizeof(int) * d->ntiles, d->stream));   /* the compaction keeps it at 0 */
-    CK(cudaMalloc(&d->slot_off, sizeof(int) * d->cap));
-    CK(cudaMalloc(&d->slot_len, sizeof(int) * d->cap));
-    CK(cudaMalloc(&d->slot_cursor, sizeof(int) * d->cap));
-    CK(cudaMalloc(&d->pair_node, sizeof(int2) * 8 * S));
-    CK(cudaMalloc(&d->scan_tmp, sizeof(int) * 2 * ((d->ntiles + 1023) / 1024 + 1)));
-    CK(cudaMalloc(&d->scan_state, sizeof(unsigned long long) * ((d->ntiles + 1023) / 1024 + 1)));
-    CK(cudaMemsetAsync(d->scan_state, 0, sizeof(unsigned long long) * ((d->ntiles + 1023) / 1024 + 1), d->stream));
+    if (lbdev_is_slab(d)) {
+      CK(cudaMalloc(&d->tile_mark, sizeof(int) * d->ntiles));
+      CK(cudaMemsetAsync(d->tile_mark, 0, sizeof(int) * d->ntiles, d->stream));   /* the compaction keeps it at 0 */
+      CK(cudaMalloc(&d->scan_tmp, sizeof(int) * ((d->ntiles + 1023) / 1024 + 1)));
+      CK(cudaMalloc(&d->scan_state, sizeof(unsigned long long) * ((d->ntiles + 1023) / 1024 + 1)));
+      CK(cudaMemsetAsync(d->scan_state, 0, sizeof(unsigned long long) * ((d->ntiles + 1023) / 1024 + 1), d->stream));
+    }
   }
   free(d->sh);
   d->sh = (lbib_sheet_dev*)malloc(sizeof(lbib_sheet_dev) * nsheets);
@@ -375,7 +387,10 @@ extern "C" int lbdev_init_df1(lbib_device* d) {
   d->have_forces = 0;
   d->have_moments = 0;
   for (int b = 0; b < 2; ++b)
-    if (d->tile_slot[b]) CK(cudaMemsetAsync(d->tile_slot[b], 0xff, sizeof(int) * d->ntiles, d->stream));
+    if (d->tile_slot[b]) {
+      CK(cudaMemsetAsync(d->tile_slot[b], 0xff, sizeof(int) * d->ntiles, d->stream));
+      CK(cudaMemsetAsync(d->tile_count[b], 0, sizeof(int), d->stream));
+    }
   return 0;
 }
 
@@ -435,73 +450,74 @@ static int prof_grow(lbib_device* d) {
   return 0;
 }
 
-/* One full step in box mode (d->overlap, a whole grid): the box of this
- * step's stencils first; the fluid step's row and bulk kernels skip the
- * box's tiles and read no force -- they need nothing from this step's
- * forces and spread, and they lose the per-cell force-map lookups and the
- * forced collision from their code -- and the box's cells are stepped by
- * the generic rules after the spread; then the tile moments and the move.
- * Every cell is stepped once by the same per-cell arithmetic (the generic
- * rules give the two-cell kernel's bits), so the results do not change.
- * d->overlap == 2 runs the row and bulk kernels on the side stream,
- * concurrently with the forces and the spread; 1 keeps one stream (the
- * spread's kernels spread over every SM, and interleaving them with the
- * bandwidth-bound bulk kernel measured slower than running them in turn). */
+/* One full step in box mode (d->overlap, a whole grid).  Only the cells of
+ * the box of this step's stencils carry a force.  The row and bulk kernels
+ * skip the box's tiles and read no force -- they need nothing from this
+ * step's forces and spread, and they lose the per-cell force-map lookups
+ * and the forced collision from their code -- and one kernel gathers the
+ * spread force of the box's tiles and steps their cells by the generic
+ * rules; then the tile moments and the move.  Every cell is stepped once by
+ * the same per-cell arithmetic (the generic rules give the two-cell kernel's
+ * bits, and a cell's slots are its own in the AA pattern, so the order of
+ * the two does not matter).
+ * The row and bulk kernels run on the side stream, beside the preparation
+ * and the spread (d->overlap == 1: in stream order).  us per step one after
+ * the other / side by side, FP64: 63 / 50 at 64x32x32, 98 / 72 at
+ * 128x64x64, 1746 / 1721 at 512x256x256; 16-bit storage: 79 / 67 at
+ * 128x64x64, 777 / 763 at 512x256x256.  (With the spread in six launches
+ * instead of two, each of which had to find room among the bulk kernel's
+ * blocks, side by side was the slower at 512x256x256.) */
 static int step_overlapped(lbib_device* d, int step_no, cudaEvent_t* ev) {
   if (!d->nodes || !d->have_df1 || !d->have_inout) return -4;
   /* the box of this step's stencils: left by the previous step's move, or
-     computed here (first step, positions set from the host, pinned rows --
-     whose nodes the move does not visit) */
-  const int pinned = (d->compat & LBIB_OPT_PIN_ROW0) != 0;
-  if (!d->box_valid || pinned)
+     computed here (first step, positions set from the host) */
+  if (!d->box_valid)
     if (lbdev_launch_stencil_box(d)) return -2;
-  d->box_next = pinned ? NULL : d->box + 6 * (d->box_cur ^ 1);
-  CK(cudaEventRecord(d->ev_box, d->stream));
+  d->box_next = d->box + 6 * (d->box_cur ^ 1);
+  d->box_valid = 0;
   /* the step's buffers: the spread fills cur, the fluid reads cur ^ 1's moments */
   d->cur ^= 1;
   d->have_forces = 1;
   d->have_moments = 0;
   d->box_mode = 1;
   const int conc = d->overlap == 2;
-  cudaStream_t fs = conc ? d->side : d->stream;
   int rc = 0;
-  if (!conc) {
-    /* the forces: in the node preparation's launch when the sheets allow */
-    d->fuse_forces = lbdev_can_fuse_forces(d);
-    for (int k = 0; k < d->nsheets && !rc && !d->fuse_forces; ++k) rc = lbdev_launch_fiber_forces(d, k);
-    if (ev) CK(cudaEventRecord(ev[1], d->stream));
-    if (!rc) rc = lbdev_launch_spread(d, step_no);
-    d->fuse_forces = 0;
-    if (ev) CK(cudaEventRecord(ev[2], d->stream));
-    if (rc) { d->box_mode = 0; d->box_next = NULL; d->box_valid = 0; return -2; }
-  }
-  d->fluid_stream = fs;
-  if (conc) CK(cudaStreamWaitEvent(d->side, d->ev_box, 0));
-  if (ev) CK(cudaEventRecord(ev[6], fs));
-  rc = lbdev_launch_fluid_step(d);
-  if (ev) CK(cudaEventRecord(ev[7], fs));
-  if (conc) CK(cudaEventRecord(d->ev_bulk, d->side));
-  d->fluid_stream = d->stream;
-  if (rc) { d->box_mode = 0; d->box_next = NULL; d->box_valid = 0; return -2; }
   if (conc) {
-    for (int k = 0; k < d->nsheets && !rc; ++k) rc = lbdev_launch_fiber_forces(d, k);
-    if (ev) CK(cudaEventRecord(ev[1], d->stream));
-    if (!rc) rc = lbdev_launch_spread(d, step_no);
-    if (ev) CK(cudaEventRecord(ev[2], d->stream));
-    CK(cudaStreamWaitEvent(d->stream, d->ev_bulk, 0));
+    CK(cudaEventRecord(d->ev_box, d->stream));
+    CK(cudaStreamWaitEvent(d->side, d->ev_box, 0));
+    d->fluid_stream = d->side;
+    if (ev) CK(cudaEventRecord(ev[6], d->side));
+    rc = lbdev_launch_fluid_step(d);
+    if (ev) CK(cudaEventRecord(ev[7], d->side));
+    d->fluid_stream = d->stream;
+    CK(cudaEventRecord(d->ev_bulk, d->side));
   }
-  if (ev) CK(cudaEventRecord(ev[8], d->stream));
-  if (!rc) rc = lbdev_launch_box_cells(d);
-  d->box_mode = 0;
-  if (rc) { d->box_next = NULL; d->box_valid = 0; return -2; }
+  /* the forces: in the node preparation's launch when the sheets allow */
+  d->fuse_forces = lbdev_can_fuse_forces(d);
+  for (int k = 0; k < d->nsheets && !rc && !d->fuse_forces; ++k) rc = lbdev_launch_fiber_forces(d, k);
+  if (ev) CK(cudaEventRecord(ev[1], d->stream));
+  if (!rc) rc = lbdev_launch_prep(d, step_no);
+  d->fuse_forces = 0;
+  if (!rc) rc = lbdev_launch_spread_box(d);
+  if (ev) CK(cudaEventRecord(ev[2], d->stream));
+  if (conc) {
+    CK(cudaStreamWaitEvent(d->stream, d->ev_bulk, 0));
+  } else {
+    if (ev) CK(cudaEventRecord(ev[6], d->stream));
+    if (!rc) rc = lbdev_launch_fluid_step(d);
+    if (ev) CK(cudaEventRecord(ev[7], d->stream));
+  }
+  d->parity ^= 1;
+  d->steps++;
   if (ev) CK(cudaEventRecord(ev[3], d->stream));
   d->have_moments = 1;
-  rc = lbdev_launch_tile_moments(d) ? -2 : 0;
+  if (!rc) rc = lbdev_launch_tile_moments(d) ? -2 : 0;
+  d->box_mode = 0;
   if (ev) CK(cudaEventRecord(ev[4], d->stream));
   if (!rc) rc = lbdev_launch_move(d) ? -2 : 0;
   if (ev) CK(cudaEventRecord(ev[5], d->stream));
   /* the move reduced the next step's box into box_next */
-  d->box_valid = !rc && d->box_next != NULL;
+  d->box_valid = !rc;
   if (d->box_valid) d->box_cur ^= 1;
   d->box_next = NULL;
   return rc;
@@ -548,11 +564,9 @@ extern "C" int lbdev_profile_end(lbib_device* d, double* stage_ms, long* steps) 
     for (int s = 0; s < LBIB_NSTAGE_TIMED; ++s) {
       float ms = 0.f;
       if (s == 2 && d->prof_overlap[t]) {
-        /* overlapped: the bulk launches (side stream) plus the box's cells */
-        float a = 0.f, b = 0.f;
-        CK(cudaEventElapsedTime(&a, ev[6], ev[7]));
-        CK(cudaEventElapsedTime(&b, ev[8], ev[3]));
-        ms = a + b;
+        /* box mode: the row and bulk launches, on their stream (the box's
+           cells are stepped in the spread's) */
+        CK(cudaEventElapsedTime(&ms, ev[6], ev[7]));
       } else {
         CK(cudaEventElapsedTime(&ms, ev[s], ev[s + 1]));
       }
@@ -801,6 +815,7 @@ extern "C" int lbdev_load_state(lbib_device* d, FILE* fp) {
   if (rc) return rc;
   CK(cudaMemcpy(d->tile_count[c], &count, sizeof(int), cudaMemcpyHostToDevice));
   CK(cudaMemset(d->tile_slot[c ^ 1], 0xff, sizeof(int) * d->ntiles));
+  CK(cudaMemset(d->tile_count[c ^ 1], 0, sizeof(int)));
   d->parity = hdr[0];
   d->cur = c;
   d->have_forces = hdr[2];

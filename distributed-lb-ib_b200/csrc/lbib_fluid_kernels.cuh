@@ -24,6 +24,7 @@
 #include "lbib_internal.h"
 #include <climits>
 
+#include "lbib_ib.cuh"
 #include "lbib_lattice.cuh"
 
 namespace lbib {
@@ -247,31 +248,96 @@ __global__ void __launch_bounds__(128, LBIB_FLUID_MINB)
   step_cell<T, PAR>(p, x, r.x, r.y);
 }
 
-/* Box mode: every cell of I in the tiles of the box, by the generic rules
- * (forced where this step's spread touched the tile), one CTA of 64
- * threads per tile, a persistent grid over the box. */
+/* The tiles of a box, and its extents in x and y; an empty box (no node
+ * inside the grid: {INT_MAX, INT_MIN} per axis) has none. */
+__device__ __forceinline__ long box_tiles(const int* __restrict__ b, int& nbx, int& nby) {
+  if (b[1] < b[0] || b[3] < b[2] || b[5] < b[4]) {
+    nbx = nby = 1;
+    return 0;
+  }
+  nbx = b[1] - b[0] + 1;
+  nby = b[3] - b[2] + 1;
+  return (long)nbx * nby * (b[5] - b[4] + 1);
+}
+
+/* Box mode: the spread force of every touched tile of the box (gather_tile)
+ * and the step of every cell of I in the box, by the generic rules, in one
+ * pass: thread t < 64 holds cell t of the CTA's tile, loads its populations
+ * and moments before the gather (whose latency hides theirs) and collides
+ * with the sum it has just formed, which is also kept for the moments.  A
+ * persistent grid over the box, in x order (neighbouring tiles share DRAM
+ * bursts; the list's order, as the tiles were met, cost the moments 17
+ * against 8.5 us at 512x256x256), with a prime number of CTAs, so that none
+ * sees one x position of the box only.  With the force written by one
+ * launch and read back by another this was 31 + 33 us at 512x256x256
+ * (FP64), and 16 + 10 us at 64x32x32, of which most is launch and latency. */
+constexpr int kBoxCtas = 1181;
 template <typename T, int PAR>
-__global__ void __launch_bounds__(64) lbib_box_cells(FluidParamsT<T> p, int* __restrict__ reset) {
+__global__ void __launch_bounds__(kGatherTPB, 4) lbib_spread_box(FluidParamsT<T> p, GatherNodes g,
+                                                                 double* __restrict__ Ftile,
+                                                                 int* __restrict__ reset,
+                                                                 int* __restrict__ super_next, long nsuper,
+                                                                 const int* err) {
+  __shared__ GatherShared sm;
   /* the next step's box starts empty; the move fills it (it runs after us) */
   if (reset && blockIdx.x == 0 && threadIdx.x < 6) reset[threadIdx.x] = (threadIdx.x & 1) ? INT_MIN : INT_MAX;
+  clear_super(super_next, nsuper);
+  if (*(volatile const int*)err) return;
   const int* b = p.box;
-  const long lbx = (long)b[1] - b[0] + 1, lby = (long)b[3] - b[2] + 1, lbz = (long)b[5] - b[4] + 1;
-  if (lbx <= 0 || lby <= 0 || lbz <= 0) return;
-  const int nbx = (int)lbx, nby = (int)lby, nbz = (int)lbz;
-  const long n = (long)nbx * nby * nbz;
+  int nbx, nby;
+  const long n = box_tiles(b, nbx, nby);
+  using R = typename Pop<T>::R;
+  using F = Form<T>;
   const int cell = threadIdx.x;
   for (long i = blockIdx.x; i < n; i += gridDim.x) {
     const int tx = b[0] + (int)(i % nbx), ty = b[2] + (int)((i / nbx) % nby), tz = b[4] + (int)(i / ((long)nbx * nby));
+    const int tile = (tz * p.nty + ty) * p.ntx + tx;
+    const int slot = p.slot_cur[tile];
     const int x = tx * 4 + (cell & 3), y = ty * 4 + ((cell >> 2) & 3), z = tz * 4 + (cell >> 4);
-    if (x >= p.xlo && x <= p.xhi && y >= 2 && y <= p.ny - 3 && z >= 2 && z <= p.nz - 3) step_cell<T, PAR>(p, x, y, z);
+    const bool in = cell < 64 && x >= p.xlo && x <= p.xhi && y >= 2 && y <= p.ny - 3 && z >= 2 && z <= p.nz - 3;
+    const long idx = sidx(p, x, y, z);
+    int kind = K_FAST;
+    R f[19];
+    Mom<R> m;
+    if (in) {
+      kind = classify(p, x, y, z);
+      load_pre<PAR>(p, x, y, z, idx, kind, f);
+      if (kind >= K_SEMI) {
+        F::initial(p, m);
+      } else if (p.first) {
+        F::initial_bulk(p, m);
+      } else {
+        const int sp = p.slot_prev[tile];
+        if (sp >= 0) F::from_tile(p, p.Uprev + (long)sp * 256, cell, m);
+        else F::moments_free(f, p, m);
+      }
+    }
+    if (slot >= 0) {
+      double Fx, Fy, Fz;
+      gather_tile(sm, g, tx * 4, ty * 4, tz * 4, Fx, Fy, Fz);
+      if (cell < 64) {
+        double* Ft = Ftile + (long)slot * 192;
+        Ft[cell] = Fx; Ft[64 + cell] = Fy; Ft[128 + cell] = Fz;
+      }
+      if (in) F::template collide<true>(f, m, (R)Fx, (R)Fy, (R)Fz, p);
+    } else if (in) {
+      F::template collide<false>(f, m, R(0), R(0), R(0), p);
+    }
+    if (in) store_post<PAR>(p, x, y, z, idx, kind, f);
   }
 }
 
 template <typename T>
-int launch_box_cells_t(lbib_device* d, const FluidParamsT<T>& p) {
-  const unsigned blocks = 148 * 16;
-  if (d->parity == 0) lbib_box_cells<T, 0><<<blocks, 64, 0, d->stream>>>(p, d->box_next);
-  else lbib_box_cells<T, 1><<<blocks, 64, 0, d->stream>>>(p, d->box_next);
+int launch_spread_box_t(lbib_device* d, const FluidParamsT<T>& p) {
+  const unsigned blocks = kBoxCtas;
+  const int c = d->cur;
+  const GatherNodes g = gather_nodes(d);
+  if (d->parity == 0)
+    lbib_spread_box<T, 0><<<blocks, kGatherTPB, 0, d->stream>>>(p, g, d->Ftile[c], d->box_next, d->super[c ^ 1],
+                                                                d->nsuper, d->err);
+  else
+    lbib_spread_box<T, 1><<<blocks, kGatherTPB, 0, d->stream>>>(p, g, d->Ftile[c], d->box_next, d->super[c ^ 1],
+                                                                d->nsuper, d->err);
   d->kernel_launches++;
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -314,11 +380,36 @@ __device__ __forceinline__ void tile_moments_cell(const FluidParamsT<T>& p, int 
   U[cell] = rho; U[64 + cell] = ux; U[128 + cell] = uy; U[192 + cell] = uz;
 }
 
+/* The next step appends to the other buffer's tile list and finds its map
+ * all -1: undo the entries the step before last left there (its moments
+ * have been read for the last time); the list's count is reset by the move. */
+__device__ __forceinline__ void clear_slots(int* __restrict__ slot, const int* __restrict__ list,
+                                            const int* __restrict__ count) {
+  if (!slot) return;
+  const int n = *count;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) slot[list[i]] = -1;
+}
+
 /* Slot i of the touched-tile list: tile list[i]. */
 template <typename T, int PAR>
 __global__ void lbib_tile_moments(FluidParamsT<T> p, const int* __restrict__ list, const int* __restrict__ count,
-                                  const double* __restrict__ Ftile, double* __restrict__ Utile) {
+                                  const double* __restrict__ Ftile, double* __restrict__ Utile,
+                                  int* __restrict__ old_slot, const int* __restrict__ old_list,
+                                  const int* __restrict__ old_count) {
+  clear_slots(old_slot, old_list, old_count);
   const int n = *count;
+  if (p.box) {
+    /* box mode: in the box's x order, not the order the tiles were met in */
+    const int* b = p.box;
+    int nbx, nby;
+    const long nb = box_tiles(b, nbx, nby);
+    for (long i = blockIdx.x; i < nb; i += gridDim.x) {
+      const int tx = b[0] + (int)(i % nbx), ty = b[2] + (int)((i / nbx) % nby), tz = b[4] + (int)(i / ((long)nbx * nby));
+      const int tile = (tz * p.nty + ty) * p.ntx + tx, slot = p.slot_cur[tile];
+      if (slot >= 0) tile_moments_cell<T, PAR>(p, tile, slot, threadIdx.x, Ftile, Utile);
+    }
+    return;
+  }
   for (int i = blockIdx.x; i < n; i += gridDim.x) tile_moments_cell<T, PAR>(p, list[i], i, threadIdx.x, Ftile, Utile);
 }
 
@@ -499,11 +590,14 @@ template <typename T>
 int launch_tile_moments_t(lbib_device* d) {
   FluidParamsT<T> p = make_params_t<T>(d, 0);
   const int c = d->cur;
-  const int blocks = 148 * 16;
+  const int blocks = 2371;   /* ~16 CTAs per SM; prime, as kBoxCtas */
+  int* old = lbdev_is_slab(d) ? nullptr : d->tile_slot[c ^ 1];
   if (d->parity == 0)
-    lbib_tile_moments<T, 0><<<blocks, 64, 0, d->stream>>>(p, d->tile_list[c], d->tile_count[c], d->Ftile[c], d->Utile[c]);
+    lbib_tile_moments<T, 0><<<blocks, 64, 0, d->stream>>>(p, d->tile_list[c], d->tile_count[c], d->Ftile[c], d->Utile[c],
+                                                          old, d->tile_list[c ^ 1], d->tile_count[c ^ 1]);
   else
-    lbib_tile_moments<T, 1><<<blocks, 64, 0, d->stream>>>(p, d->tile_list[c], d->tile_count[c], d->Ftile[c], d->Utile[c]);
+    lbib_tile_moments<T, 1><<<blocks, 64, 0, d->stream>>>(p, d->tile_list[c], d->tile_count[c], d->Ftile[c], d->Utile[c],
+                                                          old, d->tile_list[c ^ 1], d->tile_count[c ^ 1]);
   d->kernel_launches++;
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

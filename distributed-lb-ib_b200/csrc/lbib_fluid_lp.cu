@@ -271,11 +271,11 @@ int launch_words_tma(lbib_device* d, const FluidParamsT<T>& p) {
 constexpr int kTmaVariants = 3;
 constexpr int kWords8Variants = 2;
 
-/* The box's cells of a box-mode step (after the spread). */
+/* The spread and the box's cells of a box-mode step. */
 template <typename T>
-int lp_box(lbib_device* d) {
+int lp_spread_box(lbib_device* d) {
   FluidParamsT<T> p = make_params_t<T>(d, d->steps == 0);
-  return launch_box_cells_t<T>(d, p);
+  return launch_spread_box_t<T>(d, p);
 }
 
 template <typename T>
@@ -307,11 +307,11 @@ extern "C" int lbdev_lp_fluid_step(lbib_device* d) {
   }
 }
 
-extern "C" int lbdev_lp_box_cells(lbib_device* d) {
+extern "C" int lbdev_lp_spread_box(lbib_device* d) {
   switch (LBIB_PREC_TYPE(d->prec)) {
-    case LBIB_PREC_F32: return lp_box<float>(d);
-    case LBIB_PREC_F16: return lp_box<__half>(d);
-    case LBIB_PREC_BF16: return lp_box<__nv_bfloat16>(d);
+    case LBIB_PREC_F32: return lp_spread_box<float>(d);
+    case LBIB_PREC_F16: return lp_spread_box<__half>(d);
+    case LBIB_PREC_BF16: return lp_spread_box<__nv_bfloat16>(d);
     default: return -1;
   }
 }

@@ -27,13 +27,16 @@ struct SheetForces {
 };
 
 /* A block per 32-node chunk: warp p < 4 evaluates part p of the chunk's
- * nodes (node_prep_part); warp 0 also reduces the chunk's stencil box.  A
- * fifth warp, when the block has one, computes the nodes' fiber forces for
- * the sheets `sf` names (fiber_forces_node reads neighbours' positions and
- * writes the node's own force fields only, so it runs alongside). */
-__global__ void __launch_bounds__(160) lbib_node_prep(double* __restrict__ nodes, long S, int nx, int ny, int nz,
+ * nodes (node_prep_part); warp 0 also reduces the chunk's stencil box and
+ * enters the tiles its stencils touch.  A fifth warp, when the block has
+ * one, computes the nodes' fiber forces for the sheets `sf` names
+ * (fiber_forces_node reads neighbours' positions and writes the node's own
+ * force fields only, so it runs alongside).  list NULL: mark the tiles only. */
+__global__ void __launch_bounds__(160, 5) lbib_node_prep(double* __restrict__ nodes, long S, int nx, int ny, int nz,
                                                       int ntx, int nty, double* __restrict__ W, int* __restrict__ st,
-                                                      int* __restrict__ tile_cnt, int* __restrict__ chunk_box, int* err,
+                                                      int* __restrict__ chunk_box, int* __restrict__ super,
+                                                      int* __restrict__ slot, int* __restrict__ list,
+                                                      int* __restrict__ count, int* __restrict__ mark, int* err,
                                                       int step, SheetForces sf) {
   const long i = (long)blockIdx.x * 32 + (threadIdx.x & 31);
   const int part = threadIdx.x >> 5;
@@ -47,96 +50,79 @@ __global__ void __launch_bounds__(160) lbib_node_prep(double* __restrict__ nodes
       fiber_forces_node(nodes + h.offset * 12, h.rows, h.cols, h.bc, h.sc, h.sc2, h.ds1, h.ds2, sf.bend_bug, (int)li);
     return;
   }
-  int b0 = INT_MAX, b1 = INT_MIN, b2 = INT_MAX, b3 = INT_MIN, b4 = INT_MAX, b5 = INT_MIN;
-  if (i < S) node_prep_part(nodes, i, part, nx, ny, nz, ntx, nty, W, st, tile_cnt, err, step, b0, b1, b2, b3, b4, b5);
-  if (part == 0) chunk_box_reduce(i, S, chunk_box, b0, b1, b2, b3, b4, b5);
+  int is = 0, js = 0, ks = 0;
+  const bool ok = i < S && node_prep_part(nodes, i, part, nx, ny, nz, W, st, err, step, is, js, ks);
+  if (part == 0) {
+    chunk_box_reduce(i, S, chunk_box, super, is, js, ks, ok);
+    touch_tiles(is, js, ks, ok, ntx, nty, 0, slot, list, count, mark);
+  }
 }
 
-/* Tiles of columns tx in [tlo, thi) only: the slot numbering covers every
- * touched tile (so that the moment tiles of x-slabs line up), but a slab
- * lists and gathers only the tiles its own fluid cells read. */
-__global__ void lbib_pair_scatter(const int* __restrict__ st, long S, int ntx, int nty, int nx, int ny, int nz,
-                                  int tlo, int thi, const int* __restrict__ slot, const int* __restrict__ slot_off,
-                                  int* __restrict__ slot_cursor, int2* __restrict__ ent, const int* err) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (*(volatile const int*)err) return;   /* uniform: the whole warp returns */
-  pair_scatter_warp(st, i, S, ntx, nty, nx, ny, nz, tlo, thi, slot, slot_off, slot_cursor, ent);
-}
-
-/* Every listed tile: from its entries (gather_tile_ent), or, with more
- * than kListCap nodes (a crumpled sheet), by scanning the node chunks in
- * order (gather_tile_scan). */
-__global__ void __launch_bounds__(64) lbib_spread_gather(const double* __restrict__ nodes, const double* __restrict__ W,
-                                                         const int* __restrict__ st, const int* __restrict__ chunk_box,
-                                                         long S, long nchunks, const int* __restrict__ list,
-                                                         const int* __restrict__ count, const int* __restrict__ slot_off,
-                                                         const int* __restrict__ slot_len,
-                                                         const int* __restrict__ slot_cursor,
-                                                         const int2* __restrict__ ent, int ntx, int nty, int tlo,
-                                                         int thi, double* __restrict__ Ftile, const int* err) {
-  __shared__ union {
-    GatherSmemE e;
-    ScanSmem s;
-  } sm;
+/* Every listed tile of columns tx in [tlo, thi) (an x-slab gathers the
+ * tiles its own fluid cells read; the whole grid all): its force into its
+ * slot.  super_next: the super-chunk boxes of the next step, emptied. */
+__global__ void __launch_bounds__(kGatherTPB) lbib_spread_gather(GatherNodes g, const int* __restrict__ list,
+                                                                 const int* __restrict__ count, int ntx, int nty,
+                                                                 int tlo, int thi, double* __restrict__ Ftile,
+                                                                 int* __restrict__ super_next, long nsuper,
+                                                                 const int* err) {
+  __shared__ GatherShared sm;
+  clear_super(super_next, nsuper);
   if (*(volatile const int*)err) return;
   const int n = *count;
   for (int it = blockIdx.x; it < n; it += gridDim.x) {
     const int tile = list[it], tx = tile % ntx;
     if (tx < tlo || tx >= thi) continue;   /* uniform over the block */
-    const int L = slot_len[it];
-    if (L <= kListCap) {
-      gather_tile_ent(sm.e, nodes, W, st, it, tile, L, slot_cursor[it], ent + slot_off[it], ntx, nty, Ftile);
-    } else {
-      __syncthreads();   /* the union's previous contents are no longer read */
-      gather_tile_scan(sm.s, nodes, W, st, chunk_box, S, 0, nchunks, it, tile, ntx, nty, Ftile);
+    double Fx, Fy, Fz;
+    gather_tile(sm, g, tx * 4, (tile / ntx) % nty * 4, tile / (ntx * nty) * 4, Fx, Fy, Fz);
+    if (threadIdx.x < 64) {
+      double* Ft = Ftile + (long)it * 192;
+      Ft[threadIdx.x] = Fx; Ft[64 + threadIdx.x] = Fy; Ft[128 + threadIdx.x] = Fz;
     }
   }
 }
 
-/* Nodes [i0, i1) of the concatenated sheets.  With `box` (an overlapped
- * step's next box), the box in tiles of the moved nodes' stencils is
- * reduced into it (block reduction, then six atomics per block). */
-constexpr int kMoveTPB = 64;   /* two warps, each with its staged union box */
+/* Nodes [i0, i1) that stay where they are (the pinned-row option). */
+struct PinnedRows {
+  int n;
+  long lo[kFuseSheets], hi[kFuseSheets];
+};
 
+/* Nodes [i0, i1) of the concatenated sheets.  With `box` (a box-mode step's
+ * next box), the box in tiles of the nodes' stencils, pinned ones included,
+ * is reduced into it (a warp reduction, then six atomics per block). */
 __global__ void __launch_bounds__(kMoveTPB) lbib_move_nodes(double* __restrict__ nodes, const double* __restrict__ W,
                                                             const int* __restrict__ st, long i0, long i1, int ntx,
                                                             int nty, const int* __restrict__ slot,
                                                             const double* __restrict__ Utile, double dt,
                                                             const int* err, int* __restrict__ box, int nx, int ny,
-                                                            int nz) {
-  __shared__ double sU[kMoveTPB / 32][3 * kMoveCap + kMoveTiles / 2];   /* + the staged tile slots */
-  const long i = i0 + (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = i < i1 && !*(volatile const int*)err;
-  move_warp(nodes, W, st, i, live, ntx, nty, slot, Utile, dt, sU[threadIdx.x >> 5]);
-  if (!box) return;
-  int b[6] = {INT_MAX, INT_MIN, INT_MAX, INT_MIN, INT_MAX, INT_MIN};
-  if (live) {
+                                                            int nz, int* __restrict__ old_count, PinnedRows pin) {
+  __shared__ MoveSmem sm;
+  if (old_count && blockIdx.x == 0 && threadIdx.x == 0) *old_count = 0;   /* the next step's list starts empty */
+  const long i = i0 + (long)blockIdx.x * 32 + (threadIdx.x & 31);
+  if (*(volatile const int*)err) return;   /* set by earlier launches only: uniform */
+  const bool have = i < i1;
+  bool live = have;
+  for (int k = 0; k < pin.n; ++k) live = live && !(i >= pin.lo[k] && i < pin.hi[k]);
+  move_chunk(sm, nodes, W, st, i, live, ntx, nty, slot, Utile, dt);
+  if (!box || threadIdx.x >= 32) return;
+  bool in = false;
+  int is = 0, js = 0, ks = 0;
+  if (have) {
     const double* m = nodes + i * 12;
-    if (stencil_inside(m[0], nx) && stencil_inside(m[1], ny) && stencil_inside(m[2], nz)) {
-      const int is = stencil_start(m[0]), js = stencil_start(m[1]), ks = stencil_start(m[2]);
-      b[0] = is >> 2; b[1] = (is + 3) >> 2; b[2] = js >> 2; b[3] = (js + 3) >> 2; b[4] = ks >> 2; b[5] = (ks + 3) >> 2;
-    }
+    in = stencil_inside(m[0], nx) && stencil_inside(m[1], ny) && stencil_inside(m[2], nz);
+    if (in) { is = stencil_start(m[0]); js = stencil_start(m[1]); ks = stencil_start(m[2]); }
   }
-  __shared__ int red[6][4];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    int v = b[k];
-    for (int o = 16; o > 0; o >>= 1) {
-      const int u = __shfl_xor_sync(0xffffffffu, v, o);
-      v = (k & 1) ? max(v, u) : min(v, u);
-    }
-    if (lane == 0) red[k][w] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 6) {
-    const int k = threadIdx.x;
-    int v = red[k][0];
-    for (int j = 1; j < (int)(blockDim.x >> 5); ++j) v = (k & 1) ? max(v, red[k][j]) : min(v, red[k][j]);
-    if ((k & 1) ? v != INT_MIN : v != INT_MAX) {
-      if (k & 1) atomicMax(&box[k], v);
-      else atomicMin(&box[k], v);
-    }
+  const int b[6] = {__reduce_min_sync(0xffffffffu, in ? is >> 2 : INT_MAX),
+                    __reduce_max_sync(0xffffffffu, in ? (is + 3) >> 2 : INT_MIN),
+                    __reduce_min_sync(0xffffffffu, in ? js >> 2 : INT_MAX),
+                    __reduce_max_sync(0xffffffffu, in ? (js + 3) >> 2 : INT_MIN),
+                    __reduce_min_sync(0xffffffffu, in ? ks >> 2 : INT_MAX),
+                    __reduce_max_sync(0xffffffffu, in ? (ks + 3) >> 2 : INT_MIN)};
+  if (threadIdx.x == 0 && b[0] <= b[1]) {
+    atomicMin(&box[0], b[0]); atomicMax(&box[1], b[1]);
+    atomicMin(&box[2], b[2]); atomicMax(&box[3], b[3]);
+    atomicMin(&box[4], b[4]); atomicMax(&box[5], b[5]);
   }
 }
 
@@ -231,13 +217,14 @@ extern "C" int lbdev_launch_stencil_box(lbib_device* d) {
  * sheets: lbdev_launch_spread computes them when d->fuse_forces is set. */
 extern "C" int lbdev_can_fuse_forces(const lbib_device* d) { return d->nsheets <= kFuseSheets; }
 
-extern "C" int lbdev_launch_spread(lbib_device* d, int step) {
+/* Node preparation: weights, stencil starts, boxes, the touched tiles (and,
+ * with d->fuse_forces, the fiber forces).  The whole grid lists the tiles as
+ * it meets them (the slot map of this step is all -1: the step before left
+ * it so, lbib_tile_moments); an x-slab marks them and compacts the marks,
+ * because the slabs of one grid number their slots alike. */
+extern "C" int lbdev_launch_prep(lbib_device* d, int step) {
   const int c = d->cur;
   cudaStream_t st = d->stream;
-  /* tile_cnt is left at zero and tile_slot[c] fully rewritten by the
-     compaction, so the step needs no clearing pass */
-  const long S = d->S;
-  const unsigned nb = (unsigned)((S + 127) / 128);
   SheetForces sf;
   sf.n = 0;
   sf.bend_bug = (d->compat & 1) != 0;
@@ -245,58 +232,60 @@ extern "C" int lbdev_launch_spread(lbib_device* d, int step) {
     sf.n = d->nsheets;
     for (int k = 0; k < d->nsheets; ++k) sf.s[k] = d->sh[k];
   }
-  lbib_node_prep<<<(unsigned)d->nchunks, sf.n ? 160 : 128, 0, st>>>(d->nodes, S, d->nx, d->ny, d->nz, d->ntx, d->nty,
-                                                                    d->W, d->st, d->tile_cnt, d->chunk_box, d->err,
-                                                                    step, sf);
-  const unsigned nblk = (unsigned)((d->ntiles + kScanBlock - 1) / kScanBlock);
-  if (d->scan_state && d->ntiles < (1L << 22) && 8 * S < (1L << 31)) {
-    d->scan_tag = d->scan_tag % 255u + 1u;
-    const unsigned nb1 = (unsigned)((d->ntiles + kScanBlock * kOnepassTiles - 1) / (kScanBlock * kOnepassTiles));
-    lbib_compact_onepass<<<nb1, kScanBlock, 0, st>>>(d->tile_cnt, d->ntiles, (int)nb1, d->scan_state, d->scan_tag,
-                                                      d->tile_list[c], d->tile_slot[c], d->slot_off, d->slot_len,
-                                                      d->slot_cursor, d->tile_count[c], d->err);
-    d->kernel_launches -= 2;
-  } else {
-    int* block_tiles = d->scan_tmp;
-    int* block_pairs = d->scan_tmp + nblk + 1;
-    lbib_compact_count<<<nblk, kScanBlock, 0, st>>>(d->tile_cnt, d->ntiles, block_tiles, block_pairs);
-    lbib_compact_scan<<<1, kScanBlock, 0, st>>>(block_tiles, block_pairs, (int)nblk, d->tile_count[c]);
-    lbib_compact_write<<<nblk, kScanBlock, 0, st>>>(d->tile_cnt, d->ntiles, block_tiles, block_pairs,
-                                                    d->tile_list[c], d->tile_slot[c], d->slot_off, d->slot_len,
-                                                    d->slot_cursor);
+  const int slab = lbdev_is_slab(d);
+  lbib_node_prep<<<(unsigned)d->nchunks, sf.n ? 160 : 128, 0, st>>>(
+      d->nodes, d->S, d->nx, d->ny, d->nz, d->ntx, d->nty, d->W, d->st, d->chunk_box, d->super[c], d->tile_slot[c],
+      slab ? nullptr : d->tile_list[c], d->tile_count[c], d->tile_mark, d->err, step, sf);
+  d->kernel_launches++;
+  if (slab) {
+    const unsigned nblk = (unsigned)((d->ntiles + kScanBlock - 1) / kScanBlock);
+    if (d->ntiles < (1L << 31)) {
+      d->scan_tag = d->scan_tag % 255u + 1u;
+      const unsigned nb1 = (unsigned)((d->ntiles + kScanBlock * kOnepassTiles - 1) / (kScanBlock * kOnepassTiles));
+      lbib_compact_onepass<<<nb1, kScanBlock, 0, st>>>(d->tile_mark, d->ntiles, (int)nb1, d->scan_state, d->scan_tag,
+                                                        d->tile_list[c], d->tile_slot[c], d->tile_count[c], d->err);
+      d->kernel_launches++;
+    } else {
+      lbib_compact_count<<<nblk, kScanBlock, 0, st>>>(d->tile_mark, d->ntiles, d->scan_tmp);
+      lbib_compact_scan<<<1, kScanBlock, 0, st>>>(d->scan_tmp, (int)nblk, d->tile_count[c]);
+      lbib_compact_write<<<nblk, kScanBlock, 0, st>>>(d->tile_mark, d->ntiles, d->scan_tmp, d->tile_list[c],
+                                                      d->tile_slot[c]);
+      d->kernel_launches += 3;
+    }
   }
-  /* an x-slab lists and gathers the tiles of its own columns only */
-  const int tlo = d->x_lo / 4, thi = (d->x_hi + 3) / 4;
-  int2* ent = reinterpret_cast<int2*>(d->pair_node);
-  lbib_pair_scatter<<<nb, 128, 0, st>>>(d->st, S, d->ntx, d->nty, d->nx, d->ny, d->nz, tlo, thi, d->tile_slot[c],
-                                        d->slot_off, d->slot_cursor, ent, d->err);
-  lbib_spread_gather<<<148 * 12, 64, 0, st>>>(d->nodes, d->W, d->st, d->chunk_box, S, d->nchunks, d->tile_list[c],
-                                              d->tile_count[c], d->slot_off, d->slot_len, d->slot_cursor, ent,
-                                              d->ntx, d->nty, tlo, thi, d->Ftile[c], d->err);
-  d->kernel_launches += 6;
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+/* Node preparation and the gather over the listed tiles. */
+extern "C" int lbdev_launch_spread(lbib_device* d, int step) {
+  if (lbdev_launch_prep(d, step)) return -2;
+  const int c = d->cur;
+  lbib_spread_gather<<<148 * 8, kGatherTPB, 0, d->stream>>>(gather_nodes(d), d->tile_list[c], d->tile_count[c], d->ntx,
+                                                             d->nty, d->x_lo / 4, (d->x_hi + 3) / 4, d->Ftile[c],
+                                                             d->super[c ^ 1], d->nsuper, d->err);
+  d->kernel_launches++;
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 /* moveFiberSheet over all nodes; with the pinned-row option (no reference
- * counterpart) row 0 of every sheet is left where it is: one launch per
- * sheet over its rows 1 .. rows-1. */
+ * counterpart) row 0 of every sheet stays where it is: kFuseSheets sheets
+ * to a launch. */
 extern "C" int lbdev_launch_move(lbib_device* d) {
-  const int c = d->cur;
-  if (!(d->compat & LBIB_OPT_PIN_ROW0)) {
-    const unsigned nb = (unsigned)((d->S + kMoveTPB - 1) / kMoveTPB);
-    lbib_move_nodes<<<nb, kMoveTPB, 0, d->stream>>>(d->nodes, d->W, d->st, 0, d->S, d->ntx, d->nty,
-                                                    d->tile_slot[c], d->Utile[c], (double)d->dt, d->err,
-                                                    d->box_next, d->nx, d->ny, d->nz);
-    d->kernel_launches++;
-  } else {
-    for (int k = 0; k < d->nsheets; ++k) {
-      const long i0 = d->sh[k].offset + d->sh[k].cols, i1 = d->sh[k].offset + (long)d->sh[k].rows * d->sh[k].cols;
-      const unsigned nb = (unsigned)((i1 - i0 + kMoveTPB - 1) / kMoveTPB);
-      lbib_move_nodes<<<nb, kMoveTPB, 0, d->stream>>>(d->nodes, d->W, d->st, i0, i1, d->ntx, d->nty,
-                                                      d->tile_slot[c], d->Utile[c], (double)d->dt, d->err, nullptr,
-                                                      d->nx, d->ny, d->nz);
-      d->kernel_launches++;
+  const int c = d->cur, pinned = (d->compat & LBIB_OPT_PIN_ROW0) != 0;
+  const int per = pinned ? kFuseSheets : d->nsheets;
+  for (int k0 = 0; k0 < d->nsheets; k0 += per) {
+    const int k1 = k0 + per < d->nsheets ? k0 + per : d->nsheets;
+    const long i0 = d->sh[k0].offset, i1 = d->sh[k1 - 1].offset + (long)d->sh[k1 - 1].rows * d->sh[k1 - 1].cols;
+    PinnedRows pin;
+    pin.n = pinned ? k1 - k0 : 0;
+    for (int k = 0; k < pin.n; ++k) {
+      pin.lo[k] = d->sh[k0 + k].offset;
+      pin.hi[k] = pin.lo[k] + d->sh[k0 + k].cols;
     }
+    lbib_move_nodes<<<(unsigned)((i1 - i0 + 31) / 32), kMoveTPB, 0, d->stream>>>(
+        d->nodes, d->W, d->st, i0, i1, d->ntx, d->nty, d->tile_slot[c], d->Utile[c], (double)d->dt, d->err, d->box_next,
+        d->nx, d->ny, d->nz, k0 == 0 && !lbdev_is_slab(d) ? d->tile_count[c ^ 1] : nullptr, pin);
+    d->kernel_launches++;
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

@@ -6,29 +6,33 @@
  *                       compute_elasticforce (cube_pthread/lbm_ib.c:961-1318),
  *                       one node, both passes of each force in the
  *                       reference's order.
- *   node_prep_one       stencil start floor(X - 2) + 1 per axis, the twelve
+ *   node_prep_part      stencil start floor(X - 2) + 1 per axis, the twelve
  *                       delta-kernel factors 1 + cos(pi/2 r) (shared by the
- *                       spread and the interpolation of the step), the 4^3
- *                       tiles the stencil touches; chunk_box_reduce: per
- *                       32-node chunk the bounding box of its stencils.
- *   compaction kernels  touched tiles -> dense list in tile order, tile ->
- *                       slot map, and each slot's list offset
- *                       (deterministic prefix sums, three launches or one
- *                       single-pass launch); pair_scatter_warp fills the
- *                       lists with {chunk, lane mask} entries.
- *   gather_tile_ent     fiber_SpreadForce + fluid_get_SpreadForce
+ *                       spread and the interpolation of the step);
+ *                       chunk_box_reduce: per 32-node chunk (and per 1024)
+ *                       the bounding box of its stencils; touch_tiles: the
+ *                       4^3 tiles the stencils touch, appended to the
+ *                       step's tile list as they are met (or only marked,
+ *                       for the compaction below).
+ *   compaction kernels  x-slabs only: marked tiles -> dense list in tile
+ *                       order and tile -> slot map (deterministic prefix
+ *                       sums, three launches or one single-pass launch), so
+ *                       that every slab numbers the slots alike.
+ *   gather_tile         fiber_SpreadForce + fluid_get_SpreadForce
  *                       (lbm_ib.c:1323-1525) as a gather: one CTA per touched
- *                       tile sorts the tile's entries, writes its node list
- *                       in index order, then each thread (cell) sums the
- *                       contributions in that order -- the reference's
- *                       (sheet, row, col) order -- so the result is
- *                       deterministic and needs no atomics on forces.
+ *                       tile finds the nodes that touch it, in index order,
+ *                       from the boxes; then each of 64 threads (cells)
+ *                       sums its contributions in that order -- the
+ *                       reference's (sheet, row, col) order -- so the result
+ *                       is deterministic and needs no atomics on forces.
  *   move_node /         moveFiberSheet (lbm_ib.c:2540-2723): u * w summed over
  *   move_warp           the 64 stencil cells in the reference's (x, y, z)
  *                       order, then X += dt U (move_warp: a warp's nodes
  *                       with their stencils' union staged in shared memory).
  * All arithmetic keeps the reference's operation order; translation units
- * that include this file are compiled with -fmad=false.
+ * that include this file are compiled with -fmad=false, except that the
+ * gather (explicitly rounded operations) is also used by the low-precision
+ * fluid kernels, which allow contraction.
  */
 #ifndef LBIB_IB_CUH
 #define LBIB_IB_CUH
@@ -157,116 +161,117 @@ __device__ __forceinline__ int stencil_start(double p) { return (int)(floor(p / 
  * turn NaN into 0 and pass). */
 __device__ __forceinline__ bool stencil_inside(double p, int n) { return p >= 1.0 && p < (double)n - 2.0; }
 
-/* Node i: stencil start, the twelve delta-kernel factors, a count for every
- * 4^3 tile its stencil touches (tile ids offset by tile0); b0..b5 receive
- * its stencil box (left empty when the stencil leaves the grid). */
-__device__ __forceinline__ void node_prep_one(const double* __restrict__ nodes, long i, int nx, int ny, int nz,
-                                              int ntx, int nty, long tile0, double* __restrict__ W,
-                                              int* __restrict__ st, int* __restrict__ tile_cnt, int* err, int step,
-                                              int& b0, int& b1, int& b2, int& b3, int& b4, int& b5) {
-  {
-    const double* m = nodes + i * 12;
-    const bool inside = stencil_inside(m[0], nx) && stencil_inside(m[1], ny) && stencil_inside(m[2], nz);
-    const int is = inside ? stencil_start(m[0]) : 0, js = inside ? stencil_start(m[1]) : 0,
-              ks = inside ? stencil_start(m[2]) : 0;
-    st[i * 3 + 0] = is; st[i * 3 + 1] = js; st[i * 3 + 2] = ks;
-    const double cxk = kPi / (2.0 * 1.0);
-    double* w = W + i * 12;
-    for (int a = 0; a < 4; ++a) {
-      w[a] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (is + a) - m[0]));
-      w[4 + a] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (js + a) - m[1]));
-      w[8 + a] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (ks + a) - m[2]));
-    }
-    if (!inside) {
-      set_error(err, -3, step);
-    } else {
-      for (int tz = ks >> 2; tz <= (ks + 3) >> 2; ++tz)
-        for (int ty = js >> 2; ty <= (js + 3) >> 2; ++ty)
-          for (int tx = is >> 2; tx <= (is + 3) >> 2; ++tx)
-            atomicAdd(&tile_cnt[tile0 + ((long)tz * nty + ty) * ntx + tx], 1);
-      b0 = is; b1 = is + 3; b2 = js; b3 = js + 3; b4 = ks; b5 = ks + 3;
-    }
-  }
-}
-
-/* node_prep_one for the one-grid kernel, split over four threads per node:
- * part p (0..3) evaluates the three delta factors of stencil offset p (one
- * per axis); part 0 also writes the stencil start, checks the grid and
- * counts the touched tiles.  The same values as node_prep_one, with the
- * twelve dependent cosine evaluations of a node spread over four warps. */
-__device__ __forceinline__ void node_prep_part(const double* __restrict__ nodes, long i, int part, int nx, int ny,
-                                               int nz, int ntx, int nty, double* __restrict__ W,
-                                               int* __restrict__ st, int* __restrict__ tile_cnt, int* err, int step,
-                                               int& b0, int& b1, int& b2, int& b3, int& b4, int& b5) {
+/* Node i, split over four threads: part p (0..3) evaluates the three delta
+ * factors of stencil offset p (one per axis); part 0 also writes the stencil
+ * start and checks the grid.  Returns whether the stencil lies inside, its
+ * start in is, js, ks. */
+__device__ __forceinline__ bool node_prep_part(const double* __restrict__ nodes, long i, int part, int nx, int ny,
+                                               int nz, double* __restrict__ W, int* __restrict__ st, int* err,
+                                               int step, int& is, int& js, int& ks) {
   const double* m = nodes + i * 12;
   const bool inside = stencil_inside(m[0], nx) && stencil_inside(m[1], ny) && stencil_inside(m[2], nz);
-  const int is = inside ? stencil_start(m[0]) : 0, js = inside ? stencil_start(m[1]) : 0,
-            ks = inside ? stencil_start(m[2]) : 0;
+  is = inside ? stencil_start(m[0]) : 0;
+  js = inside ? stencil_start(m[1]) : 0;
+  ks = inside ? stencil_start(m[2]) : 0;
   const double cxk = kPi / (2.0 * 1.0);
   double* w = W + i * 12;
   w[part] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (is + part) - m[0]));
   w[4 + part] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (js + part) - m[1]));
   w[8 + part] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (ks + part) - m[2]));
-  if (part != 0) return;
+  if (part != 0) return inside;
   st[i * 3 + 0] = is; st[i * 3 + 1] = js; st[i * 3 + 2] = ks;
-  if (!inside) {
-    set_error(err, -3, step);
-  } else {
-    for (int tz = ks >> 2; tz <= (ks + 3) >> 2; ++tz)
-      for (int ty = js >> 2; ty <= (js + 3) >> 2; ++ty)
-        for (int tx = is >> 2; tx <= (is + 3) >> 2; ++tx)
-          atomicAdd(&tile_cnt[((long)tz * nty + ty) * ntx + tx], 1);
-    b0 = is; b1 = is + 3; b2 = js; b3 = js + 3; b4 = ks; b5 = ks + 3;
-  }
+  if (!inside) set_error(err, -3, step);
+  return inside;
 }
 
-/* The bounding box of a warp's stencils, written by lane 0 for chunk i >> 5. */
-__device__ __forceinline__ void chunk_box_reduce(long i, long S, int* __restrict__ chunk_box, int b0, int b1, int b2,
-                                                 int b3, int b4, int b5) {
+/* The 4^3 tiles (ids offset by tile0) that a warp's stencils touch, ok: the
+ * lane has one.  The lanes that touch a tile at the same stencil offset act
+ * once, through the first of them.  With `list`: the warp that meets a tile
+ * first (slot[tile] goes from -1 through -2) gives it the next slot --
+ * which one depends on timing, no result does -- so that one launch does
+ * what took a count, a prefix sum over all tiles and a scatter (22 us of a
+ * 512x256x256 step's spread).  Without: mark[tile] = 1.  The eight offsets'
+ * loads and atomics are each issued together. */
+__device__ __forceinline__ void touch_tiles(int is, int js, int ks, bool ok, int ntx, int nty, long tile0,
+                                            int* __restrict__ slot, int* __restrict__ list, int* __restrict__ count,
+                                            int* __restrict__ mark) {
   const int lane = threadIdx.x & 31;
-  for (int o = 16; o > 0; o >>= 1) {
-    b0 = min(b0, __shfl_xor_sync(0xffffffffu, b0, o));
-    b1 = max(b1, __shfl_xor_sync(0xffffffffu, b1, o));
-    b2 = min(b2, __shfl_xor_sync(0xffffffffu, b2, o));
-    b3 = max(b3, __shfl_xor_sync(0xffffffffu, b3, o));
-    b4 = min(b4, __shfl_xor_sync(0xffffffffu, b4, o));
-    b5 = max(b5, __shfl_xor_sync(0xffffffffu, b5, o));
+  long tile[8];
+  int was[8];
+#pragma unroll
+  for (int o = 0; o < 8; ++o) {
+    const int tx = (is >> 2) + (o & 1), ty = (js >> 2) + ((o >> 1) & 1), tz = (ks >> 2) + (o >> 2);
+    const bool here = ok && tx <= (is + 3) >> 2 && ty <= (js + 3) >> 2 && tz <= (ks + 3) >> 2;
+    const long id = here ? tile0 + ((long)tz * nty + ty) * ntx + tx : -1;
+    const unsigned grp = __match_any_sync(0xffffffffu, id);
+    tile[o] = here && lane == __ffs(grp) - 1 ? id : -1;
   }
-  const long chunk = i >> 5;
-  if (lane == 0 && chunk * 32 < S) {
-    int* bx = chunk_box + chunk * 6;
-    bx[0] = b0; bx[1] = b1; bx[2] = b2; bx[3] = b3; bx[4] = b4; bx[5] = b5;
+  if (!list) {
+#pragma unroll
+    for (int o = 0; o < 8; ++o)
+      if (tile[o] >= 0) mark[tile[o]] = 1;
+    return;
   }
+  volatile int* vs = slot;
+#pragma unroll
+  for (int o = 0; o < 8; ++o) was[o] = tile[o] >= 0 ? vs[tile[o]] : 0;
+#pragma unroll
+  for (int o = 0; o < 8; ++o)
+    if (tile[o] >= 0 && was[o] == -1) was[o] = atomicCAS(&slot[tile[o]], -1, -2);
+    else was[o] = 0;
+#pragma unroll
+  for (int o = 0; o < 8; ++o)
+    if (was[o] == -1) was[o] = atomicAdd(count, 1);
+    else was[o] = -1;
+#pragma unroll
+  for (int o = 0; o < 8; ++o)
+    if (was[o] >= 0) {
+      list[was[o]] = (int)tile[o];
+      slot[tile[o]] = was[o];
+    }
 }
 
-/* Deterministic compaction of the tile counts, in tile-index order:
- * per-block sums (touched tiles, node-tile pairs), a one-block scan of both,
- * then every touched tile gets its slot and the offset of its node list. */
+constexpr int kSuper = 32;   /* chunks per super-chunk */
+
+/* The bounding box of a warp's stencils (ok: the lane has one), written by
+ * lane 0 for chunk i >> 5, and merged into its super-chunk's (`super` may be
+ * NULL: few chunks). */
+__device__ __forceinline__ void chunk_box_reduce(long i, long S, int* __restrict__ chunk_box,
+                                                 int* __restrict__ super, int is, int js, int ks, bool ok) {
+  int b0 = ok ? is : INT_MAX, b1 = ok ? is + 3 : INT_MIN, b2 = ok ? js : INT_MAX, b3 = ok ? js + 3 : INT_MIN,
+      b4 = ok ? ks : INT_MAX, b5 = ok ? ks + 3 : INT_MIN;
+  b0 = __reduce_min_sync(0xffffffffu, b0); b1 = __reduce_max_sync(0xffffffffu, b1);
+  b2 = __reduce_min_sync(0xffffffffu, b2); b3 = __reduce_max_sync(0xffffffffu, b3);
+  b4 = __reduce_min_sync(0xffffffffu, b4); b5 = __reduce_max_sync(0xffffffffu, b5);
+  const long chunk = i >> 5;
+  if ((threadIdx.x & 31) != 0 || chunk * 32 >= S) return;
+  int* bx = chunk_box + chunk * 6;
+  bx[0] = b0; bx[1] = b1; bx[2] = b2; bx[3] = b3; bx[4] = b4; bx[5] = b5;
+  if (!super) return;
+  int* sx = super + chunk / kSuper * 6;
+  atomicMin(&sx[0], b0); atomicMax(&sx[1], b1);
+  atomicMin(&sx[2], b2); atomicMax(&sx[3], b3);
+  atomicMin(&sx[4], b4); atomicMax(&sx[5], b5);
+}
+
+/* Deterministic compaction of the marked tiles, in tile-index order:
+ * per-block sums, a one-block scan, then every marked tile gets its slot. */
 constexpr int kScanBlock = 1024;
 
-static __global__ void lbib_compact_count(const int* __restrict__ cnt, long n, int* __restrict__ block_tiles,
-                                   int* __restrict__ block_pairs) {
-  __shared__ int s[2][32];
+static __global__ void lbib_compact_count(const int* __restrict__ mark, long n, int* __restrict__ block_tiles) {
+  __shared__ int s[32];
   const long i = (long)blockIdx.x * kScanBlock + threadIdx.x;
-  const int c = (i < n) ? cnt[i] : 0;
-  int v = c > 0, w = c;
-  for (int o = 16; o > 0; o >>= 1) {
-    v += __shfl_xor_sync(0xffffffffu, v, o);
-    w += __shfl_xor_sync(0xffffffffu, w, o);
-  }
-  if ((threadIdx.x & 31) == 0) { s[0][threadIdx.x >> 5] = v; s[1][threadIdx.x >> 5] = w; }
+  int v = i < n && mark[i] != 0;
+  v = __reduce_add_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
   __syncthreads();
   if (threadIdx.x < 32) {
-    int a = s[0][threadIdx.x], b = s[1][threadIdx.x];
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    if (threadIdx.x == 0) { block_tiles[blockIdx.x] = a; block_pairs[blockIdx.x] = b; }
+    const int a = __reduce_add_sync(0xffffffffu, s[threadIdx.x]);
+    if (threadIdx.x == 0) block_tiles[blockIdx.x] = a;
   }
 }
 
-__device__ __forceinline__ void block_exclusive_scan(int* __restrict__ a, int n, int* total) {
+static __global__ void lbib_compact_scan(int* __restrict__ a, int n, int* __restrict__ total) {
   __shared__ int s[kScanBlock];
   int carry = 0;
   for (int base = 0; base < n; base += kScanBlock) {
@@ -285,91 +290,65 @@ __device__ __forceinline__ void block_exclusive_scan(int* __restrict__ a, int n,
     __syncthreads();
     carry += last;
   }
-  if (threadIdx.x == 0 && total) *total = carry;
+  if (threadIdx.x == 0) *total = carry;
 }
 
-static __global__ void lbib_compact_scan(int* __restrict__ block_tiles, int* __restrict__ block_pairs, int nblocks,
-                                  int* __restrict__ total_tiles) {
-  block_exclusive_scan(block_tiles, nblocks, total_tiles);
-  __syncthreads();
-  block_exclusive_scan(block_pairs, nblocks, nullptr);
-}
-
-static __global__ void lbib_compact_write(int* __restrict__ cnt, long n, const int* __restrict__ block_tiles,
-                                   const int* __restrict__ block_pairs, int* __restrict__ list,
-                                   int* __restrict__ slot, int* __restrict__ slot_off, int* __restrict__ slot_len,
-                                   int* __restrict__ slot_cursor) {
-  __shared__ int sv[32], sw[32];
+static __global__ void lbib_compact_write(int* __restrict__ mark, long n, const int* __restrict__ block_tiles,
+                                          int* __restrict__ list, int* __restrict__ slot) {
+  __shared__ int sv[32];
   const long i = (long)blockIdx.x * kScanBlock + threadIdx.x;
-  const int c = (i < n) ? cnt[i] : 0;
-  const int v = c > 0;
+  const int v = i < n && mark[i] != 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int iv = v, iw = c;  /* inclusive warp scans */
-  for (int o = 1; o < 32; o <<= 1) {
-    const int tv = __shfl_up_sync(0xffffffffu, iv, o);
-    const int tw = __shfl_up_sync(0xffffffffu, iw, o);
-    if (lane >= o) { iv += tv; iw += tw; }
-  }
-  if (lane == 31) { sv[warp] = iv; sw[warp] = iw; }
+  const unsigned m = __ballot_sync(0xffffffffu, v);
+  if (lane == 0) sv[warp] = __popc(m);
   __syncthreads();
   if (threadIdx.x < 32) {
-    const int a = sv[threadIdx.x], b = sw[threadIdx.x];
-    int ia = a, ib = b;
+    const int a = sv[threadIdx.x];
+    int ia = a;
     for (int o = 1; o < 32; o <<= 1) {
       const int ta = __shfl_up_sync(0xffffffffu, ia, o);
-      const int tb = __shfl_up_sync(0xffffffffu, ib, o);
-      if (lane >= o) { ia += ta; ib += tb; }
+      if (lane >= o) ia += ta;
     }
     sv[threadIdx.x] = ia - a;
-    sw[threadIdx.x] = ib - b;
   }
   __syncthreads();
   if (v) {
-    const int pos = block_tiles[blockIdx.x] + sv[warp] + iv - v;
+    const int pos = block_tiles[blockIdx.x] + sv[warp] + __popc(m & ((1u << lane) - 1u));
     list[pos] = (int)i;
     slot[i] = pos;
-    slot_off[pos] = block_pairs[blockIdx.x] + sw[warp] + iw - c;
-    slot_len[pos] = c;
-    slot_cursor[pos] = 0;
+    mark[i] = 0;      /* the next step starts unmarked */
   } else if (i < n) {
     slot[i] = -1;     /* the whole map is written: no clearing pass before the step */
   }
-  if (i < n && c) cnt[i] = 0;   /* counts start the next step at zero */
 }
 
 /* The same compaction in one launch: a single-pass scan with decoupled
  * look-back (Merrill & Garland, "Single-pass Parallel Prefix Scan with
  * Decoupled Look-back", 2016).  A block takes its place in tile order from
  * a ticket counter (so every block before it has started), publishes its
- * block totals, walks back over its predecessors' published totals until
+ * block total, walks back over its predecessors' published totals until
  * one carries an inclusive prefix, publishes its own inclusive prefix and
  * writes its tiles' slots.  Each published word is 64 bits: an 8-bit
  * launch tag (1..255, never 0, so a zeroed or stale word never matches),
- * a 2-bit flag (1 block totals, 2 inclusive prefix), 22 bits of tiles and
- * 32 bits of pairs; the host uses it only when the tile count fits 22
- * bits.  Every wait is bounded: a walk that runs out sets err (the step
+ * a 2-bit flag (1 block total, 2 inclusive prefix) and 32 bits of tiles.
+ * Every wait is bounded: a walk that runs out sets err (the step
  * then fails) instead of spinning on.  state[nblk] holds the ticket,
  * which the last block resets for the next launch. */
 constexpr long kLookbackSpin = 1L << 22;
 constexpr int kOnepassTiles = 4;   /* tiles per thread: a block covers 4096 tiles */
 constexpr int kErrLookback = -2;   /* the error word's code: LBIB_E_CUDA of include/lbib.h */
 
-__device__ __forceinline__ unsigned long long lookback_word(unsigned tag, unsigned flag, unsigned long long t,
-                                                            unsigned long long p) {
-  return ((unsigned long long)tag << 56) | ((unsigned long long)flag << 54) | ((t & 0x3FFFFFull) << 32) |
-         (p & 0xFFFFFFFFull);
+__device__ __forceinline__ unsigned long long lookback_word(unsigned tag, unsigned flag, unsigned long long t) {
+  return ((unsigned long long)tag << 56) | ((unsigned long long)flag << 54) | (t & 0xFFFFFFFFull);
 }
 
-static __global__ void __launch_bounds__(kScanBlock) lbib_compact_onepass(int* __restrict__ cnt, long n, int nblk,
+static __global__ void __launch_bounds__(kScanBlock) lbib_compact_onepass(int* __restrict__ mark, long n, int nblk,
                                                                           unsigned long long* __restrict__ state,
                                                                           unsigned tag, int* __restrict__ list,
                                                                           int* __restrict__ slot,
-                                                                          int* __restrict__ slot_off,
-                                                                          int* __restrict__ slot_len,
-                                                                          int* __restrict__ slot_cursor,
                                                                           int* __restrict__ total, int* err) {
-  __shared__ int sv[32], sw[32];
-  __shared__ int s_vb, s_tt, s_tp, s_pt, s_pp;
+  __shared__ int sv[32];
+  __shared__ int s_vb, s_tt, s_pt;
   unsigned* ticket = reinterpret_cast<unsigned*>(state + nblk);
   if (threadIdx.x == 0) s_vb = (int)atomicAdd(ticket, 1u);
   __syncthreads();
@@ -377,33 +356,29 @@ static __global__ void __launch_bounds__(kScanBlock) lbib_compact_onepass(int* _
   /* kOnepassTiles consecutive tiles per thread: fewer, fuller blocks, so
      that every block is resident at once and the look-back walks short */
   const long i0 = ((long)vb * kScanBlock + threadIdx.x) * kOnepassTiles;
-  int c[kOnepassTiles], tv = 0, tw = 0;
+  int c[kOnepassTiles], tv = 0;
 #pragma unroll
   for (int k = 0; k < kOnepassTiles; ++k) {
-    c[k] = (i0 + k < n) ? cnt[i0 + k] : 0;
+    c[k] = (i0 + k < n) ? mark[i0 + k] : 0;
     tv += c[k] > 0;
-    tw += c[k];
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int iv = tv, iw = tw;  /* inclusive warp scans of the threads' totals */
+  int iv = tv;  /* inclusive warp scan of the threads' totals */
   for (int o = 1; o < 32; o <<= 1) {
-    const int tv = __shfl_up_sync(0xffffffffu, iv, o);
-    const int tw = __shfl_up_sync(0xffffffffu, iw, o);
-    if (lane >= o) { iv += tv; iw += tw; }
+    const int u = __shfl_up_sync(0xffffffffu, iv, o);
+    if (lane >= o) iv += u;
   }
-  if (lane == 31) { sv[warp] = iv; sw[warp] = iw; }
+  if (lane == 31) sv[warp] = iv;
   __syncthreads();
   if (threadIdx.x < 32) {
-    const int a = sv[threadIdx.x], b = sw[threadIdx.x];
-    int ia = a, ib = b;
+    const int a = sv[threadIdx.x];
+    int ia = a;
     for (int o = 1; o < 32; o <<= 1) {
       const int ta = __shfl_up_sync(0xffffffffu, ia, o);
-      const int tb = __shfl_up_sync(0xffffffffu, ib, o);
-      if (lane >= o) { ia += ta; ib += tb; }
+      if (lane >= o) ia += ta;
     }
     sv[threadIdx.x] = ia - a;
-    sw[threadIdx.x] = ib - b;
-    if (threadIdx.x == 31) { s_tt = ia; s_tp = ib; }
+    if (threadIdx.x == 31) s_tt = ia;
   }
   __syncthreads();
   if (warp == 0) {
@@ -411,14 +386,14 @@ static __global__ void __launch_bounds__(kScanBlock) lbib_compact_onepass(int* _
        j - k; the window is summed up to its nearest inclusive word once
        every word up to there has been published */
     volatile unsigned long long* vs = state;
-    const unsigned long long at = (unsigned)s_tt, ap = (unsigned)s_tp;
-    if (vb > 0 && lane == 0) vs[vb] = lookback_word(tag, 1u, at, ap);
+    const unsigned long long at = (unsigned)s_tt;
+    if (vb > 0 && lane == 0) vs[vb] = lookback_word(tag, 1u, at);
     __syncwarp();
-    unsigned long long et = 0, ep = 0;
+    unsigned long long et = 0;
     long spins = 0;
     for (int j = vb - 1; j >= 0;) {
       const int jj = j - lane;
-      const unsigned long long w = jj >= 0 ? vs[jj] : lookback_word(tag, 2u, 0ull, 0ull);
+      const unsigned long long w = jj >= 0 ? vs[jj] : lookback_word(tag, 2u, 0ull);
       const unsigned f = (unsigned)(w >> 54) & 3u;
       const bool ready = (unsigned)(w >> 56) == tag && f != 0u;
       const unsigned incl = __ballot_sync(0xffffffffu, ready && f == 2u);
@@ -432,19 +407,13 @@ static __global__ void __launch_bounds__(kScanBlock) lbib_compact_onepass(int* _
         }
         continue;
       }
-      unsigned long long t = lane <= lim ? (w >> 32) & 0x3FFFFFull : 0ull;
-      unsigned long long q = lane <= lim ? w & 0xFFFFFFFFull : 0ull;
-      for (int o = 16; o > 0; o >>= 1) {
-        t += __shfl_xor_sync(0xffffffffu, t, o);
-        q += __shfl_xor_sync(0xffffffffu, q, o);
-      }
-      et += t; ep += q;
+      et += __reduce_add_sync(0xffffffffu, lane <= lim ? (unsigned)w : 0u);
       if (incl) break;
       j -= 32;
     }
     if (lane == 0) {
-      vs[vb] = lookback_word(tag, 2u, et + at, ep + ap);
-      s_pt = (int)et; s_pp = (int)ep;
+      vs[vb] = lookback_word(tag, 2u, et + at);
+      s_pt = (int)et;
       if (vb == nblk - 1) {
         *total = (int)(et + at);
         *ticket = 0u;   /* every block has taken its ticket */
@@ -452,62 +421,19 @@ static __global__ void __launch_bounds__(kScanBlock) lbib_compact_onepass(int* _
     }
   }
   __syncthreads();
-  int pos = s_pt + sv[warp] + iv - tv, off = s_pp + sw[warp] + iw - tw;
+  int pos = s_pt + sv[warp] + iv - tv;
 #pragma unroll
   for (int k = 0; k < kOnepassTiles; ++k) {
     const long i = i0 + k;
     if (c[k] > 0) {
       list[pos] = (int)i;
-      slot[i] = pos;
-      slot_off[pos] = off;
-      slot_len[pos] = c[k];
-      slot_cursor[pos] = 0;
-      cnt[i] = 0;     /* counts start the next step at zero */
-      ++pos;
-      off += c[k];
+      slot[i] = pos++;
+      mark[i] = 0;      /* the next step starts unmarked */
     } else if (i < n) {
       slot[i] = -1;   /* the whole map is written: no clearing pass before the step */
     }
   }
 }
-
-/* The one-grid spread's lists hold entries instead of node indices: the
- * nodes of a warp (32 consecutive nodes, chunk i >> 5) that touch a tile
- * at the same stencil offset append one entry {chunk, lane mask} with one
- * atomic.  A node touches a tile at one offset only, so the masks a chunk
- * leaves in one list are disjoint; the gather merges them.  Only the
- * tiles of columns tx in [tlo, thi) are listed (an x-slab gathers the
- * force of its own columns only; the whole grid passes [0, ntx)).  The
- * eight tile offsets are walked by every lane, inactive ones included, so
- * that the warp's lanes meet at each step.  An entry's place in its list
- * depends on timing; the gather sorts the entries. */
-__device__ __forceinline__ void pair_scatter_warp(const int* __restrict__ st, long i, long S, int ntx, int nty,
-                                                  int nx, int ny, int nz, int tlo, int thi, const int* __restrict__ slot,
-                                                  const int* __restrict__ slot_off, int* __restrict__ slot_cursor,
-                                                  int2* __restrict__ ent) {
-  const int lane = threadIdx.x & 31;
-  int is = 0, js = 0, ks = 0;
-  bool ok = i < S;
-  if (ok) {
-    is = st[i * 3 + 0]; js = st[i * 3 + 1]; ks = st[i * 3 + 2];
-    ok = !(is < 0 || is + 3 >= nx || js < 0 || js + 3 >= ny || ks < 0 || ks + 3 >= nz);
-  }
-#pragma unroll
-  for (int o = 0; o < 8; ++o) {
-    const int tx = (is >> 2) + (o & 1), ty = (js >> 2) + ((o >> 1) & 1), tz = (ks >> 2) + (o >> 2);
-    const bool here = ok && tx <= (is + 3) >> 2 && ty <= (js + 3) >> 2 && tz <= (ks + 3) >> 2 && tx >= tlo &&
-                      tx < thi;
-    const int s = here ? slot[((long)tz * nty + ty) * ntx + tx] : -1;
-    const unsigned grp = __match_any_sync(0xffffffffu, s);
-    if (!here || lane != __ffs(grp) - 1) continue;
-    const int k = atomicAdd(&slot_cursor[s], 1);
-    ent[slot_off[s] + k] = make_int2((int)(i >> 5), (int)grp);
-  }
-}
-
-/* Longest per-tile node list sorted in shared memory; longer lists take the
- * chunk-scan path below. */
-constexpr int kListCap = 1024;
 
 /* The columns [d, d + 3] of a stencil that starts d cells from a tile's
  * origin, as a 4-bit mask of the tile's columns 0..3 (0 when |d| > 3). */
@@ -529,206 +455,306 @@ __device__ __forceinline__ unsigned long long stencil_tile_mask(int dx, int dy, 
   return m;
 }
 
-/* A staged node of the entry-list gather: its x, y and z delta weights at
- * the tile's four cell positions per axis (0 where the stencil misses the
- * position), then its force.  An odd stride of 15 doubles puts 16
- * different nodes in 16 different bank pairs. */
+/* A gather CTA: warps 0 and 1 hold the tile's 64 cells, warps 2 and 3 bring
+ * the nodes. */
+constexpr int kGatherTPB = 128;
+constexpr int kGatherWarps = kGatherTPB / 32;
+constexpr int kHitCap = 256;     /* chunks whose box meets the tile  */
+constexpr int kOffHits = 64;     /* of those, with the starts kept   */
+constexpr int kListCap = 1024;   /* nodes whose stencil meets it     */
+constexpr int kBatch = 64;       /* nodes staged at once             */
+
+/* A staged node: its x, y and z delta weights at the tile's four cell
+ * positions per axis (unset where the stencil misses the position: no cell
+ * it covers reads them), then its force.  An odd stride of 15 doubles puts 16 different nodes in 16
+ * different bank pairs. */
 constexpr int kNodeRec = 15;
 
-/* Shared memory of one entry-list gather CTA (64 threads = one 4^3 tile):
- * the list's entries as sort keys (chunk << 32 | lane mask) while the node
- * list is built, then the staged node records while they are summed. */
-struct GatherSmemE {
-  int ids[kListCap];                 /* the tile's nodes in index order       */
-  int seg[kListCap];                 /* per entry: first node position, or -1 */
-  unsigned m32[2][64];               /* per node: the cells of warp 0 / 1     */
-  union {
-    unsigned long long key[kListCap];
-    double rec[64 * kNodeRec];
-  } u;
+struct GatherSmem {
+  int hit[kHitCap];                     /* chunks in index order               */
+  unsigned mask[kHitCap];               /* the nodes of each that touch        */
+  unsigned short hoff[kOffHits][32];    /* their stencil starts, the first chunks' */
+  int pos[kHitCap];                     /* their places in ids                 */
+  int ids[kListCap];                    /* the tile's nodes in index order     */
+  int off[kListCap];                    /* their stencil starts from the tile's origin */
+  unsigned cover[2][2][kBatch];         /* per staged node: cells of warp 0, 1 */
+  double rec[2][kBatch * kNodeRec];
+  int warp_n[kGatherWarps];
+  int n;
 };
 
-/* Slot `it` (local tile `tile`) from its E entries {chunk, lane mask}: the
- * entries are sorted by chunk (bitonic, in shared memory), the masks of a
- * chunk merged, and the node list written in index order; then each of
- * the 64 threads sums its cell's contributions in node order -- the
- * reference's (sheet, row, col) order -- into Ftile[it].  The same values
- * as gather_tile. */
-__device__ __forceinline__ void gather_tile_ent(GatherSmemE& sm, const double* __restrict__ nodes,
-                                                const double* __restrict__ W, const int* __restrict__ st, int it,
-                                                int tile, int L, int E, const int2* __restrict__ ent,
-                                                int ntx, int nty, double* __restrict__ Ftile) {
-  const int t = threadIdx.x;
-  const double cf = 1.0 / (64.0 * 1.0 * 1.0 * 1.0);
-  unsigned long long* key = sm.u.key;
-  int P = 1;
-  while (P < E) P <<= 1;
-  __syncthreads();   /* the previous tile's data is no longer read */
-  for (int k = t; k < P; k += 64) {
-    unsigned long long v = ~0ull;
-    if (k < E) {
-      const int2 e = ent[k];
-      v = ((unsigned long long)(unsigned)e.x << 32) | (unsigned)e.y;
-    }
-    key[k] = v;
-  }
-  __syncthreads();
-  for (int k = 2; k <= P; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int a = t; a < P; a += 64) {
-        const int b = a ^ j;
-        if (b > a) {
-          const unsigned long long va = key[a], vb = key[b];
-          const bool up = (a & k) == 0;
-          if ((va > vb) == up) { key[a] = vb; key[b] = va; }
-        }
-      }
-      __syncthreads();
-    }
-  /* entries of one chunk are now adjacent: the first of each run takes the
-     run's merged mask and its first position (a short serial pass) */
-  if (t == 0) {
-    int pos = 0;
-    for (int e = 0; e < E;) {
-      const unsigned ch = (unsigned)(key[e] >> 32);
-      unsigned m = (unsigned)key[e];
-      int f = e + 1;
-      while (f < E && (unsigned)(key[f] >> 32) == ch) { m |= (unsigned)key[f]; sm.seg[f] = -1; ++f; }
-      key[e] = ((unsigned long long)ch << 32) | m;
-      sm.seg[e] = pos;
-      pos += __popc(m);
-      e = f;
-    }
-  }
-  __syncthreads();
-  for (int e = t; e < E; e += 64) {
-    int pos = sm.seg[e];
-    if (pos < 0) continue;
-    const int base = (int)(key[e] >> 32) * 32;
-    for (unsigned m = (unsigned)key[e]; m; m &= m - 1) sm.ids[pos++] = base + __ffs(m) - 1;
-  }
-  __syncthreads();   /* ids complete; key no longer read (aliases the node records) */
-  double* rec = sm.u.rec;
-  const int tx = tile % ntx, ty = (tile / ntx) % nty, tz = tile / (ntx * nty);
-  const int x0 = tx * 4, y0 = ty * 4, z0 = tz * 4;
-  /* the thread's cell in a record: its x, y and z weight positions */
-  const int ox = t & 3, oy = 4 + ((t >> 2) & 3), oz = 8 + (t >> 4);
-  const int lane = t & 31;
-  const unsigned* mw = sm.m32[t >> 5];
-  double Fx = 0.0, Fy = 0.0, Fz = 0.0;
-  for (int b0 = 0; b0 < L; b0 += 64) {
-    const int nb = min(64, L - b0);
-    if (t < nb) {
-      const long nd = sm.ids[b0 + t];
-      const int sx = st[nd * 3 + 0], sy = st[nd * 3 + 1], sz = st[nd * 3 + 2];
-      double* r = rec + t * kNodeRec;
-      const double* w = W + nd * 12;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        /* cell position c of the tile is stencil position c + (x0 - sx) */
-        const int a = c + x0 - sx, b = c + y0 - sy, e = c + z0 - sz;
-        r[c] = (unsigned)a < 4u ? w[a] : 0.0;
-        r[4 + c] = (unsigned)b < 4u ? w[4 + b] : 0.0;
-        r[8 + c] = (unsigned)e < 4u ? w[8 + e] : 0.0;
-      }
-      r[12] = nodes[nd * 12 + 9]; r[13] = nodes[nd * 12 + 10]; r[14] = nodes[nd * 12 + 11];
-      const unsigned long long m = stencil_tile_mask(sx - x0, sy - y0, sz - z0);
-      sm.m32[0][t] = (unsigned)m;
-      sm.m32[1][t] = (unsigned)(m >> 32);
-    }
-    __syncthreads();
-    /* 32 nodes at a time: the warp's 32 x 32 cover bits (node j covers
-       lane l's cell) are transposed with five shuffle stages, so that
-       each lane walks only the nodes that cover its cell, in node order */
-    for (int j0 = 0; j0 < nb; j0 += 32) {
-      unsigned x = j0 + lane < nb ? mw[j0 + lane] : 0u;
-#pragma unroll
-      for (int k = 16; k >= 1; k >>= 1) {
-        const unsigned M = k == 16 ? 0x0000FFFFu : k == 8 ? 0x00FF00FFu : k == 4 ? 0x0F0F0F0Fu
-                         : k == 2 ? 0x33333333u : 0x55555555u;
-        const unsigned y = __shfl_xor_sync(0xffffffffu, x, k);
-        x = (lane & k) ? (x & ~M) | ((y & ~M) >> k) : (x & M) | ((y & M) << k);
-      }
-      for (unsigned bits = x; bits; bits &= bits - 1u) {
-        const double* r = rec + (j0 + __ffs(bits) - 1) * kNodeRec;
-        const double tmp = cf * r[ox] * r[oy] * r[oz];
-        Fx = Fx + r[12] * tmp;
-        Fy = Fy + r[13] * tmp;
-        Fz = Fz + r[14] * tmp;
-      }
-    }
-    __syncthreads();
-  }
-  double* Ft = Ftile + (long)it * 192;
-  Ft[t] = Fx; Ft[64 + t] = Fy; Ft[128 + t] = Fz;
+__device__ __forceinline__ bool box_meets(const int* __restrict__ b, int x0, int y0, int z0) {
+  const int2 x = *reinterpret_cast<const int2*>(b), y = *reinterpret_cast<const int2*>(b + 2),
+             z = *reinterpret_cast<const int2*>(b + 4);
+  return !(x.y < x0 || x.x > x0 + 3 || y.y < y0 || y.x > y0 + 3 || z.y < z0 || z.x > z0 + 3);
 }
 
-/* Crowded tiles (more than kListCap nodes, e.g. a crumpled sheet): visit the
- * nodes chunk by chunk in global order, skipping chunks whose stencil box
- * misses the tile.  Same summation order, no list needed. */
+/* Where the sheet's nodes are found: stencil starts and weights, the boxes
+ * of chunks [c_lo, c_hi) and (NULL: few chunks) of the super-chunks; nodes
+ * end at S. */
+struct GatherNodes {
+  const double* nodes;
+  const double* W;
+  const int* st;
+  const int* chunk_box;
+  const int* super;
+  long S, c_lo, c_hi;
+};
+
+/* What the gather of grid d's current step reads. */
+inline GatherNodes gather_nodes(const lbib_device* d) {
+  return GatherNodes{d->nodes, d->W, d->st, d->chunk_box, d->super[d->cur], d->S, 0, d->nchunks};
+}
+
+/* The next step's super-chunk boxes start empty (its node preparation
+ * merges into them); by the whole grid, in a launch after the last reader. */
+__device__ __forceinline__ void clear_super(int* __restrict__ super, long n) {
+  if (!super) return;
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < 6 * n; i += (long)gridDim.x * blockDim.x)
+    super[i] = (i % 6) & 1 ? INT_MIN : INT_MAX;
+}
+
+/* The CTA's threads with `flag` set append `value` in thread order to
+ * out[*n ..) (up to cap); *n grows by their number.  Ends with a barrier. */
+__device__ __forceinline__ void append_in_order(GatherSmem& sm, bool flag, int value, int* out, int cap, int& n) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned m = __ballot_sync(0xffffffffu, flag);
+  if (lane == 0) sm.warp_n[warp] = __popc(m);
+  __syncthreads();
+  int at = n;
+#pragma unroll
+  for (int w = 0; w < kGatherWarps; ++w) {
+    if (w == warp && flag) {
+      const int k = at + __popc(m & ((1u << lane) - 1u));
+      if (k < cap) out[k] = value;
+    }
+    at += sm.warp_n[w];
+  }
+  n = at;
+  __syncthreads();
+}
+
+/* The nodes that touch the tile at (x0, y0, z0), in index order, into
+ * sm.ids; returns their number, or -1 when a list overflows (a crumpled
+ * sheet).  Boxes of 1024 nodes first (sheets of more than 128 chunks),
+ * then of 32, then the nodes themselves: every level is a handful of
+ * coalesced loads per CTA, nothing is sorted, and no list has to be built
+ * beforehand. */
+__device__ __forceinline__ int gather_list(GatherSmem& sm, const GatherNodes& g, int x0, int y0, int z0) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  int nh = 0;
+  if (!g.super || g.c_hi - g.c_lo <= kGatherTPB) {
+    for (long c0 = g.c_lo; c0 < g.c_hi; c0 += kGatherTPB) {
+      const long c = c0 + t;
+      append_in_order(sm, c < g.c_hi && box_meets(g.chunk_box + c * 6, x0, y0, z0), (int)c, sm.hit, kHitCap, nh);
+    }
+  } else {
+    int ns = 0;
+    const long s1 = (g.c_hi + kSuper - 1) / kSuper;
+    for (long s0 = g.c_lo / kSuper; s0 < s1; s0 += kGatherTPB) {
+      const long s = s0 + t;
+      append_in_order(sm, s < s1 && box_meets(g.super + s * 6, x0, y0, z0), (int)s, sm.pos, kHitCap, ns);
+    }
+    if (ns > kHitCap) return -1;
+    for (int k = 0; k < ns; k += kGatherWarps) {
+      const long c = k + warp < ns ? (long)sm.pos[k + warp] * kSuper + lane : -1;
+      append_in_order(sm, c >= g.c_lo && c < g.c_hi && box_meets(g.chunk_box + c * 6, x0, y0, z0), (int)c, sm.hit,
+                      kHitCap, nh);
+    }
+  }
+  if (nh > kHitCap) return -1;
+  for (int h = warp; h < nh; h += kGatherWarps) {
+    const long i = (long)sm.hit[h] * 32 + lane;
+    unsigned dx = 8u, dy = 8u, dz = 8u;   /* start - origin + 3: 0..6 where they meet */
+    if (i < g.S) {
+      const int* s = g.st + i * 3;
+      dx = (unsigned)(s[0] - x0 + 3); dy = (unsigned)(s[1] - y0 + 3); dz = (unsigned)(s[2] - z0 + 3);
+    }
+    const bool in = dx < 7u && dy < 7u && dz < 7u;
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    if (lane == 0) sm.mask[h] = m;
+    if (h < kOffHits) sm.hoff[h][lane] = (unsigned short)(dx | dy << 4 | dz << 8);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int run = 0;
+    for (int h0 = 0; h0 < nh; h0 += 32) {
+      const int v = h0 + lane < nh ? __popc(sm.mask[h0 + lane]) : 0;
+      int iv = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, iv, o);
+        if (lane >= o) iv += u;
+      }
+      if (h0 + lane < nh) sm.pos[h0 + lane] = run + iv - v;
+      run += __shfl_sync(0xffffffffu, iv, 31);
+    }
+    if (lane == 0) sm.n = run;
+  }
+  __syncthreads();
+  const int L = sm.n;
+  if (L > kListCap) return -1;
+  for (int h = warp; h < nh; h += kGatherWarps) {
+    const unsigned m = sm.mask[h];
+    if ((m >> lane) & 1u) {
+      const int k = sm.pos[h] + __popc(m & ((1u << lane) - 1u)), i = sm.hit[h] * 32 + lane;
+      unsigned o;
+      if (h < kOffHits) {
+        o = sm.hoff[h][lane];
+      } else {
+        const int* s = g.st + (long)i * 3;
+        o = (unsigned)(s[0] - x0 + 3) | (unsigned)(s[1] - y0 + 3) << 4 | (unsigned)(s[2] - z0 + 3) << 8;
+      }
+      sm.ids[k] = i;
+      sm.off[k] = (int)o;
+    }
+  }
+  __syncthreads();
+  return L;
+}
+
+/* 8 bytes global -> shared, asynchronously. */
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+/* Bring nodes b0 .. b0 + kBatch - 1 of the list to buffer `buf`, a thread of
+ * warps 2 and 3 per node, asynchronously: a record goes to its place without
+ * passing through registers (the cell's own state needs them). */
+__device__ __forceinline__ void gather_stage(GatherSmem& sm, const GatherNodes& g, int L, int b0, int buf) {
+  const int k = (int)threadIdx.x - 64;
+  if (b0 + k >= L) return;
+  const long nd = sm.ids[b0 + k];
+  const int off = sm.off[b0 + k];
+  double* r = sm.rec[buf] + k * kNodeRec;
+  const double* w = g.W + nd * 12;
+  const int d[3] = {(off & 15) - 3, ((off >> 4) & 15) - 3, (off >> 8) - 3};
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int c = 0; c < 4; ++c)   /* cell position c of the tile is stencil position c - d */
+      if ((unsigned)(c - d[a]) < 4u) cp_async8(r + 4 * a + c, w + 4 * a + c - d[a]);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) cp_async8(r + 12 + a, g.nodes + nd * 12 + 9 + a);
+  const unsigned long long cov = stencil_tile_mask(d[0], d[1], d[2]);
+  sm.cover[buf][0][k] = (unsigned)cov;
+  sm.cover[buf][1][k] = (unsigned)(cov >> 32);
+}
+
+/* Too many nodes for the lists: visit the chunks in order, skipping those
+ * whose box misses the tile.  Same summation order. */
 struct ScanSmem {
-  int hit[64];
+  int hit[kGatherTPB];
   int st[32][3];
   double w[32][12];
   double fe[32][3];
 };
 
-/* Slot `it` with more than kListCap nodes: visit the node chunks
- * [c_lo, c_hi) (32 nodes each, nodes below S) in order, skipping chunks
- * whose stencil box misses the tile. */
-__device__ __forceinline__ void gather_tile_scan(ScanSmem& sm, const double* __restrict__ nodes,
-                                                 const double* __restrict__ W, const int* __restrict__ st,
-                                                 const int* __restrict__ chunk_box, long S, long c_lo, long c_hi,
-                                                 int it, int tile, int ntx, int nty, double* __restrict__ Ftile) {
-  int* hit = sm.hit;
-  auto& s_st = sm.st;
-  auto& s_w = sm.w;
-  auto& s_fe = sm.fe;
-  const int cell = threadIdx.x;
+__device__ __forceinline__ void gather_scan(ScanSmem& sm, const GatherNodes& g, int x0, int y0, int z0, double& Fx,
+                                            double& Fy, double& Fz) {
+  const int t = threadIdx.x;
   const double cf = 1.0 / (64.0 * 1.0 * 1.0 * 1.0);
-  {
-    const int tx = tile % ntx, ty = (tile / ntx) % nty, tz = tile / (ntx * nty);
-    const int x0 = tx * 4, y0 = ty * 4, z0 = tz * 4;
-    const int gx = x0 + (cell & 3), gy = y0 + ((cell >> 2) & 3), gz = z0 + (cell >> 4);
-    double Fx = 0.0, Fy = 0.0, Fz = 0.0;
-    for (long c0 = c_lo; c0 < c_hi; c0 += 64) {
-      const long c = c0 + cell;
-      int h = 0;
-      if (c < c_hi) {
-        const int* bx = chunk_box + c * 6;
-        h = !(bx[1] < x0 || bx[0] > x0 + 3 || bx[3] < y0 || bx[2] > y0 + 3 || bx[5] < z0 || bx[4] > z0 + 3);
+  const int gx = x0 + (t & 3), gy = y0 + ((t >> 2) & 3), gz = z0 + ((t & 63) >> 4);
+  for (long c0 = g.c_lo; c0 < g.c_hi; c0 += kGatherTPB) {
+    const long c = c0 + t;
+    __syncthreads();
+    sm.hit[t] = c < g.c_hi && box_meets(g.chunk_box + c * 6, x0, y0, z0);
+    __syncthreads();
+    for (int k = 0; k < kGatherTPB; ++k) {
+      if (!sm.hit[k]) continue;
+      if (t < 32) {
+        const long nd = (c0 + k) * 32 + t;
+        if (nd < g.S) {
+          for (int a = 0; a < 3; ++a) sm.st[t][a] = g.st[nd * 3 + a];
+          for (int a = 0; a < 12; ++a) sm.w[t][a] = g.W[nd * 12 + a];
+          for (int a = 0; a < 3; ++a) sm.fe[t][a] = g.nodes[nd * 12 + 9 + a];
+        } else {
+          sm.st[t][0] = sm.st[t][1] = sm.st[t][2] = INT_MIN / 2;
+        }
       }
       __syncthreads();
-      hit[cell] = h;
+      for (int j = 0; j < 32 && t < 64; ++j) {
+        const int a = gx - sm.st[j][0], b = gy - sm.st[j][1], e = gz - sm.st[j][2];
+        if ((unsigned)a < 4u && (unsigned)b < 4u && (unsigned)e < 4u) {
+          const double tmp = __dmul_rn(__dmul_rn(__dmul_rn(cf, sm.w[j][a]), sm.w[j][4 + b]), sm.w[j][8 + e]);
+          Fx = __dadd_rn(Fx, __dmul_rn(sm.fe[j][0], tmp));
+          Fy = __dadd_rn(Fy, __dmul_rn(sm.fe[j][1], tmp));
+          Fz = __dadd_rn(Fz, __dmul_rn(sm.fe[j][2], tmp));
+        }
+      }
       __syncthreads();
-      for (int k = 0; k < 64; ++k) {
-        if (!hit[k]) continue;
-        const long base = (c0 + k) * 32;
-        if (cell < 32) {
-          const long nd = base + cell;
-          if (nd < S) {
-            s_st[cell][0] = st[nd * 3 + 0]; s_st[cell][1] = st[nd * 3 + 1]; s_st[cell][2] = st[nd * 3 + 2];
-            for (int a = 0; a < 12; ++a) s_w[cell][a] = W[nd * 12 + a];
-            s_fe[cell][0] = nodes[nd * 12 + 9]; s_fe[cell][1] = nodes[nd * 12 + 10]; s_fe[cell][2] = nodes[nd * 12 + 11];
-          } else {
-            s_st[cell][0] = INT_MIN / 2; s_st[cell][1] = INT_MIN / 2; s_st[cell][2] = INT_MIN / 2;
+    }
+  }
+}
+
+union GatherShared {
+  GatherSmem g;
+  ScanSmem s;
+};
+
+/* The spread force of the tile at (x0, y0, z0): thread t < 64 gets its
+ * cell's sum over the nodes in index order (cell = 16 z + 4 y + x).  Called
+ * by all kGatherTPB threads.  Warps 2 and 3 stage the next 64 nodes while
+ * warps 0 and 1 sum the last: each sum is a serial chain (its order is the
+ * reference's), so latency is kept out of it. */
+__device__ __forceinline__ void gather_tile(GatherShared& sh, const GatherNodes& g, int x0, int y0, int z0,
+                                            double& Fx, double& Fy, double& Fz) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const double cf = 1.0 / (64.0 * 1.0 * 1.0 * 1.0);
+  Fx = Fy = Fz = 0.0;
+  __syncthreads();   /* the previous tile's data is no longer read */
+  GatherSmem& sm = sh.g;
+  const int L = gather_list(sm, g, x0, y0, z0);
+  if (L < 0) {
+    gather_scan(sh.s, g, x0, y0, z0, Fx, Fy, Fz);
+    return;
+  }
+  /* the thread's cell in a record: its x, y and z weight positions */
+  const int ox = t & 3, oy = 4 + ((t >> 2) & 3), oz = 8 + ((t & 63) >> 4);
+  if (warp >= 2) {
+    gather_stage(sm, g, L, 0, 0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  __syncthreads();
+  for (int b0 = 0, buf = 0; b0 < L; b0 += kBatch, buf ^= 1) {
+    if (warp >= 2) {
+      gather_stage(sm, g, L, b0 + kBatch, buf ^ 1);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+#pragma unroll 1
+      for (int j0 = 0; j0 < kBatch && b0 + j0 < L; j0 += 32) {
+        /* the warp's 32 x 32 cover bits (node j covers lane l's cell) are
+           transposed with five shuffle stages, so that each lane walks only
+           the nodes that cover its cell, in node order, two at a time */
+        unsigned x = b0 + j0 + lane < L ? sm.cover[buf][warp][j0 + lane] : 0u;
+#pragma unroll
+        for (int k = 16; k >= 1; k >>= 1) {
+          const unsigned M = k == 16 ? 0x0000FFFFu : k == 8 ? 0x00FF00FFu : k == 4 ? 0x0F0F0F0Fu
+                           : k == 2 ? 0x33333333u : 0x55555555u;
+          const unsigned y = __shfl_xor_sync(0xffffffffu, x, k);
+          x = (lane & k) ? (x & ~M) | ((y & ~M) >> k) : (x & M) | ((y & M) << k);
+        }
+        const double* rec = sm.rec[buf] + j0 * kNodeRec;
+        for (unsigned bits = x; bits;) {
+          const double* r = rec + (__ffs(bits) - 1) * kNodeRec;
+          bits &= bits - 1u;
+          const bool two = bits != 0u;
+          const double* q = two ? rec + (__ffs(bits) - 1) * kNodeRec : r;
+          bits &= bits - 1u;   /* 0 stays 0 */
+          const double tr = __dmul_rn(__dmul_rn(__dmul_rn(cf, r[ox]), r[oy]), r[oz]);
+          const double tq = __dmul_rn(__dmul_rn(__dmul_rn(cf, q[ox]), q[oy]), q[oz]);
+          Fx = __dadd_rn(Fx, __dmul_rn(r[12], tr));
+          Fy = __dadd_rn(Fy, __dmul_rn(r[13], tr));
+          Fz = __dadd_rn(Fz, __dmul_rn(r[14], tr));
+          if (two) {
+            Fx = __dadd_rn(Fx, __dmul_rn(q[12], tq));
+            Fy = __dadd_rn(Fy, __dmul_rn(q[13], tq));
+            Fz = __dadd_rn(Fz, __dmul_rn(q[14], tq));
           }
         }
-        __syncthreads();
-        for (int j = 0; j < 32; ++j) {
-          const int a = gx - s_st[j][0], b = gy - s_st[j][1], e = gz - s_st[j][2];
-          if ((unsigned)a < 4u && (unsigned)b < 4u && (unsigned)e < 4u) {
-            const double tmp = cf * s_w[j][a] * s_w[j][4 + b] * s_w[j][8 + e];
-            Fx = Fx + s_fe[j][0] * tmp;
-            Fy = Fy + s_fe[j][1] * tmp;
-            Fz = Fz + s_fe[j][2] * tmp;
-          }
-        }
-        __syncthreads();
       }
     }
-    double* Ft = Ftile + (long)it * 192;
-    Ft[cell] = Fx; Ft[64 + cell] = Fy; Ft[128 + cell] = Fz;
+    __syncthreads();
   }
 }
 
@@ -776,104 +802,105 @@ __device__ __forceinline__ void move_node(double* __restrict__ nodes, const doub
 }
 
 
-/* Cells a warp's staged move holds in shared memory: the union box of its
- * 32 nodes' stencils (along a fiber row ~5 x 20 x 5 cells); a larger
- * union (a warp straddling two rows, a crumpled sheet) takes move_node. */
+/* A move CTA: the 32 nodes of a chunk, four warps. */
+constexpr int kMoveTPB = 128;
+/* Cells a CTA's staged move holds in shared memory: the union box of its 32
+ * nodes' stencils (along a fiber row ~5 x 20 x 5 cells); a larger union (a
+ * chunk straddling two rows, a crumpled sheet) takes move_node. */
 constexpr int kMoveCap = 640;
 constexpr int kMoveTiles = 64;   /* tiles of the union box whose slots are staged */
 
-__device__ __forceinline__ int warp_min(int v) {
-  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-__device__ __forceinline__ int warp_max(int v) {
-  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
+struct MoveSmem {
+  double U[3][kMoveCap];
+  int slot[kMoveTiles];
+};
 
-/* move_node for the 32 nodes of a warp (node i on this lane, `live` if it
- * moves), with the velocity of the union box of their stencils staged once
- * in shared memory (sU: 3 x kMoveCap doubles for this warp): the lanes
- * read each box cell's u from its moment tile with coalesced loads, then
- * every lane sums its own 64 terms from shared memory -- the same values
- * in the same order as move_node, with ~5x fewer L2 requests (neighbouring
- * nodes' stencils overlap by 3 cells of 4).  Called by all 32 lanes. */
-__device__ __forceinline__ void move_warp(double* __restrict__ nodes, const double* __restrict__ W,
-                                          const int* __restrict__ st, long i, bool live, int ntx, int nty,
-                                          const int* __restrict__ slot, const double* __restrict__ Utile, double dt,
-                                          double* __restrict__ sU) {
-  const int lane = threadIdx.x & 31;
+/* The move of the 32 nodes of a chunk (node i on lane l of every warp,
+ * `live` if it moves), with the velocity of the union box of their stencils
+ * staged once in shared memory: the four warps read each box cell's u from
+ * its moment tile, then warp a < 3 sums component a of every node's 64
+ * terms from shared memory -- the same values in the same order as
+ * move_node, with ~5x fewer L2 requests (neighbouring nodes' stencils
+ * overlap by 3 cells of 4).  A node's sum is a serial chain of 64 terms, so
+ * a thread holds one component only; with one warp that staged and summed
+ * all three for its nodes the launch took 10 us at 16 x 16 nodes, this 6.
+ * Called by all kMoveTPB threads; ends with a barrier. */
+__device__ __forceinline__ void move_chunk(MoveSmem& sm, double* __restrict__ nodes, const double* __restrict__ W,
+                                           const int* __restrict__ st, long i, bool live, int ntx, int nty,
+                                           const int* __restrict__ slot, const double* __restrict__ Utile, double dt) {
+  const int t = threadIdx.x, warp = t >> 5;
   int is = 0, js = 0, ks = 0;
   if (live) { is = st[i * 3 + 0]; js = st[i * 3 + 1]; ks = st[i * 3 + 2]; }
-  const int x0 = warp_min(live ? is : INT_MAX), x1 = warp_max(live ? is + 3 : INT_MIN);
-  if (x0 > x1) return;   /* no live lane */
-  const int y0 = warp_min(live ? js : INT_MAX), y1 = warp_max(live ? js + 3 : INT_MIN);
-  const int z0 = warp_min(live ? ks : INT_MAX), z1 = warp_max(live ? ks + 3 : INT_MIN);
+  const int x0 = __reduce_min_sync(0xffffffffu, live ? is : INT_MAX), x1 = __reduce_max_sync(0xffffffffu, live ? is + 3 : INT_MIN);
+  const int y0 = __reduce_min_sync(0xffffffffu, live ? js : INT_MAX), y1 = __reduce_max_sync(0xffffffffu, live ? js + 3 : INT_MIN);
+  const int z0 = __reduce_min_sync(0xffffffffu, live ? ks : INT_MAX), z1 = __reduce_max_sync(0xffffffffu, live ? ks + 3 : INT_MIN);
+  if (x0 > x1) {   /* no live node: uniform over the CTA */
+    __syncthreads();
+    return;
+  }
   const int bx = x1 - x0 + 1, by = y1 - y0 + 1, bz = z1 - z0 + 1;
   const long vol = (long)bx * by * bz;
-  const int ntiles_box = ((x1 >> 2) - (x0 >> 2) + 1) * ((y1 >> 2) - (y0 >> 2) + 1) * ((z1 >> 2) - (z0 >> 2) + 1);
-  if (vol > kMoveCap || ntiles_box > kMoveTiles) {   /* uniform over the warp */
-    if (live) move_node(nodes, W, st, i, ntx, nty, slot, Utile, dt);
+  const int tx0 = x0 >> 2, ty0 = y0 >> 2, tz0 = z0 >> 2;
+  const int tbx = (x1 >> 2) - tx0 + 1, tby = (y1 >> 2) - ty0 + 1;
+  const long ntb = (long)tbx * tby * ((z1 >> 2) - tz0 + 1);
+  if (vol > kMoveCap || ntb > kMoveTiles) {   /* uniform over the CTA */
+    if (live && warp == 0) move_node(nodes, W, st, i, ntx, nty, slot, Utile, dt);
+    __syncthreads();
     return;
+  }
+  /* the weights this thread will need, on their way while the box is staged */
+  double w[12];
+  double at = 0.0;
+  if (live && warp < 3) {
+    const double2* p = reinterpret_cast<const double2*>(W + i * 12);
+#pragma unroll
+    for (int a = 0; a < 6; ++a) { w[2 * a] = p[a].x; w[2 * a + 1] = p[a].y; }
+    at = nodes[i * 12 + warp];
   }
   /* the slots of the box's tiles first (at most 3 x 7 x 3 for a box that
      fits), so that the cell loads below depend on one shared-memory read */
-  int* sslot = reinterpret_cast<int*>(sU + 3 * kMoveCap);
-  const int tx0 = x0 >> 2, ty0 = y0 >> 2, tz0 = z0 >> 2;
-  const int tbx = (x1 >> 2) - tx0 + 1, tby = (y1 >> 2) - ty0 + 1, ntb = tbx * tby * ((z1 >> 2) - tz0 + 1);
-  for (int j = lane; j < ntb; j += 32) {
-    const int tx = tx0 + j % tbx, ty = ty0 + (j / tbx) % tby, tz = tz0 + j / (tbx * tby);
-    sslot[j] = slot[(tz * nty + ty) * ntx + tx];
+  if (t < (int)ntb) {
+    const int tx = tx0 + t % tbx, ty = ty0 + (t / tbx) % tby, tz = tz0 + t / (tbx * tby);
+    sm.slot[t] = slot[(tz * nty + ty) * ntx + tx];
   }
-  __syncwarp();
+  __syncthreads();
   /* the box's longest axis (the fiber direction: neighbouring lanes'
      stencils are offset along it) is stored fastest, so that the lanes'
      reads below fall on consecutive words, not on one bank */
   const int f = (bx >= by && bx >= bz) ? 0 : (by >= bz ? 1 : 2);
-  const int a = f == 0 ? 1 : 0, b = f == 2 ? 1 : 2;
-  const int ext[3] = {bx, by, bz};
-  int str[3];
-  str[f] = 1; str[a] = ext[f]; str[b] = ext[f] * ext[a];
-#pragma unroll 4
-  for (int j = lane; j < (int)vol; j += 32) {
-    int u[3];
-    u[f] = j % ext[f]; u[a] = (j / ext[f]) % ext[a]; u[b] = j / (ext[f] * ext[a]);
-    const int cx = x0 + u[0], cy = y0 + u[1], cz = z0 + u[2];
+  const int ef = f == 0 ? bx : f == 1 ? by : bz, ea = f == 0 ? by : bx;
+  const int sx = f == 0 ? 1 : ef, sy = f == 1 ? 1 : f == 0 ? ef : ef * ea, sz = f == 2 ? 1 : ef * ea;
+  /* j / ef and j / ea by reciprocals: exact for j < 640, divisors < 100 */
+  const unsigned rf = (65535u + ef) / ef, ra = (65535u + ea) / ea;
+#pragma unroll 5
+  for (int j = t; j < (int)vol; j += kMoveTPB) {   /* 640 / 128: the loads of all rounds in flight */
+    const int q = ef < 100 ? (int)(j * rf >> 16) : j / ef, uf = j - q * ef;
+    const int ub = ea < 100 ? (int)(q * ra >> 16) : q / ea, ua = q - ub * ea;
+    const int cx = x0 + (f == 0 ? uf : ua), cy = y0 + (f == 1 ? uf : f == 0 ? ua : ub), cz = z0 + (f == 2 ? uf : ub);
     /* a box corner no stencil covers may lie in an untouched tile: never read */
-    const int sp = sslot[((cz >> 2) - tz0) * tbx * tby + ((cy >> 2) - ty0) * tbx + ((cx >> 2) - tx0)];
+    const int sp = sm.slot[((cz >> 2) - tz0) * tbx * tby + ((cy >> 2) - ty0) * tbx + ((cx >> 2) - tx0)];
     double vx = 0.0, vy = 0.0, vz = 0.0;
     if (sp >= 0) {
-      const double* U = Utile + (long)sp * 256;
-      const int cell = lbib::cell_in_tile(cx, cy, cz);
-      vx = U[64 + cell]; vy = U[128 + cell]; vz = U[192 + cell];
+      const double* U = Utile + (long)sp * 256 + lbib::cell_in_tile(cx, cy, cz);
+      vx = U[64]; vy = U[128]; vz = U[192];
     }
-    sU[j] = vx; sU[kMoveCap + j] = vy; sU[2 * kMoveCap + j] = vz;
+    sm.U[0][j] = vx; sm.U[1][j] = vy; sm.U[2][j] = vz;
   }
-  __syncwarp();
-  if (live) {
+  __syncthreads();
+  if (live && warp < 3) {
     const double c_64 = 1.0 / (6.4e1);
-    const double* w = W + i * 12;
-    double s1 = 0, s2 = 0, s3 = 0;
+    const double* u = sm.U[warp] + (is - x0) * sx + (js - y0) * sy + (ks - z0) * sz;
+    double s = 0;
 #pragma unroll
-    for (int i2 = 0; i2 <= 3; i2++) {
+    for (int i2 = 0; i2 <= 3; i2++)
 #pragma unroll
-      for (int j2 = 0; j2 <= 3; j2++) {
+      for (int j2 = 0; j2 <= 3; j2++)
 #pragma unroll
-        for (int k2 = 0; k2 <= 3; k2++) {
-          const int c = (is + i2 - x0) * str[0] + (js + j2 - y0) * str[1] + (ks + k2 - z0) * str[2];
-          const double vx = sU[c], vy = sU[kMoveCap + c], vz = sU[2 * kMoveCap + c];
-          s1 += vx * w[i2] * w[4 + j2] * w[8 + k2] * c_64;
-          s2 += vy * w[i2] * w[4 + j2] * w[8 + k2] * c_64;
-          s3 += vz * w[i2] * w[4 + j2] * w[8 + k2] * c_64;
-        }
-      }
-    }
-    double* m = nodes + i * 12;
-    m[0] += dt * s1;
-    m[1] += dt * s2;
-    m[2] += dt * s3;
+        for (int k2 = 0; k2 <= 3; k2++)
+          s += u[i2 * sx + j2 * sy + k2 * sz] * w[i2] * w[4 + j2] * w[8 + k2] * c_64;
+    nodes[i * 12 + warp] = at + dt * s;
   }
-  __syncwarp();
+  __syncthreads();
 }
 
 }  // namespace lbib

@@ -32,6 +32,7 @@ extern "C" {
 #define LBIB_TILE 4
 #define LBIB_TILE_CELLS 64
 #define LBIB_CHUNK 32
+#define LBIB_SUPER_MIN 128       /* more node chunks than this: super-chunk boxes too */
 
 #ifndef LBIB_PREC_F64
 #define LBIB_PREC_F64 0   /* population storage precisions, as in include/lbib.h */
@@ -101,15 +102,11 @@ typedef struct lbib_device {
   int ntx, nty, ntz;
   long ntiles;
   long cap;                      /* slots per buffer                          */
-  int* tile_cnt;                 /* [ntiles] nodes whose stencil touches it   */
-  int* slot_off;                 /* [cap] start of the slot's node list       */
-  int* slot_len;                 /* [cap] length of the slot's node list      */
-  int* slot_cursor;              /* [cap] fill cursor                         */
-  int* pair_node;                /* [8 S] int2 entry lists of the touched tiles */
+  int* tile_mark;                /* [ntiles] x-slabs: touched this step       */
   int* tile_slot[2];             /* [ntiles] slot or -1                       */
-  int* tile_list[2];             /* [cap] touched tiles in index order        */
+  int* tile_list[2];             /* [cap] touched tiles, slot by slot         */
   int* tile_count[2];            /* [1]                                       */
-  int* scan_tmp;                 /* block sums for the compaction             */
+  int* scan_tmp;                 /* x-slabs: block sums for the compaction    */
   unsigned long long* scan_state; /* one-pass compaction: per-block words + ticket */
   unsigned scan_tag;             /* the one-pass compaction's launch tag (1..255) */
   double* Ftile[2];              /* [cap][3][64]                              */
@@ -127,6 +124,9 @@ typedef struct lbib_device {
   int* st;                       /* [S][3]                                    */
   int* chunk_box;                /* [nchunks][6]                              */
   long nchunks;
+  int* super[2];                 /* [nsuper][6] boxes of 32 chunks, double buffered
+                                    by step; NULL for few chunks */
+  long nsuper;
   /* errors and plumbing */
   int* err;                      /* [2]: code, step                           */
   int* h_err;                    /* pinned mirror                             */
@@ -159,7 +159,7 @@ typedef struct lbib_device {
 } lbib_device;
 
 #define LBIB_NSTAGE_TIMED 5      /* forces, spread, fluid, moments, move */
-#define LBIB_PROF_EV 9           /* events per profiled step                 */
+#define LBIB_PROF_EV 8           /* events per profiled step                 */
 
 typedef struct lbdev_config {
   int nx, ny, nz, cube_size, compat, prec;
@@ -169,6 +169,8 @@ typedef struct lbdev_config {
 } lbdev_config;
 
 int  lbdev_create(lbib_device** out, const lbdev_config* cfg);
+/* d holds part of the grid's columns. */
+static inline int lbdev_is_slab(const lbib_device* d) { return d->x_lo > 0 || d->x_hi < d->nx; }
 /* Columns [x_lo, x_hi) of the grid held by d (x_hi <= 0: all); sets the
  * storage geometry, allocates nothing. */
 int  lbdev_set_columns(lbib_device* d, int x_lo, int x_hi);
