@@ -46,35 +46,33 @@ using namespace lbib;
 /* ------------------------------------------------------------ kernels */
 namespace {
 
-/* A block per 32-node chunk, all of one problem (every problem's nodes start
- * at a multiple of 32), as the one-grid lbib_node_prep: four warps evaluate
- * the delta factors, the first also reduces the chunk's box and enters the
- * touched tiles, the fifth computes the fiber forces.  step_no: the batch's
- * device step counter (graph replays see the live value), 1 for the first
- * step. */
-__global__ void __launch_bounds__(160, 5) lbib_b_node_prep(double* __restrict__ nodes, const int* __restrict__ node_inst,
+/* A CTA per 32-node chunk, all of one problem (every problem's nodes start
+ * at a multiple of 32), as the one-grid lbib_node_prep: four warps of
+ * node_prep_warp and two for the fiber forces.  step_no: the batch's device
+ * step counter (graph replays see the live value), 1 for the first step. */
+__global__ void __launch_bounds__(192, 4) lbib_b_node_prep(double* __restrict__ nodes, const int* __restrict__ node_inst,
                                                         const BatchDesc* __restrict__ D, double* __restrict__ W,
                                                         int* __restrict__ st, int* __restrict__ chunk_box,
                                                         int* __restrict__ slot, int* __restrict__ list,
                                                         int* __restrict__ count, int* err, long SP,
                                                         const int* __restrict__ step_no, int bend_bug) {
+  __shared__ double x[6][32];
+  __shared__ int s_skip;
   const long i0 = (long)blockIdx.x * 32, i = i0 + (threadIdx.x & 31);
   const int part = threadIdx.x >> 5, k = node_inst[i0];
-  if (k < 0 || *(volatile int*)(err + 2 * k)) return;   /* uniform over the block, but for a node that fails right now */
+  /* one read for the CTA: another chunk of the problem may fail meanwhile */
+  if (threadIdx.x == 0) s_skip = k < 0 || *(volatile int*)(err + 2 * k);
+  __syncthreads();
+  if (s_skip) return;
   const BatchDesc& d = D[k];
   const bool mine = i < d.node0 + d.S;
-  if (part == 4) {
-    if (mine)
-      fiber_forces_node(nodes + d.node0 * 12, d.rows, d.cols, d.bc, d.sc, d.sc2, d.ds1, d.ds2, bend_bug,
-                        (int)(i - d.node0));
+  if (part >= 4) {
+    fiber_forces_pair(nodes + d.node0 * 12, d.rows, d.cols, d.bc, d.sc, d.sc2, d.ds1, d.ds2, bend_bug,
+                      (int)(i - d.node0), mine, part - 4, x);
     return;
   }
-  int is = 0, js = 0, ks = 0;
-  const bool ok = mine && node_prep_part(nodes, i, part, d.nx, d.ny, d.nz, W, st, err + 2 * k, *step_no, is, js, ks);
-  if (part == 0) {
-    chunk_box_reduce(i, SP, chunk_box, nullptr, is, js, ks, ok);
-    touch_tiles(is, js, ks, ok, d.ntx, d.nty, d.tile0, slot, list, count, nullptr);
-  }
+  node_prep_warp(nodes, i, mine, SP, part, d.nx, d.ny, d.nz, d.ntx, d.nty, d.tile0, W, st, chunk_box, nullptr, slot,
+                 list, count, nullptr, err + 2 * k, *step_no);
 }
 
 /* Every listed tile of the batch: its force into its slot. */
@@ -120,21 +118,23 @@ __global__ void __launch_bounds__(kMoveTPB) lbib_b_move(double* __restrict__ nod
   move_chunk(sm, nodes, W, st, i, live, d.ntx, d.nty, slot + d.tile0, Utile, d.dt);
 }
 
-/* FP64 rows away from the walls: the two-cell step, a block per 128 pairs of
- * a problem's (row, pair) range, the parameters in shared memory. */
+/* FP64 rows away from the walls: the two-cell step over runs of blocks of 128
+ * pairs of a problem's (row, pair) range, the parameters in shared memory. */
 template <int PAR>
-__global__ void __launch_bounds__(128, 3) lbib_b_x2(const FluidParams* __restrict__ P, const int2* __restrict__ blk,
+__global__ void __launch_bounds__(128, 3) lbib_b_x2(const FluidParams* __restrict__ P, const int4* __restrict__ blk,
                                                     const int* __restrict__ err) {
   __shared__ __align__(16) FluidParams sp;
-  const int2 m = blk[blockIdx.x];
+  const int4 m = blk[blockIdx.x];
   if (err[2 * m.x]) return;
   block_copy(sp, P + m.x);
   const int npairs = (sp.xhi - sp.xlo + 1) / 2, nry = sp.ny - 6;
-  const long g = (long)m.y * 128 + threadIdx.x;
-  const long row = g / npairs;
-  if (row >= (long)nry * x2_rows_z(sp.nz, sp.zin_hi)) return;
-  const int pr = (int)(g - row * npairs);
-  x2_pair<PAR>(sp, sp.xlo + 2 * pr, 3 + (int)(row % nry), 3 + (int)(row / nry));
+  const int rows = nry * x2_rows_z(sp.nz, sp.zin_hi);
+#pragma unroll 1
+  for (int j = 0; j < m.z; ++j) {
+    const int g = (m.y + j) * 128 + threadIdx.x, row = g / npairs;
+    if (row >= rows) return;
+    x2_pair<PAR>(sp, sp.xlo + 2 * (g - row * npairs), 3 + row % nry, 3 + row / nry);
+  }
 }
 
 template <int PAR>
@@ -278,10 +278,10 @@ struct lbib_batch {
   int2* rowyz;                   /* generic rows (y, z), each problem's contiguous */
   int4* rblk;                    /* generic-row blocks */
   long nrblk;
-  int2* xblk;                    /* FP64 two-cell blocks (problem, block) */
+  int4* xblk;                    /* FP64 two-cell items (problem, first block, blocks) */
   long nxblk;
   int* variant;                  /* word-kernel variant per problem */
-  int2* wblk[MAXV];              /* word blocks of each variant group */
+  int4* wblk[MAXV];              /* word items of each variant group, as xblk */
   long nwblk[MAXV];
   long steps;
   int parity, cur;
@@ -344,34 +344,41 @@ int upload_tables(lbib_batch* b) {
   return rc;
 }
 
-/* Word blocks of each variant group: (problem, block within the problem). */
+/* Runs of `run` of n blocks of problem k. */
+long run_count(long n, int run) { return (n + run - 1) / run; }
+long fill_runs(int4* out, int k, long n, int run) {
+  for (long j = 0; j < n; j += run) *out++ = make_int4(k, (int)j, (int)(n - j < run ? n - j : run), 0);
+  return run_count(n, run);
+}
+
+/* Word blocks of problem k (words_geometry: rows end to end); 0 for none. */
+long word_blocks(const lbib_batch* b, int k) {
+  int nry = 0, nrz = 0;
+  if (b->variant[k] < 0 || !b->h_desc[k].bulk || !lbdev_bulk_rows(b->sh[k], &nry, &nrz)) return 0;
+  const int V = batch_variant_cells_lp(b->prec, b->variant[k]);
+  return ((long)nry * nrz * (b->sh[k]->nx / V) + WTPB - 1) / WTPB;
+}
+
+/* Word items of each variant group. */
 int build_word_blocks(lbib_batch* b) {
   for (int v = 0; v < MAXV; ++v) { cudaFree(b->wblk[v]); b->wblk[v] = NULL; b->nwblk[v] = 0; }
   if (!is_lp(b)) return 0;
+  long total = 0;
+  for (int k = 0; k < b->B; ++k) total += word_blocks(b, k);
+  const int run = run_length(total);
   for (int v = 0; v < batch_variants_lp(b->prec); ++v) {
     long n = 0;
-    for (int k = 0; k < b->B; ++k) {
-      int nry = 0, nrz = 0;
-      if (b->variant[k] != v || !b->h_desc[k].bulk || !lbdev_bulk_rows(b->sh[k], &nry, &nrz)) continue;
-      const int V = batch_variant_cells_lp(b->prec, v);
-      const long gpr = b->sh[k]->nx / V;   /* words_geometry: rows end to end */
-      n += ((long)nry * nrz * gpr + WTPB - 1) / WTPB;
-    }
+    for (int k = 0; k < b->B; ++k)
+      if (b->variant[k] == v) n += run_count(word_blocks(b, k), run);
     if (!n) continue;
-    int2* h = (int2*)malloc(sizeof(int2) * n);
+    int4* h = (int4*)malloc(sizeof(int4) * n);
     if (!h) return -5;
     long i = 0;
-    for (int k = 0; k < b->B; ++k) {
-      int nry = 0, nrz = 0;
-      if (b->variant[k] != v || !b->h_desc[k].bulk || !lbdev_bulk_rows(b->sh[k], &nry, &nrz)) continue;
-      const int V = batch_variant_cells_lp(b->prec, v);
-      const long gpr = b->sh[k]->nx / V;   /* words_geometry: rows end to end */
-      const long nb = ((long)nry * nrz * gpr + WTPB - 1) / WTPB;
-      for (long j = 0; j < nb; ++j) h[i++] = make_int2(k, (int)j);
-    }
+    for (int k = 0; k < b->B; ++k)
+      if (b->variant[k] == v) i += fill_runs(h + i, k, word_blocks(b, k), run);
     int rc = 0;
-    if (cudaMalloc(&b->wblk[v], sizeof(int2) * n) != cudaSuccess) rc = -5;
-    else if (cudaMemcpy(b->wblk[v], h, sizeof(int2) * n, cudaMemcpyHostToDevice) != cudaSuccess) rc = -2;
+    if (cudaMalloc(&b->wblk[v], sizeof(int4) * n) != cudaSuccess) rc = -5;
+    else if (cudaMemcpy(b->wblk[v], h, sizeof(int4) * n, cudaMemcpyHostToDevice) != cudaSuccess) rc = -2;
     free(h);
     if (rc) return rc;
     b->nwblk[v] = n;
@@ -385,7 +392,7 @@ int build_word_blocks(lbib_batch* b) {
  * also step the plane-adjacent cells, come from build_word_blocks). */
 int build_rows(lbib_batch* b) {
   const int lp = is_lp(b);
-  long n = 0, nr = 0, nxb = 0;
+  long n = 0, nr = 0, nxb = 0, pair_blocks = 0;
   for (int k = 0; k < b->B; ++k) {
     const lbib_device* d = b->sh[k];
     int ry = 0, rz = 0;
@@ -393,11 +400,17 @@ int build_rows(lbib_batch* b) {
     const long rows = (long)(d->ny - 4) * (d->nz - 4) - (bulk ? (long)ry * rz : 0);
     n += rows;
     nr += (rows * (d->nx - 4) + 127) / 128;
-    if (bulk && !lp) nxb += ((long)ry * rz * ((d->nx - 4) / 2) + 127) / 128;
+    if (bulk && !lp) pair_blocks += ((long)ry * rz * ((d->nx - 4) / 2) + 127) / 128;
+  }
+  const int run = run_length(pair_blocks);
+  for (int k = 0; k < b->B && !lp; ++k) {
+    int ry = 0, rz = 0;
+    if (b->h_desc[k].bulk && lbdev_bulk_rows(b->sh[k], &ry, &rz))
+      nxb += run_count(((long)ry * rz * ((b->sh[k]->nx - 4) / 2) + 127) / 128, run);
   }
   int2* h = (int2*)malloc(sizeof(int2) * (n ? n : 1));
   int4* rb = (int4*)malloc(sizeof(int4) * (nr ? nr : 1));
-  int2* xo = (int2*)malloc(sizeof(int2) * (nxb ? nxb : 1));
+  int4* xo = (int4*)malloc(sizeof(int4) * (nxb ? nxb : 1));
   if (!h || !rb || !xo) { free(h); free(rb); free(xo); return -5; }
   long r = 0, ir = 0, ix = 0;
   for (int k = 0; k < b->B; ++k) {
@@ -413,8 +426,7 @@ int build_rows(lbib_batch* b) {
       }
     const long rows = r - r0;
     for (long j = 0; j < (rows * (d->nx - 4) + 127) / 128; ++j) rb[ir++] = make_int4(k, (int)r0, (int)rows, (int)j);
-    if (bulk && !lp)
-      for (long j = 0; j < ((long)ry * rz * ((d->nx - 4) / 2) + 127) / 128; ++j) xo[ix++] = make_int2(k, (int)j);
+    if (bulk && !lp) ix += fill_runs(xo + ix, k, ((long)ry * rz * ((d->nx - 4) / 2) + 127) / 128, run);
   }
   b->nrblk = nr;
   b->nxblk = nxb;
@@ -423,8 +435,8 @@ int build_rows(lbib_batch* b) {
   else if (n && cudaMemcpy(b->rowyz, h, sizeof(int2) * n, cudaMemcpyHostToDevice) != cudaSuccess) rc = -2;
   if (!rc && cudaMalloc(&b->rblk, sizeof(int4) * (nr ? nr : 1)) != cudaSuccess) rc = -5;
   else if (!rc && nr && cudaMemcpy(b->rblk, rb, sizeof(int4) * nr, cudaMemcpyHostToDevice) != cudaSuccess) rc = -2;
-  if (!rc && cudaMalloc(&b->xblk, sizeof(int2) * (nxb ? nxb : 1)) != cudaSuccess) rc = -5;
-  else if (!rc && nxb && cudaMemcpy(b->xblk, xo, sizeof(int2) * nxb, cudaMemcpyHostToDevice) != cudaSuccess) rc = -2;
+  if (!rc && cudaMalloc(&b->xblk, sizeof(int4) * (nxb ? nxb : 1)) != cudaSuccess) rc = -5;
+  else if (!rc && nxb && cudaMemcpy(b->xblk, xo, sizeof(int4) * nxb, cudaMemcpyHostToDevice) != cudaSuccess) rc = -2;
   free(h);
   free(rb);
   free(xo);
@@ -464,7 +476,7 @@ int batch_step(lbib_batch* b) {
   const int c = b->cur ^ 1, par = b->parity, first = b->steps == 0;
   cudaStream_t s = b->stream;
   const long SP = b->SP;
-  lbib_b_node_prep<<<(unsigned)(SP / 32), 160, 0, s>>>(b->nodes, b->node_inst, b->desc, b->W, b->st, b->chunk_box,
+  lbib_b_node_prep<<<(unsigned)(SP / 32), 192, 0, s>>>(b->nodes, b->node_inst, b->desc, b->W, b->st, b->chunk_box,
                                                        b->tile_slot[c], b->tile_list[c], b->tile_count[c], b->err, SP,
                                                        b->step_no, (b->compat & 1) != 0);
   b->launches += 1;
@@ -576,6 +588,7 @@ lbib_batch* lbib_batch_create(int n, const lbib_problem* problems, int precision
   b->variant = (int*)calloc(n, sizeof(int));
   if (!b->sh || !b->prob || !b->h_desc || !b->variant) rc = -5;
   if (!rc) memcpy(b->prob, problems, sizeof(lbib_problem) * n);
+  for (int k = 0; k < n && !rc && t != LBIB_PREC_F64; ++k) b->variant[k] = batch_default_variant_lp(precision);
   if (!rc && cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) rc = -2;
   /* sizes and offsets */
   const size_t pb = pop_bytes(precision), rb = t == LBIB_PREC_F64 ? 8 : 4;

@@ -40,6 +40,18 @@ struct BatchDesc {
   double bc, sc, sc2, ds1, ds2, dt;
 };
 
+/* A CTA's share of the pair and word kernels: a run of consecutive blocks of
+ * one problem, {problem, first block, blocks, 0}.  Before its first load a
+ * CTA waits for its item, the problem's error word and its parameters, one
+ * after the other; with one block to a CTA that was a third of its life (FP64
+ * pairs of 24 problems: 415 us per step against TODO).  Up to kRun blocks,
+ * fewer where the batch would not fill the chip several times over. */
+constexpr int kRun = 8;
+inline int run_length(long blocks) {
+  const long r = blocks / (148 * 24);
+  return r < 1 ? 1 : r > kRun ? kRun : (int)r;
+}
+
 /* Copy a parameter struct into shared memory with the whole block. */
 template <typename S>
 __device__ __forceinline__ void block_copy(S& dst, const S* __restrict__ src) {
@@ -78,15 +90,16 @@ __global__ void __launch_bounds__(128) lbib_b_rows(const FluidParamsT<T>* __rest
  * does not matter. */
 template <typename T, int V, int PAR, int MINB>
 __global__ void __launch_bounds__(WTPB, MINB) lbib_b_words(const WordsParams<T>* __restrict__ WP,
-                                                           const int2* __restrict__ blk, const int* __restrict__ err) {
+                                                           const int4* __restrict__ blk, const int* __restrict__ err) {
   __shared__ __align__(16) WordsParams<T> sb;
-  const int2 m = blk[blockIdx.x];
+  const int4 m = blk[blockIdx.x];
   if (err[2 * m.x]) return;
   block_copy(sb, WP + m.x);
-  const long first = (long)m.y * WTPB;
-  words_item<T, V, PAR>(sb, first + threadIdx.x);
+  const long first = (long)m.y * WTPB, end = first + (long)m.z * WTPB;
+#pragma unroll 1
+  for (long t = first; t < end; t += WTPB) words_item<T, V, PAR>(sb, t + threadIdx.x);
   const long r0 = fdiv((unsigned)(first + sb.gpr - 1), sb.dgpr);
-  long r1 = fdiv((unsigned)(first + WTPB + sb.gpr - 1), sb.dgpr);
+  long r1 = fdiv((unsigned)(end + sb.gpr - 1), sb.dgpr);
   if (r1 > sb.nrows) r1 = sb.nrows;
   for (long i = threadIdx.x; i < 4 * (r1 - r0); i += WTPB) edge_cell<T, PAR>(sb.p, sb.nry, (int)(r0 + i / 4), (int)(i & 3));
 }

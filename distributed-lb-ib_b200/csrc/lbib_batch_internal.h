@@ -26,7 +26,7 @@ struct BatchFluid {
   const int2* rowyz;       /* generic rows (y, z), each problem's contiguous */
   const int4* rblk;        /* generic-row blocks: (problem, first row, rows, chunk) */
   long nrblk;
-  const int2* xblk;        /* FP64 two-cell blocks: (problem, block) */
+  const int4* xblk;        /* FP64 two-cell items: (problem, first block, blocks) */
   long nxblk;
   const int* list;         /* touched tiles (global ids) */
   const int* count;
@@ -47,8 +47,10 @@ int batch_gather_lp(const BatchFluid& f);
 /* Generic rows (FP64: two-cell blocks too). */
 int batch_rows_lp(const BatchFluid& f);
 int batch_rows_f64(const BatchFluid& f);
-/* Word-kernel blocks of one variant. */
-int batch_words_lp(const BatchFluid& f, int variant, const int2* blk, long nblk);
+/* Word-kernel items (problem, first block, blocks) of one variant; the
+ * variant a problem starts with. */
+int batch_words_lp(const BatchFluid& f, int variant, const int4* blk, long nblk);
+int batch_default_variant_lp(int prec);
 int batch_variants_lp(int prec);
 int batch_variant_cells_lp(int prec, int variant);   /* V of a variant */
 /* Tile moments after the step (parity = the next step's). */

@@ -33,7 +33,7 @@ int rows(const BatchFluid& f) {
 }
 
 template <typename T, int V, int MINB>
-int words(const BatchFluid& f, const int2* blk, long nblk) {
+int words(const BatchFluid& f, const int4* blk, long nblk) {
   if (nblk <= 0) return 0;
   const WordsParams<T>* WP = static_cast<const WordsParams<T>*>(f.WP);
   if (f.par == 0) lbib_b_words<T, V, 0, MINB><<<(unsigned)nblk, WTPB, 0, f.stream>>>(WP, blk, f.err);
@@ -42,7 +42,7 @@ int words(const BatchFluid& f, const int2* blk, long nblk) {
 }
 
 template <typename T>
-int words_v(const BatchFluid& f, int v, const int2* blk, long nblk) {
+int words_v(const BatchFluid& f, int v, const int4* blk, long nblk) {
   return with_variant<T>(v, [&](auto V, auto MINB) { return words<T, V, MINB>(f, blk, nblk); });
 }
 
@@ -78,7 +78,7 @@ int batch_rows_lp(const BatchFluid& f) {
   }
 }
 
-int batch_words_lp(const BatchFluid& f, int variant, const int2* blk, long nblk) {
+int batch_words_lp(const BatchFluid& f, int variant, const int4* blk, long nblk) {
   switch (LBIB_PREC_TYPE(f.prec)) {
     case LBIB_PREC_F32: return words_v<float>(f, variant, blk, nblk);
     case LBIB_PREC_F16: return words_v<__half>(f, variant, blk, nblk);
@@ -86,6 +86,11 @@ int batch_words_lp(const BatchFluid& f, int variant, const int2* blk, long nblk)
     default: return -1;
   }
 }
+
+/* {4, 4} for 16-bit storage, {2, 5} for FP32: per step of a 128-problem
+ * sweep 1130 us, against 1133 to 1439 of the others, and 1376 us against
+ * 1536 and 1587; the autotuner's per-class choice gains another 3%. */
+int batch_default_variant_lp(int prec) { return LBIB_PREC_TYPE(prec) == LBIB_PREC_F32 ? 2 : 1; }
 
 int batch_variants_lp(int prec) { return word_variants(prec); }
 

@@ -23,6 +23,7 @@
 
 #include "lbib_internal.h"
 #include <climits>
+#include <cmath>
 
 #include "lbib_ib.cuh"
 #include "lbib_lattice.cuh"
@@ -535,6 +536,12 @@ __global__ void lbib_init_table(FluidParamsT<T> p, typename Pop<T>::R* __restric
   for (int q = 0; q < 19; ++q) t[q * count + i] = Form<T>::stored_initial(q, p.rho0, p.ux0, p);
 }
 
+/* 1/c for div_const, or 0 where c does not qualify (|c y - 1| >= 2^-54). */
+inline double div_const_inverse(double c) {
+  const double y = 1.0 / c;
+  return fabs(fma(c, y, -1.0)) < 0x1p-54 ? y : 0.0;
+}
+
 template <typename T>
 FluidParamsT<T> make_params_t(lbib_device* d, int first) {
   using R = typename Pop<T>::R;
@@ -550,6 +557,7 @@ FluidParamsT<T> make_params_t(lbib_device* d, int first) {
   p.ux_rest = (d->compat & LBIB_OPT_REST_START) ? 0.0 : d->u_l;
   p.omtau = d->omtau; p.invtau = d->invtau;
   p.kw0 = d->kw[0]; p.kw1 = d->kw[1]; p.kw2 = d->kw[2];
+  p.cs2_inv = div_const_inverse(d->cs2); p.cs4_inv = div_const_inverse(d->cs4);
   p.cs2 = d->cs2; p.cs4 = d->cs4; p.half_dt = d->half_dt; p.g = d->g_l;
   const int c = d->cur;
   p.slot_cur = d->tile_slot[c]; p.Fcur = d->Ftile[c];

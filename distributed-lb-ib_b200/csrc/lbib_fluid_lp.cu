@@ -278,12 +278,25 @@ int lp_spread_box(lbib_device* d) {
   return launch_spread_box_t<T>(d, p);
 }
 
+/* The variant of a state that has not been autotuned: by the autotuner's
+ * times at three sizes.  us per fluid step, {4,3} / {2,6} / {4,5} / {4,5}
+ * even with {8,4} odd: 21 20 21 23 at 64x32x32, 28 28 29 28 at 128x64x64,
+ * 135 127 107 107 at 256x128x128, 942 766 682 657 at 512x256x256 (FP16);
+ * FP32, {2,3} {2,4} {2,5}: 33 30 30, 182 159 148 and 1158 1024 966 at the
+ * last three. */
+template <typename T>
+int default_variant(const lbib_device* d) {
+  if (sizeof(T) == 4) return 2;
+  if (d->N < (1L << 20)) return 4;
+  return d->nx % 8 == 0 ? word_variants(d->prec) + kTmaVariants + 1 : 5;
+}
+
 template <typename T>
 int lp_step(lbib_device* d) {
   FluidParamsT<T> p = make_params_t<T>(d, d->steps == 0);
   if (launch_step_rows_t<T>(d, p)) return -2;
   if (!d->use_bulk) return 0;
-  const int v = d->lp_variant < 0 ? 0 : d->lp_variant;
+  const int v = d->lp_variant < 0 ? default_variant<T>(d) : d->lp_variant;
   if constexpr (sizeof(T) == 2) {
     const int nw = word_variants(d->prec);
     if (v == nw) return launch_words_tma<T, 2, 4>(d, p);

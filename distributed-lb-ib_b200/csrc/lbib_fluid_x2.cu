@@ -27,6 +27,8 @@ struct X2Params {
   int nry;       /* interior rows in y: ny - 6 */
   int npairs;    /* pairs per row: (xhi - xlo + 1) / 2 */
   long pf;       /* L2 prefetch distance in blocks (0: none) */
+  unsigned flat; /* pairs in all, rows end to end; 0: blocks per row */
+  FastDiv dpairs, dnry;
 };
 
 /* Threads 0..18 ask L2 for plane q of the rows of the block pf blocks
@@ -48,6 +50,13 @@ __device__ __forceinline__ void x2_prefetch(const X2Params& b, int q) {
 
 template <int PAR>
 __global__ void __launch_bounds__(TPB, PAR ? LBIB_X2_MINB1 : LBIB_X2_MINB0) lbib_fluid_step_x2(X2Params b) {
+  if (b.flat) {
+    const unsigned t = blockIdx.x * TPB + threadIdx.x;
+    if (t >= b.flat) return;
+    const unsigned row = fdiv(t, b.dpairs), z = fdiv(row, b.dnry);
+    x2_pair<PAR>(b.p, b.p.xlo + 2 * (int)(t - row * b.npairs), 3 + (int)(row - z * b.nry), 3 + (int)z);
+    return;
+  }
   if (b.pf > 0 && threadIdx.x < 19) x2_prefetch<PAR>(b, threadIdx.x);
   const int pr = blockIdx.y * TPB + threadIdx.x;
   if (pr >= b.npairs) return;
@@ -81,6 +90,18 @@ extern "C" int lbdev_launch_fluid_bulk(lbib_device* d, const void* fluid_params)
     b.pf = (long)d->l2_pf * sms * (d->parity ? LBIB_X2_MINB1 : LBIB_X2_MINB0);
   }
   dim3 grid((unsigned)((long)b.nry * nrz), (unsigned)((b.npairs + TPB - 1) / TPB));
+  /* a block per TPB pairs of a row keeps every warp on one row; where that
+     leaves more than 5% of the threads without a pair (62 pairs in rows of
+     128 cells: half), the rows are laid end to end instead.  us per step
+     of the kernel, per row / end to end: TODO */
+  const long pairs = (long)b.nry * nrz * b.npairs, slots = (long)grid.x * grid.y * TPB;
+  b.flat = 0;
+  if (pairs < 0.95 * slots && pairs + TPB < (1L << 31)) {
+    b.flat = (unsigned)pairs;
+    b.dpairs = fast_div((unsigned)b.npairs);
+    b.dnry = fast_div((unsigned)b.nry);
+    grid = dim3((unsigned)((pairs + TPB - 1) / TPB));
+  }
   if (d->parity == 0) lbib_fluid_step_x2<0><<<grid, TPB, 0, d->fluid_stream>>>(b);
   else lbib_fluid_step_x2<1><<<grid, TPB, 0, d->fluid_stream>>>(b);
   d->kernel_launches++;

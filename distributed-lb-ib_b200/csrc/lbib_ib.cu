@@ -26,36 +26,31 @@ struct SheetForces {
   lbib_sheet_dev s[kFuseSheets];
 };
 
-/* A block per 32-node chunk: warp p < 4 evaluates part p of the chunk's
- * nodes (node_prep_part); warp 0 also reduces the chunk's stencil box and
- * enters the tiles its stencils touch.  A fifth warp, when the block has
- * one, computes the nodes' fiber forces for the sheets `sf` names
- * (fiber_forces_node reads neighbours' positions and writes the node's own
- * force fields only, so it runs alongside).  list NULL: mark the tiles only. */
-__global__ void __launch_bounds__(160, 5) lbib_node_prep(double* __restrict__ nodes, long S, int nx, int ny, int nz,
+/* A CTA per 32-node chunk: node_prep_warp by warps 0 to 3; warps 4 and 5,
+ * when it has them, compute the nodes' fiber forces for the sheets `sf`
+ * names (they read neighbours' positions and write the node's own force
+ * fields only, so they run alongside).  list NULL: mark the tiles only.
+ * Bound by the latency of one chunk's chain at any size that matters:
+ * 16,000 cycles with one warp for the forces and for all tiles, TODO. */
+__global__ void __launch_bounds__(192, 4) lbib_node_prep(double* __restrict__ nodes, long S, int nx, int ny, int nz,
                                                       int ntx, int nty, double* __restrict__ W, int* __restrict__ st,
                                                       int* __restrict__ chunk_box, int* __restrict__ super,
                                                       int* __restrict__ slot, int* __restrict__ list,
                                                       int* __restrict__ count, int* __restrict__ mark, int* err,
                                                       int step, SheetForces sf) {
+  __shared__ double x[6][32];
   const long i = (long)blockIdx.x * 32 + (threadIdx.x & 31);
   const int part = threadIdx.x >> 5;
-  if (part == 4) {
-    if (sf.n == 0 || i >= S) return;
+  if (part >= 4) {
     int k = 0;
     while (k + 1 < sf.n && i >= sf.s[k + 1].offset) ++k;
     const lbib_sheet_dev& h = sf.s[k];
-    const long li = i - h.offset;
-    if (li < (long)h.rows * h.cols)
-      fiber_forces_node(nodes + h.offset * 12, h.rows, h.cols, h.bc, h.sc, h.sc2, h.ds1, h.ds2, sf.bend_bug, (int)li);
+    fiber_forces_pair(nodes + h.offset * 12, h.rows, h.cols, h.bc, h.sc, h.sc2, h.ds1, h.ds2, sf.bend_bug,
+                      (int)(i - h.offset), i < S, part - 4, x);
     return;
   }
-  int is = 0, js = 0, ks = 0;
-  const bool ok = i < S && node_prep_part(nodes, i, part, nx, ny, nz, W, st, err, step, is, js, ks);
-  if (part == 0) {
-    chunk_box_reduce(i, S, chunk_box, super, is, js, ks, ok);
-    touch_tiles(is, js, ks, ok, ntx, nty, 0, slot, list, count, mark);
-  }
+  node_prep_warp(nodes, i, i < S, S, part, nx, ny, nz, ntx, nty, 0, W, st, chunk_box, super, slot, list, count, mark,
+                 err, step);
 }
 
 /* Every listed tile of columns tx in [tlo, thi) (an x-slab gathers the
@@ -233,7 +228,7 @@ extern "C" int lbdev_launch_prep(lbib_device* d, int step) {
     for (int k = 0; k < d->nsheets; ++k) sf.s[k] = d->sh[k];
   }
   const int slab = lbdev_is_slab(d);
-  lbib_node_prep<<<(unsigned)d->nchunks, sf.n ? 160 : 128, 0, st>>>(
+  lbib_node_prep<<<(unsigned)d->nchunks, sf.n ? 192 : 128, 0, st>>>(
       d->nodes, d->S, d->nx, d->ny, d->nz, d->ntx, d->nty, d->W, d->st, d->chunk_box, d->super[c], d->tile_slot[c],
       slab ? nullptr : d->tile_list[c], d->tile_count[c], d->tile_mark, d->err, step, sf);
   d->kernel_launches++;

@@ -6,11 +6,11 @@
  *                       compute_elasticforce (cube_pthread/lbm_ib.c:961-1318),
  *                       one node, both passes of each force in the
  *                       reference's order.
- *   node_prep_part      stencil start floor(X - 2) + 1 per axis, the twelve
+ *   node_prep_warp      stencil start floor(X - 2) + 1 per axis, the twelve
  *                       delta-kernel factors 1 + cos(pi/2 r) (shared by the
  *                       spread and the interpolation of the step);
  *                       chunk_box_reduce: per 32-node chunk (and per 1024)
- *                       the bounding box of its stencils; touch_tiles: the
+ *                       the bounding box of its stencils; TouchTiles: the
  *                       4^3 tiles the stencils touch, appended to the
  *                       step's tile list as they are met (or only marked,
  *                       for the compaction below).
@@ -53,103 +53,98 @@ __device__ __forceinline__ void set_error(int* err, int code, int step) {
   if (atomicCAS(err, 0, code) == 0) err[1] = step;
 }
 
+/* One direction's share of a node's bending and stretching force: along the
+ * fiber (k = c, n = C nodes, stride 1 node, rest length ds1) or across the
+ * fibers (k = r, n = R, stride C, ds2).  `slip`: at the last node but one
+ * the x component takes the node's own position for the one two nodes back
+ * (lbm_ib.c:1032-1035, the row pass only).  The node and its neighbours
+ * k - 2 .. k + 2 are loaded together before any is used.  Bending lbm_ib.c:1002-1052 and 1062-1145, stretching 1179-1221 and
+ * 1233-1278. */
+__device__ __forceinline__ void fiber_line_forces(const double* __restrict__ m, int k, int n, long stride, double bc,
+                                                  double sc, double rest, bool slip, double b[3], double s[3]) {
+  double p[5][3];
+#pragma unroll
+  for (int o = -2; o <= 2; ++o) {
+    /* the neighbours its formula reads; its own place for the others */
+    const bool used = o == 0 || (k == 0 ? o > 0 : k == 1 ? o != -2 : k == n - 1 ? o < 0 : k == n - 2 ? o != 2 : true);
+    const double* q = m + (used ? (long)o * stride * 12 : 0);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) p[o + 2][d] = q[d];
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double a2 = p[0][d], a1 = p[1][d], x = p[2][d], c1 = p[3][d], c2 = p[4][d];
+    if (k == 0) b[d] = bc * (-c2 + 2 * c1 - x);
+    else if (k == 1) b[d] = bc * (-c2 + 4 * c1 - 5 * x + 2 * a1);
+    else if (k == n - 1) b[d] = bc * (-x + 2 * a1 - a2);
+    else if (k == n - 2) b[d] = bc * (2 * c1 - 5 * x + 4 * a1 - (d == 0 && slip ? x : a2));
+    else b[d] = bc * (-c2 + 4.0 * c1 - 6.0 * x + 4.0 * a1 - a2);
+  }
+  /* towards the next node (k = 0), from the previous one (the last: the
+     reference's reversed tangent), or both */
+  const bool first = k == 0, last = k == n - 1;
+  double u[3], v[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    u[d] = last ? p[2][d] - p[1][d] : p[3][d] - p[2][d];
+    v[d] = p[1][d] - p[2][d];
+  }
+  const double lu = sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+  if (first || last) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) s[d] = sc * ((lu - rest) * (u[d] / lu));
+  } else {
+    const double lv = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) s[d] = sc * ((lu - rest) * (u[d] / lu) + (lv - rest) * (v[d] / lv));
+  }
+}
+
+/* The node's record: the along-fiber shares plus the across-fiber ones, and
+ * compute_elasticforce (lbm_ib.c:1303-1308): stretch + bend. */
+__device__ __forceinline__ void fiber_store(double* __restrict__ o, const double b1[3], const double s1[3],
+                                            const double b2[3], const double s2[3]) {
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double b = b1[d] + b2[d], s = s1[d] + s2[d];
+    o[3 + d] = b;
+    o[6 + d] = s;
+    o[9 + d] = s + b;
+  }
+}
+
 /* compute_bendingforce + compute_stretchingforce + compute_elasticforce for
  * node i of one R x C sheet whose records start at `nodes`. */
 __device__ __forceinline__ void fiber_forces_node(double* __restrict__ nodes, int R, int C, double bc, double sc,
                                                   double sc2, double ds1, double ds2, int bend_bug, int i) {
-  const int r = i / C, c = i % C;
-#define P(rr, cc) (nodes + ((long)(rr) * C + (cc)) * 12)
-  const double* m = P(r, c);
+  double* m = nodes + (long)i * 12;
+  double b1[3], s1[3], b2[3], s2[3];
+  fiber_line_forces(m, i % C, C, 1, bc, sc, ds1, bend_bug, b1, s1);
+  fiber_line_forces(m, i / C, R, C, bc, sc2, ds2, false, b2, s2);
+  fiber_store(m, b1, s1, b2, s2);
+}
+
+/* The same by two warps of a CTA, a lane of each for node i (`ok`: there is
+ * one): warp `half` 0 the along-fiber share, 1 the across-fiber one, which it
+ * hands over through shared memory x[6][32]; named barrier 1 is theirs. */
+__device__ __forceinline__ void fiber_forces_pair(double* __restrict__ nodes, int R, int C, double bc, double sc,
+                                                  double sc2, double ds1, double ds2, int bend_bug, int i, bool ok,
+                                                  int half, double (*x)[32]) {
+  const int lane = threadIdx.x & 31;
+  double* m = nodes + (long)i * 12;
   double b[3], s[3];
-  /* bending along the fiber (row), lbm_ib.c:1002-1052 */
-  for (int d = 0; d < 3; ++d) {
-    if (c == 0) {
-      b[d] = bc * (-P(r, 2)[d] + 2 * P(r, 1)[d] - P(r, 0)[d]);
-    } else if (c == 1) {
-      b[d] = bc * (-P(r, 3)[d] + 4 * P(r, 2)[d] - 5 * P(r, 1)[d] + 2 * P(r, 0)[d]);
-    } else if (c == C - 1) {
-      b[d] = bc * (-P(r, c)[d] + 2 * P(r, c - 1)[d] - P(r, c - 2)[d]);
-    } else if (c == C - 2) {
-      const double last = (d == 0 && bend_bug) ? P(r, c)[d] : P(r, c - 2)[d];
-      b[d] = bc * (2 * P(r, c + 1)[d] - 5 * P(r, c)[d] + 4 * P(r, c - 1)[d] - last);
-    } else {
-      b[d] = bc * (-P(r, c + 2)[d] + 4.0 * P(r, c + 1)[d] - 6.0 * P(r, c)[d] + 4.0 * P(r, c - 1)[d] - P(r, c - 2)[d]);
-    }
+  if (ok) {
+    if (half) fiber_line_forces(m, i / C, R, C, bc, sc2, ds2, false, b, s);
+    else fiber_line_forces(m, i % C, C, 1, bc, sc, ds1, bend_bug, b, s);
   }
-  /* bending across fibers (column), lbm_ib.c:1062-1145 */
-  for (int d = 0; d < 3; ++d) {
-    double v;
-    if (r == 0) {
-      v = bc * (-P(2, c)[d] + 2 * (P(1, c)[d]) - (P(0, c)[d]));
-    } else if (r == 1) {
-      v = bc * (-P(3, c)[d] + 4 * (P(2, c)[d]) - 5 * (P(1, c)[d]) + 2 * (P(0, c)[d]));
-    } else if (r == R - 1) {
-      v = bc * (-(P(r, c)[d]) + 2 * (P(r - 1, c)[d]) - (P(r - 2, c)[d]));
-    } else if (r == R - 2) {
-      v = bc * (2 * P(r + 1, c)[d] - 5 * (P(r, c)[d]) + 4 * (P(r - 1, c)[d]) - (P(r - 2, c)[d]));
-    } else {
-      v = bc * (-P(r + 2, c)[d] + 4.0 * (P(r + 1, c)[d]) - 6.0 * (P(r, c)[d]) + 4.0 * (P(r - 1, c)[d]) - (P(r - 2, c)[d]));
-    }
-    b[d] = b[d] + v;
+  if (half && ok)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) { x[d][lane] = b[d]; x[3 + d][lane] = s[d]; }
+  asm volatile("bar.sync 1, 64;" ::: "memory");
+  if (!half && ok) {
+    const double b2[3] = {x[0][lane], x[1][lane], x[2][lane]}, s2[3] = {x[3][lane], x[4][lane], x[5][lane]};
+    fiber_store(m, b, s, b2, s2);
   }
-  /* stretching along the fiber (row), lbm_ib.c:1179-1221 */
-  if (c == 0) {
-    const double* p = P(r, 1);
-    const double t0 = p[0] - m[0], t1 = p[1] - m[1], t2 = p[2] - m[2];
-    const double dr = sqrt(t0 * t0 + t1 * t1 + t2 * t2);
-    s[0] = sc * ((dr - ds1) * (t0 / dr));
-    s[1] = sc * ((dr - ds1) * (t1 / dr));
-    s[2] = sc * ((dr - ds1) * (t2 / dr));
-  } else if (c == C - 1) {
-    const double* q = P(r, C - 2);
-    const double t0 = m[0] - q[0], t1 = m[1] - q[1], t2 = m[2] - q[2];
-    const double dl = sqrt(t0 * t0 + t1 * t1 + t2 * t2);
-    s[0] = sc * ((dl - ds1) * (t0 / dl));
-    s[1] = sc * ((dl - ds1) * (t1 / dl));
-    s[2] = sc * ((dl - ds1) * (t2 / dl));
-  } else {
-    const double* p = P(r, c + 1);
-    const double* q = P(r, c - 1);
-    const double r0 = p[0] - m[0], r1 = p[1] - m[1], r2 = p[2] - m[2];
-    const double l0 = q[0] - m[0], l1 = q[1] - m[1], l2 = q[2] - m[2];
-    const double dr = sqrt(r0 * r0 + r1 * r1 + r2 * r2);
-    const double dl = sqrt(l0 * l0 + l1 * l1 + l2 * l2);
-    s[0] = sc * ((dr - ds1) * (r0 / dr) + (dl - ds1) * (l0 / dl));
-    s[1] = sc * ((dr - ds1) * (r1 / dr) + (dl - ds1) * (l1 / dl));
-    s[2] = sc * ((dr - ds1) * (r2 / dr) + (dl - ds1) * (l2 / dl));
-  }
-  /* stretching across fibers (column), lbm_ib.c:1233-1278 */
-  if (r == 0) {
-    const double* p = P(1, c);
-    const double t0 = p[0] - m[0], t1 = p[1] - m[1], t2 = p[2] - m[2];
-    const double dt = sqrt(t0 * t0 + t1 * t1 + t2 * t2);
-    s[0] = s[0] + sc2 * ((dt - ds2) * (t0 / dt));
-    s[1] = s[1] + sc2 * ((dt - ds2) * (t1 / dt));
-    s[2] = s[2] + sc2 * ((dt - ds2) * (t2 / dt));
-  } else if (r == R - 1) {
-    const double* q = P(R - 2, c);
-    const double t0 = m[0] - q[0], t1 = m[1] - q[1], t2 = m[2] - q[2];
-    const double db = sqrt(t0 * t0 + t1 * t1 + t2 * t2);
-    s[0] = s[0] + sc2 * ((db - ds2) * (t0 / db));
-    s[1] = s[1] + sc2 * ((db - ds2) * (t1 / db));
-    s[2] = s[2] + sc2 * ((db - ds2) * (t2 / db));
-  } else {
-    const double* p = P(r + 1, c);
-    const double* q = P(r - 1, c);
-    const double a0 = p[0] - m[0], a1 = p[1] - m[1], a2 = p[2] - m[2];
-    const double e0 = q[0] - m[0], e1 = q[1] - m[1], e2 = q[2] - m[2];
-    const double dt = sqrt(a0 * a0 + a1 * a1 + a2 * a2);
-    const double db = sqrt(e0 * e0 + e1 * e1 + e2 * e2);
-    s[0] = s[0] + sc2 * ((dt - ds2) * (a0 / dt) + (db - ds2) * (e0 / db));
-    s[1] = s[1] + sc2 * ((dt - ds2) * (a1 / dt) + (db - ds2) * (e1 / db));
-    s[2] = s[2] + sc2 * ((dt - ds2) * (a2 / dt) + (db - ds2) * (e2 / db));
-  }
-#undef P
-  double* o = nodes + (long)i * 12;
-  o[3] = b[0]; o[4] = b[1]; o[5] = b[2];
-  o[6] = s[0]; o[7] = s[1]; o[8] = s[2];
-  /* compute_elasticforce, lbm_ib.c:1303-1308: stretch + bend */
-  o[9] = s[0] + b[0]; o[10] = s[1] + b[1]; o[11] = s[2] + b[2];
 }
 
 __device__ __forceinline__ int stencil_start(double p) { return (int)(floor(p / 1.0 - 2) + 1); }
@@ -161,74 +156,74 @@ __device__ __forceinline__ int stencil_start(double p) { return (int)(floor(p / 
  * turn NaN into 0 and pass). */
 __device__ __forceinline__ bool stencil_inside(double p, int n) { return p >= 1.0 && p < (double)n - 2.0; }
 
-/* Node i, split over four threads: part p (0..3) evaluates the three delta
- * factors of stencil offset p (one per axis); part 0 also writes the stencil
- * start and checks the grid.  Returns whether the stencil lies inside, its
- * start in is, js, ks. */
-__device__ __forceinline__ bool node_prep_part(const double* __restrict__ nodes, long i, int part, int nx, int ny,
-                                               int nz, double* __restrict__ W, int* __restrict__ st, int* err,
-                                               int step, int& is, int& js, int& ks) {
-  const double* m = nodes + i * 12;
+/* The 4^3 tiles (ids offset by tile0) that a warp's stencils touch at offsets
+ * 2 part and 2 part + 1 of the eight (the four warps of a chunk share them;
+ * ok: the lane has a stencil).  The lanes that touch a tile at the same
+ * offset act once, through the first of them.  With `list`: the warp that
+ * meets a tile first (slot[tile] goes from -1 through -2) gives it the next
+ * slot -- which one depends on timing, no result does -- so that one launch
+ * does what took a count, a prefix sum over all tiles and a scatter (22 us
+ * of a 512x256x256 step's spread).  Without: mark[tile] = 1.  begin sends
+ * the atomics off, finish uses their answers: the cosines come in between.
+ * (All eight offsets by one warp after its cosines: 8,000 of the
+ * launch's 16,000 cycles.) */
+struct TouchTiles {
+  int tile[2], was[2];
+  __device__ __forceinline__ void begin(int part, int is, int js, int ks, bool ok, int ntx, int nty, int tile0,
+                                        int* __restrict__ slot, bool listed, int* __restrict__ mark) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int tx = (is >> 2) + u, ty = (js >> 2) + (part & 1), tz = (ks >> 2) + (part >> 1);
+      const bool here = ok && tx <= (is + 3) >> 2 && ty <= (js + 3) >> 2 && tz <= (ks + 3) >> 2;
+      const int id = here ? tile0 + (tz * nty + ty) * ntx + tx : -1;
+      const unsigned grp = __match_any_sync(0xffffffffu, id);
+      tile[u] = here && lane == __ffs(grp) - 1 ? id : -1;
+      was[u] = 0;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (tile[u] < 0) continue;
+      if (listed) was[u] = atomicCAS(&slot[tile[u]], -1, -2);
+      else mark[tile[u]] = 1;
+    }
+  }
+  __device__ __forceinline__ void finish(int* __restrict__ slot, int* __restrict__ list, int* __restrict__ count) {
+    const int lane = threadIdx.x & 31;
+    const unsigned a = __ballot_sync(0xffffffffu, was[0] == -1), b = __ballot_sync(0xffffffffu, was[1] == -1);
+    const int na = __popc(a), n = na + __popc(b);
+    if (!n) return;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(count, n);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (was[u] != -1) continue;
+      const int k = base + (u ? na + __popc(b & below) : __popc(a & below));
+      list[k] = tile[u];
+      slot[tile[u]] = k;
+    }
+  }
+};
+
+/* A node's stencil start per axis; false when it leaves the grid. */
+__device__ __forceinline__ bool node_stencil(const double m[3], int nx, int ny, int nz, int& is, int& js, int& ks) {
   const bool inside = stencil_inside(m[0], nx) && stencil_inside(m[1], ny) && stencil_inside(m[2], nz);
   is = inside ? stencil_start(m[0]) : 0;
   js = inside ? stencil_start(m[1]) : 0;
   ks = inside ? stencil_start(m[2]) : 0;
-  const double cxk = kPi / (2.0 * 1.0);
-  double* w = W + i * 12;
-  w[part] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (is + part) - m[0]));
-  w[4 + part] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (js + part) - m[1]));
-  w[8 + part] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (ks + part) - m[2]));
-  if (part != 0) return inside;
-  st[i * 3 + 0] = is; st[i * 3 + 1] = js; st[i * 3 + 2] = ks;
-  if (!inside) set_error(err, -3, step);
   return inside;
 }
 
-/* The 4^3 tiles (ids offset by tile0) that a warp's stencils touch, ok: the
- * lane has one.  The lanes that touch a tile at the same stencil offset act
- * once, through the first of them.  With `list`: the warp that meets a tile
- * first (slot[tile] goes from -1 through -2) gives it the next slot --
- * which one depends on timing, no result does -- so that one launch does
- * what took a count, a prefix sum over all tiles and a scatter (22 us of a
- * 512x256x256 step's spread).  Without: mark[tile] = 1.  The eight offsets'
- * loads and atomics are each issued together. */
-__device__ __forceinline__ void touch_tiles(int is, int js, int ks, bool ok, int ntx, int nty, long tile0,
-                                            int* __restrict__ slot, int* __restrict__ list, int* __restrict__ count,
-                                            int* __restrict__ mark) {
-  const int lane = threadIdx.x & 31;
-  long tile[8];
-  int was[8];
-#pragma unroll
-  for (int o = 0; o < 8; ++o) {
-    const int tx = (is >> 2) + (o & 1), ty = (js >> 2) + ((o >> 1) & 1), tz = (ks >> 2) + (o >> 2);
-    const bool here = ok && tx <= (is + 3) >> 2 && ty <= (js + 3) >> 2 && tz <= (ks + 3) >> 2;
-    const long id = here ? tile0 + ((long)tz * nty + ty) * ntx + tx : -1;
-    const unsigned grp = __match_any_sync(0xffffffffu, id);
-    tile[o] = here && lane == __ffs(grp) - 1 ? id : -1;
-  }
-  if (!list) {
-#pragma unroll
-    for (int o = 0; o < 8; ++o)
-      if (tile[o] >= 0) mark[tile[o]] = 1;
-    return;
-  }
-  volatile int* vs = slot;
-#pragma unroll
-  for (int o = 0; o < 8; ++o) was[o] = tile[o] >= 0 ? vs[tile[o]] : 0;
-#pragma unroll
-  for (int o = 0; o < 8; ++o)
-    if (tile[o] >= 0 && was[o] == -1) was[o] = atomicCAS(&slot[tile[o]], -1, -2);
-    else was[o] = 0;
-#pragma unroll
-  for (int o = 0; o < 8; ++o)
-    if (was[o] == -1) was[o] = atomicAdd(count, 1);
-    else was[o] = -1;
-#pragma unroll
-  for (int o = 0; o < 8; ++o)
-    if (was[o] >= 0) {
-      list[was[o]] = (int)tile[o];
-      slot[tile[o]] = was[o];
-    }
+/* The three delta factors (one per axis) of stencil offset `part` of a node
+ * at m whose stencil starts at is, js, ks. */
+__device__ __forceinline__ void delta_factors(double* __restrict__ w, const double m[3], int part, int is, int js,
+                                              int ks) {
+  const double cxk = kPi / (2.0 * 1.0);
+  w[part] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (is + part) - m[0]));
+  w[4 + part] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (js + part) - m[1]));
+  w[8 + part] = 1.0e0 + lbib_cos_2phase(cxk * (1.0 * (ks + part) - m[2]));
 }
 
 constexpr int kSuper = 32;   /* chunks per super-chunk */
@@ -252,6 +247,33 @@ __device__ __forceinline__ void chunk_box_reduce(long i, long S, int* __restrict
   atomicMin(&sx[0], b0); atomicMax(&sx[1], b1);
   atomicMin(&sx[2], b2); atomicMax(&sx[3], b3);
   atomicMin(&sx[4], b4); atomicMax(&sx[5], b5);
+}
+
+/* Node preparation of a chunk's 32 nodes (node i on lane l of each of the
+ * four warps, `have`: there is one): warp `part` evaluates its delta factors
+ * and enters its share of the touched tiles; the first also writes the
+ * stencil starts, checks the grid and reduces the chunk's box. */
+__device__ __forceinline__ void node_prep_warp(const double* __restrict__ nodes, long i, bool have, long S, int part,
+                                               int nx, int ny, int nz, int ntx, int nty, long tile0,
+                                               double* __restrict__ W, int* __restrict__ st,
+                                               int* __restrict__ chunk_box, int* __restrict__ super,
+                                               int* __restrict__ slot, int* __restrict__ list,
+                                               int* __restrict__ count, int* __restrict__ mark, int* err, int step) {
+  double m[3] = {-1.0, 0.0, 0.0};
+  if (have) { m[0] = nodes[i * 12]; m[1] = nodes[i * 12 + 1]; m[2] = nodes[i * 12 + 2]; }
+  int is, js, ks;
+  const bool ok = node_stencil(m, nx, ny, nz, is, js, ks);
+  TouchTiles t;
+  t.begin(part, is, js, ks, ok, ntx, nty, (int)tile0, slot, list != nullptr, mark);
+  if (part == 0) {
+    if (have) {
+      st[i * 3 + 0] = is; st[i * 3 + 1] = js; st[i * 3 + 2] = ks;
+      if (!ok) set_error(err, -3, step);
+    }
+    chunk_box_reduce(i, S, chunk_box, super, is, js, ks, ok);
+  }
+  if (have) delta_factors(W + i * 12, m, part, is, js, ks);
+  if (list) t.finish(slot, list, count);
 }
 
 /* Deterministic compaction of the marked tiles, in tile-index order:
@@ -461,14 +483,14 @@ constexpr int kGatherTPB = 128;
 constexpr int kGatherWarps = kGatherTPB / 32;
 constexpr int kHitCap = 256;     /* chunks whose box meets the tile  */
 constexpr int kOffHits = 64;     /* of those, with the starts kept   */
+constexpr int kHitsAhead = 4;
 constexpr int kListCap = 1024;   /* nodes whose stencil meets it     */
 constexpr int kBatch = 64;       /* nodes staged at once             */
 
 /* A staged node: its x, y and z delta weights at the tile's four cell
  * positions per axis (unset where the stencil misses the position: no cell
- * it covers reads them), then its force.  An odd stride of 15 doubles puts 16 different nodes in 16
- * different bank pairs. */
-constexpr int kNodeRec = 15;
+ * it covers reads them), then its force. */
+constexpr int kNodeRec = 16;
 
 struct GatherSmem {
   int hit[kHitCap];                     /* chunks in index order               */
@@ -478,7 +500,7 @@ struct GatherSmem {
   int ids[kListCap];                    /* the tile's nodes in index order     */
   int off[kListCap];                    /* their stencil starts from the tile's origin */
   unsigned cover[2][2][kBatch];         /* per staged node: cells of warp 0, 1 */
-  double rec[2][kBatch * kNodeRec];
+  alignas(16) double rec[2][kBatch * kNodeRec];
   int warp_n[kGatherWarps];
   int n;
 };
@@ -563,17 +585,27 @@ __device__ __forceinline__ int gather_list(GatherSmem& sm, const GatherNodes& g,
     }
   }
   if (nh > kHitCap) return -1;
-  for (int h = warp; h < nh; h += kGatherWarps) {
-    const long i = (long)sm.hit[h] * 32 + lane;
-    unsigned dx = 8u, dy = 8u, dz = 8u;   /* start - origin + 3: 0..6 where they meet */
-    if (i < g.S) {
-      const int* s = g.st + i * 3;
-      dx = (unsigned)(s[0] - x0 + 3); dy = (unsigned)(s[1] - y0 + 3); dz = (unsigned)(s[2] - z0 + 3);
+  /* kHitsAhead chunks of a warp at a time: their loads in flight together */
+  for (int h0 = warp; h0 < nh; h0 += kGatherWarps * kHitsAhead) {
+    unsigned o[kHitsAhead][3];
+#pragma unroll
+    for (int u = 0; u < kHitsAhead; ++u) {
+      const int h = h0 + u * kGatherWarps;
+      const long i = h < nh ? (long)sm.hit[h] * 32 + lane : g.S;
+      o[u][0] = o[u][1] = o[u][2] = 8u;   /* start - origin + 3: 0..6 where they meet */
+      if (i < g.S) {
+        const int* s = g.st + i * 3;
+        o[u][0] = (unsigned)(s[0] - x0 + 3); o[u][1] = (unsigned)(s[1] - y0 + 3); o[u][2] = (unsigned)(s[2] - z0 + 3);
+      }
     }
-    const bool in = dx < 7u && dy < 7u && dz < 7u;
-    const unsigned m = __ballot_sync(0xffffffffu, in);
-    if (lane == 0) sm.mask[h] = m;
-    if (h < kOffHits) sm.hoff[h][lane] = (unsigned short)(dx | dy << 4 | dz << 8);
+#pragma unroll
+    for (int u = 0; u < kHitsAhead; ++u) {
+      const int h = h0 + u * kGatherWarps;
+      const unsigned m = __ballot_sync(0xffffffffu, o[u][0] < 7u && o[u][1] < 7u && o[u][2] < 7u);
+      if (h >= nh) break;   /* uniform over the warp */
+      if (lane == 0) sm.mask[h] = m;
+      if (h < kOffHits) sm.hoff[h][lane] = (unsigned short)(o[u][0] | o[u][1] << 4 | o[u][2] << 8);
+    }
   }
   __syncthreads();
   if (warp == 0) {
@@ -696,7 +728,11 @@ union GatherShared {
  * cell's sum over the nodes in index order (cell = 16 z + 4 y + x).  Called
  * by all kGatherTPB threads.  Warps 2 and 3 stage the next 64 nodes while
  * warps 0 and 1 sum the last: each sum is a serial chain (its order is the
- * reference's), so latency is kept out of it. */
+ * reference's), so latency is kept out of it.  The 32 cells of a warp go
+ * through the nodes together, a lane adding those that cover its cell: at
+ * 128x64x64 (182 nodes on a tile, 64 of them on each cell) 21,000 cycles
+ * with each lane on its own list of covering nodes -- scattered shared
+ * memory reads, one long chain -- against TODO. */
 __device__ __forceinline__ void gather_tile(GatherShared& sh, const GatherNodes& g, int x0, int y0, int z0,
                                             double& Fx, double& Fy, double& Fz) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -721,36 +757,20 @@ __device__ __forceinline__ void gather_tile(GatherShared& sh, const GatherNodes&
       gather_stage(sm, g, L, b0 + kBatch, buf ^ 1);
       asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
-#pragma unroll 1
-      for (int j0 = 0; j0 < kBatch && b0 + j0 < L; j0 += 32) {
-        /* the warp's 32 x 32 cover bits (node j covers lane l's cell) are
-           transposed with five shuffle stages, so that each lane walks only
-           the nodes that cover its cell, in node order, two at a time */
-        unsigned x = b0 + j0 + lane < L ? sm.cover[buf][warp][j0 + lane] : 0u;
-#pragma unroll
-        for (int k = 16; k >= 1; k >>= 1) {
-          const unsigned M = k == 16 ? 0x0000FFFFu : k == 8 ? 0x00FF00FFu : k == 4 ? 0x0F0F0F0Fu
-                           : k == 2 ? 0x33333333u : 0x55555555u;
-          const unsigned y = __shfl_xor_sync(0xffffffffu, x, k);
-          x = (lane & k) ? (x & ~M) | ((y & ~M) >> k) : (x & M) | ((y & M) << k);
-        }
-        const double* rec = sm.rec[buf] + j0 * kNodeRec;
-        for (unsigned bits = x; bits;) {
-          const double* r = rec + (__ffs(bits) - 1) * kNodeRec;
-          bits &= bits - 1u;
-          const bool two = bits != 0u;
-          const double* q = two ? rec + (__ffs(bits) - 1) * kNodeRec : r;
-          bits &= bits - 1u;   /* 0 stays 0 */
-          const double tr = __dmul_rn(__dmul_rn(__dmul_rn(cf, r[ox]), r[oy]), r[oz]);
-          const double tq = __dmul_rn(__dmul_rn(__dmul_rn(cf, q[ox]), q[oy]), q[oz]);
-          Fx = __dadd_rn(Fx, __dmul_rn(r[12], tr));
-          Fy = __dadd_rn(Fy, __dmul_rn(r[13], tr));
-          Fz = __dadd_rn(Fz, __dmul_rn(r[14], tr));
-          if (two) {
-            Fx = __dadd_rn(Fx, __dmul_rn(q[12], tq));
-            Fy = __dadd_rn(Fy, __dmul_rn(q[13], tq));
-            Fz = __dadd_rn(Fz, __dmul_rn(q[14], tq));
-          }
+      const double* rec = sm.rec[buf];
+      const unsigned* cov = sm.cover[buf][warp];
+      const int n = min(kBatch, L - b0);
+#pragma unroll 4
+      for (int k = 0; k < n; ++k) {
+        const double* r = rec + k * kNodeRec;
+        const double2 fxy = *reinterpret_cast<const double2*>(r + 12);
+        const double fz = r[14];
+        const double tmp = __dmul_rn(__dmul_rn(__dmul_rn(cf, r[ox]), r[oy]), r[oz]);
+        const double ax = __dmul_rn(fxy.x, tmp), ay = __dmul_rn(fxy.y, tmp), az = __dmul_rn(fz, tmp);
+        if ((cov[k] >> lane) & 1u) {
+          Fx = __dadd_rn(Fx, ax);
+          Fy = __dadd_rn(Fy, ay);
+          Fz = __dadd_rn(Fz, az);
         }
       }
     }
@@ -805,8 +825,8 @@ __device__ __forceinline__ void move_node(double* __restrict__ nodes, const doub
 /* A move CTA: the 32 nodes of a chunk, four warps. */
 constexpr int kMoveTPB = 128;
 /* Cells a CTA's staged move holds in shared memory: the union box of its 32
- * nodes' stencils (along a fiber row ~5 x 20 x 5 cells); a larger union (a
- * chunk straddling two rows, a crumpled sheet) takes move_node. */
+ * nodes' stencils (along a fiber row ~5 x 20 x 5 cells); a group of nodes
+ * with a larger union (a crumpled sheet) takes move_node. */
 constexpr int kMoveCap = 640;
 constexpr int kMoveTiles = 64;   /* tiles of the union box whose slots are staged */
 
@@ -824,39 +844,50 @@ struct MoveSmem {
  * overlap by 3 cells of 4).  A node's sum is a serial chain of 64 terms, so
  * a thread holds one component only; with one warp that staged and summed
  * all three for its nodes the launch took 10 us at 16 x 16 nodes, this 6.
- * Called by all kMoveTPB threads; ends with a barrier. */
+ * Nodes whose stencils lie too far apart for one box (a chunk that straddles
+ * two rows of its sheet) are taken in groups near one another.  Called by
+ * all kMoveTPB threads; ends with a barrier. */
 __device__ __forceinline__ void move_chunk(MoveSmem& sm, double* __restrict__ nodes, const double* __restrict__ W,
                                            const int* __restrict__ st, long i, bool live, int ntx, int nty,
                                            const int* __restrict__ slot, const double* __restrict__ Utile, double dt) {
   const int t = threadIdx.x, warp = t >> 5;
   int is = 0, js = 0, ks = 0;
-  if (live) { is = st[i * 3 + 0]; js = st[i * 3 + 1]; ks = st[i * 3 + 2]; }
-  const int x0 = __reduce_min_sync(0xffffffffu, live ? is : INT_MAX), x1 = __reduce_max_sync(0xffffffffu, live ? is + 3 : INT_MIN);
-  const int y0 = __reduce_min_sync(0xffffffffu, live ? js : INT_MAX), y1 = __reduce_max_sync(0xffffffffu, live ? js + 3 : INT_MIN);
-  const int z0 = __reduce_min_sync(0xffffffffu, live ? ks : INT_MAX), z1 = __reduce_max_sync(0xffffffffu, live ? ks + 3 : INT_MIN);
-  if (x0 > x1) {   /* no live node: uniform over the CTA */
-    __syncthreads();
-    return;
+  double w[12], at = 0.0;
+  if (live) {
+    is = st[i * 3 + 0]; js = st[i * 3 + 1]; ks = st[i * 3 + 2];
+    if (warp < 3) {   /* the weights this thread will need, on their way while the box is staged */
+      const double2* p = reinterpret_cast<const double2*>(W + i * 12);
+#pragma unroll
+      for (int a = 0; a < 6; ++a) { w[2 * a] = p[a].x; w[2 * a + 1] = p[a].y; }
+      at = nodes[i * 12 + warp];
+    }
   }
+  /* every warp holds the same 32 stencils, so what follows is uniform over
+     the CTA */
+  unsigned left = __ballot_sync(0xffffffffu, live);
+  bool now = live;   /* the lane's node is in the group being moved */
+  while (left) {
+  const int x0 = __reduce_min_sync(0xffffffffu, now ? is : INT_MAX), x1 = __reduce_max_sync(0xffffffffu, now ? is + 3 : INT_MIN);
+  const int y0 = __reduce_min_sync(0xffffffffu, now ? js : INT_MAX), y1 = __reduce_max_sync(0xffffffffu, now ? js + 3 : INT_MIN);
+  const int z0 = __reduce_min_sync(0xffffffffu, now ? ks : INT_MAX), z1 = __reduce_max_sync(0xffffffffu, now ? ks + 3 : INT_MIN);
   const int bx = x1 - x0 + 1, by = y1 - y0 + 1, bz = z1 - z0 + 1;
   const long vol = (long)bx * by * bz;
   const int tx0 = x0 >> 2, ty0 = y0 >> 2, tz0 = z0 >> 2;
   const int tbx = (x1 >> 2) - tx0 + 1, tby = (y1 >> 2) - ty0 + 1;
   const long ntb = (long)tbx * tby * ((z1 >> 2) - tz0 + 1);
-  if (vol > kMoveCap || ntb > kMoveTiles) {   /* uniform over the CTA */
-    if (live && warp == 0) move_node(nodes, W, st, i, ntx, nty, slot, Utile, dt);
-    __syncthreads();
-    return;
-  }
-  /* the weights this thread will need, on their way while the box is staged */
-  double w[12];
-  double at = 0.0;
-  if (live && warp < 3) {
-    const double2* p = reinterpret_cast<const double2*>(W + i * 12);
-#pragma unroll
-    for (int a = 0; a < 6; ++a) { w[2 * a] = p[a].x; w[2 * a + 1] = p[a].y; }
-    at = nodes[i * 12 + warp];
-  }
+  if (vol > kMoveCap || ntb > kMoveTiles) {
+    /* too large: the nodes near the first one, or if that is this group
+       already, each on its own */
+    const int f = __ffs(left) - 1;
+    const int fx = __shfl_sync(0xffffffffu, is, f), fy = __shfl_sync(0xffffffffu, js, f),
+              fz = __shfl_sync(0xffffffffu, ks, f);
+    const bool near = ((left >> (t & 31)) & 1u) && abs(is - fx) <= 16 && abs(js - fy) <= 16 && abs(ks - fz) <= 16;
+    if (__any_sync(0xffffffffu, near != now)) {
+      now = near;
+      continue;
+    }
+    if (now && warp == 0) move_node(nodes, W, st, i, ntx, nty, slot, Utile, dt);
+  } else {
   /* the slots of the box's tiles first (at most 3 x 7 x 3 for a box that
      fits), so that the cell loads below depend on one shared-memory read */
   if (t < (int)ntb) {
@@ -887,7 +918,7 @@ __device__ __forceinline__ void move_chunk(MoveSmem& sm, double* __restrict__ no
     sm.U[0][j] = vx; sm.U[1][j] = vy; sm.U[2][j] = vz;
   }
   __syncthreads();
-  if (live && warp < 3) {
+  if (now && warp < 3) {
     const double c_64 = 1.0 / (6.4e1);
     const double* u = sm.U[warp] + (is - x0) * sx + (js - y0) * sy + (ks - z0) * sz;
     double s = 0;
@@ -900,7 +931,11 @@ __device__ __forceinline__ void move_chunk(MoveSmem& sm, double* __restrict__ no
           s += u[i2 * sx + j2 * sy + k2 * sz] * w[i2] * w[4 + j2] * w[8 + k2] * c_64;
     nodes[i * 12 + warp] = at + dt * s;
   }
+  }
+  left &= ~__ballot_sync(0xffffffffu, now);
+  now = (left >> (t & 31)) & 1u;
   __syncthreads();
+  }
 }
 
 }  // namespace lbib

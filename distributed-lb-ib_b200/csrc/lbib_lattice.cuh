@@ -44,6 +44,27 @@
 
 namespace lbib {
 
+/* Division of n < 2^31 by a fixed d in [1, 2^31) with one multiply-high and
+ * one add (the round-up method for invariant divisors, Granlund and
+ * Montgomery 1994): l = ceil(log2 d), m = floor(2^32 (2^l - d) / d) + 1,
+ * n / d = (umulhi(n, m) + n) >> l.  The kernels' thread indices are below
+ * 2^31, and a 64-bit division costs tens of instructions per thread. */
+struct FastDiv {
+  unsigned d, m, l;
+};
+
+__host__ __forceinline__ FastDiv fast_div(unsigned d) {
+  FastDiv f;
+  unsigned l = 0;
+  while ((1ull << l) < d) ++l;
+  f.d = d;
+  f.l = l;
+  f.m = (unsigned)((((1ull << 32) * ((1ull << l) - d)) / d) + 1);
+  return f;
+}
+
+__device__ __forceinline__ unsigned fdiv(unsigned n, const FastDiv& f) { return (__umulhi(n, f.m) + n) >> f.l; }
+
 /* cube_pthread/lbm_ib.c:777-833 */
 __host__ __device__ constexpr int cx(int q) {
   return (q == 1 || q == 7 || q == 9 || q == 15 || q == 17) ? 1
@@ -110,6 +131,7 @@ struct FluidParamsT {
   double rho0, ux0;      /* moments of the plane cells and the tables (the inflow)     */
   double ux_rest;        /* initial u_x of the cells x in [3, nx-4]: ux0, 0 from rest  */
   double omtau, invtau, kw0, kw1, kw2, cs2, cs4, half_dt, g;
+  double cs2_inv, cs4_inv;   /* 1/cs2, 1/cs4 for div_const, or 0 */
   const int* slot_cur;   /* F(t) tiles */
   const double* Fcur;
   const int* slot_prev;  /* (rho, u)(t-1) tiles */
@@ -313,6 +335,22 @@ __device__ __forceinline__ void velocity_dots(R ux, R uy, R uz, R cu[19]) {
  * and BGK relaxation, in place on f.  With a force the Guo term is added as
  * written there (true divisions by cs^2 and cs^4); without one that term is
  * +-0 in the reference and is skipped. */
+/* a / c, correctly rounded, for a constant c with y = 1/c rounded to nearest:
+ * q = a y, the residual a - c q by FMA, q + y times that (Markstein, "Computation
+ * of elementary functions on the IBM RISC System/6000 processor", 1990).  It is
+ * the rounded quotient when q is within one ulp of it and the residual is
+ * exact: the first holds if |c y - 1| < 2^-54 (the host checks it and passes
+ * y = 0 otherwise), the second away from overflow and underflow; other
+ * operands, zeros apart, take the division.  A forced cell divides 38
+ * times: 14,000 cycles of its CTA's 46,000 were the collision, mostly
+ * divisions, this way TODO. */
+__device__ __forceinline__ double div_const(double a, double c, double y) {
+  const double m = fabs(a);
+  if (y == 0.0 || !(m < 0x1p900) || (m < 0x1p-900 && m != 0.0)) return a / c;
+  const double q = __dmul_rn(a, y);
+  return __fma_rn(__fma_rn(-q, c, a), y, q);
+}
+
 /* Guo forcing term of direction q as lbm_ib.c:1740-1754 writes it. */
 template <typename R, typename P>
 __device__ __forceinline__ R guo(int q, R ux, R uy, R uz, R Fx, R Fy, R Fzg, const P& p) {
@@ -321,7 +359,7 @@ __device__ __forceinline__ R guo(int q, R ux, R uy, R uz, R Fx, R Fy, R Fzg, con
   const R A = (c0 - ux) * Fx + (c1 - uy) * Fy + (c2 - uz) * Fzg;
   const R B = c0 * ux + c1 * uy + c2 * uz;
   const R C = c0 * Fx + c1 * Fy + c2 * Fzg;
-  return kw * (A / (R)p.cs2 + B / (R)p.cs4 * C);
+  return kw * (div_const(A, (R)p.cs2, p.cs2_inv) + div_const(B, (R)p.cs4, p.cs4_inv) * C);
 }
 
 template <typename R>

@@ -167,27 +167,6 @@ struct Word {
   }
 };
 
-/* Division of n < 2^31 by a fixed d in [1, 2^31) with one multiply-high and
- * one add (the round-up method for invariant divisors, Granlund and
- * Montgomery 1994): l = ceil(log2 d), m = floor(2^32 (2^l - d) / d) + 1,
- * n / d = (umulhi(n, m) + n) >> l.  The kernels' thread indices are below
- * 2^31, and a 64-bit division costs tens of instructions per thread. */
-struct FastDiv {
-  unsigned d, m, l;
-};
-
-__host__ __forceinline__ FastDiv fast_div(unsigned d) {
-  FastDiv f;
-  unsigned l = 0;
-  while ((1ull << l) < d) ++l;
-  f.d = d;
-  f.l = l;
-  f.m = (unsigned)((((1ull << 32) * ((1ull << l) - d)) / d) + 1);
-  return f;
-}
-
-__device__ __forceinline__ unsigned fdiv(unsigned n, const FastDiv& f) { return (__umulhi(n, f.m) + n) >> f.l; }
-
 template <typename T>
 struct WordsParams {
   FluidParamsT<T> p;
