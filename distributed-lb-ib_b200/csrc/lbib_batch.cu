@@ -75,29 +75,6 @@ __global__ void __launch_bounds__(192, 4) lbib_b_node_prep(double* __restrict__ 
                  list, count, nullptr, err + 2 * k, *step_no);
 }
 
-/* Every listed tile of the batch: its force into its slot. */
-__global__ void __launch_bounds__(kGatherTPB) lbib_b_gather(GatherNodes g, const int* __restrict__ list,
-                                                            const int* __restrict__ count,
-                                                            const int* __restrict__ tile_inst,
-                                                            const BatchDesc* __restrict__ D,
-                                                            double* __restrict__ Ftile, const int* err) {
-  __shared__ GatherShared sm;
-  const int n = *count;
-  for (int it = blockIdx.x; it < n; it += gridDim.x) {
-    const int k = tile_inst[list[it]];
-    if (*(volatile const int*)(err + 2 * k)) continue;
-    const BatchDesc& d = D[k];
-    const int tile = (int)(list[it] - d.tile0);
-    double Fx, Fy, Fz;
-    gather_tile(sm, batch_nodes(g, d), tile % d.ntx * 4, tile / d.ntx % d.nty * 4, tile / (d.ntx * d.nty) * 4, Fx, Fy,
-                Fz);
-    if (threadIdx.x < 64) {
-      double* Ft = Ftile + (long)it * 192;
-      Ft[threadIdx.x] = Fx; Ft[64 + threadIdx.x] = Fy; Ft[128 + threadIdx.x] = Fz;
-    }
-  }
-}
-
 /* The move, a CTA per 32-node chunk of one problem (move_chunk); a pinned
  * leading row stays. */
 __global__ void __launch_bounds__(kMoveTPB) lbib_b_move(double* __restrict__ nodes, const double* __restrict__ W,
@@ -118,29 +95,31 @@ __global__ void __launch_bounds__(kMoveTPB) lbib_b_move(double* __restrict__ nod
   move_chunk(sm, nodes, W, st, i, live, d.ntx, d.nty, slot + d.tile0, Utile, d.dt);
 }
 
-/* FP64 rows away from the walls: the two-cell step over runs of blocks of 128
- * pairs of a problem's (row, pair) range, the parameters in shared memory. */
+/* FP64 rows away from the walls: the two-cell step, a block per 128 pairs of
+ * a problem's (row, pair) range, the parameters in shared memory; the tiles
+ * that carry force are stepped with their gather, so that the forced
+ * collision and its registers are not in this kernel (415 us per step at 24
+ * problems with them, TODO without). */
 template <int PAR>
-__global__ void __launch_bounds__(128, 3) lbib_b_x2(const FluidParams* __restrict__ P, const int4* __restrict__ blk,
-                                                    const int* __restrict__ err) {
-  __shared__ __align__(16) FluidParams sp;
+__global__ void __launch_bounds__(128, 3) lbib_b_x2(const WordsParams<double>* __restrict__ WP,
+                                                    const int4* __restrict__ blk, const int* __restrict__ err) {
+  __shared__ __align__(16) WordsParams<double> sb;
   const int4 m = blk[blockIdx.x];
   if (err[2 * m.x]) return;
-  block_copy(sp, P + m.x);
-  const int npairs = (sp.xhi - sp.xlo + 1) / 2, nry = sp.ny - 6;
-  const int rows = nry * x2_rows_z(sp.nz, sp.zin_hi);
-#pragma unroll 1
-  for (int j = 0; j < m.z; ++j) {
-    const int g = (m.y + j) * 128 + threadIdx.x, row = g / npairs;
-    if (row >= rows) return;
-    x2_pair<PAR>(sp, sp.xlo + 2 * (g - row * npairs), 3 + row % nry, 3 + row / nry);
-  }
+  block_copy(sb, WP + m.x);
+  const FluidParams& sp = sb.p;
+  const int npairs = sb.gpr, nry = sb.nry;
+  const unsigned g = (unsigned)m.y * 128 + threadIdx.x, row = fdiv(g, sb.dgpr);
+  if (row >= (unsigned)sb.nrows) return;
+  const unsigned z = fdiv(row, sb.dnry);
+  x2_pair<PAR, true>(sp, sp.xlo + 2 * (int)(g - row * npairs), 3 + (int)(row - z * nry), 3 + (int)z);
 }
 
 template <int PAR>
 int rest_f64_t(const BatchFluid& f) {
   const FluidParams* P = static_cast<const FluidParams*>(f.P);
-  if (f.nxblk > 0) lbib_b_x2<PAR><<<(unsigned)f.nxblk, 128, 0, f.stream>>>(P, f.xblk, f.err);
+  if (f.nxblk > 0)
+    lbib_b_x2<PAR><<<(unsigned)f.nxblk, 128, 0, f.stream>>>(static_cast<const WordsParams<double>*>(f.WP), f.xblk, f.err);
   if (f.nrblk > 0) lbib_b_rows<double, PAR><<<(unsigned)f.nrblk, 128, 0, f.stream>>>(P, f.rowyz, f.rblk, f.err);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -148,6 +127,17 @@ int rest_f64_t(const BatchFluid& f) {
 }  // namespace
 
 namespace lbib {
+
+int batch_gather_f64(const BatchFluid& f) {
+  const FluidParams* P = static_cast<const FluidParams*>(f.P);
+  if (f.par == 0)
+    lbib_b_gather_step<double, 0><<<f.grid_tiles, kGatherTPB, 0, f.stream>>>(P, f.desc, f.nodes, f.list, f.count,
+                                                                             f.tile_inst, f.Ftile, f.err);
+  else
+    lbib_b_gather_step<double, 1><<<f.grid_tiles, kGatherTPB, 0, f.stream>>>(P, f.desc, f.nodes, f.list, f.count,
+                                                                             f.tile_inst, f.Ftile, f.err);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
 
 int batch_rows_f64(const BatchFluid& f) { return f.par ? rest_f64_t<1>(f) : rest_f64_t<0>(f); }
 
@@ -315,6 +305,10 @@ void fill_tables(lbib_batch* b, int c, int first, void* P, void* WP) {
     if (lbdev_bulk_rows(d, &nry, &nrz)) {
       const int V = is_lp(b) ? batch_variant_cells_lp(b->prec, b->variant[k]) : 2;
       words_geometry(w[k], V, d->nx, nry, nrz);
+      if (!is_lp(b)) {   /* the pairs x = 2 .. nx-3 of a row */
+        w[k].gpr = (d->nx - 4) / 2;
+        w[k].dgpr = fast_div((unsigned)w[k].gpr);
+      }
     } else {
       memset(&w[k].nry, 0, sizeof(WordsParams<T>) - offsetof(WordsParams<T>, nry));
     }
@@ -392,7 +386,7 @@ int build_word_blocks(lbib_batch* b) {
  * also step the plane-adjacent cells, come from build_word_blocks). */
 int build_rows(lbib_batch* b) {
   const int lp = is_lp(b);
-  long n = 0, nr = 0, nxb = 0, pair_blocks = 0;
+  long n = 0, nr = 0, nxb = 0;
   for (int k = 0; k < b->B; ++k) {
     const lbib_device* d = b->sh[k];
     int ry = 0, rz = 0;
@@ -400,13 +394,7 @@ int build_rows(lbib_batch* b) {
     const long rows = (long)(d->ny - 4) * (d->nz - 4) - (bulk ? (long)ry * rz : 0);
     n += rows;
     nr += (rows * (d->nx - 4) + 127) / 128;
-    if (bulk && !lp) pair_blocks += ((long)ry * rz * ((d->nx - 4) / 2) + 127) / 128;
-  }
-  const int run = run_length(pair_blocks);
-  for (int k = 0; k < b->B && !lp; ++k) {
-    int ry = 0, rz = 0;
-    if (b->h_desc[k].bulk && lbdev_bulk_rows(b->sh[k], &ry, &rz))
-      nxb += run_count(((long)ry * rz * ((b->sh[k]->nx - 4) / 2) + 127) / 128, run);
+    if (bulk && !lp) nxb += ((long)ry * rz * ((d->nx - 4) / 2) + 127) / 128;
   }
   int2* h = (int2*)malloc(sizeof(int2) * (n ? n : 1));
   int4* rb = (int4*)malloc(sizeof(int4) * (nr ? nr : 1));
@@ -426,7 +414,7 @@ int build_rows(lbib_batch* b) {
       }
     const long rows = r - r0;
     for (long j = 0; j < (rows * (d->nx - 4) + 127) / 128; ++j) rb[ir++] = make_int4(k, (int)r0, (int)rows, (int)j);
-    if (bulk && !lp) ix += fill_runs(xo + ix, k, ((long)ry * rz * ((d->nx - 4) / 2) + 127) / 128, run);
+    if (bulk && !lp) ix += fill_runs(xo + ix, k, ((long)ry * rz * ((d->nx - 4) / 2) + 127) / 128, 1);
   }
   b->nrblk = nr;
   b->nxblk = nxb;
@@ -487,8 +475,7 @@ int batch_step(lbib_batch* b) {
   if (is_lp(b)) {
     if (batch_gather_lp(f)) return -2;
   } else {
-    lbib_b_gather<<<b->grid_tiles, kGatherTPB, 0, s>>>(f.nodes, f.list, f.count, b->tile_inst, b->desc, b->Ftile[c],
-                                                       b->err);
+    if (batch_gather_f64(f)) return -2;
   }
   b->launches++;
   if (is_lp(b)) {

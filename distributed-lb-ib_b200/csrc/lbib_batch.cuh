@@ -113,11 +113,11 @@ __device__ __forceinline__ GatherNodes batch_nodes(GatherNodes g, const BatchDes
 }
 
 /* Every listed tile: its spread force into its slot, and the step of its
- * cells in the word kernel's range (which leaves them out), by the CTA that
- * has just written the force.  Launched before the word blocks and the
+ * cells in the word or pair kernel's range (which leaves them out), by the
+ * CTA that has just written the force.  Launched before the word blocks and the
  * generic rows, which read the forces of their own cells. */
 template <typename T, int PAR>
-__global__ void __launch_bounds__(kGatherTPB, 5) lbib_b_gather_step(const FluidParamsT<T>* __restrict__ P,
+__global__ void __launch_bounds__(kGatherTPB, sizeof(T) == 8 ? 4 : 5) lbib_b_gather_step(const FluidParamsT<T>* __restrict__ P,
                                                                     const BatchDesc* __restrict__ D, GatherNodes g,
                                                                     const int* __restrict__ list,
                                                                     const int* __restrict__ count,
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kGatherTPB, 5) lbib_b_gather_step(const FluidP
     Ft[t] = Fx; Ft[64 + t] = Fy; Ft[128 + t] = Fz;
     const FluidParamsT<T>& p = P[k];
     /* the thread reads back the force it has just written */
-    if (d.bulk) forced_cell<T, PAR>(p, tile, t, min(p.nz - 4, p.zin_hi));
+    if (d.bulk) forced_cell<T, PAR>(p, tile, t, min(p.nz - 4, p.zin_hi), sizeof(T) == 8 ? 2 : 4);
   }
 }
 

@@ -41,9 +41,10 @@ struct BatchFluid {
   int grid_tiles;          /* persistent grid for tile-list kernels */
 };
 
-/* The spread's gather, and in low precision the forced cells with it: before
- * everything that reads the forces. */
+/* The spread's gather and the forced cells: before everything else that reads
+ * the forces. */
 int batch_gather_lp(const BatchFluid& f);
+int batch_gather_f64(const BatchFluid& f);
 /* Generic rows (FP64: two-cell blocks too). */
 int batch_rows_lp(const BatchFluid& f);
 int batch_rows_f64(const BatchFluid& f);

@@ -206,8 +206,9 @@ struct Form<T, true> {
   }
 };
 
-/* One cell of I through the generic rules: load, moments, collision, store. */
-template <typename T, int PAR>
+/* One cell of I through the generic rules: load, moments, collision, store.
+ * FORCES false: the caller knows that the cell carries none. */
+template <typename T, int PAR, bool FORCES = true>
 __device__ __forceinline__ void step_cell(const FluidParamsT<T>& p, int x, int y, int z) {
   using R = typename Pop<T>::R;
   const long idx = sidx(p, x, y, z);
@@ -229,7 +230,7 @@ __device__ __forceinline__ void step_cell(const FluidParamsT<T>& p, int x, int y
   }
   /* box mode: a cell outside the box carries no force, and this step's
      tile map may still be under construction by the concurrent spread */
-  const int sc = (p.box && !in_box(p.box, x, y, z)) ? -1 : p.slot_cur[tile];
+  const int sc = !FORCES || (p.box && !in_box(p.box, x, y, z)) ? -1 : p.slot_cur[tile];
   if (sc >= 0) {
     const double* Ft = p.Fcur + (long)sc * 192;
     F::template collide<true>(f, m, (R)Ft[cell], (R)Ft[64 + cell], (R)Ft[128 + cell], p);
@@ -239,14 +240,14 @@ __device__ __forceinline__ void step_cell(const FluidParamsT<T>& p, int x, int y
   store_post<PAR>(p, x, y, z, idx, kind, f);
 }
 
-template <typename T, int PAR>
+template <typename T, int PAR, bool FORCES>
 __global__ void __launch_bounds__(128, LBIB_FLUID_MINB)
     lbib_fluid_step(FluidParamsT<T> p, const int2* __restrict__ rows) {
   const int x = blockIdx.y * blockDim.x + threadIdx.x + p.xlo;
   const int2 r = rows[blockIdx.x];
   if (x > p.xhi) return;
   if (p.box && in_box(p.box, x, r.x, r.y)) return;
-  step_cell<T, PAR>(p, x, r.x, r.y);
+  step_cell<T, PAR, FORCES>(p, x, r.x, r.y);
 }
 
 /* The tiles of a box, and its extents in x and y; an empty box (no node
@@ -588,8 +589,18 @@ int launch_step_rows_t(lbib_device* d, const FluidParamsT<T>& p) {
   if (d->nrows <= 0) return 0;
   dim3 block(128);
   dim3 grid((unsigned)d->nrows, (unsigned)((p.xhi - p.xlo + 1 + 127) / 128));
-  if (d->parity == 0) lbib_fluid_step<T, 0><<<grid, block, 0, d->fluid_stream>>>(p, (const int2*)d->rows);
-  else lbib_fluid_step<T, 1><<<grid, block, 0, d->fluid_stream>>>(p, (const int2*)d->rows);
+  /* box mode leaves the forced cells out (FP64: without their code, which
+     costs the rows at 128x64x64 TODO; the low-precision forms keep one body,
+     whose contraction into FMA must not differ between the modes) */
+  const int2* rows = (const int2*)d->rows;
+  if (sizeof(T) == 8 && p.box) {
+    if (d->parity == 0) lbib_fluid_step<T, 0, sizeof(T) != 8><<<grid, block, 0, d->fluid_stream>>>(p, rows);
+    else lbib_fluid_step<T, 1, sizeof(T) != 8><<<grid, block, 0, d->fluid_stream>>>(p, rows);
+  } else if (d->parity == 0) {
+    lbib_fluid_step<T, 0, true><<<grid, block, 0, d->fluid_stream>>>(p, rows);
+  } else {
+    lbib_fluid_step<T, 1, true><<<grid, block, 0, d->fluid_stream>>>(p, rows);
+  }
   d->kernel_launches++;
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

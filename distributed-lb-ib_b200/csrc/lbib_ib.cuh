@@ -866,6 +866,7 @@ __device__ __forceinline__ void move_chunk(MoveSmem& sm, double* __restrict__ no
      the CTA */
   unsigned left = __ballot_sync(0xffffffffu, live);
   bool now = live;   /* the lane's node is in the group being moved */
+  int reach = 16;
   while (left) {
   const int x0 = __reduce_min_sync(0xffffffffu, now ? is : INT_MAX), x1 = __reduce_max_sync(0xffffffffu, now ? is + 3 : INT_MIN);
   const int y0 = __reduce_min_sync(0xffffffffu, now ? js : INT_MAX), y1 = __reduce_max_sync(0xffffffffu, now ? js + 3 : INT_MIN);
@@ -876,14 +877,14 @@ __device__ __forceinline__ void move_chunk(MoveSmem& sm, double* __restrict__ no
   const int tbx = (x1 >> 2) - tx0 + 1, tby = (y1 >> 2) - ty0 + 1;
   const long ntb = (long)tbx * tby * ((z1 >> 2) - tz0 + 1);
   if (vol > kMoveCap || ntb > kMoveTiles) {
-    /* too large: the nodes near the first one, or if that is this group
-       already, each on its own */
-    const int f = __ffs(left) - 1;
-    const int fx = __shfl_sync(0xffffffffu, is, f), fy = __shfl_sync(0xffffffffu, js, f),
-              fz = __shfl_sync(0xffffffffu, ks, f);
-    const bool near = ((left >> (t & 31)) & 1u) && abs(is - fx) <= 16 && abs(js - fy) <= 16 && abs(ks - fz) <= 16;
-    if (__any_sync(0xffffffffu, near != now)) {
-      now = near;
+    /* too large: the nodes within `reach` of the first one, nearer and
+       nearer until the box fits, or, at the end, each on its own */
+    if (reach > 0) {
+      const int f = __ffs(left) - 1;
+      const int fx = __shfl_sync(0xffffffffu, is, f), fy = __shfl_sync(0xffffffffu, js, f),
+                fz = __shfl_sync(0xffffffffu, ks, f);
+      now = ((left >> (t & 31)) & 1u) && abs(is - fx) <= reach && abs(js - fy) <= reach && abs(ks - fz) <= reach;
+      reach >>= 1;
       continue;
     }
     if (now && warp == 0) move_node(nodes, W, st, i, ntx, nty, slot, Utile, dt);
@@ -934,6 +935,7 @@ __device__ __forceinline__ void move_chunk(MoveSmem& sm, double* __restrict__ no
   }
   left &= ~__ballot_sync(0xffffffffu, now);
   now = (left >> (t & 31)) & 1u;
+  reach = 16;
   __syncthreads();
   }
 }

@@ -567,10 +567,10 @@ __device__ __forceinline__ Word<__half, 4> smem_word(const uint16_t* w, int e0, 
 /* A cell of a forced tile inside the word kernel's range (bulk rows,
  * x in [4, nx-5]; zb = last bulk z row), by the generic per-cell rules. */
 template <typename T, int PAR>
-__device__ __forceinline__ void forced_cell(const FluidParamsT<T>& p, int tile, int cell, int zb) {
+__device__ __forceinline__ void forced_cell(const FluidParamsT<T>& p, int tile, int cell, int zb, int xlo = 4) {
   const int tx = tile % p.ntx, ty = (tile / p.ntx) % p.nty, tz = tile / (p.ntx * p.nty);
   const int x = tx * 4 + (cell & 3), y = ty * 4 + ((cell >> 2) & 3), z = tz * 4 + (cell >> 4);
-  if (y >= 3 && y <= p.ny - 4 && z >= 3 && z <= zb && x >= 4 && x <= p.nx - 5) step_cell<T, PAR>(p, x, y, z);
+  if (y >= 3 && y <= p.ny - 4 && z >= 3 && z <= zb && x >= xlo && x <= p.nx - 1 - xlo) step_cell<T, PAR>(p, x, y, z);
 }
 
 /* Cell k in {0..3} -> x in {2, 3, nx-4, nx-3} of bulk row r. */

@@ -32,6 +32,7 @@ __host__ __device__ inline int x2_rows_z(int nz, int zin_hi) {
 }
 
 /* Moments (previous step) and force of one cell, then the collision. */
+template <bool FORCES>
 __device__ __forceinline__ void x2_relax_cell(const FluidParams& p, int x, int y, int z, bool plane, double f[19]) {
   const int tile = tile_of(x, y, z, p.ntx, p.nty);
   const int cell = cell_in_tile(x, y, z);
@@ -49,7 +50,9 @@ __device__ __forceinline__ void x2_relax_cell(const FluidParams& p, int x, int y
       moments(f, 0.0, 0.0, 0.0, p.half_dt, p.g, rho, ux, uy, uz);
     }
   }
-  const int sc = p.box ? -1 : p.slot_cur[tile];   /* box mode: only unforced cells get here */
+  /* box mode, and where the pairs of touched tiles are left out: only
+     unforced cells get here */
+  const int sc = !FORCES || p.box ? -1 : p.slot_cur[tile];
   if (sc >= 0) {
     const double* Ft = p.Fcur + (long)sc * 192;
     collide<true>(f, rho, ux, uy, uz, Ft[cell], Ft[64 + cell], Ft[128 + cell], p);
@@ -72,7 +75,8 @@ __device__ __forceinline__ void x2_plane_table(const FluidParams& p, int y, int 
   }
 }
 
-/* The step of the pair (x, x+1) of row (y, z); x even.  In an odd step a
+/* The step of the pair (x, x+1) of row (y, z); x even.  LEAVE: pairs of tiles
+ * that carry force this step are left to another kernel.  In an odd step a
  * pair holding a plane cell runs the same loads and stores as every other
  * pair -- the plane cell's pulled values are then replaced by its table, and
  * its pushes that would leave I (c_x = -1 at x = 2, +1 at x = nx-3) go to
@@ -80,9 +84,10 @@ __device__ __forceinline__ void x2_plane_table(const FluidParams& p, int y, int 
  * holding it does not diverge into the per-cell rules (1.89 -> 1.79 ms per
  * FP64 step at 512x256x256).  Its even-step loads keep the per-cell rules,
  * which measured faster there (even-step fluid 1.75 -> 1.67 ms). */
-template <int PAR>
+template <int PAR, bool LEAVE = false>
 __device__ __forceinline__ void x2_pair(const FluidParams& p, int x, int y, int z) {
-  if (p.box && in_box(p.box, x, y, z)) return;    /* both cells share a tile (x even) */
+  /* both cells share a tile (x even) */
+  if (LEAVE ? p.slot_cur[tile_of(x, y, z, p.ntx, p.nty)] >= 0 : p.box && in_box(p.box, x, y, z)) return;
   const long idx = sidx(p, x, y, z);
   const bool pa = (x == 2), pb = (x + 1 == p.nx - 3);
   double* __restrict__ F = p.f;
@@ -106,8 +111,8 @@ __device__ __forceinline__ void x2_pair(const FluidParams& p, int x, int y, int 
     }
     if (pa || pb) x2_plane_table(p, y, z, pa, fa, fb);
   }
-  x2_relax_cell(p, x, y, z, pa, fa);
-  x2_relax_cell(p, x + 1, y, z, pb, fb);
+  x2_relax_cell<!LEAVE>(p, x, y, z, pa, fa);
+  x2_relax_cell<!LEAVE>(p, x + 1, y, z, pb, fb);
   if (PAR == 0) {
 #pragma unroll
     for (int q = 0; q < 19; ++q)
