@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(kMoveTPB) lbib_b_move(double* __restrict__ nod
  * a problem's (row, pair) range, the parameters in shared memory; the tiles
  * that carry force are stepped with their gather, so that the forced
  * collision and its registers are not in this kernel (415 us per step at 24
- * problems with them, TODO without). */
+ * problems with them, 252 without). */
 template <int PAR>
 __global__ void __launch_bounds__(128, 3) lbib_b_x2(const WordsParams<double>* __restrict__ WP,
                                                     const int4* __restrict__ blk, const int* __restrict__ err) {
@@ -116,10 +116,15 @@ __global__ void __launch_bounds__(128, 3) lbib_b_x2(const WordsParams<double>* _
 }
 
 template <int PAR>
-int rest_f64_t(const BatchFluid& f) {
-  const FluidParams* P = static_cast<const FluidParams*>(f.P);
+int pairs_f64_t(const BatchFluid& f) {
   if (f.nxblk > 0)
     lbib_b_x2<PAR><<<(unsigned)f.nxblk, 128, 0, f.stream>>>(static_cast<const WordsParams<double>*>(f.WP), f.xblk, f.err);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+template <int PAR>
+int rows_f64_t(const BatchFluid& f) {
+  const FluidParams* P = static_cast<const FluidParams*>(f.P);
   if (f.nrblk > 0) lbib_b_rows<double, PAR><<<(unsigned)f.nrblk, 128, 0, f.stream>>>(P, f.rowyz, f.rblk, f.err);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -139,7 +144,8 @@ int batch_gather_f64(const BatchFluid& f) {
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-int batch_rows_f64(const BatchFluid& f) { return f.par ? rest_f64_t<1>(f) : rest_f64_t<0>(f); }
+int batch_pairs_f64(const BatchFluid& f) { return f.par ? pairs_f64_t<1>(f) : pairs_f64_t<0>(f); }
+int batch_rows_f64(const BatchFluid& f) { return f.par ? rows_f64_t<1>(f) : rows_f64_t<0>(f); }
 
 int batch_tile_moments_f64(const BatchFluid& f) {
   const FluidParamsT<double>* P = static_cast<const FluidParamsT<double>*>(f.P);
@@ -247,6 +253,8 @@ void big_free(void* p) {
 struct lbib_batch {
   int B, prec, compat;
   cudaStream_t stream;
+  cudaStream_t side;             /* FP64: the pair kernel, beside the spread and the rows */
+  cudaEvent_t ev_prep, ev_bulk;
   lbib_device** sh;              /* host-only shadows, pointers into the pools */
   lbib_problem* prob;
   BatchDesc* h_desc;
@@ -468,28 +476,35 @@ int batch_step(lbib_batch* b) {
                                                        b->tile_slot[c], b->tile_list[c], b->tile_count[c], b->err, SP,
                                                        b->step_no, (b->compat & 1) != 0);
   b->launches += 1;
-  /* the fused fluid step */
+  /* the fused fluid step.  The word / pair kernels need this step's tile map
+     only, the gather steps the touched tiles' cells, the generic rows read
+     the forces.  FP64: the pairs run on the side stream beside gather and
+     rows (24 problems: 414 -> 403 us per step); in 16-bit storage that was
+     the slower order (128 problems: 1045 -> 1108 us), the word kernel being
+     bound by issue, not by memory */
   const void* P = first ? b->P_first : b->P[c];
   const void* WP = first ? b->WP_first : b->WP[c];
   BatchFluid f = fluid_args(b, par, P, WP, c);
   if (is_lp(b)) {
     if (batch_gather_lp(f)) return -2;
-  } else {
-    if (batch_gather_f64(f)) return -2;
-  }
-  b->launches++;
-  if (is_lp(b)) {
     for (int v = 0; v < MAXV; ++v)
       if (b->nwblk[v]) {
         if (batch_words_lp(f, v, b->wblk[v], b->nwblk[v])) return -2;
         b->launches++;
       }
     if (batch_rows_lp(f)) return -2;
-    b->launches += b->nrblk > 0;
   } else {
-    if (batch_rows_f64(f)) return -2;
-    b->launches += (b->nxblk > 0) + (b->nrblk > 0);
+    CK(cudaEventRecord(b->ev_prep, s));
+    CK(cudaStreamWaitEvent(b->side, b->ev_prep, 0));
+    f.stream = b->side;
+    if (batch_pairs_f64(f)) return -2;
+    b->launches += b->nxblk > 0;
+    CK(cudaEventRecord(b->ev_bulk, b->side));
+    f.stream = s;
+    if (batch_gather_f64(f) || batch_rows_f64(f)) return -2;
+    CK(cudaStreamWaitEvent(s, b->ev_bulk, 0));
   }
+  b->launches += 1 + (b->nrblk > 0);
   /* moments of the touched tiles, read by the next step and the move */
   BatchFluid g = fluid_args(b, par ^ 1, b->P[c], b->WP[c], c);
   if ((is_lp(b) ? batch_tile_moments_lp(g) : batch_tile_moments_f64(g))) return -2;
@@ -576,7 +591,14 @@ lbib_batch* lbib_batch_create(int n, const lbib_problem* problems, int precision
   if (!b->sh || !b->prob || !b->h_desc || !b->variant) rc = -5;
   if (!rc) memcpy(b->prob, problems, sizeof(lbib_problem) * n);
   for (int k = 0; k < n && !rc && t != LBIB_PREC_F64; ++k) b->variant[k] = batch_default_variant_lp(precision);
-  if (!rc && cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) rc = -2;
+  /* the spread and the rows take SMs ahead of the bulk beside them */
+  int prio_lo = 0, prio_hi = 0;
+  cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
+  if (!rc && (cudaStreamCreateWithPriority(&b->stream, cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
+              cudaStreamCreateWithPriority(&b->side, cudaStreamNonBlocking, prio_lo) != cudaSuccess ||
+              cudaEventCreateWithFlags(&b->ev_prep, cudaEventDisableTiming) != cudaSuccess ||
+              cudaEventCreateWithFlags(&b->ev_bulk, cudaEventDisableTiming) != cudaSuccess))
+    rc = -2;
   /* sizes and offsets */
   const size_t pb = pop_bytes(precision), rb = t == LBIB_PREC_F64 ? 8 : 4;
   long foff = 0, toff = 0, tile0 = 0, cap = 0, node0 = 0;
@@ -765,6 +787,9 @@ void lbib_batch_free(lbib_batch* b) {
   if (b->h_err) cudaFreeHost(b->h_err);
   cudaFree(b->desc); cudaFree(b->rowyz); cudaFree(b->rblk); cudaFree(b->xblk);
   for (int v = 0; v < MAXV; ++v) cudaFree(b->wblk[v]);
+  if (b->side) cudaStreamDestroy(b->side);
+  if (b->ev_prep) cudaEventDestroy(b->ev_prep);
+  if (b->ev_bulk) cudaEventDestroy(b->ev_bulk);
   if (b->stream) cudaStreamDestroy(b->stream);
   free(b->prob); free(b->h_desc); free(b->variant);
   free(b);

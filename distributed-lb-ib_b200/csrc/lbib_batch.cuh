@@ -40,12 +40,13 @@ struct BatchDesc {
   double bc, sc, sc2, ds1, ds2, dt;
 };
 
-/* A CTA's share of the pair and word kernels: a run of consecutive blocks of
- * one problem, {problem, first block, blocks, 0}.  Before its first load a
- * CTA waits for its item, the problem's error word and its parameters, one
- * after the other; with one block to a CTA that was a third of its life (FP64
- * pairs of 24 problems: 415 us per step against TODO).  Up to kRun blocks,
- * fewer where the batch would not fill the chip several times over. */
+/* A CTA's share of the word kernel: a run of consecutive blocks of one
+ * problem, {problem, first block, blocks, 0}.  Before its first load a CTA
+ * waits for its item, the problem's error word and its parameters, one after
+ * the other; runs took a 128-problem 16-bit step from 1130 to 1050 us.  Up to
+ * kRun blocks, fewer where the batch would not fill the chip several times
+ * over.  (The FP64 pair kernel lost by it, 415 -> 475 us at 24 problems: its
+ * loop spilled; its items have one block.) */
 constexpr int kRun = 8;
 inline int run_length(long blocks) {
   const long r = blocks / (148 * 24);
@@ -114,8 +115,8 @@ __device__ __forceinline__ GatherNodes batch_nodes(GatherNodes g, const BatchDes
 
 /* Every listed tile: its spread force into its slot, and the step of its
  * cells in the word or pair kernel's range (which leaves them out), by the
- * CTA that has just written the force.  Launched before the word blocks and the
- * generic rows, which read the forces of their own cells. */
+ * CTA that has just written the force.  Launched before the generic rows,
+ * which read the forces of their own cells. */
 template <typename T, int PAR>
 __global__ void __launch_bounds__(kGatherTPB, sizeof(T) == 8 ? 4 : 5) lbib_b_gather_step(const FluidParamsT<T>* __restrict__ P,
                                                                     const BatchDesc* __restrict__ D, GatherNodes g,
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(kGatherTPB, sizeof(T) == 8 ? 4 : 5) lbib_b_gat
     Ft[t] = Fx; Ft[64 + t] = Fy; Ft[128 + t] = Fz;
     const FluidParamsT<T>& p = P[k];
     /* the thread reads back the force it has just written */
-    if (d.bulk) forced_cell<T, PAR>(p, tile, t, min(p.nz - 4, p.zin_hi), sizeof(T) == 8 ? 2 : 4);
+    if (d.bulk) forced_cell<T, PAR>(p, tile, t, min(p.nz - 4, p.zin_hi));
   }
 }
 

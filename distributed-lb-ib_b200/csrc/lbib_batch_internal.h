@@ -45,9 +45,11 @@ struct BatchFluid {
  * the forces. */
 int batch_gather_lp(const BatchFluid& f);
 int batch_gather_f64(const BatchFluid& f);
-/* Generic rows (FP64: two-cell blocks too). */
+/* Generic rows. */
 int batch_rows_lp(const BatchFluid& f);
 int batch_rows_f64(const BatchFluid& f);
+/* FP64 two-cell blocks. */
+int batch_pairs_f64(const BatchFluid& f);
 /* Word-kernel items (problem, first block, blocks) of one variant; the
  * variant a problem starts with. */
 int batch_words_lp(const BatchFluid& f, int variant, const int4* blk, long nblk);

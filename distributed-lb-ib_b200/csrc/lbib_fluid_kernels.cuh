@@ -301,18 +301,20 @@ __global__ void __launch_bounds__(kGatherTPB, 4) lbib_spread_box(FluidParamsT<T>
     int kind = K_FAST;
     R f[19];
     Mom<R> m;
+    /* the moments of t - 1: before the gather, or in FP64 (where moving
+       arithmetic cannot change its rounding) after it, so that the
+       populations' latency passes behind the gather */
+    const int sp = in && !p.first ? p.slot_prev[tile] : -1;
+    auto moments = [&]() {
+      if (kind >= K_SEMI) F::initial(p, m);
+      else if (p.first) F::initial_bulk(p, m);
+      else if (sp >= 0) F::from_tile(p, p.Uprev + (long)sp * 256, cell, m);
+      else F::moments_free(f, p, m);
+    };
     if (in) {
       kind = classify(p, x, y, z);
       load_pre<PAR>(p, x, y, z, idx, kind, f);
-      if (kind >= K_SEMI) {
-        F::initial(p, m);
-      } else if (p.first) {
-        F::initial_bulk(p, m);
-      } else {
-        const int sp = p.slot_prev[tile];
-        if (sp >= 0) F::from_tile(p, p.Uprev + (long)sp * 256, cell, m);
-        else F::moments_free(f, p, m);
-      }
+      if (sizeof(T) != 8) moments();
     }
     if (slot >= 0) {
       double Fx, Fy, Fz;
@@ -321,8 +323,12 @@ __global__ void __launch_bounds__(kGatherTPB, 4) lbib_spread_box(FluidParamsT<T>
         double* Ft = Ftile + (long)slot * 192;
         Ft[cell] = Fx; Ft[64 + cell] = Fy; Ft[128 + cell] = Fz;
       }
-      if (in) F::template collide<true>(f, m, (R)Fx, (R)Fy, (R)Fz, p);
+      if (in) {
+        if (sizeof(T) == 8) moments();
+        F::template collide<true>(f, m, (R)Fx, (R)Fy, (R)Fz, p);
+      }
     } else if (in) {
+      if (sizeof(T) == 8) moments();
       F::template collide<false>(f, m, R(0), R(0), R(0), p);
     }
     if (in) store_post<PAR>(p, x, y, z, idx, kind, f);
@@ -590,7 +596,7 @@ int launch_step_rows_t(lbib_device* d, const FluidParamsT<T>& p) {
   dim3 block(128);
   dim3 grid((unsigned)d->nrows, (unsigned)((p.xhi - p.xlo + 1 + 127) / 128));
   /* box mode leaves the forced cells out (FP64: without their code, which
-     costs the rows at 128x64x64 TODO; the low-precision forms keep one body,
+     cost the rows at 128x64x64 11.2 against 8.2 us in odd steps; the low-precision forms keep one body,
      whose contraction into FMA must not differ between the modes) */
   const int2* rows = (const int2*)d->rows;
   if (sizeof(T) == 8 && p.box) {

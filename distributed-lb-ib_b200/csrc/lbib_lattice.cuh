@@ -340,74 +340,130 @@ __device__ __forceinline__ void velocity_dots(R ux, R uy, R uz, R cu[19]) {
  * of elementary functions on the IBM RISC System/6000 processor", 1990).  It is
  * the rounded quotient when q is within one ulp of it and the residual is
  * exact: the first holds if |c y - 1| < 2^-54 (the host checks it and passes
- * y = 0 otherwise), the second away from overflow and underflow; other
- * operands, zeros apart, take the division.  A forced cell divides 38
- * times: 14,000 cycles of its CTA's 46,000 were the collision, mostly
- * divisions, this way TODO. */
+ * y = 0 otherwise), the second away from overflow and underflow, a = 0
+ * included (div_safe).  A forced cell divided 38 times, now 28 this way;
+ * at 128x64x64 the divisions were most of the 14,000 cycles that a tile
+ * CTA's collision took of its 46,000 (now ~4,000). */
 __device__ __forceinline__ double div_const(double a, double c, double y) {
-  const double m = fabs(a);
-  if (y == 0.0 || !(m < 0x1p900) || (m < 0x1p-900 && m != 0.0)) return a / c;
   const double q = __dmul_rn(a, y);
   return __fma_rn(__fma_rn(-q, c, a), y, q);
 }
 
-/* Guo forcing term of direction q as lbm_ib.c:1740-1754 writes it. */
-template <typename R, typename P>
-__device__ __forceinline__ R guo(int q, R ux, R uy, R uz, R Fx, R Fy, R Fzg, const P& p) {
-  const R c0 = (R)cx(q), c1 = (R)cy(q), c2 = (R)cz(q);
-  const R kw = (R)((q == 0) ? p.kw0 : ((q <= 6) ? p.kw1 : p.kw2));
-  const R A = (c0 - ux) * Fx + (c1 - uy) * Fy + (c2 - uz) * Fzg;
-  const R B = c0 * ux + c1 * uy + c2 * uz;
-  const R C = c0 * Fx + c1 * Fy + c2 * Fzg;
-  return kw * (div_const(A, (R)p.cs2, p.cs2_inv) + div_const(B, (R)p.cs4, p.cs4_inv) * C);
+/* v is 0 or 2^-400 <= |v| < 2^400.  Where that holds for u and F, the
+ * dividends formed from them -- sums of u, of (c - u) F -- are 0 or between
+ * 2^-900 and 2^900. */
+__device__ __forceinline__ bool div_safe(double v) {
+  const unsigned h = (unsigned)__double2hiint(v) & 0x7fffffffu;
+  return h - 0x26F00000u < 0x32000000u || v == 0.0;
 }
 
+/* The Guo forcing term of direction q (lbm_ib.c:1740-1754),
+ *   kw (A / cs^2 + B / cs^4 C),  A = (c - u).F,  B = c.u,  C = c.F,
+ * with what directions share formed once: the products (c_d - u_d) F_d for
+ * c_d = -1, 0, 1 per axis, and B / cs^4 C per opposite pair (both signs
+ * change).  Dropping the products with c_d = 0 from B and C changes them by
+ * a signed zero at most. */
 template <typename R>
 struct Relax {
-  R ux, uy, uz, Fx, Fy, Fzg, t6, om, it;
+  R t6, om, it;
+  R px[3], py[3], pz[3];   /* (c_d - u_d) F_d, c_d = -1, 0, 1 */
 };
+
+/* The constants of a collision; cs2_inv, cs4_inv as div_const takes them. */
+template <typename R>
+struct CollideConst {
+  R om, it, kw0, kw1, kw2, cs2, cs4, cs2_inv, cs4_inv, g;
+};
+
+template <bool FAST>
+__device__ __forceinline__ double guo_div(double a, double c, double y) {
+  return FAST ? div_const(a, c, y) : a / c;
+}
 
 /* One opposite pair (qa, qb) with c_qa . u = cu: both equilibria share
  * 3cu, cu^2 and 1.5 u^2, and 1 + (-3cu) == 1 - 3cu exactly.  With a force
- * the Guo term is added after the relaxation, as the reference sums it. */
-template <bool FORCED, int QA, int QB, typename R, typename P>
-__device__ __forceinline__ void relax_pair(R* f, R cu, R wr, const Relax<R>& r, const P& p) {
+ * (c_qa . F = cF) the Guo term is added after the relaxation, as the
+ * reference sums it. */
+template <bool FORCED, bool FAST, int QA, int QB, typename R>
+__device__ __forceinline__ void relax_pair(R* f, R cu, R cF, R wr, const Relax<R>& r, const CollideConst<R>& p) {
   const R a3 = R(3.0) * cu;
   const R sq = R(4.5) * (cu * cu);
   const R ea = wr * (R(1.0) + a3 + sq - r.t6);
   const R eb = wr * (R(1.0) + (-a3) + sq - r.t6);
   R va = f[QA] * r.om + r.it * ea;
   R vb = f[QB] * r.om + r.it * eb;
-  if (FORCED) {
-    va = va + guo(QA, r.ux, r.uy, r.uz, r.Fx, r.Fy, r.Fzg, p);
-    vb = vb + guo(QB, r.ux, r.uy, r.uz, r.Fx, r.Fy, r.Fzg, p);
+  if constexpr (FORCED) {
+    const R kw = QA <= 6 ? p.kw1 : p.kw2;
+    const R bc = guo_div<FAST>(cu, p.cs4, p.cs4_inv) * cF;
+    const R Aa = r.px[cx(QA) + 1] + r.py[cy(QA) + 1] + r.pz[cz(QA) + 1];
+    const R Ab = r.px[cx(QB) + 1] + r.py[cy(QB) + 1] + r.pz[cz(QB) + 1];
+    va = va + kw * (guo_div<FAST>(Aa, p.cs2, p.cs2_inv) + bc);
+    vb = vb + kw * (guo_div<FAST>(Ab, p.cs2, p.cs2_inv) + bc);
   }
   f[QA] = va;
   f[QB] = vb;
 }
 
-template <bool FORCED, typename R, typename P>
-__device__ __forceinline__ void collide(R f[19], R rho, R ux, R uy, R uz, R Fx, R Fy, R Fz, const P& p) {
+template <bool FORCED, bool FAST, typename R>
+__device__ __forceinline__ void collide_body(R f[19], R rho, R ux, R uy, R uz, R Fx, R Fy, R Fz,
+                                             const CollideConst<R>& p) {
   Relax<R> r;
-  r.ux = ux; r.uy = uy; r.uz = uz;
-  r.Fx = Fx; r.Fy = Fy; r.Fzg = FORCED ? Fz + rho * (R)p.g : R(0);
+  const R Fzg = FORCED ? Fz + rho * p.g : R(0);
+  if constexpr (FORCED) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const R c = R(k - 1);
+      r.px[k] = (c - ux) * Fx;
+      r.py[k] = (c - uy) * Fy;
+      r.pz[k] = (c - uz) * Fzg;
+    }
+  }
   r.t6 = R(1.5) * (ux * ux + uy * uy + uz * uz);
-  r.om = (R)p.omtau; r.it = (R)p.invtau;
+  r.om = p.om; r.it = p.it;
   const R wr0 = R(1.0 / 3.0) * rho;
   const R wr1 = R(1.0 / 18.0) * rho;
   const R wr2 = R(1.0 / 36.0) * rho;
   R v0 = f[0] * r.om + r.it * (wr0 * (R(1.0) - r.t6));
-  if (FORCED) v0 = v0 + guo(0, ux, uy, uz, Fx, Fy, r.Fzg, p);
+  if constexpr (FORCED) v0 = v0 + p.kw0 * guo_div<FAST>(r.px[1] + r.py[1] + r.pz[1], p.cs2, p.cs2_inv);
   f[0] = v0;
-  relax_pair<FORCED, 1, 2>(f, ux, wr1, r, p);
-  relax_pair<FORCED, 3, 4>(f, uz, wr1, r, p);
-  relax_pair<FORCED, 6, 5>(f, uy, wr1, r, p);
-  relax_pair<FORCED, 7, 8>(f, ux + uz, wr2, r, p);
-  relax_pair<FORCED, 9, 10>(f, ux - uz, wr2, r, p);
-  relax_pair<FORCED, 11, 12>(f, uz - uy, wr2, r, p);
-  relax_pair<FORCED, 13, 14>(f, uy + uz, wr2, r, p);
-  relax_pair<FORCED, 15, 16>(f, ux - uy, wr2, r, p);
-  relax_pair<FORCED, 17, 18>(f, ux + uy, wr2, r, p);
+  relax_pair<FORCED, FAST, 1, 2>(f, ux, Fx, wr1, r, p);
+  relax_pair<FORCED, FAST, 3, 4>(f, uz, Fzg, wr1, r, p);
+  relax_pair<FORCED, FAST, 6, 5>(f, uy, Fy, wr1, r, p);
+  relax_pair<FORCED, FAST, 7, 8>(f, ux + uz, Fx + Fzg, wr2, r, p);
+  relax_pair<FORCED, FAST, 9, 10>(f, ux - uz, Fx - Fzg, wr2, r, p);
+  relax_pair<FORCED, FAST, 11, 12>(f, uz - uy, Fzg - Fy, wr2, r, p);
+  relax_pair<FORCED, FAST, 13, 14>(f, uy + uz, Fy + Fzg, wr2, r, p);
+  relax_pair<FORCED, FAST, 15, 16>(f, ux - uy, Fx - Fy, wr2, r, p);
+  relax_pair<FORCED, FAST, 17, 18>(f, ux + uy, Fx + Fy, wr2, r, p);
+}
+
+/* The collision of a forced cell by true divisions: operands that div_const
+ * does not take (not finite, or beyond any flow). */
+template <typename R>
+__device__ __noinline__ void collide_rare(R* f, R rho, R ux, R uy, R uz, R Fx, R Fy, R Fz, CollideConst<R> c) {
+  collide_body<true, false>(f, rho, ux, uy, uz, Fx, Fy, Fz, c);
+}
+
+template <bool FORCED, typename R, typename P>
+__device__ __forceinline__ void collide(R f[19], R rho, R ux, R uy, R uz, R Fx, R Fy, R Fz, const P& p) {
+  CollideConst<R> c;
+  c.om = (R)p.omtau; c.it = (R)p.invtau;
+  if constexpr (FORCED) {
+    c.kw0 = (R)p.kw0; c.kw1 = (R)p.kw1; c.kw2 = (R)p.kw2;
+    c.cs2 = (R)p.cs2; c.cs4 = (R)p.cs4; c.cs2_inv = p.cs2_inv; c.cs4_inv = p.cs4_inv; c.g = (R)p.g;
+    const R Fzg = Fz + rho * c.g;
+    if (!(div_safe(ux) && div_safe(uy) && div_safe(uz) && div_safe(Fx) && div_safe(Fy) && div_safe(Fzg) &&
+          c.cs2_inv != 0.0 && c.cs4_inv != 0.0)) {
+      R h[19];   /* a copy: f stays in registers on the other path */
+#pragma unroll
+      for (int q = 0; q < 19; ++q) h[q] = f[q];
+      collide_rare(h, rho, ux, uy, uz, Fx, Fy, Fz, c);
+#pragma unroll
+      for (int q = 0; q < 19; ++q) f[q] = h[q];
+      return;
+    }
+  }
+  collide_body<FORCED, true>(f, rho, ux, uy, uz, Fx, Fy, Fz, c);
 }
 
 /* Cell (x, y, z) lies in a tile of the box (box mode). */

@@ -564,13 +564,14 @@ __device__ __forceinline__ Word<__half, 4> smem_word(const uint16_t* w, int e0, 
   return o;
 }
 
-/* A cell of a forced tile inside the word kernel's range (bulk rows,
- * x in [4, nx-5]; zb = last bulk z row), by the generic per-cell rules. */
+/* A cell of a forced tile in the bulk rows (zb = the last in z), by the
+ * generic per-cell rules; the word and pair kernels and edge_cell leave it
+ * out. */
 template <typename T, int PAR>
-__device__ __forceinline__ void forced_cell(const FluidParamsT<T>& p, int tile, int cell, int zb, int xlo = 4) {
+__device__ __forceinline__ void forced_cell(const FluidParamsT<T>& p, int tile, int cell, int zb) {
   const int tx = tile % p.ntx, ty = (tile / p.ntx) % p.nty, tz = tile / (p.ntx * p.nty);
   const int x = tx * 4 + (cell & 3), y = ty * 4 + ((cell >> 2) & 3), z = tz * 4 + (cell >> 4);
-  if (y >= 3 && y <= p.ny - 4 && z >= 3 && z <= zb && x >= xlo && x <= p.nx - 1 - xlo) step_cell<T, PAR>(p, x, y, z);
+  if (y >= 3 && y <= p.ny - 4 && z >= 3 && z <= zb && x >= 2 && x <= p.nx - 3) step_cell<T, PAR>(p, x, y, z);
 }
 
 /* Cell k in {0..3} -> x in {2, 3, nx-4, nx-3} of bulk row r. */
@@ -578,7 +579,8 @@ template <typename T, int PAR>
 __device__ __forceinline__ void edge_cell(const FluidParamsT<T>& p, int nry, int r, int k) {
   const int y = 3 + r % nry, z = 3 + r / nry;
   const int x = k < 2 ? 2 + k : p.nx - 6 + k;
-  if (p.box && in_box(p.box, x, y, z)) return;
+  /* forced cells are stepped elsewhere: with the box, or by forced_cell */
+  if (p.box ? in_box(p.box, x, y, z) : p.slot_cur[tile_of(x, y, z, p.ntx, p.nty)] >= 0) return;
   step_cell<T, PAR>(p, x, y, z);
 }
 

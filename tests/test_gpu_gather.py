@@ -59,3 +59,14 @@ def test_five_pinned_sheets(gpu, oracle_built):
     sheets = [_sheet(9 + k, 11, 5.0 + 4 * k, 8.0, 6.0) for k in range(5)]
     case = P.Case(NX, NY, NZ, sheets, Ks_l=0.01, Kb_l=0.001, compat=P.COMPAT_ALL | 0x400)
     _run(case, [None] * 5, steps=5)
+
+
+@pytest.mark.parametrize("ks", [1e-150, 1e-305])
+def test_tiny_forces(gpu, oracle_built, ks):
+    """Forces too small for the divisions by a multiplication with the
+    reciprocal (residuals would underflow) take true divisions."""
+    rng = np.random.default_rng(3)
+    case = P.Case(NX, NY, NZ, [_sheet(12, 14, 12.0)], Ks_l=ks, Kb_l=ks / 10)
+    y, z = np.meshgrid(np.linspace(8, 30, 12), np.linspace(8, 34, 14), indexing="ij")
+    pos = np.stack([np.full_like(y, 12.0), y, z], axis=-1) + rng.uniform(-0.3, 0.3, y.shape + (3,))
+    _run(case, [pos])
