@@ -45,8 +45,8 @@ struct BatchDesc {
  * waits for its item, the problem's error word and its parameters, one after
  * the other; runs took a 128-problem 16-bit step from 1130 to 1050 us.  Up to
  * kRun blocks, fewer where the batch would not fill the chip several times
- * over.  (The FP64 pair kernel lost by it, 415 -> 475 us at 24 problems: its
- * loop spilled; its items have one block.) */
+ * over.  (The FP64 pair kernel lost by it, 415 -> 435 and 519 us in even and odd
+ * steps at 24 problems; its items have one block.) */
 constexpr int kRun = 8;
 inline int run_length(long blocks) {
   const long r = blocks / (148 * 24);

@@ -93,8 +93,9 @@ extern "C" int lbdev_launch_fluid_bulk(lbib_device* d, const void* fluid_params)
   /* a block per TPB pairs of a row keeps every warp on one row; where that
      leaves more than 5% of the threads without a pair (62 pairs in rows of
      128 cells: half), the rows are laid end to end instead.  us of the
-     kernel, per row / end to end: 9.3 / 7.2 at 64x32x32, 30 / 23 at
-     128x64x64, 36 / 22 at 100x55x75 */
+     kernel in even, odd steps, per row -> end to end: 9.3, 9.8 -> 7.2, 7.7
+     at 64x32x32, 29, 32 -> 23, 25 at 128x64x64, 34, 39 -> 19, 24 at
+     100x55x75 */
   const long pairs = (long)b.nry * nrz * b.npairs, slots = (long)grid.x * grid.y * TPB;
   b.flat = 0;
   if (pairs < 0.95 * slots && pairs + TPB < (1L << 31)) {

@@ -30,9 +30,9 @@ struct SheetForces {
  * when it has them, compute the nodes' fiber forces for the sheets `sf`
  * names (they read neighbours' positions and write the node's own force
  * fields only, so they run alongside).  list NULL: mark the tiles only.
- * Bound by the latency of one chunk's chain: 16,000 cycles with one warp for
- * the forces and one for all tiles after its cosines, 8,000 so; 10.7 -> 6.0
- * us a launch at 64x32x32, 22 -> 17.5 at 512x256x256. */
+ * Bound by the latency of one chunk's chain, 16,000 cycles when one warp took
+ * all of its tiles: 11.1 -> 6.1 us a launch at 64x32x32, 23 -> 17.4 at
+ * 512x256x256. */
 __global__ void __launch_bounds__(192, 4) lbib_node_prep(double* __restrict__ nodes, long S, int nx, int ny, int nz,
                                                       int ntx, int nty, double* __restrict__ W, int* __restrict__ st,
                                                       int* __restrict__ chunk_box, int* __restrict__ super,

@@ -341,9 +341,11 @@ __device__ __forceinline__ void velocity_dots(R ux, R uy, R uz, R cu[19]) {
  * the rounded quotient when q is within one ulp of it and the residual is
  * exact: the first holds if |c y - 1| < 2^-54 (the host checks it and passes
  * y = 0 otherwise), the second away from overflow and underflow, a = 0
- * included (div_safe).  A forced cell divided 38 times, now 28 this way;
- * at 128x64x64 the divisions were most of the 14,000 cycles that a tile
- * CTA's collision took of its 46,000 (now ~4,000). */
+ * included (div_safe).  A forced cell divided 38 times, now 28 this way.
+ * At 128x64x64 the collision was 14,000 of a tile CTA's 46,000 cycles, 5,500
+ * with a first form of this that checked each division; with the one check
+ * per cell, the hit loads ahead and the moments after the gather, the launch
+ * went on from 19.6 to 16.2 us (15.1 to 12.1 at 64x32x32). */
 __device__ __forceinline__ double div_const(double a, double c, double y) {
   const double q = __dmul_rn(a, y);
   return __fma_rn(__fma_rn(-q, c, a), y, q);
