@@ -28,6 +28,7 @@ int lbdev_launch_prep(lbib_device* d, int step);
 int lbdev_launch_spread(lbib_device* d, int step);
 int lbdev_launch_move(lbib_device* d);
 int lbdev_launch_stencil_box(lbib_device* d);
+int lbdev_launch_clear_tiles(lbib_device* d);
 int lbdev_launch_spread_box(lbib_device* d);
 int lbdev_launch_scatter_force(lbib_device* d, double* fx, double* fy, double* fz);
 }
@@ -227,13 +228,22 @@ extern "C" int lbdev_create(lbib_device** out, const lbdev_config* c) {
   d->l2_pf = pf ? atoi(pf) : 0;
   d->fluid_stream = d->stream;
   /* box-mode steps for a whole grid: 2 with the fluid's bulk beside the
-     spread (default), 1 in stream order, 0 off (LBIB_OVERLAP) */
+     spread, 3 beside the moments and the move too (lbdev_late_join), 1 in
+     stream order, 0 off (LBIB_OVERLAP).  Default 3 for the grids whose bulk
+     kernel outlasts the spread but not the whole chain: joining late saves
+     the wait, and costs the ring's tiles and a launch.  FP64, us per step 2 /
+     3: 37.2 / 39.1 at 64x32x32, 41.6 / 44.9 at 96x48x48, 47.4 / 47.2 at
+     100x55x75, 57.4 / 52.3 at 128x64x64, 92.9 / 83.8 at 128x128x64, 159.6 /
+     154.9 at 192x128x96, 251.4 / 249.7 at 256x128x128, 742 / 754 at
+     384x192x192, 1719 / 1749 at 512x256x256 */
   const char* ov = getenv("LBIB_OVERLAP");
-  d->overlap = lbdev_is_slab(d) ? 0 : (ov ? atoi(ov) : 2);
+  const long cells = (long)d->nx * d->ny * d->nz;
+  d->overlap = lbdev_is_slab(d) ? 0 : (ov ? atoi(ov) : cells >= 1L << 19 && cells <= 1L << 22 ? 3 : 2);
   if (d->overlap &&
       (cudaStreamCreateWithPriority(&d->side, cudaStreamNonBlocking, prio_lo) != cudaSuccess ||
        cudaEventCreateWithFlags(&d->ev_box, cudaEventDisableTiming) != cudaSuccess ||
        cudaEventCreateWithFlags(&d->ev_bulk, cudaEventDisableTiming) != cudaSuccess ||
+       cudaEventCreateWithFlags(&d->ev_spread, cudaEventDisableTiming) != cudaSuccess ||
        cudaMalloc(&d->box, sizeof(int) * 12) != cudaSuccess)) {
     lbdev_free(d);
     return -2;
@@ -299,6 +309,7 @@ extern "C" void lbdev_free(lbib_device* d) {
   if (d->side) cudaStreamDestroy(d->side);
   if (d->ev_box) cudaEventDestroy(d->ev_box);
   if (d->ev_bulk) cudaEventDestroy(d->ev_bulk);
+  if (d->ev_spread) cudaEventDestroy(d->ev_spread);
   cudaFree(d->box);
   if (d->stream) cudaStreamDestroy(d->stream);
   free(d);
@@ -466,7 +477,12 @@ static int prof_grow(lbib_device* d) {
  * 128x64x64, 1746 / 1721 at 512x256x256; 16-bit storage: 79 / 67 at
  * 128x64x64, 777 / 763 at 512x256x256.  (With the spread in six launches
  * instead of two, each of which had to find room among the bulk kernel's
- * blocks, side by side was the slower at 512x256x256.) */
+ * blocks, side by side was the slower at 512x256x256.)
+ * The streams join before the moments, whose cells' slots the bulk kernel
+ * may be writing, or, with a ring of tiles around the box (lbdev_late_join),
+ * after the move; the map of the step before, which the bulk kernel reads to
+ * its end, is then cleared behind it on the side stream and not by the
+ * moments. */
 static int step_overlapped(lbib_device* d, int step_no, cudaEvent_t* ev) {
   if (!d->nodes || !d->have_df1 || !d->have_inout) return -4;
   /* the box of this step's stencils: left by the previous step's move, or
@@ -480,7 +496,8 @@ static int step_overlapped(lbib_device* d, int step_no, cudaEvent_t* ev) {
   d->have_forces = 1;
   d->have_moments = 0;
   d->box_mode = 1;
-  const int conc = d->overlap == 2;
+  const int conc = d->overlap >= 2, late = lbdev_late_join(d);
+  d->late = late;
   int rc = 0;
   if (conc) {
     CK(cudaEventRecord(d->ev_box, d->stream));
@@ -490,7 +507,7 @@ static int step_overlapped(lbib_device* d, int step_no, cudaEvent_t* ev) {
     rc = lbdev_launch_fluid_step(d);
     if (ev) CK(cudaEventRecord(ev[7], d->side));
     d->fluid_stream = d->stream;
-    CK(cudaEventRecord(d->ev_bulk, d->side));
+    if (!late) CK(cudaEventRecord(d->ev_bulk, d->side));
   }
   /* the forces: in the node preparation's launch when the sheets allow */
   d->fuse_forces = lbdev_can_fuse_forces(d);
@@ -500,7 +517,13 @@ static int step_overlapped(lbib_device* d, int step_no, cudaEvent_t* ev) {
   d->fuse_forces = 0;
   if (!rc) rc = lbdev_launch_spread_box(d);
   if (ev) CK(cudaEventRecord(ev[2], d->stream));
-  if (conc) {
+  if (late) {
+    /* the old map has readers on both streams; its clearing leaves the chain */
+    CK(cudaEventRecord(d->ev_spread, d->stream));
+    CK(cudaStreamWaitEvent(d->side, d->ev_spread, 0));
+    if (!rc) rc = lbdev_launch_clear_tiles(d);
+    CK(cudaEventRecord(d->ev_bulk, d->side));
+  } else if (conc) {
     CK(cudaStreamWaitEvent(d->stream, d->ev_bulk, 0));
   } else {
     if (ev) CK(cudaEventRecord(ev[6], d->stream));
@@ -516,6 +539,8 @@ static int step_overlapped(lbib_device* d, int step_no, cudaEvent_t* ev) {
   if (ev) CK(cudaEventRecord(ev[4], d->stream));
   if (!rc) rc = lbdev_launch_move(d) ? -2 : 0;
   if (ev) CK(cudaEventRecord(ev[5], d->stream));
+  if (late) CK(cudaStreamWaitEvent(d->stream, d->ev_bulk, 0));
+  d->late = 0;
   /* the move reduced the next step's box into box_next */
   d->box_valid = !rc;
   if (d->box_valid) d->box_cur ^= 1;

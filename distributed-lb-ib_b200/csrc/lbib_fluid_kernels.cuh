@@ -616,7 +616,7 @@ int launch_tile_moments_t(lbib_device* d) {
   FluidParamsT<T> p = make_params_t<T>(d, 0);
   const int c = d->cur;
   const int blocks = 2371;   /* ~16 CTAs per SM; prime, as kBoxCtas */
-  int* old = lbdev_is_slab(d) ? nullptr : d->tile_slot[c ^ 1];
+  int* old = lbdev_is_slab(d) || d->late ? nullptr : d->tile_slot[c ^ 1];
   if (d->parity == 0)
     lbib_tile_moments<T, 0><<<blocks, 64, 0, d->stream>>>(p, d->tile_list[c], d->tile_count[c], d->Ftile[c], d->Utile[c],
                                                           old, d->tile_list[c ^ 1], d->tile_count[c ^ 1]);

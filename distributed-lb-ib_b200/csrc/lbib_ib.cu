@@ -86,13 +86,15 @@ struct PinnedRows {
 
 /* Nodes [i0, i1) of the concatenated sheets.  With `box` (a box-mode step's
  * next box), the box in tiles of the nodes' stencils, pinned ones included,
- * is reduced into it (a warp reduction, then six atomics per block). */
+ * and `ring` tiles around them, is reduced into it (a warp reduction, then
+ * six atomics per block). */
 __global__ void __launch_bounds__(kMoveTPB) lbib_move_nodes(double* __restrict__ nodes, const double* __restrict__ W,
                                                             const int* __restrict__ st, long i0, long i1, int ntx,
                                                             int nty, const int* __restrict__ slot,
                                                             const double* __restrict__ Utile, double dt,
-                                                            const int* err, int* __restrict__ box, int nx, int ny,
-                                                            int nz, int* __restrict__ old_count, PinnedRows pin) {
+                                                            const int* err, int* __restrict__ box, int ring, int nx,
+                                                            int ny, int nz, int* __restrict__ old_count,
+                                                            PinnedRows pin) {
   __shared__ MoveSmem sm;
   if (old_count && blockIdx.x == 0 && threadIdx.x == 0) *old_count = 0;   /* the next step's list starts empty */
   const long i = i0 + (long)blockIdx.x * 32 + (threadIdx.x & 31);
@@ -116,10 +118,24 @@ __global__ void __launch_bounds__(kMoveTPB) lbib_move_nodes(double* __restrict__
                     __reduce_min_sync(0xffffffffu, in ? ks >> 2 : INT_MAX),
                     __reduce_max_sync(0xffffffffu, in ? (ks + 3) >> 2 : INT_MIN)};
   if (threadIdx.x == 0 && b[0] <= b[1]) {
-    atomicMin(&box[0], b[0]); atomicMax(&box[1], b[1]);
-    atomicMin(&box[2], b[2]); atomicMax(&box[3], b[3]);
-    atomicMin(&box[4], b[4]); atomicMax(&box[5], b[5]);
+    const int t[6] = {b[0], b[1], b[2], b[3], b[4], b[5]};
+    const int n[3] = {(nx + 3) / 4, (ny + 3) / 4, (nz + 3) / 4};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      atomicMin(&box[2 * a], max(t[2 * a] - ring, 0));
+      atomicMax(&box[2 * a + 1], min(t[2 * a + 1] + ring, n[a] - 1));
+    }
   }
+}
+
+/* A late-joined step's old tile map and list: every entry out of the map,
+ * the list empty (one block: the count is reset after its last read). */
+__global__ void __launch_bounds__(1024) lbib_clear_tiles(int* __restrict__ slot, const int* __restrict__ list,
+                                                         int* __restrict__ count) {
+  const int n = *count;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) slot[list[i]] = -1;
+  __syncthreads();
+  if (threadIdx.x == 0) *count = 0;
 }
 
 /* The box, in tiles, of all stencils of the current node positions (one
@@ -127,7 +143,7 @@ __global__ void __launch_bounds__(kMoveTPB) lbib_move_nodes(double* __restrict__
  * runs after the spread.  Nodes whose stencil leaves the grid are left out
  * (the spread reports them).  No valid node: an empty box. */
 __global__ void __launch_bounds__(1024) lbib_stencil_box(const double* __restrict__ nodes, long S, int nx, int ny,
-                                                         int nz, int* __restrict__ box) {
+                                                         int nz, int ring, int* __restrict__ box) {
   __shared__ int red[6][32];
   int b0 = INT_MAX, b1 = INT_MIN, b2 = INT_MAX, b3 = INT_MIN, b4 = INT_MAX, b5 = INT_MIN;
   for (long i0 = threadIdx.x; i0 < S; i0 += 4L * blockDim.x) {
@@ -166,7 +182,11 @@ __global__ void __launch_bounds__(1024) lbib_stencil_box(const double* __restric
     }
     if (lane == 0) {
       if (b0 > b1) { box[0] = 1; box[1] = 0; box[2] = 1; box[3] = 0; box[4] = 1; box[5] = 0; }
-      else { box[0] = b0 >> 2; box[1] = b1 >> 2; box[2] = b2 >> 2; box[3] = b3 >> 2; box[4] = b4 >> 2; box[5] = b5 >> 2; }
+      else {
+        box[0] = max((b0 >> 2) - ring, 0); box[1] = min((b1 >> 2) + ring, (nx + 3) / 4 - 1);
+        box[2] = max((b2 >> 2) - ring, 0); box[3] = min((b3 >> 2) + ring, (ny + 3) / 4 - 1);
+        box[4] = max((b4 >> 2) - ring, 0); box[5] = min((b5 >> 2) + ring, (nz + 3) / 4 - 1);
+      }
     }
   }
 }
@@ -204,7 +224,15 @@ extern "C" int lbdev_launch_fiber_forces(lbib_device* d, int k) {
 }
 
 extern "C" int lbdev_launch_stencil_box(lbib_device* d) {
-  lbib_stencil_box<<<1, 1024, 0, d->stream>>>(d->nodes, d->S, d->nx, d->ny, d->nz, d->box + 6 * d->box_cur);
+  lbib_stencil_box<<<1, 1024, 0, d->stream>>>(d->nodes, d->S, d->nx, d->ny, d->nz, lbdev_late_join(d), d->box + 6 * d->box_cur);
+  d->kernel_launches++;
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+/* On the side stream, after the launches that read the old map. */
+extern "C" int lbdev_launch_clear_tiles(lbib_device* d) {
+  const int o = d->cur ^ 1;
+  lbib_clear_tiles<<<1, 1024, 0, d->side>>>(d->tile_slot[o], d->tile_list[o], d->tile_count[o]);
   d->kernel_launches++;
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -280,7 +308,8 @@ extern "C" int lbdev_launch_move(lbib_device* d) {
     }
     lbib_move_nodes<<<(unsigned)((i1 - i0 + 31) / 32), kMoveTPB, 0, d->stream>>>(
         d->nodes, d->W, d->st, i0, i1, d->ntx, d->nty, d->tile_slot[c], d->Utile[c], (double)d->dt, d->err, d->box_next,
-        d->nx, d->ny, d->nz, k0 == 0 && !lbdev_is_slab(d) ? d->tile_count[c ^ 1] : nullptr, pin);
+        lbdev_late_join(d), d->nx, d->ny, d->nz, k0 == 0 && !lbdev_is_slab(d) && !d->late ? d->tile_count[c ^ 1] : nullptr,
+        pin);
     d->kernel_launches++;
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

@@ -141,13 +141,14 @@ typedef struct lbib_device {
      the box's cells run on `stream` after the spread */
   cudaStream_t fluid_stream;     /* == stream unless a step is overlapped     */
   cudaStream_t side;
-  cudaEvent_t ev_box, ev_bulk;
+  cudaEvent_t ev_box, ev_bulk, ev_spread;
   int* box;                      /* [2][6]: this step's box and the next's    */
   int box_cur;                   /* which of the two this step uses           */
   int box_valid;                 /* box[box_cur] holds the current positions' */
   int* box_next;                 /* the move accumulates the next box here    */
   int box_mode;                  /* 1 inside an overlapped step               */
   int overlap;                   /* overlapped steps allowed (LBIB_OVERLAP)   */
+  int late;                      /* 1 inside a step whose streams join after the move */
   int fuse_forces;               /* the spread's node preparation also computes the fiber forces */
   int device;
   long kernel_launches;          /* kernels this state has launched           */
@@ -171,6 +172,15 @@ typedef struct lbdev_config {
 int  lbdev_create(lbib_device** out, const lbdev_config* cfg);
 /* d holds part of the grid's columns. */
 static inline int lbdev_is_slab(const lbib_device* d) { return d->x_lo > 0 || d->x_hi < d->nx; }
+
+/* An overlapped step may join its streams after the move: the box then has a
+ * ring of tiles around the touched ones, so that every cell whose slots the
+ * moments read is stepped by the box's launch (not with periodic z, whose
+ * neighbours across the edge no ring covers; nor in the low-precision forms,
+ * where a cell's bits depend on which kernel steps it: FMA contraction). */
+static inline int lbdev_late_join(const lbib_device* d) {
+  return d->overlap == 3 && LBIB_PREC_TYPE(d->prec) == LBIB_PREC_F64 && !(d->compat & LBIB_OPT_PERIODIC_Z);
+}
 /* Columns [x_lo, x_hi) of the grid held by d (x_hi <= 0: all); sets the
  * storage geometry, allocates nothing. */
 int  lbdev_set_columns(lbib_device* d, int x_lo, int x_hi);

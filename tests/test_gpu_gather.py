@@ -70,3 +70,36 @@ def test_tiny_forces(gpu, oracle_built, ks):
     y, z = np.meshgrid(np.linspace(8, 30, 12), np.linspace(8, 34, 14), indexing="ij")
     pos = np.stack([np.full_like(y, 12.0), y, z], axis=-1) + rng.uniform(-0.3, 0.3, y.shape + (3,))
     _run(case, [pos])
+
+
+@pytest.mark.parametrize("nx,ny,nz,where", [
+    (32, 40, 44, (3.0, 6.0, 8.0)),           # at the inlet
+    (32, 40, 44, (NX - 4.0, 6.0, 8.0)),      # at the outlet
+    (32, 40, 44, (14.0, 3.0, 4.0)),          # in a corner of the walls
+    (36, 40, 44, (17.5, 16.0, 15.0)),
+    (128, 64, 64, (40.0, 20.0, 18.0)),       # large enough to join late by itself
+])
+@pytest.mark.parametrize("options", [0, 0x100, 0x400])
+def test_streams_joined_after_the_move(gpu, monkeypatch, nx, ny, nz, where, options):
+    """The step whose streams join after the move against the stages in order,
+    bit for bit, with a sheet that jumps from one end of the grid to another
+    (the map of the step before lies outside the box) and back."""
+    def run(mode):
+        monkeypatch.setenv("LBIB_OVERLAP", mode)
+        case = P.Case(nx, ny, nz, [P.Sheet(18, 20, 17.0, 14.0, *where)], Ks_l=0.01, Kb_l=0.001,
+                      compat=P.COMPAT_ALL | options)
+        s = lbib.Solver(case)
+        s.run(4)
+        rec = s.sheet(0)
+        rec[..., 0] = (nx - 1) - rec[..., 0]
+        s.set_sheet(0, rec)
+        s.run(3)
+        rec = s.sheet(0)
+        rec[..., 0] = (nx - 1) - rec[..., 0]
+        s.set_sheet(0, rec)
+        s.run(4)
+        out = [*s.moments(), s.sheet(0)]
+        s.close()
+        return out
+    for a, b in zip(run("3"), run("0")):
+        np.testing.assert_array_equal(a, b)
