@@ -406,7 +406,9 @@ long lbib_kernel_launches(GV gv);                /* CUDA kernels launched so far
 /* Stage timing with CUDA events on the library's stream: between begin and
  * end every step records events around its five stages; end synchronises and
  * returns the summed milliseconds of [fiber forces, spread, fused fluid step,
- * tile moments, interpolate+move] and the number of steps timed. */
+ * tile moments, interpolate+move] and the number of steps timed.  A whole
+ * grid's steps run the fluid kernels beside the spread, so the stages overlap,
+ * and the cells near the sheets are stepped in the spread's launch. */
 int lbib_profile_begin(GV gv);
 int lbib_profile_end(GV gv, double* stage_ms, long* steps);
 
