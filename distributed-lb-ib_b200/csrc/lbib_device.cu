@@ -473,9 +473,9 @@ static int prof_grow(lbib_device* d) {
  * the two does not matter).
  * The row and bulk kernels run on the side stream, beside the preparation
  * and the spread (d->overlap == 1: in stream order).  us per step one after
- * the other / side by side, FP64: 63 / 50 at 64x32x32, 98 / 72 at
- * 128x64x64, 1746 / 1721 at 512x256x256; 16-bit storage: 79 / 67 at
- * 128x64x64, 777 / 763 at 512x256x256.  (With the spread in six launches
+ * the other / side by side, FP64: 46.9 / 34.3 at 64x32x32, 70.4 / 57.4
+ * at 128x64x64, 1730 / 1719 at 512x256x256; 16-bit storage: 62.1 / 52.3 at
+ * 128x64x64, 760 / 750 at 512x256x256.  (With the spread in six launches
  * instead of two, each of which had to find room among the bulk kernel's
  * blocks, side by side was the slower at 512x256x256.)
  * The streams join before the moments, whose cells' slots the bulk kernel
