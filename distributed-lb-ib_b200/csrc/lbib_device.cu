@@ -28,7 +28,7 @@ int lbdev_launch_prep(lbib_device* d, int step);
 int lbdev_launch_spread(lbib_device* d, int step);
 int lbdev_launch_move(lbib_device* d);
 int lbdev_launch_stencil_box(lbib_device* d);
-int lbdev_launch_clear_tiles(lbib_device* d);
+int lbdev_launch_clear_tiles(lbib_device* d, int b, cudaStream_t st);
 int lbdev_launch_spread_box(lbib_device* d);
 int lbdev_launch_scatter_force(lbib_device* d, double* fx, double* fy, double* fz);
 }
@@ -357,6 +357,7 @@ extern "C" int lbdev_set_sheets(lbib_device* d, int nsheets, const lbib_sheet_de
       CK(cudaMalloc(&d->Utile[b], sizeof(double) * 256 * d->cap));
       CK(cudaMemsetAsync(d->tile_slot[b], 0xff, sizeof(int) * d->ntiles, d->stream));
       CK(cudaMemsetAsync(d->tile_count[b], 0, sizeof(int), d->stream));
+      d->tiles_left[b] = 0;
     }
     if (lbdev_is_slab(d)) {
       CK(cudaMalloc(&d->tile_mark, sizeof(int) * d->ntiles));
@@ -401,6 +402,7 @@ extern "C" int lbdev_init_df1(lbib_device* d) {
     if (d->tile_slot[b]) {
       CK(cudaMemsetAsync(d->tile_slot[b], 0xff, sizeof(int) * d->ntiles, d->stream));
       CK(cudaMemsetAsync(d->tile_count[b], 0, sizeof(int), d->stream));
+      d->tiles_left[b] = 0;
     }
   return 0;
 }
@@ -497,7 +499,6 @@ static int step_overlapped(lbib_device* d, int step_no, cudaEvent_t* ev) {
   d->have_moments = 0;
   d->box_mode = 1;
   const int conc = d->overlap >= 2, late = lbdev_late_join(d);
-  d->late = late;
   int rc = 0;
   if (conc) {
     CK(cudaEventRecord(d->ev_box, d->stream));
@@ -521,7 +522,7 @@ static int step_overlapped(lbib_device* d, int step_no, cudaEvent_t* ev) {
     /* the old map has readers on both streams; its clearing leaves the chain */
     CK(cudaEventRecord(d->ev_spread, d->stream));
     CK(cudaStreamWaitEvent(d->side, d->ev_spread, 0));
-    if (!rc) rc = lbdev_launch_clear_tiles(d);
+    if (!rc) rc = lbdev_launch_clear_tiles(d, d->cur ^ 1, d->side);
     CK(cudaEventRecord(d->ev_bulk, d->side));
   } else if (conc) {
     CK(cudaStreamWaitEvent(d->stream, d->ev_bulk, 0));
@@ -540,7 +541,6 @@ static int step_overlapped(lbib_device* d, int step_no, cudaEvent_t* ev) {
   if (!rc) rc = lbdev_launch_move(d) ? -2 : 0;
   if (ev) CK(cudaEventRecord(ev[5], d->stream));
   if (late) CK(cudaStreamWaitEvent(d->stream, d->ev_bulk, 0));
-  d->late = 0;
   /* the move reduced the next step's box into box_next */
   d->box_valid = !rc;
   if (d->box_valid) d->box_cur ^= 1;
@@ -841,6 +841,8 @@ extern "C" int lbdev_load_state(lbib_device* d, FILE* fp) {
   CK(cudaMemcpy(d->tile_count[c], &count, sizeof(int), cudaMemcpyHostToDevice));
   CK(cudaMemset(d->tile_slot[c ^ 1], 0xff, sizeof(int) * d->ntiles));
   CK(cudaMemset(d->tile_count[c ^ 1], 0, sizeof(int)));
+  d->tiles_left[c] = LBIB_TILES_ALL;
+  d->tiles_left[c ^ 1] = 0;
   d->parity = hdr[0];
   d->cur = c;
   d->have_forces = hdr[2];

@@ -618,7 +618,10 @@ int launch_tile_moments_t(lbib_device* d) {
   FluidParamsT<T> p = make_params_t<T>(d, 0);
   const int c = d->cur;
   const int blocks = 2371;   /* ~16 CTAs per SM; prime, as kBoxCtas */
-  int* old = lbdev_is_slab(d) || d->late ? nullptr : d->tile_slot[c ^ 1];
+  /* a box-mode step's old map: read for the last time before this launch (a
+     host that calls the stages may still collide with it) */
+  int* old = d->box_mode && d->tiles_left[c ^ 1] == LBIB_TILES_ALL ? d->tile_slot[c ^ 1] : nullptr;
+  if (old) d->tiles_left[c ^ 1] = LBIB_TILES_LIST;
   if (d->parity == 0)
     lbib_tile_moments<T, 0><<<blocks, 64, 0, d->stream>>>(p, d->tile_list[c], d->tile_count[c], d->Ftile[c], d->Utile[c],
                                                           old, d->tile_list[c ^ 1], d->tile_count[c ^ 1]);

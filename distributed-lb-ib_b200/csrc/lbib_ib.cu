@@ -128,8 +128,8 @@ __global__ void __launch_bounds__(kMoveTPB) lbib_move_nodes(double* __restrict__
   }
 }
 
-/* A late-joined step's old tile map and list: every entry out of the map,
- * the list empty (one block: the count is reset after its last read). */
+/* A tile map and its list: every entry out of the map, the list empty (one
+ * block: the count is reset after its last read). */
 __global__ void __launch_bounds__(1024) lbib_clear_tiles(int* __restrict__ slot, const int* __restrict__ list,
                                                          int* __restrict__ count) {
   const int n = *count;
@@ -229,11 +229,13 @@ extern "C" int lbdev_launch_stencil_box(lbib_device* d) {
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-/* On the side stream, after the launches that read the old map. */
-extern "C" int lbdev_launch_clear_tiles(lbib_device* d) {
-  const int o = d->cur ^ 1;
-  lbib_clear_tiles<<<1, 1024, 0, d->side>>>(d->tile_slot[o], d->tile_list[o], d->tile_count[o]);
+/* Buffer b's map and list emptied on `st`, after the launches that read them;
+ * nothing to do where the last spread's entries are gone already. */
+extern "C" int lbdev_launch_clear_tiles(lbib_device* d, int b, cudaStream_t st) {
+  if (!d->tiles_left[b]) return 0;
+  lbib_clear_tiles<<<1, 1024, 0, st>>>(d->tile_slot[b], d->tile_list[b], d->tile_count[b]);
   d->kernel_launches++;
+  d->tiles_left[b] = 0;
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -243,9 +245,12 @@ extern "C" int lbdev_can_fuse_forces(const lbib_device* d) { return d->nsheets <
 
 /* Node preparation: weights, stencil starts, boxes, the touched tiles (and,
  * with d->fuse_forces, the fiber forces).  The whole grid lists the tiles as
- * it meets them (the slot map of this step is all -1: the step before left
- * it so, lbib_tile_moments); an x-slab marks them and compacts the marks,
- * because the slabs of one grid number their slots alike. */
+ * it meets them, from an empty list and a map that is all -1: a box-mode step
+ * empties the buffer its successor fills, whatever else ran before (the
+ * stages one by one, with some of them left out or repeated) is cleared here.
+ * Every tile enters the list once and a node touches at most eight, so the
+ * list ends below its d->cap entries.  An x-slab marks the tiles and compacts
+ * the marks, because the slabs of one grid number their slots alike. */
 extern "C" int lbdev_launch_prep(lbib_device* d, int step) {
   const int c = d->cur;
   cudaStream_t st = d->stream;
@@ -257,6 +262,10 @@ extern "C" int lbdev_launch_prep(lbib_device* d, int step) {
     for (int k = 0; k < d->nsheets; ++k) sf.s[k] = d->sh[k];
   }
   const int slab = lbdev_is_slab(d);
+  if (!slab) {
+    if (lbdev_launch_clear_tiles(d, c, st)) return -2;
+    d->tiles_left[c] = LBIB_TILES_ALL;
+  }
   lbib_node_prep<<<(unsigned)d->nchunks, sf.n ? 192 : 128, 0, st>>>(
       d->nodes, d->S, d->nx, d->ny, d->nz, d->ntx, d->nty, d->W, d->st, d->chunk_box, d->super[c], d->tile_slot[c],
       slab ? nullptr : d->tile_list[c], d->tile_count[c], d->tile_mark, d->err, step, sf);
@@ -296,6 +305,8 @@ extern "C" int lbdev_launch_spread(lbib_device* d, int step) {
  * to a launch. */
 extern "C" int lbdev_launch_move(lbib_device* d) {
   const int c = d->cur, pinned = (d->compat & LBIB_OPT_PIN_ROW0) != 0;
+  /* the old list is emptied only once its map has been (a box-mode step) */
+  int* old_count = d->tiles_left[c ^ 1] == LBIB_TILES_LIST ? d->tile_count[c ^ 1] : nullptr;
   const int per = pinned ? kFuseSheets : d->nsheets;
   for (int k0 = 0; k0 < d->nsheets; k0 += per) {
     const int k1 = k0 + per < d->nsheets ? k0 + per : d->nsheets;
@@ -308,10 +319,10 @@ extern "C" int lbdev_launch_move(lbib_device* d) {
     }
     lbib_move_nodes<<<(unsigned)((i1 - i0 + 31) / 32), kMoveTPB, 0, d->stream>>>(
         d->nodes, d->W, d->st, i0, i1, d->ntx, d->nty, d->tile_slot[c], d->Utile[c], (double)d->dt, d->err, d->box_next,
-        lbdev_late_join(d), d->nx, d->ny, d->nz, k0 == 0 && !lbdev_is_slab(d) && !d->late ? d->tile_count[c ^ 1] : nullptr,
-        pin);
+        lbdev_late_join(d), d->nx, d->ny, d->nz, k0 == 0 ? old_count : nullptr, pin);
     d->kernel_launches++;
   }
+  if (old_count) d->tiles_left[c ^ 1] = 0;
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -34,6 +34,9 @@ extern "C" {
 #define LBIB_CHUNK 32
 #define LBIB_SUPER_MIN 128       /* more node chunks than this: super-chunk boxes too */
 
+#define LBIB_TILES_LIST 1        /* the list and its count; the map is all -1 again */
+#define LBIB_TILES_ALL 2         /* the map too                                 */
+
 #ifndef LBIB_PREC_F64
 #define LBIB_PREC_F64 0   /* population storage precisions, as in include/lbib.h */
 #define LBIB_PREC_F32 1
@@ -106,6 +109,8 @@ typedef struct lbib_device {
   int* tile_slot[2];             /* [ntiles] slot or -1                       */
   int* tile_list[2];             /* [cap] touched tiles, slot by slot         */
   int* tile_count[2];            /* [1]                                       */
+  int tiles_left[2];             /* whole grids: what the last spread into the buffer left
+                                    there: LBIB_TILES_ALL, _LIST or 0 (nothing)  */
   int* scan_tmp;                 /* x-slabs: block sums for the compaction    */
   unsigned long long* scan_state; /* one-pass compaction: per-block words + ticket */
   unsigned scan_tag;             /* the one-pass compaction's launch tag (1..255) */
@@ -148,7 +153,6 @@ typedef struct lbib_device {
   int* box_next;                 /* the move accumulates the next box here    */
   int box_mode;                  /* 1 inside an overlapped step               */
   int overlap;                   /* overlapped steps allowed (LBIB_OVERLAP)   */
-  int late;                      /* 1 inside a step whose streams join after the move */
   int fuse_forces;               /* the spread's node preparation also computes the fiber forces */
   int device;
   long kernel_launches;          /* kernels this state has launched           */
