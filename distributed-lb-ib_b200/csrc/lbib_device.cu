@@ -161,6 +161,9 @@ static int build_rows(lbib_device* d) {
 extern "C" int lbdev_set_physics(lbib_device* d, const lbdev_config* c) {
   d->tau = c->tau; d->u_l = c->u_l; d->rho_l = c->rho_l; d->Ks_l = c->Ks_l; d->Kb_l = c->Kb_l;
   d->g_l = c->g_l; d->cs_l = c->cs_l; d->dt = c->dt; d->compat = c->compat;
+  /* the next step's box, with or without a ring of tiles, was reduced under
+     the options so far (lbdev_late_join) */
+  d->box_valid = 0;
   derive_constants(d);
   derive_boundaries(d);
   return d->stream ? build_rows(d) : 0;

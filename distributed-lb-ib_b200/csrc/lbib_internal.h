@@ -149,7 +149,8 @@ typedef struct lbib_device {
   cudaEvent_t ev_box, ev_bulk, ev_spread;
   int* box;                      /* [2][6]: this step's box and the next's    */
   int box_cur;                   /* which of the two this step uses           */
-  int box_valid;                 /* box[box_cur] holds the current positions' */
+  int box_valid;                 /* box[box_cur] holds the current positions',
+                                    with the ring that lbdev_late_join asks for */
   int* box_next;                 /* the move accumulates the next box here    */
   int box_mode;                  /* 1 inside an overlapped step               */
   int overlap;                   /* overlapped steps allowed (LBIB_OVERLAP)   */
