@@ -49,7 +49,9 @@ namespace {
 /* A CTA per 32-node chunk, all of one problem (every problem's nodes start
  * at a multiple of 32), as the one-grid lbib_node_prep: four warps of
  * node_prep_warp and two for the fiber forces.  step_no: the batch's device
- * step counter (graph replays see the live value), 1 for the first step. */
+ * step counter (graph replays see the live value), 1 for the first step.
+ * Every chunk of a problem that stops in this step is still done, so that the
+ * sheet's records do not depend on which chunk found the error. */
 __global__ void __launch_bounds__(192, 4) lbib_b_node_prep(double* __restrict__ nodes, const int* __restrict__ node_inst,
                                                         const BatchDesc* __restrict__ D, double* __restrict__ W,
                                                         int* __restrict__ st, int* __restrict__ chunk_box,
@@ -60,8 +62,8 @@ __global__ void __launch_bounds__(192, 4) lbib_b_node_prep(double* __restrict__ 
   __shared__ int s_skip;
   const long i0 = (long)blockIdx.x * 32, i = i0 + (threadIdx.x & 31);
   const int part = threadIdx.x >> 5, k = node_inst[i0];
-  /* one read for the CTA: another chunk of the problem may fail meanwhile */
-  if (threadIdx.x == 0) s_skip = k < 0 || *(volatile int*)(err + 2 * k);
+  const int step = *step_no;
+  if (threadIdx.x == 0) s_skip = k < 0 || failed_before(err + 2 * k, step);
   __syncthreads();
   if (s_skip) return;
   const BatchDesc& d = D[k];
@@ -72,7 +74,7 @@ __global__ void __launch_bounds__(192, 4) lbib_b_node_prep(double* __restrict__ 
     return;
   }
   node_prep_warp(nodes, i, mine, SP, part, d.nx, d.ny, d.nz, d.ntx, d.nty, d.tile0, W, st, chunk_box, nullptr, slot,
-                 list, count, nullptr, err + 2 * k, *step_no);
+                 list, count, nullptr, err + 2 * k, step);
 }
 
 /* The move, a CTA per 32-node chunk of one problem (move_chunk); a pinned

@@ -49,8 +49,18 @@ namespace lbib {
 /* PI as truncated in the reference, cube_pthread/lbm_ib.c:33. */
 constexpr double kPi = 3.14159265358979;
 
+/* The error words {code, step} in one go, the first one to come; no reader
+ * sees a code without its step. */
 __device__ __forceinline__ void set_error(int* err, int code, int step) {
-  if (atomicCAS(err, 0, code) == 0) err[1] = step;
+  atomicCAS(reinterpret_cast<unsigned long long*>(err), 0ull,
+            (unsigned long long)(unsigned)step << 32 | (unsigned)code);
+}
+
+/* An error from before this step: one that another CTA of this launch sets
+ * meanwhile does not count. */
+__device__ __forceinline__ bool failed_before(const int* err, int step) {
+  const unsigned long long w = *reinterpret_cast<const volatile unsigned long long*>(err);
+  return (unsigned)w != 0u && (int)(w >> 32) != step;
 }
 
 /* One direction's share of a node's bending and stretching force: along the
