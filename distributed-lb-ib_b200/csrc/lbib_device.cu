@@ -791,6 +791,20 @@ static int dev_in(lbib_device* d, FILE* fp, void* dp, size_t n, void* buf, size_
   return 0;
 }
 
+/* The same for ints in [lo, hi). */
+static int dev_in_ints(lbib_device* d, FILE* fp, int* dp, long n, long lo, long hi, int* buf, size_t cap) {
+  const long per = (long)(cap / sizeof(int));
+  for (long o = 0; o < n; o += per) {
+    const long k = n - o < per ? n - o : per;
+    if (get(fp, buf, sizeof(int) * k)) return -7;
+    for (long i = 0; i < k; ++i)
+      if (buf[i] < lo || buf[i] >= hi) return -1;
+    CK(cudaMemcpy(dp + o, buf, sizeof(int) * k, cudaMemcpyHostToDevice));
+  }
+  (void)d;
+  return 0;
+}
+
 extern "C" int lbdev_save_state(lbib_device* d, FILE* fp) {
   if (!d->nodes || !d->tile_slot[0]) return -4;
   CK(cudaStreamSynchronize(d->stream));
@@ -834,13 +848,23 @@ extern "C" int lbdev_load_state(lbib_device* d, FILE* fp) {
   int rc = dev_in(d, fp, d->f, lbdev_pop_bytes(d->prec) * 19 * d->Ns, buf, cap);
   if (!rc) rc = dev_in(d, fp, d->inlet, real * 19 * P, buf, cap);
   if (!rc) rc = dev_in(d, fp, d->outlet, real * 19 * P, buf, cap);
-  if (!rc) rc = dev_in(d, fp, d->tile_slot[c], sizeof(int) * d->ntiles, buf, cap);
-  if (!rc) rc = dev_in(d, fp, d->tile_list[c], sizeof(int) * count, buf, cap);
+  /* the map and the list are indices: out-of-range ones are refused */
+  if (!rc) rc = dev_in_ints(d, fp, d->tile_slot[c], d->ntiles, -1, count, (int*)buf, cap);
+  if (!rc) rc = dev_in_ints(d, fp, d->tile_list[c], count, 0, d->ntiles, (int*)buf, cap);
   if (!rc) rc = dev_in(d, fp, d->Ftile[c], sizeof(double) * 192 * count, buf, cap);
   if (!rc) rc = dev_in(d, fp, d->Utile[c], sizeof(double) * 256 * count, buf, cap);
   if (!rc) rc = dev_in(d, fp, d->nodes, sizeof(double) * 12 * d->S, buf, cap);
   free(buf);
-  if (rc) return rc;
+  if (rc) {
+    /* half a map would keep its tiles out of later lists */
+    for (int b = 0; b < 2; ++b) {
+      CK(cudaMemset(d->tile_slot[b], 0xff, sizeof(int) * d->ntiles));
+      CK(cudaMemset(d->tile_count[b], 0, sizeof(int)));
+      d->tiles_left[b] = 0;
+    }
+    d->have_forces = d->have_moments = 0;
+    return rc;
+  }
   CK(cudaMemcpy(d->tile_count[c], &count, sizeof(int), cudaMemcpyHostToDevice));
   CK(cudaMemset(d->tile_slot[c ^ 1], 0xff, sizeof(int) * d->ntiles));
   CK(cudaMemset(d->tile_count[c ^ 1], 0, sizeof(int)));
