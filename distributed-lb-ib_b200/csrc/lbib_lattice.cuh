@@ -331,10 +331,6 @@ __device__ __forceinline__ void velocity_dots(R ux, R uy, R uz, R cu[19]) {
   cu[17] = ux + uy;  cu[18] = -cu[17];
 }
 
-/* compute_eqlbrmdistrfuncDF1, cube_pthread/lbm_ib.c:1713-1807: equilibrium
- * and BGK relaxation, in place on f.  With a force the Guo term is added as
- * written there (true divisions by cs^2 and cs^4); without one that term is
- * +-0 in the reference and is skipped. */
 /* a / c, correctly rounded, for a constant c with y = 1/c rounded to nearest:
  * q = a y, the residual a - c q by FMA, q + y times that (Markstein, "Computation
  * of elementary functions on the IBM RISC System/6000 processor", 1990).  It is
@@ -363,12 +359,14 @@ __device__ __forceinline__ bool div_safe(double v) {
  *   kw (A / cs^2 + B / cs^4 C),  A = (c - u).F,  B = c.u,  C = c.F,
  * with what directions share formed once: the products (c_d - u_d) F_d for
  * c_d = -1, 0, 1 per axis, and B / cs^4 C per opposite pair (both signs
- * change).  Dropping the products with c_d = 0 from B and C changes them by
- * a signed zero at most. */
+ * change).  Dropping the products with c_d = 0 from B and C changes finite
+ * ones by a signed zero at most; operands that are not finite (0 times them
+ * is NaN) take guo_as_written. */
 template <typename R>
 struct Relax {
   R t6, om, it;
   R px[3], py[3], pz[3];   /* (c_d - u_d) F_d, c_d = -1, 0, 1 */
+  R ux, uy, uz, Fx, Fy, Fzg;   /* guo_as_written's */
 };
 
 /* The constants of a collision; cs2_inv, cs4_inv as div_const takes them. */
@@ -377,9 +375,15 @@ struct CollideConst {
   R om, it, kw0, kw1, kw2, cs2, cs4, cs2_inv, cs4_inv, g;
 };
 
-template <bool FAST>
-__device__ __forceinline__ double guo_div(double a, double c, double y) {
-  return FAST ? div_const(a, c, y) : a / c;
+/* The term with every product and with true divisions. */
+template <typename R>
+__device__ __forceinline__ R guo_as_written(int q, const Relax<R>& r, const CollideConst<R>& p) {
+  const R c0 = (R)cx(q), c1 = (R)cy(q), c2 = (R)cz(q);
+  const R kw = q == 0 ? p.kw0 : q <= 6 ? p.kw1 : p.kw2;
+  const R A = (c0 - r.ux) * r.Fx + (c1 - r.uy) * r.Fy + (c2 - r.uz) * r.Fzg;
+  const R B = c0 * r.ux + c1 * r.uy + c2 * r.uz;
+  const R C = c0 * r.Fx + c1 * r.Fy + c2 * r.Fzg;
+  return kw * (A / p.cs2 + B / p.cs4 * C);
 }
 
 /* One opposite pair (qa, qb) with c_qa . u = cu: both equilibria share
@@ -394,13 +398,16 @@ __device__ __forceinline__ void relax_pair(R* f, R cu, R cF, R wr, const Relax<R
   const R eb = wr * (R(1.0) + (-a3) + sq - r.t6);
   R va = f[QA] * r.om + r.it * ea;
   R vb = f[QB] * r.om + r.it * eb;
-  if constexpr (FORCED) {
+  if constexpr (FORCED && !FAST) {
+    va = va + guo_as_written(QA, r, p);
+    vb = vb + guo_as_written(QB, r, p);
+  } else if constexpr (FORCED) {
     const R kw = QA <= 6 ? p.kw1 : p.kw2;
-    const R bc = guo_div<FAST>(cu, p.cs4, p.cs4_inv) * cF;
+    const R bc = div_const(cu, p.cs4, p.cs4_inv) * cF;
     const R Aa = r.px[cx(QA) + 1] + r.py[cy(QA) + 1] + r.pz[cz(QA) + 1];
     const R Ab = r.px[cx(QB) + 1] + r.py[cy(QB) + 1] + r.pz[cz(QB) + 1];
-    va = va + kw * (guo_div<FAST>(Aa, p.cs2, p.cs2_inv) + bc);
-    vb = vb + kw * (guo_div<FAST>(Ab, p.cs2, p.cs2_inv) + bc);
+    va = va + kw * (div_const(Aa, p.cs2, p.cs2_inv) + bc);
+    vb = vb + kw * (div_const(Ab, p.cs2, p.cs2_inv) + bc);
   }
   f[QA] = va;
   f[QB] = vb;
@@ -411,7 +418,9 @@ __device__ __forceinline__ void collide_body(R f[19], R rho, R ux, R uy, R uz, R
                                              const CollideConst<R>& p) {
   Relax<R> r;
   const R Fzg = FORCED ? Fz + rho * p.g : R(0);
-  if constexpr (FORCED) {
+  if constexpr (FORCED && !FAST) {
+    r.ux = ux; r.uy = uy; r.uz = uz; r.Fx = Fx; r.Fy = Fy; r.Fzg = Fzg;
+  } else if constexpr (FORCED) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       const R c = R(k - 1);
@@ -426,7 +435,8 @@ __device__ __forceinline__ void collide_body(R f[19], R rho, R ux, R uy, R uz, R
   const R wr1 = R(1.0 / 18.0) * rho;
   const R wr2 = R(1.0 / 36.0) * rho;
   R v0 = f[0] * r.om + r.it * (wr0 * (R(1.0) - r.t6));
-  if constexpr (FORCED) v0 = v0 + p.kw0 * guo_div<FAST>(r.px[1] + r.py[1] + r.pz[1], p.cs2, p.cs2_inv);
+  if constexpr (FORCED && !FAST) v0 = v0 + guo_as_written(0, r, p);
+  else if constexpr (FORCED) v0 = v0 + p.kw0 * div_const(r.px[1] + r.py[1] + r.pz[1], p.cs2, p.cs2_inv);
   f[0] = v0;
   relax_pair<FORCED, FAST, 1, 2>(f, ux, Fx, wr1, r, p);
   relax_pair<FORCED, FAST, 3, 4>(f, uz, Fzg, wr1, r, p);
@@ -446,6 +456,10 @@ __device__ __noinline__ void collide_rare(R* f, R rho, R ux, R uy, R uz, R Fx, R
   collide_body<true, false>(f, rho, ux, uy, uz, Fx, Fy, Fz, c);
 }
 
+/* compute_eqlbrmdistrfuncDF1, cube_pthread/lbm_ib.c:1713-1807: equilibrium
+ * and BGK relaxation, in place on f.  With a force the Guo term is added, the
+ * rounded quotients by cs^2 and cs^4 as there; without one that term is +-0
+ * in the reference and is skipped. */
 template <bool FORCED, typename R, typename P>
 __device__ __forceinline__ void collide(R f[19], R rho, R ux, R uy, R uz, R Fx, R Fy, R Fz, const P& p) {
   CollideConst<R> c;
