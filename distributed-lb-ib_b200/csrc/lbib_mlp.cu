@@ -8,7 +8,9 @@
  * Matrices: see lbib_mlp_tc.cuh for the chunk layout of the BF16 ones
  * (activations, dZ, weights); Z (FP32) has the same order, 8 consecutive
  * columns of a row together.  Row padding (to 128) is written as zeros by
- * every epilogue, column padding (to 128) is zero from the start.
+ * every epilogue; columns are padded to 16 only.  Device memory of a net, per
+ * batch row: 2 bytes for each width that is a layer's input, 4 more for each
+ * hidden one, and twice 2 for the widest output.
  *
  * Shapes: widths w_0 .. w_L (input, hidden..., output); layer l maps w_l to
  * w_{l+1}.  Every width is padded to a multiple of 16 inside (the padded
@@ -145,7 +147,7 @@ __device__ __forceinline__ void gemm_tile(const Gemm& g, int tile, int z, uint8_
   auto fetch = [&](int kk) {   /* one thread: the copies of slice kk */
     const int b = kk % kStages, kn = extent(kk), k0 = k00 + kk * BK;
     const uint32_t s = s0 + b * kStageBytes;
-    mbar_expect(&c.full[b], (fp32_in ? 0 : slice_bytes<BM>(g.A, kn)) + slice_bytes<BN>(g.B, kn));
+    mbar_expect(&c.full[b], (fp32_in ? 0 : slice_bytes<BM>(g.A, m0, kn)) + slice_bytes<BN>(g.B, n0, kn));
     if (!fp32_in) fetch_slice<BM>(s, g.A, m0, k0, kn, &c.full[b]);
     fetch_slice<BN>(s + BM * BK * 2, g.B, n0, k0, kn, &c.full[b]);
   };
@@ -482,8 +484,8 @@ struct lbib_mlp {
   long* woff;           /* [L] offset of W_l in p (padded) */
   long* boff;           /* [L] offset of b_l in p */
   long* wbo;            /* [2 L] offsets of W_l and its transpose in wbf  */
-  __nv_bfloat16** act;  /* [L] activations, rows x wp_l (to 128); act[0] = input */
-  __nv_bfloat16** dz;   /* [L] dZ, rows x wp_{l+1} (to 128)               */
+  __nv_bfloat16** act;  /* [L] activations, rows x wp_l; act[0] = input   */
+  __nv_bfloat16* dz[2]; /* layer l's dZ, rows x wp_{l+1}, in dz[l & 1]    */
   float** z;            /* [L-1] pre-activations fp32, rows x wp_{l+1}    */
   float* part;          /* squared-error sums of the output layer's tiles */
   float* d_loss;
@@ -525,13 +527,10 @@ int launch(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem,
   return cudaLaunchKernelEx(&c, kernel, (P)args...) == cudaSuccess ? 0 : -2;
 }
 
-/* Chunks of a row of a rows x wp matrix. */
-int row_chunks(int wp) { return (int)(align_up(wp, 128) / 8); }
-
 /* Layer l's matrices as operands: rows as the tile's rows, or columns; W_l
  * [out][in] or its transpose. */
-Operand act_op(const lbib_mlp* n, int l, int mn) { return Operand{n->act[l], row_chunks(n->wp[l]), BM, mn}; }
-Operand dz_op(const lbib_mlp* n, int l, int mn) { return Operand{n->dz[l], row_chunks(n->wp[l + 1]), BM, mn}; }
+Operand act_op(const lbib_mlp* n, int l, int mn) { return Operand{n->act[l], n->wp[l] / 8, BM, mn}; }
+Operand dz_op(const lbib_mlp* n, int l, int mn) { return Operand{n->dz[l & 1], n->wp[l + 1] / 8, BM, mn}; }
 Operand w_op(const lbib_mlp* n, int l, int transposed) {
   return Operand{n->wbf + n->wbo[2 * l + transposed], n->wp[l + transposed] / 8, BN, 0};
 }
@@ -552,7 +551,7 @@ Gemm layer_product(lbib_mlp* n, int l, const float* X, int batch) {
   Gemm g = product(act_op(n, l, 0), w_op(n, l, 0), batch, n->wp[l + 1], n->wp[l]);
   if (l == 0) { g.X = X; g.xw = n->w[0]; }
   g.aux = n->p + n->boff[l];
-  g.oC = row_chunks(n->wp[l + 1]);
+  g.oC = n->wp[l + 1] / 8;
   if (l + 1 < n->L) g.out1 = n->act[l + 1];
   return g;
 }
@@ -585,7 +584,7 @@ int gradients(lbib_mlp* n, const float* X, const float* T, int batch, bool want_
       g.out0 = n->z[l];
       rc = launch(mlp_layer<EPI_GELU_KEEP>, g.tiles, NT, kSmem, n->stream, 1, g, n->d_err);
     } else {
-      g.out1 = n->dz[l]; g.T = T; g.w = n->w[L];
+      g.out1 = n->dz[l & 1]; g.T = T; g.w = n->w[L];
       g.loss = want_loss ? n->part : NULL;
       rc = launch(mlp_layer<EPI_MSE>, g.tiles, NT, kSmem, n->stream, 1, g, n->d_err);
       if (!rc && want_loss)
@@ -615,8 +614,8 @@ int gradients(lbib_mlp* n, const float* X, const float* T, int batch, bool want_
     if (l > 0) {
       /* dZ_{l-1} = (dZ W) * gelu'(Z_{l-1}): M = batch, N = in, K = out */
       a.dA = product(dz_op(n, l, 0), w_op(n, l, 1), batch, in, out);
-      a.dA.out1 = n->dz[l - 1];
-      a.dA.oC = row_chunks(in);
+      a.dA.out1 = n->dz[(l - 1) & 1];
+      a.dA.oC = in / 8;
       a.dA.z = n->z[l - 1];
       a.n_dA = (a.dA.tiles + sk - 1) / sk * sk;
     }
@@ -692,9 +691,8 @@ lbib_mlp* lbib_mlp_create(int n_layers, const int* widths, int max_batch, unsign
   n->boff = (long*)calloc(L, sizeof(long));
   n->wbo = (long*)calloc(2 * L, sizeof(long));
   n->act = (__nv_bfloat16**)calloc(L + 1, sizeof(void*));
-  n->dz = (__nv_bfloat16**)calloc(L, sizeof(void*));
   n->z = (float**)calloc(L, sizeof(void*));
-  int rc = (!n->w || !n->wp || !n->woff || !n->boff || !n->wbo || !n->act || !n->dz || !n->z) ? -5 : 0;
+  int rc = (!n->w || !n->wp || !n->woff || !n->boff || !n->wbo || !n->act || !n->z) ? -5 : 0;
   n->rows = align_up(max_batch, BM);
   long np = 0, nw = 0;
   for (int l = 0; l <= L && !rc; ++l) {
@@ -727,12 +725,13 @@ lbib_mlp* lbib_mlp_create(int n_layers, const int* widths, int max_batch, unsign
     part(n->p, fp); part(n->g, fp); part(n->m, fp); part(n->v, fp);
     part(n->wmap, sizeof(int2) * np);
     part(n->wbf, sizeof(__nv_bfloat16) * nw);
+    long dzw[2] = {0, 0};
     for (int l = 0; l < L; ++l) {
-      const size_t z = n->rows * align_up(n->wp[l + 1], 128);
-      part(n->act[l], sizeof(__nv_bfloat16) * n->rows * align_up(n->wp[l], 128));
-      part(n->dz[l], sizeof(__nv_bfloat16) * z);
-      if (l + 1 < L) part(n->z[l], sizeof(float) * z);
+      part(n->act[l], sizeof(__nv_bfloat16) * n->rows * n->wp[l]);
+      if (l + 1 < L) part(n->z[l], sizeof(float) * n->rows * n->wp[l + 1]);
+      if (n->wp[l + 1] > dzw[l & 1]) dzw[l & 1] = n->wp[l + 1];
     }
+    for (int k = 0; k < 2; ++k) part(n->dz[k], sizeof(__nv_bfloat16) * n->rows * dzw[k]);
     part(n->part, sizeof(float) * out_tiles);
     part(n->d_loss, sizeof(float));
     part(n->d_err, sizeof(int));
@@ -777,7 +776,7 @@ void lbib_mlp_free(lbib_mlp* n) {
   if (n->stream) cudaStreamSynchronize(n->stream);
   cudaFree(n->mem);
   if (n->own_stream) cudaStreamDestroy(n->own_stream);
-  free(n->w); free(n->wp); free(n->woff); free(n->boff); free(n->wbo); free(n->act); free(n->dz); free(n->z);
+  free(n->w); free(n->wp); free(n->woff); free(n->boff); free(n->wbo); free(n->act); free(n->z);
   free(n);
 }
 

@@ -180,15 +180,17 @@ __device__ __forceinline__ float ld_cluster(const float* p, uint32_t rank) {
 /* The operand's rows [r0, r0 + R) (r0 a multiple of R; R = blk when K-major)
  * at K elements [k0, k0 + kn), k0 a multiple of BK and kn <= BK of 16: its
  * bytes, and their copy to shared memory at s.  MN-major copies the whole
- * block of BK rows. */
+ * block of BK matrix rows, of the columns that exist: what lies in the buffer
+ * for the others only reaches rows or columns of the tile that are not
+ * written. */
 template <int R>
-__device__ __forceinline__ uint32_t slice_bytes(const Operand& X, int kn) {
-  return X.mn ? R * BK * 2 : R * kn * 2;
+__device__ __forceinline__ uint32_t slice_bytes(const Operand& X, int r0, int kn) {
+  return X.mn ? min(R / 8, X.C - r0 / 8) * BK * 16 : R * kn * 2;
 }
 template <int R>
 __device__ __forceinline__ void fetch_slice(uint32_t s, const Operand& X, int r0, int k0, int kn, uint64_t* bar) {
   const long chunk = X.mn ? ((long)(k0 / BK) * X.C + r0 / 8) * BK : ((long)(r0 / R) * X.C + k0 / 8) * R;
-  bulk_copy(s, X.p + chunk * 8, slice_bytes<R>(X, kn), bar);
+  bulk_copy(s, X.p + chunk * 8, slice_bytes<R>(X, r0, kn), bar);
 }
 
 /* The descriptor of a staged operand's K = 16 step j: core matrices along K
