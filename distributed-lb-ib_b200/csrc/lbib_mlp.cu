@@ -25,7 +25,8 @@
  * reduction.  A training step is one
  * launch per layer forward, one per layer backward (that layer's dW, db and
  * the dZ of the layer below, which all need only its dZ) and Adam: 2L + 1
- * launches, chained by programmatic dependent launch.
+ * launches, chained by programmatic dependent launch, and one more for an
+ * input of more than 16 columns.
  */
 #include <math.h>
 #include <stdint.h>
@@ -81,7 +82,7 @@ static_assert(NT == 32 * 4 * kChunks, "an epilogue thread per chunk");
 /* One product and what is done with it. */
 struct Gemm {
   Operand A, B;           /* A(m, k), and B as X(n, k)                      */
-  const float* X;         /* A instead: FP32 rows [M][xw], rounded on the way in */
+  const float* X;         /* A instead: FP32 rows [M][xw] of few columns, rounded on the way in */
   int xw;
   __nv_bfloat16* copy;    /* with X: the rounded rows, in A's layout, or NULL */
   int M, N, K;
@@ -151,18 +152,16 @@ __device__ __forceinline__ void gemm_tile(const Gemm& g, int tile, int z, uint8_
     if (!fp32_in) fetch_slice<BM>(s, g.A, m0, k0, kn, &c.full[b]);
     fetch_slice<BN>(s + BM * BK * 2, g.B, n0, k0, kn, &c.full[b]);
   };
-  /* the FP32 input's slice kk (a layer of few columns: rarely more than
-     one), by all threads */
-  auto convert = [&](int kk) {
-    const int b = kk % kStages, kn = extent(kk), k0 = k00 + kk * BK;
-    for (int v = t; v < BM * (kn / 8); v += NT) {
-      const int r = v % BM, kb = v / BM, m = m0 + r, k = k0 + kb * 8;
+  /* the FP32 input (kInlineInput columns at most: one slice), by all threads */
+  auto convert = [&]() {
+    for (int v = t; v < BM * (g.K / 8); v += NT) {
+      const int r = v % BM, kb = v / BM, m = m0 + r, k = kb * 8;
       float x[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) x[i] = m < g.M && k + i < g.xw ? g.X[(long)m * g.xw + k + i] : 0.0f;
       const uint4 u = pack8(x);
-      *reinterpret_cast<uint4*>(smem + b * kStageBytes + (kb * BM + r) * 16) = u;
-      if (g.copy && n0 == 0) *reinterpret_cast<uint4*>(g.copy + (((long)(m0 / BM) * g.A.C + k / 8) * BM + r) * 8) = u;
+      *reinterpret_cast<uint4*>(smem + (kb * BM + r) * 16) = u;
+      if (g.copy && n0 == 0) *reinterpret_cast<uint4*>(g.copy + (((long)(m0 / BM) * g.A.C + kb) * BM + r) * 8) = u;
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   };
@@ -171,7 +170,7 @@ __device__ __forceinline__ void gemm_tile(const Gemm& g, int tile, int z, uint8_
   if (t == 0)
     for (int kk = 0; kk < lead; ++kk) fetch(kk);
   if (fp32_in) {
-    for (int kk = 0; kk < lead; ++kk) convert(kk);
+    convert();
     __syncthreads();
   }
   const uint32_t idesc = instr_desc_bf16(BM, BN, g.A.mn, g.B.mn);
@@ -188,27 +187,14 @@ __device__ __forceinline__ void gemm_tile(const Gemm& g, int tile, int z, uint8_
     mma_commit(&c.done[b]);
     return true;
   };
-  if (!fp32_in) {
-    if (t == 32)
-      for (int kk = 0; kk < nk && ok; ++kk) ok = multiply(kk);
-    /* refills, each once the MMAs that read the buffer are done */
-    if (t == 0)
-      for (int kk = kStages; kk < nk && ok; ++kk) {
-        ok = mbar_wait(&c.done[kk % kStages], (kk / kStages - 1) & 1);
-        if (ok) fetch(kk);
-      }
-  } else {
-    /* a wide FP32 input: the later slices in step, all threads converting */
-    for (int kk = 0; kk < nk; ++kk) {
-      if (kk >= kStages) {
-        if (!__syncthreads_and(ok && mbar_wait(&c.done[kk % kStages], (kk / kStages - 1) & 1))) { ok = false; break; }
-        if (t == 0) fetch(kk);
-        convert(kk);
-        __syncthreads();
-      }
-      if (t == 32) ok = ok && multiply(kk);
+  if (t == 32)
+    for (int kk = 0; kk < nk && ok; ++kk) ok = multiply(kk);
+  /* refills, each once the MMAs that read the buffer are done */
+  if (t == 0)
+    for (int kk = kStages; kk < nk && ok; ++kk) {
+      ok = mbar_wait(&c.done[kk % kStages], (kk / kStages - 1) & 1);
+      if (ok) fetch(kk);
     }
-  }
   /* warp w holds TMEM lanes 32 (w % 4) .., columns 8 (w / 4) .. */
   const int row = (warp & 3) * 32 + lane, ch = warp >> 2;
   const int m = m0 + row, n = n0 + 8 * ch;
@@ -347,6 +333,29 @@ __device__ __forceinline__ void tile_end(uint32_t tmem) {
   lbib_tc::tc_fence_before();
   __syncthreads();
   if (threadIdx.x < 32) lbib_tc::tmem_free<BN>(tmem);
+}
+
+/* FP32 rows [M][w] rounded into the chunk layout of `out` (C chunks a row, the
+ * rows up to a multiple of 128 and the columns past w zero): 32 rows of 8
+ * chunks a CTA, 256 bytes read and 64 written at a time. */
+constexpr int kInputRows = 32, kInputChunks = 8;
+__global__ void __launch_bounds__(kInputRows * kInputChunks) mlp_input(const float* __restrict__ X, int M, int w, int C,
+                                                                      __nv_bfloat16* __restrict__ out) {
+  lbib_tc::pdl_trigger();
+  const int nc = (C + kInputChunks - 1) / kInputChunks;
+  const int c = blockIdx.x % nc * kInputChunks + threadIdx.x % kInputChunks;
+  const long r = (long)(blockIdx.x / nc) * kInputRows + threadIdx.x / kInputChunks;
+  lbib_tc::pdl_wait();
+  if (c >= C) return;
+  const float* p = X + r * w + 8 * c;
+  float x[8];
+  if (r < M && 8 * c + 8 <= w && ((reinterpret_cast<uintptr_t>(X) | (uintptr_t)w * 4) & 15) == 0) {
+    load8(p, x);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = r < M && 8 * c + i < w ? p[i] : 0.0f;
+  }
+  *reinterpret_cast<uint4*>(out + ((r / BM * C + c) * BM + r % BM) * 8) = pack8(x);
 }
 
 /* A layer forward: C = A W^T + b and its epilogue, a CTA per tile.  At
@@ -546,10 +555,27 @@ Gemm product(Operand A, Operand B, int M, int N, int K) {
   return g;
 }
 
-/* Layer l forward of `batch` rows; layer 0 reads the caller's FP32 rows. */
+/* Layer 0 rounds up to kInlineInput columns of the caller's FP32 rows itself,
+ * in every column tile; wider ones are rounded once by a launch before it.  us
+ * of a forward, itself / launch before, batch 1024: 16 -> 64 columns 30.6 /
+ * 29.2 (batch 128: 27.2 / 28.3; training steps 22.0 / 23.1 and 16.4 / 16.6),
+ * 32 -> 64 35.1 / 29.2, 256 -> 256 47 / 37, 4096 -> 4096 2400 / 148. */
+constexpr int kInlineInput = 16;
+static_assert(kInlineInput <= BK, "one slice");
+bool inline_input(const lbib_mlp* n) { return n->wp[0] <= kInlineInput; }
+
+/* `batch` wider FP32 rows into act[0]. */
+int stage_input(lbib_mlp* n, const float* X, int batch) {
+  if (inline_input(n)) return 0;
+  const int C = n->wp[0] / 8;
+  const long blocks = align_up(batch, BM) / kInputRows * ((C + kInputChunks - 1) / kInputChunks);
+  return launch(mlp_input, (unsigned)blocks, kInputRows * kInputChunks, 0, n->stream, 1, X, batch, n->w[0], C, n->act[0]);
+}
+
+/* Layer l forward of `batch` rows; X: layer 0's input, if it reads it itself. */
 Gemm layer_product(lbib_mlp* n, int l, const float* X, int batch) {
   Gemm g = product(act_op(n, l, 0), w_op(n, l, 0), batch, n->wp[l + 1], n->wp[l]);
-  if (l == 0) { g.X = X; g.xw = n->w[0]; }
+  if (l == 0 && inline_input(n)) { g.X = X; g.xw = n->w[0]; }
   g.aux = n->p + n->boff[l];
   g.oC = n->wp[l + 1] / 8;
   if (l + 1 < n->L) g.out1 = n->act[l + 1];
@@ -558,6 +584,7 @@ Gemm layer_product(lbib_mlp* n, int l, const float* X, int batch) {
 
 /* Y [batch][w_L] of `batch` rows. */
 int forward(lbib_mlp* n, const float* X, int batch, float* Y) {
+  if (stage_input(n, X, batch)) return -2;
   for (int l = 0; l < n->L; ++l) {
     Gemm g = layer_product(n, l, X, batch);
     int rc;
@@ -576,9 +603,10 @@ int forward(lbib_mlp* n, const float* X, int batch, float* Y) {
  * layout), and the loss into n->d_loss when it is wanted. */
 int gradients(lbib_mlp* n, const float* X, const float* T, int batch, bool want_loss) {
   const int L = n->L;
+  if (stage_input(n, X, batch)) return -2;
   for (int l = 0; l < L; ++l) {
     Gemm g = layer_product(n, l, X, batch);
-    if (l == 0) g.copy = n->act[0];                     /* read again by dW of layer 0 */
+    if (l == 0 && g.X) g.copy = n->act[0];                     /* read again by dW of layer 0 */
     int rc;
     if (l + 1 < L) {
       g.out0 = n->z[l];
