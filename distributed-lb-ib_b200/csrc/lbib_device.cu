@@ -47,7 +47,6 @@ static void free_tiles(lbib_device* d) {
     cudaFree(d->Utile[b]); d->Utile[b] = NULL;
   }
   cudaFree(d->tile_mark); d->tile_mark = NULL;
-  cudaFree(d->scan_tmp); d->scan_tmp = NULL;
   cudaFree(d->scan_state); d->scan_state = NULL;
 }
 
@@ -365,7 +364,6 @@ extern "C" int lbdev_set_sheets(lbib_device* d, int nsheets, const lbib_sheet_de
     if (lbdev_is_slab(d)) {
       CK(cudaMalloc(&d->tile_mark, sizeof(int) * d->ntiles));
       CK(cudaMemsetAsync(d->tile_mark, 0, sizeof(int) * d->ntiles, d->stream));   /* the compaction keeps it at 0 */
-      CK(cudaMalloc(&d->scan_tmp, sizeof(int) * ((d->ntiles + 1023) / 1024 + 1)));
       CK(cudaMalloc(&d->scan_state, sizeof(unsigned long long) * ((d->ntiles + 1023) / 1024 + 1)));
       CK(cudaMemsetAsync(d->scan_state, 0, sizeof(unsigned long long) * ((d->ntiles + 1023) / 1024 + 1), d->stream));
     }

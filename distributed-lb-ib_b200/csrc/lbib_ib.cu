@@ -271,20 +271,11 @@ extern "C" int lbdev_launch_prep(lbib_device* d, int step) {
       slab ? nullptr : d->tile_list[c], d->tile_count[c], d->tile_mark, d->err, step, sf);
   d->kernel_launches++;
   if (slab) {
-    const unsigned nblk = (unsigned)((d->ntiles + kScanBlock - 1) / kScanBlock);
-    if (d->ntiles < (1L << 31)) {
-      d->scan_tag = d->scan_tag % 255u + 1u;
-      const unsigned nb1 = (unsigned)((d->ntiles + kScanBlock * kOnepassTiles - 1) / (kScanBlock * kOnepassTiles));
-      lbib_compact_onepass<<<nb1, kScanBlock, 0, st>>>(d->tile_mark, d->ntiles, (int)nb1, d->scan_state, d->scan_tag,
-                                                        d->tile_list[c], d->tile_slot[c], d->tile_count[c], d->err);
-      d->kernel_launches++;
-    } else {
-      lbib_compact_count<<<nblk, kScanBlock, 0, st>>>(d->tile_mark, d->ntiles, d->scan_tmp);
-      lbib_compact_scan<<<1, kScanBlock, 0, st>>>(d->scan_tmp, (int)nblk, d->tile_count[c]);
-      lbib_compact_write<<<nblk, kScanBlock, 0, st>>>(d->tile_mark, d->ntiles, d->scan_tmp, d->tile_list[c],
-                                                      d->tile_slot[c]);
-      d->kernel_launches += 3;
-    }
+    d->scan_tag = d->scan_tag % 255u + 1u;
+    const unsigned nb = (unsigned)((d->ntiles + kScanBlock * kOnepassTiles - 1) / (kScanBlock * kOnepassTiles));
+    lbib_compact_onepass<<<nb, kScanBlock, 0, st>>>(d->tile_mark, d->ntiles, (int)nb, d->scan_state, d->scan_tag,
+                                                     d->tile_list[c], d->tile_slot[c], d->tile_count[c], d->err);
+    d->kernel_launches++;
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

@@ -14,10 +14,9 @@
  *                       4^3 tiles the stencils touch, appended to the
  *                       step's tile list as they are met (or only marked,
  *                       for the compaction below).
- *   compaction kernels  x-slabs only: marked tiles -> dense list in tile
+ *   lbib_compact_onepass  x-slabs only: marked tiles -> dense list in tile
  *                       order and tile -> slot map (deterministic prefix
- *                       sums, three launches or one single-pass launch), so
- *                       that every slab numbers the slots alike.
+ *                       sums), so that every slab numbers the slots alike.
  *   gather_tile         fiber_SpreadForce + fluid_get_SpreadForce
  *                       (lbm_ib.c:1323-1525) as a gather: one CTA per touched
  *                       tile finds the nodes that touch it, in index order,
@@ -25,10 +24,10 @@
  *                       sums its contributions in that order -- the
  *                       reference's (sheet, row, col) order -- so the result
  *                       is deterministic and needs no atomics on forces.
- *   move_node /         moveFiberSheet (lbm_ib.c:2540-2723): u * w summed over
- *   move_warp           the 64 stencil cells in the reference's (x, y, z)
- *                       order, then X += dt U (move_warp: a warp's nodes
- *                       with their stencils' union staged in shared memory).
+ *   move_chunk          moveFiberSheet (lbm_ib.c:2540-2723): u * w summed over
+ *                       the 64 stencil cells in the reference's (x, y, z)
+ *                       order, then X += dt U, with the union of a chunk's
+ *                       stencils staged in shared memory.
  * All arithmetic keeps the reference's operation order; translation units
  * that include this file are compiled with -fmad=false, except that the
  * gather (explicitly rounded operations) is also used by the low-precision
@@ -286,79 +285,13 @@ __device__ __forceinline__ void node_prep_warp(const double* __restrict__ nodes,
   if (list) t.finish(slot, list, count);
 }
 
-/* Deterministic compaction of the marked tiles, in tile-index order:
- * per-block sums, a one-block scan, then every marked tile gets its slot. */
 constexpr int kScanBlock = 1024;
 
-static __global__ void lbib_compact_count(const int* __restrict__ mark, long n, int* __restrict__ block_tiles) {
-  __shared__ int s[32];
-  const long i = (long)blockIdx.x * kScanBlock + threadIdx.x;
-  int v = i < n && mark[i] != 0;
-  v = __reduce_add_sync(0xffffffffu, v);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int a = __reduce_add_sync(0xffffffffu, s[threadIdx.x]);
-    if (threadIdx.x == 0) block_tiles[blockIdx.x] = a;
-  }
-}
-
-static __global__ void lbib_compact_scan(int* __restrict__ a, int n, int* __restrict__ total) {
-  __shared__ int s[kScanBlock];
-  int carry = 0;
-  for (int base = 0; base < n; base += kScanBlock) {
-    const int i = base + threadIdx.x;
-    const int v = (i < n) ? a[i] : 0;
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 1; o < kScanBlock; o <<= 1) {
-      const int t = (threadIdx.x >= (unsigned)o) ? s[threadIdx.x - o] : 0;
-      __syncthreads();
-      s[threadIdx.x] += t;
-      __syncthreads();
-    }
-    if (i < n) a[i] = carry + s[threadIdx.x] - v;
-    const int last = s[kScanBlock - 1];
-    __syncthreads();
-    carry += last;
-  }
-  if (threadIdx.x == 0) *total = carry;
-}
-
-static __global__ void lbib_compact_write(int* __restrict__ mark, long n, const int* __restrict__ block_tiles,
-                                          int* __restrict__ list, int* __restrict__ slot) {
-  __shared__ int sv[32];
-  const long i = (long)blockIdx.x * kScanBlock + threadIdx.x;
-  const int v = i < n && mark[i] != 0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned m = __ballot_sync(0xffffffffu, v);
-  if (lane == 0) sv[warp] = __popc(m);
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int a = sv[threadIdx.x];
-    int ia = a;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int ta = __shfl_up_sync(0xffffffffu, ia, o);
-      if (lane >= o) ia += ta;
-    }
-    sv[threadIdx.x] = ia - a;
-  }
-  __syncthreads();
-  if (v) {
-    const int pos = block_tiles[blockIdx.x] + sv[warp] + __popc(m & ((1u << lane) - 1u));
-    list[pos] = (int)i;
-    slot[i] = pos;
-    mark[i] = 0;      /* the next step starts unmarked */
-  } else if (i < n) {
-    slot[i] = -1;     /* the whole map is written: no clearing pass before the step */
-  }
-}
-
-/* The same compaction in one launch: a single-pass scan with decoupled
- * look-back (Merrill & Garland, "Single-pass Parallel Prefix Scan with
- * Decoupled Look-back", 2016).  A block takes its place in tile order from
- * a ticket counter (so every block before it has started), publishes its
- * block total, walks back over its predecessors' published totals until
+/* Deterministic compaction of the marked tiles, in tile-index order, in one
+ * launch: a single-pass scan with decoupled look-back (Merrill & Garland,
+ * "Single-pass Parallel Prefix Scan with Decoupled Look-back", 2016).  A block
+ * takes its place in tile order from a ticket counter (so every block before
+ * it has started), publishes its block total, walks back over its predecessors' published totals until
  * one carries an inclusive prefix, publishes its own inclusive prefix and
  * writes its tiles' slots.  Each published word is 64 bits: an 8-bit
  * launch tag (1..255, never 0, so a zeroed or stale word never matches),
@@ -790,57 +723,14 @@ __device__ __forceinline__ void gather_tile(GatherShared& sh, const GatherNodes&
   }
 }
 
-/* moveFiberSheet for node i; slot maps local tiles to global slots. */
-__device__ __forceinline__ void move_node(double* __restrict__ nodes, const double* __restrict__ W,
-                                          const int* __restrict__ st, long i, int ntx, int nty,
-                                          const int* __restrict__ slot, const double* __restrict__ Utile, double dt) {
-  const double c_64 = 1.0 / (6.4e1);
-  const int is = st[i * 3 + 0], js = st[i * 3 + 1], ks = st[i * 3 + 2];
-  const double* w = W + i * 12;
-  /* the stencil spans at most 2 tiles per axis: look their slots up first,
-     so that the 64 cells' loads below do not wait on one another */
-  const int tx0 = is >> 2, ty0 = js >> 2, tz0 = ks >> 2;
-  int sp8[8];
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const int tx = tx0 + (a & 1), ty = ty0 + ((a >> 1) & 1), tz = tz0 + (a >> 2);
-    const bool need = tx * 4 <= is + 3 && ty * 4 <= js + 3 && tz * 4 <= ks + 3;
-    sp8[a] = need ? slot[(tz * nty + ty) * ntx + tx] : 0;
-  }
-  double s1 = 0, s2 = 0, s3 = 0;
-#pragma unroll
-  for (int i2 = 0; i2 <= 3; i2++) {
-    const int gi = is + i2;
-#pragma unroll
-    for (int j2 = 0; j2 <= 3; j2++) {
-      const int gj = js + j2;
-#pragma unroll
-      for (int k2 = 0; k2 <= 3; k2++) {
-        const int gk = ks + k2;
-        const int sp = sp8[((gi >> 2) - tx0) | (((gj >> 2) - ty0) << 1) | (((gk >> 2) - tz0) << 2)];
-        const double* U = Utile + (long)sp * 256;
-        const int cell = lbib::cell_in_tile(gi, gj, gk);
-        const double vx = U[64 + cell], vy = U[128 + cell], vz = U[192 + cell];
-        s1 += vx * w[i2] * w[4 + j2] * w[8 + k2] * c_64;
-        s2 += vy * w[i2] * w[4 + j2] * w[8 + k2] * c_64;
-        s3 += vz * w[i2] * w[4 + j2] * w[8 + k2] * c_64;
-      }
-    }
-  }
-  double* m = nodes + i * 12;
-  m[0] += dt * s1;
-  m[1] += dt * s2;
-  m[2] += dt * s3;
-}
-
-
 /* A move CTA: the 32 nodes of a chunk, four warps. */
 constexpr int kMoveTPB = 128;
 /* Cells a CTA's staged move holds in shared memory: the union box of its 32
- * nodes' stencils (along a fiber row ~5 x 20 x 5 cells); a group of nodes
- * with a larger union (a crumpled sheet) takes move_node. */
+ * nodes' stencils (along a fiber row ~5 x 20 x 5 cells).  Nodes whose starts
+ * differ by 1 from one node's always fit. */
 constexpr int kMoveCap = 640;
 constexpr int kMoveTiles = 64;   /* tiles of the union box whose slots are staged */
+static_assert(6 * 6 * 6 <= kMoveCap && 3 * 3 * 3 <= kMoveTiles, "a group of reach 1");
 
 struct MoveSmem {
   double U[3][kMoveCap];
@@ -851,11 +741,11 @@ struct MoveSmem {
  * `live` if it moves), with the velocity of the union box of their stencils
  * staged once in shared memory: the four warps read each box cell's u from
  * its moment tile, then warp a < 3 sums component a of every node's 64
- * terms from shared memory -- the same values in the same order as
- * move_node, with ~5x fewer L2 requests (neighbouring nodes' stencils
- * overlap by 3 cells of 4).  A node's sum is a serial chain of 64 terms, so
- * a thread holds one component only; with one warp that staged and summed
- * all three for its nodes the launch took 10 us at 16 x 16 nodes, this 6.
+ * terms from shared memory, with ~5x fewer L2 requests than a node at a time
+ * (neighbouring nodes' stencils overlap by 3 cells of 4).  A node's sum is a
+ * serial chain of 64 terms, so a thread holds one component only; with one
+ * warp that staged and summed all three for its nodes the launch took 10 us
+ * at 16 x 16 nodes, this 6.
  * Nodes whose stencils lie too far apart for one box (a chunk that straddles
  * two rows of its sheet) are taken in groups near one another.  Called by
  * all kMoveTPB threads; ends with a barrier. */
@@ -880,18 +770,17 @@ __device__ __forceinline__ void move_chunk(MoveSmem& sm, double* __restrict__ no
   bool now = live;   /* the lane's node is in the group being moved */
   int reach = 16;
   while (left) {
-  const int x0 = __reduce_min_sync(0xffffffffu, now ? is : INT_MAX), x1 = __reduce_max_sync(0xffffffffu, now ? is + 3 : INT_MIN);
-  const int y0 = __reduce_min_sync(0xffffffffu, now ? js : INT_MAX), y1 = __reduce_max_sync(0xffffffffu, now ? js + 3 : INT_MIN);
-  const int z0 = __reduce_min_sync(0xffffffffu, now ? ks : INT_MAX), z1 = __reduce_max_sync(0xffffffffu, now ? ks + 3 : INT_MIN);
-  const int bx = x1 - x0 + 1, by = y1 - y0 + 1, bz = z1 - z0 + 1;
-  const long vol = (long)bx * by * bz;
-  const int tx0 = x0 >> 2, ty0 = y0 >> 2, tz0 = z0 >> 2;
-  const int tbx = (x1 >> 2) - tx0 + 1, tby = (y1 >> 2) - ty0 + 1;
-  const long ntb = (long)tbx * tby * ((z1 >> 2) - tz0 + 1);
-  if (vol > kMoveCap || ntb > kMoveTiles) {
-    /* too large: the nodes within `reach` of the first one, nearer and
-       nearer until the box fits, or, at the end, each on its own */
-    if (reach > 0) {
+    const int x0 = __reduce_min_sync(0xffffffffu, now ? is : INT_MAX), x1 = __reduce_max_sync(0xffffffffu, now ? is + 3 : INT_MIN);
+    const int y0 = __reduce_min_sync(0xffffffffu, now ? js : INT_MAX), y1 = __reduce_max_sync(0xffffffffu, now ? js + 3 : INT_MIN);
+    const int z0 = __reduce_min_sync(0xffffffffu, now ? ks : INT_MAX), z1 = __reduce_max_sync(0xffffffffu, now ? ks + 3 : INT_MIN);
+    const int bx = x1 - x0 + 1, by = y1 - y0 + 1, bz = z1 - z0 + 1;
+    const long vol = (long)bx * by * bz;
+    const int tx0 = x0 >> 2, ty0 = y0 >> 2, tz0 = z0 >> 2;
+    const int tbx = (x1 >> 2) - tx0 + 1, tby = (y1 >> 2) - ty0 + 1;
+    const long ntb = (long)tbx * tby * ((z1 >> 2) - tz0 + 1);
+    if (vol > kMoveCap || ntb > kMoveTiles) {
+      /* too large: the nodes within `reach` of the first one, nearer and
+         nearer until the box fits (at the latest at 1) */
       const int f = __ffs(left) - 1;
       const int fx = __shfl_sync(0xffffffffu, is, f), fy = __shfl_sync(0xffffffffu, js, f),
                 fz = __shfl_sync(0xffffffffu, ks, f);
@@ -899,56 +788,53 @@ __device__ __forceinline__ void move_chunk(MoveSmem& sm, double* __restrict__ no
       reach >>= 1;
       continue;
     }
-    if (now && warp == 0) move_node(nodes, W, st, i, ntx, nty, slot, Utile, dt);
-  } else {
-  /* the slots of the box's tiles first (at most 3 x 7 x 3 for a box that
-     fits), so that the cell loads below depend on one shared-memory read */
-  if (t < (int)ntb) {
-    const int tx = tx0 + t % tbx, ty = ty0 + (t / tbx) % tby, tz = tz0 + t / (tbx * tby);
-    sm.slot[t] = slot[(tz * nty + ty) * ntx + tx];
-  }
-  __syncthreads();
-  /* the box's longest axis (the fiber direction: neighbouring lanes'
-     stencils are offset along it) is stored fastest, so that the lanes'
-     reads below fall on consecutive words, not on one bank */
-  const int f = (bx >= by && bx >= bz) ? 0 : (by >= bz ? 1 : 2);
-  const int ef = f == 0 ? bx : f == 1 ? by : bz, ea = f == 0 ? by : bx;
-  const int sx = f == 0 ? 1 : ef, sy = f == 1 ? 1 : f == 0 ? ef : ef * ea, sz = f == 2 ? 1 : ef * ea;
-  /* j / ef and j / ea by reciprocals: exact for j < 640, divisors < 100 */
-  const unsigned rf = (65535u + ef) / ef, ra = (65535u + ea) / ea;
-#pragma unroll 5
-  for (int j = t; j < (int)vol; j += kMoveTPB) {   /* 640 / 128: the loads of all rounds in flight */
-    const int q = ef < 100 ? (int)(j * rf >> 16) : j / ef, uf = j - q * ef;
-    const int ub = ea < 100 ? (int)(q * ra >> 16) : q / ea, ua = q - ub * ea;
-    const int cx = x0 + (f == 0 ? uf : ua), cy = y0 + (f == 1 ? uf : f == 0 ? ua : ub), cz = z0 + (f == 2 ? uf : ub);
-    /* a box corner no stencil covers may lie in an untouched tile: never read */
-    const int sp = sm.slot[((cz >> 2) - tz0) * tbx * tby + ((cy >> 2) - ty0) * tbx + ((cx >> 2) - tx0)];
-    double vx = 0.0, vy = 0.0, vz = 0.0;
-    if (sp >= 0) {
-      const double* U = Utile + (long)sp * 256 + lbib::cell_in_tile(cx, cy, cz);
-      vx = U[64]; vy = U[128]; vz = U[192];
+    /* the slots of the box's tiles first (at most 3 x 7 x 3 for a box that
+       fits), so that the cell loads below depend on one shared-memory read */
+    if (t < (int)ntb) {
+      const int tx = tx0 + t % tbx, ty = ty0 + (t / tbx) % tby, tz = tz0 + t / (tbx * tby);
+      sm.slot[t] = slot[(tz * nty + ty) * ntx + tx];
     }
-    sm.U[0][j] = vx; sm.U[1][j] = vy; sm.U[2][j] = vz;
-  }
-  __syncthreads();
-  if (now && warp < 3) {
-    const double c_64 = 1.0 / (6.4e1);
-    const double* u = sm.U[warp] + (is - x0) * sx + (js - y0) * sy + (ks - z0) * sz;
-    double s = 0;
+    __syncthreads();
+    /* the box's longest axis (the fiber direction: neighbouring lanes'
+       stencils are offset along it) is stored fastest, so that the lanes'
+       reads below fall on consecutive words, not on one bank */
+    const int f = (bx >= by && bx >= bz) ? 0 : (by >= bz ? 1 : 2);
+    const int ef = f == 0 ? bx : f == 1 ? by : bz, ea = f == 0 ? by : bx;
+    const int sx = f == 0 ? 1 : ef, sy = f == 1 ? 1 : f == 0 ? ef : ef * ea, sz = f == 2 ? 1 : ef * ea;
+    /* j / ef and j / ea by reciprocals: exact for j < 640, divisors < 100 */
+    const unsigned rf = (65535u + ef) / ef, ra = (65535u + ea) / ea;
+#pragma unroll 5
+    for (int j = t; j < (int)vol; j += kMoveTPB) {   /* 640 / 128: the loads of all rounds in flight */
+      const int q = ef < 100 ? (int)(j * rf >> 16) : j / ef, uf = j - q * ef;
+      const int ub = ea < 100 ? (int)(q * ra >> 16) : q / ea, ua = q - ub * ea;
+      const int cx = x0 + (f == 0 ? uf : ua), cy = y0 + (f == 1 ? uf : f == 0 ? ua : ub), cz = z0 + (f == 2 ? uf : ub);
+      /* a box corner no stencil covers may lie in an untouched tile: never read */
+      const int sp = sm.slot[((cz >> 2) - tz0) * tbx * tby + ((cy >> 2) - ty0) * tbx + ((cx >> 2) - tx0)];
+      double vx = 0.0, vy = 0.0, vz = 0.0;
+      if (sp >= 0) {
+        const double* U = Utile + (long)sp * 256 + lbib::cell_in_tile(cx, cy, cz);
+        vx = U[64]; vy = U[128]; vz = U[192];
+      }
+      sm.U[0][j] = vx; sm.U[1][j] = vy; sm.U[2][j] = vz;
+    }
+    __syncthreads();
+    if (now && warp < 3) {
+      const double c_64 = 1.0 / (6.4e1);
+      const double* u = sm.U[warp] + (is - x0) * sx + (js - y0) * sy + (ks - z0) * sz;
+      double s = 0;
 #pragma unroll
-    for (int i2 = 0; i2 <= 3; i2++)
+      for (int i2 = 0; i2 <= 3; i2++)
 #pragma unroll
-      for (int j2 = 0; j2 <= 3; j2++)
+        for (int j2 = 0; j2 <= 3; j2++)
 #pragma unroll
-        for (int k2 = 0; k2 <= 3; k2++)
-          s += u[i2 * sx + j2 * sy + k2 * sz] * w[i2] * w[4 + j2] * w[8 + k2] * c_64;
-    nodes[i * 12 + warp] = at + dt * s;
-  }
-  }
-  left &= ~__ballot_sync(0xffffffffu, now);
-  now = (left >> (t & 31)) & 1u;
-  reach = 16;
-  __syncthreads();
+          for (int k2 = 0; k2 <= 3; k2++)
+            s += u[i2 * sx + j2 * sy + k2 * sz] * w[i2] * w[4 + j2] * w[8 + k2] * c_64;
+      nodes[i * 12 + warp] = at + dt * s;
+    }
+    left &= ~__ballot_sync(0xffffffffu, now);
+    now = (left >> (t & 31)) & 1u;
+    reach = 16;
+    __syncthreads();
   }
 }
 

@@ -111,7 +111,6 @@ typedef struct lbib_device {
   int* tile_count[2];            /* [1]                                       */
   int tiles_left[2];             /* whole grids: what the last spread into the buffer left
                                     there: LBIB_TILES_ALL, _LIST or 0 (nothing)  */
-  int* scan_tmp;                 /* x-slabs: block sums for the compaction    */
   unsigned long long* scan_state; /* one-pass compaction: per-block words + ticket */
   unsigned scan_tag;             /* the one-pass compaction's launch tag (1..255) */
   double* Ftile[2];              /* [cap][3][64]                              */
