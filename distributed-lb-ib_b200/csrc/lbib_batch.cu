@@ -576,7 +576,9 @@ lbib_batch* lbib_batch_create(int n, const lbib_problem* problems, int precision
     return NULL;
   for (int k = 0; k < n; ++k) {
     const lbib_problem* p = problems + k;
-    if (p->nx < 8 || p->ny < 8 || p->nz < 8 || p->nx % 4 || p->ny % 4 || p->nz % 4 || p->rows < 2 || p->cols < 2 ||
+    /* fewer than 4 nodes: the bending formulas (node 0 reads 2, node 1 reads 3) would
+       leave the sheet, and the last problem's the pool */
+    if (p->nx < 8 || p->ny < 8 || p->nz < 8 || p->nx % 4 || p->ny % 4 || p->nz % 4 || p->rows < 4 || p->cols < 4 ||
         !(p->tau > 0.5))
       return NULL;
   }

@@ -485,7 +485,7 @@ int lbib_spread_force_noalloc(const double* nodes, long num_nodes, int nx, int n
 typedef struct lbib_problem {
   int nx, ny, nz;                  /* lattice, x = flow direction            */
   double tau, u_l, Ks_l, Kb_l;
-  int rows, cols;                  /* the sheet, as Fibersheet               */
+  int rows, cols;                  /* the sheet, as Fibersheet; at least 4 each */
   double width, height, x0, y0, z0;
   int pinned;                      /* 1: row 0 of the sheet does not move (a
                                       flap hinged at its leading edge; not in
