@@ -278,12 +278,15 @@ int lp_spread_box(lbib_device* d) {
   return launch_spread_box_t<T>(d, p);
 }
 
-/* The variant of a state that has not been autotuned: by the autotuner's
- * times at three sizes.  us per fluid step, {4,3} / {2,6} / {4,5} / {4,5}
- * even with {8,4} odd: 21 20 21 23 at 64x32x32, 28 28 29 28 at 128x64x64,
- * 135 127 107 107 at 256x128x128, 942 766 682 657 at 512x256x256 (FP16);
- * FP32, {2,3} {2,4} {2,5}: 33 30 30, 182 159 148 and 1158 1024 966 at the
- * last three. */
+/* The variant of a state that has not been autotuned.  us per fluid step by
+ * the autotuner, FP16, {4,3} / {2,6} / {4,5} / {4,5} even with {8,4} odd: 21
+ * 20 21 23 at 64x32x32, 28 28 29 28 at 128x64x64, 135 127 107 107 at
+ * 256x128x128, 942 766 682 657 at 512x256x256; FP32, {2,3} {2,4} {2,5}: 33 30
+ * 30, 182 159 148 and 1158 1024 966 at the last three.  Whole steps between
+ * those sizes, FP16 in the same order: 56 54 53 54 at 160x80x80, 60 58 54 55
+ * at 160x84x84, 73 70 65 66 at 192x96x96, 428 362 333 332 at 384x192x192, so
+ * that the line at 2^20 cells costs at most a microsecond or two on either
+ * side; BF16 is within 2% of FP16 at every size and variant. */
 template <typename T>
 int default_variant(const lbib_device* d) {
   if (sizeof(T) == 4) return 2;
