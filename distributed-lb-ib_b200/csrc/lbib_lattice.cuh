@@ -361,12 +361,11 @@ __device__ __forceinline__ bool div_safe(double v) {
  * c_d = -1, 0, 1 per axis, and B / cs^4 C per opposite pair (both signs
  * change).  Dropping the products with c_d = 0 from B and C changes finite
  * ones by a signed zero at most; operands that are not finite (0 times them
- * is NaN) take guo_as_written. */
+ * is NaN) take collide_rare. */
 template <typename R>
 struct Relax {
   R t6, om, it;
   R px[3], py[3], pz[3];   /* (c_d - u_d) F_d, c_d = -1, 0, 1 */
-  R ux, uy, uz, Fx, Fy, Fzg;   /* guo_as_written's */
 };
 
 /* The constants of a collision; cs2_inv, cs4_inv as div_const takes them. */
@@ -375,22 +374,11 @@ struct CollideConst {
   R om, it, kw0, kw1, kw2, cs2, cs4, cs2_inv, cs4_inv, g;
 };
 
-/* The term with every product and with true divisions. */
-template <typename R>
-__device__ __forceinline__ R guo_as_written(int q, const Relax<R>& r, const CollideConst<R>& p) {
-  const R c0 = (R)cx(q), c1 = (R)cy(q), c2 = (R)cz(q);
-  const R kw = q == 0 ? p.kw0 : q <= 6 ? p.kw1 : p.kw2;
-  const R A = (c0 - r.ux) * r.Fx + (c1 - r.uy) * r.Fy + (c2 - r.uz) * r.Fzg;
-  const R B = c0 * r.ux + c1 * r.uy + c2 * r.uz;
-  const R C = c0 * r.Fx + c1 * r.Fy + c2 * r.Fzg;
-  return kw * (A / p.cs2 + B / p.cs4 * C);
-}
-
 /* One opposite pair (qa, qb) with c_qa . u = cu: both equilibria share
  * 3cu, cu^2 and 1.5 u^2, and 1 + (-3cu) == 1 - 3cu exactly.  With a force
  * (c_qa . F = cF) the Guo term is added after the relaxation, as the
  * reference sums it. */
-template <bool FORCED, bool FAST, int QA, int QB, typename R>
+template <bool FORCED, int QA, int QB, typename R>
 __device__ __forceinline__ void relax_pair(R* f, R cu, R cF, R wr, const Relax<R>& r, const CollideConst<R>& p) {
   const R a3 = R(3.0) * cu;
   const R sq = R(4.5) * (cu * cu);
@@ -398,10 +386,7 @@ __device__ __forceinline__ void relax_pair(R* f, R cu, R cF, R wr, const Relax<R
   const R eb = wr * (R(1.0) + (-a3) + sq - r.t6);
   R va = f[QA] * r.om + r.it * ea;
   R vb = f[QB] * r.om + r.it * eb;
-  if constexpr (FORCED && !FAST) {
-    va = va + guo_as_written(QA, r, p);
-    vb = vb + guo_as_written(QB, r, p);
-  } else if constexpr (FORCED) {
+  if constexpr (FORCED) {
     const R kw = QA <= 6 ? p.kw1 : p.kw2;
     const R bc = div_const(cu, p.cs4, p.cs4_inv) * cF;
     const R Aa = r.px[cx(QA) + 1] + r.py[cy(QA) + 1] + r.pz[cz(QA) + 1];
@@ -413,14 +398,12 @@ __device__ __forceinline__ void relax_pair(R* f, R cu, R cF, R wr, const Relax<R
   f[QB] = vb;
 }
 
-template <bool FORCED, bool FAST, typename R>
+template <bool FORCED, typename R>
 __device__ __forceinline__ void collide_body(R f[19], R rho, R ux, R uy, R uz, R Fx, R Fy, R Fz,
                                              const CollideConst<R>& p) {
   Relax<R> r;
   const R Fzg = FORCED ? Fz + rho * p.g : R(0);
-  if constexpr (FORCED && !FAST) {
-    r.ux = ux; r.uy = uy; r.uz = uz; r.Fx = Fx; r.Fy = Fy; r.Fzg = Fzg;
-  } else if constexpr (FORCED) {
+  if constexpr (FORCED) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       const R c = R(k - 1);
@@ -435,25 +418,50 @@ __device__ __forceinline__ void collide_body(R f[19], R rho, R ux, R uy, R uz, R
   const R wr1 = R(1.0 / 18.0) * rho;
   const R wr2 = R(1.0 / 36.0) * rho;
   R v0 = f[0] * r.om + r.it * (wr0 * (R(1.0) - r.t6));
-  if constexpr (FORCED && !FAST) v0 = v0 + guo_as_written(0, r, p);
-  else if constexpr (FORCED) v0 = v0 + p.kw0 * div_const(r.px[1] + r.py[1] + r.pz[1], p.cs2, p.cs2_inv);
+  if constexpr (FORCED) v0 = v0 + p.kw0 * div_const(r.px[1] + r.py[1] + r.pz[1], p.cs2, p.cs2_inv);
   f[0] = v0;
-  relax_pair<FORCED, FAST, 1, 2>(f, ux, Fx, wr1, r, p);
-  relax_pair<FORCED, FAST, 3, 4>(f, uz, Fzg, wr1, r, p);
-  relax_pair<FORCED, FAST, 6, 5>(f, uy, Fy, wr1, r, p);
-  relax_pair<FORCED, FAST, 7, 8>(f, ux + uz, Fx + Fzg, wr2, r, p);
-  relax_pair<FORCED, FAST, 9, 10>(f, ux - uz, Fx - Fzg, wr2, r, p);
-  relax_pair<FORCED, FAST, 11, 12>(f, uz - uy, Fzg - Fy, wr2, r, p);
-  relax_pair<FORCED, FAST, 13, 14>(f, uy + uz, Fy + Fzg, wr2, r, p);
-  relax_pair<FORCED, FAST, 15, 16>(f, ux - uy, Fx - Fy, wr2, r, p);
-  relax_pair<FORCED, FAST, 17, 18>(f, ux + uy, Fx + Fy, wr2, r, p);
+  relax_pair<FORCED, 1, 2>(f, ux, Fx, wr1, r, p);
+  relax_pair<FORCED, 3, 4>(f, uz, Fzg, wr1, r, p);
+  relax_pair<FORCED, 6, 5>(f, uy, Fy, wr1, r, p);
+  relax_pair<FORCED, 7, 8>(f, ux + uz, Fx + Fzg, wr2, r, p);
+  relax_pair<FORCED, 9, 10>(f, ux - uz, Fx - Fzg, wr2, r, p);
+  relax_pair<FORCED, 11, 12>(f, uz - uy, Fzg - Fy, wr2, r, p);
+  relax_pair<FORCED, 13, 14>(f, uy + uz, Fy + Fzg, wr2, r, p);
+  relax_pair<FORCED, 15, 16>(f, ux - uy, Fx - Fy, wr2, r, p);
+  relax_pair<FORCED, 17, 18>(f, ux + uy, Fx + Fy, wr2, r, p);
 }
 
-/* The collision of a forced cell by true divisions: operands that div_const
- * does not take (not finite, or beyond any flow). */
+/* The collision of a forced cell with operands that div_const does not take
+ * (not finite, or beyond any flow): every product of the Guo term and true
+ * divisions, as lbm_ib.c:1740-1754 writes it.  In memory and one direction at
+ * a time: what the call needs in registers its callers have to spare, and the
+ * pair kernel, which hardly ever gets here, has none (unrolled over the
+ * directions: 588 bytes of spills there, 111.1 against 105.1 ms for 50 steps
+ * at 512x256x256). */
 template <typename R>
-__device__ __noinline__ void collide_rare(R* f, R rho, R ux, R uy, R uz, R Fx, R Fy, R Fz, CollideConst<R> c) {
-  collide_body<true, false>(f, rho, ux, uy, uz, Fx, Fy, Fz, c);
+struct RareCell {
+  R f[19], rho, ux, uy, uz, Fx, Fy, Fzg;
+  CollideConst<R> c;
+};
+
+template <typename R>
+__device__ __noinline__ void collide_rare(RareCell<R>* a) {
+  const CollideConst<R>& c = a->c;
+#pragma unroll 1
+  for (int q = 0; q < 19; ++q) {
+    const R ux = a->ux, uy = a->uy, uz = a->uz, Fx = a->Fx, Fy = a->Fy, Fzg = a->Fzg;
+    const R c0 = (R)cx(q), c1 = (R)cy(q), c2 = (R)cz(q);
+    const R t6 = R(1.5) * (ux * ux + uy * uy + uz * uz);
+    /* c . u of the components that count: at most two, 0 + v is v */
+    const R cu = (cx(q) ? c0 * ux : R(0)) + (cy(q) ? c1 * uy : R(0)) + (cz(q) ? c2 * uz : R(0));
+    const R w = q == 0 ? R(1.0 / 3.0) : q <= 6 ? R(1.0 / 18.0) : R(1.0 / 36.0);
+    const R kw = q == 0 ? c.kw0 : q <= 6 ? c.kw1 : c.kw2;
+    const R e = w * a->rho * (R(1.0) + R(3.0) * cu + R(4.5) * (cu * cu) - t6);
+    const R A = (c0 - ux) * Fx + (c1 - uy) * Fy + (c2 - uz) * Fzg;
+    const R B = c0 * ux + c1 * uy + c2 * uz;
+    const R C = c0 * Fx + c1 * Fy + c2 * Fzg;
+    a->f[q] = a->f[q] * c.om + c.it * e + kw * (A / c.cs2 + B / c.cs4 * C);
+  }
 }
 
 /* compute_eqlbrmdistrfuncDF1, cube_pthread/lbm_ib.c:1713-1807: equilibrium
@@ -470,16 +478,17 @@ __device__ __forceinline__ void collide(R f[19], R rho, R ux, R uy, R uz, R Fx, 
     const R Fzg = Fz + rho * c.g;
     if (!(div_safe(ux) && div_safe(uy) && div_safe(uz) && div_safe(Fx) && div_safe(Fy) && div_safe(Fzg) &&
           c.cs2_inv != 0.0 && c.cs4_inv != 0.0)) {
-      R h[19];   /* a copy: f stays in registers on the other path */
+      RareCell<R> a;   /* a copy: f stays in registers on the other path */
+      a.rho = rho; a.ux = ux; a.uy = uy; a.uz = uz; a.Fx = Fx; a.Fy = Fy; a.Fzg = Fzg; a.c = c;
 #pragma unroll
-      for (int q = 0; q < 19; ++q) h[q] = f[q];
-      collide_rare(h, rho, ux, uy, uz, Fx, Fy, Fz, c);
+      for (int q = 0; q < 19; ++q) a.f[q] = f[q];
+      collide_rare(&a);
 #pragma unroll
-      for (int q = 0; q < 19; ++q) f[q] = h[q];
+      for (int q = 0; q < 19; ++q) f[q] = a.f[q];
       return;
     }
   }
-  collide_body<FORCED, true>(f, rho, ux, uy, uz, Fx, Fy, Fz, c);
+  collide_body<FORCED>(f, rho, ux, uy, uz, Fx, Fy, Fz, c);
 }
 
 /* Cell (x, y, z) lies in a tile of the box (box mode). */
