@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kGatherTPB, sizeof(T) == 8 ? 4 : 5) lbib_b_gat
                                                                     const int* __restrict__ tile_inst,
                                                                     double* __restrict__ Ftile,
                                                                     const int* __restrict__ err) {
-  __shared__ GatherShared sm;
+  __shared__ GatherSmem sm;
   const int n = *count, t = threadIdx.x;
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
     const int k = tile_inst[list[i]];

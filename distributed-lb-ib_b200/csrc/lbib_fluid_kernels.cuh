@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kGatherTPB, 4) lbib_spread_box(FluidParamsT<T>
                                                                  int* __restrict__ reset,
                                                                  int* __restrict__ super_next, long nsuper,
                                                                  const int* err) {
-  __shared__ GatherShared sm;
+  __shared__ GatherSmem sm;
   /* the next step's box starts empty; the move fills it (it runs after us) */
   if (reset && blockIdx.x == 0 && threadIdx.x < 6) reset[threadIdx.x] = (threadIdx.x & 1) ? INT_MIN : INT_MAX;
   clear_super(super_next, nsuper);

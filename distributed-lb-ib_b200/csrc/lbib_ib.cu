@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kGatherTPB) lbib_spread_gather(GatherNodes g, 
                                                                  int tlo, int thi, double* __restrict__ Ftile,
                                                                  int* __restrict__ super_next, long nsuper,
                                                                  const int* err) {
-  __shared__ GatherShared sm;
+  __shared__ GatherSmem sm;
   clear_super(super_next, nsuper);
   if (*(volatile const int*)err) return;
   const int n = *count;

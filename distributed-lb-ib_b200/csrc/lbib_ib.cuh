@@ -424,11 +424,12 @@ __device__ __forceinline__ unsigned long long stencil_tile_mask(int dx, int dy, 
  * the nodes. */
 constexpr int kGatherTPB = 128;
 constexpr int kGatherWarps = kGatherTPB / 32;
-constexpr int kHitCap = 256;     /* chunks whose box meets the tile  */
+constexpr int kHitCap = 256;     /* chunks whose box meets the tile, at once */
 constexpr int kOffHits = 64;     /* of those, with the starts kept   */
 constexpr int kHitsAhead = 8;
-constexpr int kListCap = 1024;   /* nodes whose stencil meets it     */
+constexpr int kListCap = 1024;   /* nodes whose stencil meets it, at once */
 constexpr int kBatch = 64;       /* nodes staged at once             */
+static_assert(kHitCap >= kGatherTPB && kListCap >= 32, "a round of candidates, a chunk");
 
 /* A staged node: its x, y and z delta weights at the tile's four cell
  * positions per axis (unset where the stencil misses the position: no cell
@@ -439,13 +440,12 @@ struct GatherSmem {
   int hit[kHitCap];                     /* chunks in index order               */
   unsigned mask[kHitCap];               /* the nodes of each that touch        */
   unsigned short hoff[kOffHits][32];    /* their stencil starts, the first chunks' */
-  int pos[kHitCap];                     /* their places in ids                 */
+  int pos[kHitCap + 1];                 /* nodes before each                   */
   int ids[kListCap];                    /* the tile's nodes in index order     */
   int off[kListCap];                    /* their stencil starts from the tile's origin */
   unsigned cover[2][2][kBatch];         /* per staged node: cells 0..31, 32..63 */
   alignas(16) double rec[2][kBatch * kNodeRec];
   int warp_n[kGatherWarps];
-  int n;
 };
 
 __device__ __forceinline__ bool box_meets(const int* __restrict__ b, int x0, int y0, int z0) {
@@ -480,8 +480,8 @@ __device__ __forceinline__ void clear_super(int* __restrict__ super, long n) {
 }
 
 /* The CTA's threads with `flag` set append `value` in thread order to
- * out[*n ..) (up to cap); *n grows by their number.  Ends with a barrier. */
-__device__ __forceinline__ void append_in_order(GatherSmem& sm, bool flag, int value, int* out, int cap, int& n) {
+ * out[n ..) (up to kHitCap); n grows by their number.  Ends with a barrier. */
+__device__ __forceinline__ void append_in_order(GatherSmem& sm, bool flag, int value, int* out, int& n) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned m = __ballot_sync(0xffffffffu, flag);
   if (lane == 0) sm.warp_n[warp] = __popc(m);
@@ -491,7 +491,7 @@ __device__ __forceinline__ void append_in_order(GatherSmem& sm, bool flag, int v
   for (int w = 0; w < kGatherWarps; ++w) {
     if (w == warp && flag) {
       const int k = at + __popc(m & ((1u << lane) - 1u));
-      if (k < cap) out[k] = value;
+      if (k < kHitCap) out[k] = value;
     }
     at += sm.warp_n[w];
   }
@@ -499,35 +499,39 @@ __device__ __forceinline__ void append_in_order(GatherSmem& sm, bool flag, int v
   __syncthreads();
 }
 
-/* The nodes that touch the tile at (x0, y0, z0), in index order, into
- * sm.ids; returns their number, or -1 when a list overflows (a crumpled
- * sheet).  Boxes of 1024 nodes first (sheets of more than 128 chunks),
- * then of 32, then the nodes themselves: every level is a handful of
- * coalesced loads per CTA, nothing is sorted, and no list has to be built
- * beforehand. */
-__device__ __forceinline__ int gather_list(GatherSmem& sm, const GatherNodes& g, int x0, int y0, int z0) {
+/* The chunks whose box meets the tile at (x0, y0, z0), in index order, into
+ * sm.hit; returns their number, above kHitCap when they do not fit.  Boxes of
+ * 1024 nodes first (sheets of more than 128 chunks), then of 32. */
+__device__ __forceinline__ int gather_chunks(GatherSmem& sm, const GatherNodes& g, int x0, int y0, int z0) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   int nh = 0;
   if (!g.super || g.c_hi - g.c_lo <= kGatherTPB) {
     for (long c0 = g.c_lo; c0 < g.c_hi; c0 += kGatherTPB) {
       const long c = c0 + t;
-      append_in_order(sm, c < g.c_hi && box_meets(g.chunk_box + c * 6, x0, y0, z0), (int)c, sm.hit, kHitCap, nh);
+      append_in_order(sm, c < g.c_hi && box_meets(g.chunk_box + c * 6, x0, y0, z0), (int)c, sm.hit, nh);
     }
   } else {
     int ns = 0;
     const long s1 = (g.c_hi + kSuper - 1) / kSuper;
     for (long s0 = g.c_lo / kSuper; s0 < s1; s0 += kGatherTPB) {
       const long s = s0 + t;
-      append_in_order(sm, s < s1 && box_meets(g.super + s * 6, x0, y0, z0), (int)s, sm.pos, kHitCap, ns);
+      append_in_order(sm, s < s1 && box_meets(g.super + s * 6, x0, y0, z0), (int)s, sm.pos, ns);
     }
-    if (ns > kHitCap) return -1;
+    if (ns > kHitCap) return kHitCap + 1;
     for (int k = 0; k < ns; k += kGatherWarps) {
       const long c = k + warp < ns ? (long)sm.pos[k + warp] * kSuper + lane : -1;
-      append_in_order(sm, c >= g.c_lo && c < g.c_hi && box_meets(g.chunk_box + c * 6, x0, y0, z0), (int)c, sm.hit,
-                      kHitCap, nh);
+      append_in_order(sm, c >= g.c_lo && c < g.c_hi && box_meets(g.chunk_box + c * 6, x0, y0, z0), (int)c, sm.hit, nh);
     }
   }
-  if (nh > kHitCap) return -1;
+  return nh;
+}
+
+/* The nodes of the nh chunks in sm.hit that touch the tile: a mask per chunk
+ * and the number of nodes before it.  Returns their number.  Every level is a
+ * handful of coalesced loads per CTA, nothing is sorted, and no list has to be
+ * built beforehand. */
+__device__ __forceinline__ int gather_masks(GatherSmem& sm, const GatherNodes& g, int nh, int x0, int y0, int z0) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   /* kHitsAhead chunks of a warp at a time: their loads in flight together */
   for (int h0 = warp; h0 < nh; h0 += kGatherWarps * kHitsAhead) {
     unsigned o[kHitsAhead][3];
@@ -563,16 +567,21 @@ __device__ __forceinline__ int gather_list(GatherSmem& sm, const GatherNodes& g,
       if (h0 + lane < nh) sm.pos[h0 + lane] = run + iv - v;
       run += __shfl_sync(0xffffffffu, iv, 31);
     }
-    if (lane == 0) sm.n = run;
+    if (lane == 0) sm.pos[nh] = run;
   }
   __syncthreads();
-  const int L = sm.n;
-  if (L > kListCap) return -1;
+  return sm.pos[nh];
+}
+
+/* The nodes of chunks [h0, h1) of sm.hit, in index order, into sm.ids. */
+__device__ __forceinline__ void gather_ids(GatherSmem& sm, const GatherNodes& g, int h0, int h1, int x0, int y0,
+                                           int z0) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, first = sm.pos[h0];
 #pragma unroll 4
-  for (int h = warp; h < nh; h += kGatherWarps) {
+  for (int h = h0 + warp; h < h1; h += kGatherWarps) {
     const unsigned m = sm.mask[h];
     if ((m >> lane) & 1u) {
-      const int k = sm.pos[h] + __popc(m & ((1u << lane) - 1u)), i = sm.hit[h] * 32 + lane;
+      const int k = sm.pos[h] - first + __popc(m & ((1u << lane) - 1u)), i = sm.hit[h] * 32 + lane;
       unsigned o;
       if (h < kOffHits) {
         o = sm.hoff[h][lane];
@@ -585,7 +594,6 @@ __device__ __forceinline__ int gather_list(GatherSmem& sm, const GatherNodes& g,
     }
   }
   __syncthreads();
-  return L;
 }
 
 /* 8 bytes global -> shared, asynchronously. */
@@ -617,79 +625,12 @@ __device__ __forceinline__ void gather_stage(GatherSmem& sm, const GatherNodes& 
   sm.cover[buf][1][k] = (unsigned)(cov >> 32);
 }
 
-/* Too many nodes for the lists: visit the chunks in order, skipping those
- * whose box misses the tile.  Same summation order. */
-struct ScanSmem {
-  int hit[kGatherTPB];
-  int st[32][3];
-  double w[32][12];
-  double fe[32][3];
-};
-
-__device__ __forceinline__ void gather_scan(ScanSmem& sm, const GatherNodes& g, int x0, int y0, int z0, double& Fx,
-                                            double& Fy, double& Fz) {
-  const int t = threadIdx.x;
-  const double cf = 1.0 / (64.0 * 1.0 * 1.0 * 1.0);
-  const int gx = x0 + (t & 3), gy = y0 + ((t >> 2) & 3), gz = z0 + ((t & 63) >> 4);
-  for (long c0 = g.c_lo; c0 < g.c_hi; c0 += kGatherTPB) {
-    const long c = c0 + t;
-    __syncthreads();
-    sm.hit[t] = c < g.c_hi && box_meets(g.chunk_box + c * 6, x0, y0, z0);
-    __syncthreads();
-    for (int k = 0; k < kGatherTPB; ++k) {
-      if (!sm.hit[k]) continue;
-      if (t < 32) {
-        const long nd = (c0 + k) * 32 + t;
-        if (nd < g.S) {
-          for (int a = 0; a < 3; ++a) sm.st[t][a] = g.st[nd * 3 + a];
-          for (int a = 0; a < 12; ++a) sm.w[t][a] = g.W[nd * 12 + a];
-          for (int a = 0; a < 3; ++a) sm.fe[t][a] = g.nodes[nd * 12 + 9 + a];
-        } else {
-          sm.st[t][0] = sm.st[t][1] = sm.st[t][2] = INT_MIN / 2;
-        }
-      }
-      __syncthreads();
-      for (int j = 0; j < 32 && t < 64; ++j) {
-        const int a = gx - sm.st[j][0], b = gy - sm.st[j][1], e = gz - sm.st[j][2];
-        if ((unsigned)a < 4u && (unsigned)b < 4u && (unsigned)e < 4u) {
-          const double tmp = __dmul_rn(__dmul_rn(__dmul_rn(cf, sm.w[j][a]), sm.w[j][4 + b]), sm.w[j][8 + e]);
-          Fx = __dadd_rn(Fx, __dmul_rn(sm.fe[j][0], tmp));
-          Fy = __dadd_rn(Fy, __dmul_rn(sm.fe[j][1], tmp));
-          Fz = __dadd_rn(Fz, __dmul_rn(sm.fe[j][2], tmp));
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-union GatherShared {
-  GatherSmem g;
-  ScanSmem s;
-};
-
-/* The spread force of the tile at (x0, y0, z0): thread t < 64 gets its
- * cell's sum over the nodes in index order (cell = 16 z + 4 y + x).  Called
- * by all kGatherTPB threads.  Warps 2 and 3 stage the next 64 nodes while
- * warps 0 and 1 sum the last: each sum is a serial chain (its order is the
- * reference's), so latency is kept out of it.  The 32 cells of a warp go
- * through the nodes together, a lane adding those that cover its cell: at
- * 128x64x64 (182 nodes on a tile, 64 of them on each cell) 11,500 cycles,
- * against 21,000 with each lane on its own list of covering nodes
- * (scattered shared-memory reads).  One warp with two cells per lane, which
- * halves those reads, took the launch at 128x64x64 from 17 to 20 us. */
-__device__ __forceinline__ void gather_tile(GatherShared& sh, const GatherNodes& g, int x0, int y0, int z0,
-                                            double& Fx, double& Fy, double& Fz) {
+/* Chunks [h0, h1) of sm.hit, L <= kListCap nodes, added to the threads' sums. */
+__device__ __forceinline__ void gather_sum(GatherSmem& sm, const GatherNodes& g, int h0, int h1, int L, int x0, int y0,
+                                           int z0, double& Fx, double& Fy, double& Fz) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const double cf = 1.0 / (64.0 * 1.0 * 1.0 * 1.0);
-  Fx = Fy = Fz = 0.0;
-  __syncthreads();   /* the previous tile's data is no longer read */
-  GatherSmem& sm = sh.g;
-  const int L = gather_list(sm, g, x0, y0, z0);
-  if (L < 0) {
-    gather_scan(sh.s, g, x0, y0, z0, Fx, Fy, Fz);
-    return;
-  }
+  gather_ids(sm, g, h0, h1, x0, y0, z0);
   /* the thread's cell in a record: its x, y and z weight positions */
   const int ox = t & 3, oy = 4 + ((t >> 2) & 3), oz = 8 + ((t & 63) >> 4);
   if (warp >= 2) {
@@ -721,6 +662,53 @@ __device__ __forceinline__ void gather_tile(GatherShared& sh, const GatherNodes&
     }
     __syncthreads();
   }
+}
+
+/* gather_tile of a tile with more chunks or nodes than the lists hold (a
+ * crumpled sheet): a list at a time, from the start.  Apart from the common
+ * form, because what it keeps over a sum would cost that one registers which
+ * hold the cell's state (2% of a 128x64x64 step).  10,816 nodes strewn over a
+ * 128x96x96 grid, us per step, with every chunk that meets the tile visited by
+ * itself / a list at a time: 12,240 / 1,020; strewn over 30^3 690 / 193, over
+ * 12^3 612 / 214, on a plane at 0.1 cells 558 / 268. */
+__device__ __forceinline__ void gather_long(GatherSmem& sm, const GatherNodes& g, int x0, int y0, int z0, double& Fx,
+                                            double& Fy, double& Fz) {
+  for (long c0 = g.c_lo; c0 < g.c_hi;) {
+    int nh = 0;
+    __syncthreads();   /* the lists are no longer read */
+    for (; c0 < g.c_hi && nh <= kHitCap - kGatherTPB; c0 += kGatherTPB) {
+      const long c = c0 + threadIdx.x;
+      append_in_order(sm, c < g.c_hi && box_meets(g.chunk_box + c * 6, x0, y0, z0), (int)c, sm.hit, nh);
+    }
+    const int n = gather_masks(sm, g, nh, x0, y0, z0);
+    for (int h0 = 0, h1; h0 < nh; h0 = h1) {
+      /* all of these chunks' nodes, or as many chunks as the list holds */
+      h1 = nh;
+      if (n - sm.pos[h0] > kListCap)
+        for (h1 = h0 + 1; sm.pos[h1 + 1] - sm.pos[h0] <= kListCap;) ++h1;
+      gather_sum(sm, g, h0, h1, sm.pos[h1] - sm.pos[h0], x0, y0, z0, Fx, Fy, Fz);
+    }
+  }
+}
+
+/* The spread force of the tile at (x0, y0, z0): thread t < 64 gets its
+ * cell's sum over the nodes in index order (cell = 16 z + 4 y + x).  Called
+ * by all kGatherTPB threads.  Warps 2 and 3 stage the next 64 nodes while
+ * warps 0 and 1 sum the last: each sum is a serial chain (its order is the
+ * reference's), so latency is kept out of it.  The 32 cells of a warp go
+ * through the nodes together, a lane adding those that cover its cell: at
+ * 128x64x64 (182 nodes on a tile, 64 of them on each cell) 11,500 cycles,
+ * against 21,000 with each lane on its own list of covering nodes
+ * (scattered shared-memory reads).  One warp with two cells per lane, which
+ * halves those reads, took the launch at 128x64x64 from 17 to 20 us. */
+__device__ __forceinline__ void gather_tile(GatherSmem& sm, const GatherNodes& g, int x0, int y0, int z0, double& Fx,
+                                            double& Fy, double& Fz) {
+  __syncthreads();   /* the previous tile's data is no longer read */
+  const int nh = gather_chunks(sm, g, x0, y0, z0);
+  const int n = nh <= kHitCap ? gather_masks(sm, g, nh, x0, y0, z0) : kListCap + 1;
+  Fx = Fy = Fz = 0.0;
+  if (n <= kListCap) gather_sum(sm, g, 0, nh, n, x0, y0, z0, Fx, Fy, Fz);
+  else gather_long(sm, g, x0, y0, z0, Fx, Fy, Fz);
 }
 
 /* A move CTA: the 32 nodes of a chunk, four warps. */
