@@ -483,7 +483,7 @@ int batch_step(lbib_batch* b) {
      the forces.  FP64: the pairs run on the side stream beside gather and
      rows (24 problems: 414 -> 403 us per step); in 16-bit storage that was
      the slower order (128 problems: 1045 -> 1108 us), the word kernel being
-     bound by issue, not by memory */
+     bound by the latency of its loads at the warps it has, not by memory */
   const void* P = first ? b->P_first : b->P[c];
   const void* WP = first ? b->WP_first : b->WP[c];
   BatchFluid f = fluid_args(b, par, P, WP, c);

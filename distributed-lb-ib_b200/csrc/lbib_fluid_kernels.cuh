@@ -272,7 +272,7 @@ __device__ __forceinline__ long box_tiles(const int* __restrict__ b, int& nbx, i
  * against 8.5 us at 512x256x256), with a prime number of CTAs, so that none
  * sees one x position of the box only.  With the force written by one
  * launch and read back by another this was 31 + 33 us at 512x256x256
- * (FP64), and 16 + 10 us at 64x32x32; now 57 and 12.  Bound by the latency
+ * (FP64), and 16 + 10 us at 64x32x32; now 54 to 56 and 12.  Bound by the latency
  * of one tile's chain on small grids (at 128x64x64 the SMs' throughput is at
  * 9% and DRAM's at 5%), which a late join's ring lengthens from 16 to 18 us. */
 constexpr int kBoxCtas = 1181;

@@ -526,6 +526,9 @@ int lbib_batch_autotune(lbib_batch* b, int steps, double* ms, int max_ms, int* c
  * [out][in] row-major, then b [out].  X, T, Y of forward/train/gradient are
  * device pointers to row-major FP32 [batch][width] arrays; grad and loss of
  * lbib_mlp_gradient are host memory; the work runs on the MLP's stream.
+ * Device memory per row of max_batch (to a multiple of 128), widths to
+ * multiples of 16: 2 bytes for each layer's input, 4 for each hidden output
+ * and twice 2 for the widest output.
  * Returns NULL / error codes as above. */
 typedef struct lbib_mlp lbib_mlp;
 lbib_mlp* lbib_mlp_create(int n_layers, const int* widths, int max_batch, unsigned long long seed);
